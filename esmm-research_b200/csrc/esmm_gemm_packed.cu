@@ -170,32 +170,23 @@ __device__ __forceinline__ KFrag load_kfrag(const char *pa, const char *pb)
     return f;
 }
 
-// The thread's 8 x 8 outputs are held as 2 x 2 blocks for the packed FP32 multiply-add of sm_100
-// (fma.rn.f32x2: two independent IEEE FMAs per instruction, half the issue slots of scalar FFMA).
-// Block (p, q) covers rows 2p, 2p+1 and columns 2q, 2q+1 of the thread tile:
-//   diag[p][q] = (c[2p][2q],   c[2p+1][2q+1])        anti[p][q] = (c[2p][2q+1], c[2p+1][2q])
-// so both use the row pair (a[2p], a[2p+1]) as it comes from shared memory, with the column pair
-// (b[2q], b[2q+1]) as loaded for diag and swapped for anti.  Row pairs 0, 1 are the top 32-row
-// block, 2, 3 the bottom one.  Every output still sees one FMA per live k, in ascending k.
+// The thread's 8 x 8 outputs are held as row pairs for the packed FP32 multiply-add of sm_100 (fma.rn.f32x2: two
+// independent IEEE FMAs per instruction, half the issue slots of scalar FFMA):
+//   c[p][j] = (c of row 2p, column j; c of row 2p + 1, column j)
+// so an FMA takes the row pair (a[2p], a[2p+1]) as it comes from shared memory and one column of B in both halves.  Row
+// pairs 0, 1 are the top 32-row block, 2, 3 the bottom one.  Every output still sees one FMA per live k, in ascending k.
+// The row pair is the outer loop, so that eight instructions in a row use the same pair: this loop alone, operands in
+// shared memory, reaches 67.6 TFLOP/s, which is what fma.rn.f32x2 does with no loads at all; 63.3 with the column as
+// the outer loop, and 62.4 with the columns kept as pairs too (diagonal and anti-diagonal of 2 x 2 blocks).
 struct Acc {
-    float2 diag[4][4], anti[4][4];
+    float2 c[4][8];
 };
-
-// One 2 x 2 block: the diagonal pair and the anti-diagonal pair, one two-wide FMA each (the second on the swapped column
-// pair).  (The anti-diagonal pair as two scalar FMAs instead - no swapped operands, 48 instead of 32 multiply-add
-// instructions per row - was measured 23 % slower on the dense path.)
-__device__ __forceinline__ void fma_block(float2 &diag, float2 &anti, float2 ar, float bx, float by)
-{
-    diag = __ffma2_rn(ar, make_float2(bx, by), diag);
-    anti = __ffma2_rn(ar, make_float2(by, bx), anti);
-}
 
 __device__ __forceinline__ void fma_pair_row(Acc &c, int p, float2 ar, const KFrag &f)
 {
-    fma_block(c.diag[p][0], c.anti[p][0], ar, f.b0.x, f.b0.y);
-    fma_block(c.diag[p][1], c.anti[p][1], ar, f.b0.z, f.b0.w);
-    fma_block(c.diag[p][2], c.anti[p][2], ar, f.b1.x, f.b1.y);
-    fma_block(c.diag[p][3], c.anti[p][3], ar, f.b1.z, f.b1.w);
+    const float b[8] = {f.b0.x, f.b0.y, f.b0.z, f.b0.w, f.b1.x, f.b1.y, f.b1.z, f.b1.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c.c[p][j] = __ffma2_rn(ar, make_float2(b[j], b[j]), c.c[p][j]);
 }
 
 __device__ __forceinline__ void fma_top(Acc &c, const KFrag &f)
@@ -870,10 +861,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc.diag[i][j] = make_float2(0.0f, 0.0f);
-                    acc.anti[i][j] = make_float2(0.0f, 0.0f);
-                }
+                for (int j = 0; j < 8; ++j) acc.c[i][j] = make_float2(0.0f, 0.0f);
 
             // joint masks of a stage: bit r = row r is live for (top | bottom) block x my columns.  The
             // masks of the next stage are formed under the multiply-adds of the current one (the list's
@@ -928,7 +916,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             if (lane == 0) mbar_arrive(lempty0 + 8 * buf);
             if (warp == 0) ESMM_STAMP(601 + 4 * it);
 
-            // epilogue: C is overwritten (beta = 0); un-scramble the 2 x 2 blocks into rows
+            // epilogue: C is overwritten (beta = 0)
             const int row0 = tm * TM_ROWS + wm * 32 * WMB + lm * 4;
             const int col0 = tn * TILE_N + wn * 32 + ln * 4;
 #pragma unroll
@@ -939,10 +927,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
                     const int row = row0 + (i & 3) + 32 * (i >> 2);
                     float v[8];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        v[2 * q] = e == 0 ? acc.diag[pr][q].x : acc.anti[pr][q].y;
-                        v[2 * q + 1] = e == 0 ? acc.anti[pr][q].x : acc.diag[pr][q].y;
-                    }
+                    for (int j = 0; j < 8; ++j) v[j] = e == 0 ? acc.c[pr][j].x : acc.c[pr][j].y;
                     if (row < p.M) {
                         float *c = p.C + (size_t)row * p.N + col0;
                         const size_t c_floats = (size_t)p.M * p.N, off = (size_t)row * p.N + col0;
