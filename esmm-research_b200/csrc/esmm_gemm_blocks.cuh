@@ -1,0 +1,412 @@
+// Block mode of the packed joint-sparse SGEMM: every warp of the CTA works on its own blocks of C, with its own list of live k
+// and its own copies.
+//
+// The tiled pipeline (esmm_gemm_packed.cu) fetches every k that is live for any part of a 128 x 128 tile and moves in steps
+// of 32 such rows, eight warps together.  On operands whose 32-row and 32-column blocks are zero in different places most of
+// a fetched row is of no use to most of the warps, and a step lasts as long as its busiest warp.  Here nothing is shared:
+//
+//   * an item is a pair of adjacent 32 x 32 blocks of C: 64 rows x 32 columns, or 32 rows x 64 columns where B's patterns agree in
+//     pairs of column blocks more often than A's in pairs of row blocks.  The operand that spans 64 is called X, the one that
+//     spans 32 Y;
+//   * a warp joins the pattern bytes of each block to a list of its live k (ascending, 16 bits each, a ring of 512
+//     that is refilled as it is used up).  Lanes
+//     0-15 own the first block and walk its list, lanes 16-31 the second: a step is one live k of EACH block, 4 sixteen-byte
+//     loads and 32 two-wide FMAs per thread for its 8 x 8 outputs, whether the two k are the same or not.  (One block after the
+//     other on the whole warp, 4 x 8 outputs per thread, takes 6 loads for the same work.)
+//   * the rows of 16 steps are one stage of the warp's own ring of two, fetched with 16-byte cp.async copies: 128 bytes of X and
+//     128 of Y per block and k, Y only once where the blocks have the same list.  No copy is spent on a k that is dead for the
+//     block, and no multiply-add unless one list is longer than the other;
+//   * the warps of a CTA draw items from a counter in shared memory; the last ones come as single blocks spread over the whole
+//     warp, so that the warps finish together (a problem with few blocks consists of nothing else).
+//
+// What bounds it: the FMA pipe, 74 % busy where the lists are long (the pipeline on dense tiles: 76 %); what is lost goes to the
+// copies, which take issue slots and shared-memory bandwidth from the same warps (without them, a probe, 12 % faster at long
+// lists, 6 % at short ones), and to the listing.  Measured, whole calls, the tiled pipeline before -> block mode: 2048 x 11008 x 4096
+// pruned MLP 1016 -> 739 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 167 and at 0.5 / 0.5 921 -> 718,
+// 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 59.7.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 / 0.5 824),
+// 8 k per stage (971), lists made for all of K before the first copy (762), rows past a list's end skipped in a second code
+// path instead of multiplied by zeros (752: the accumulators are then moved between registers at every stage).
+//
+// There is no barrier between warps and nothing to wait for but a warp's own copies.  Every output sees one FMA per live k, in
+// ascending k, as in the tiled pipeline: the results are the same bits.
+#pragma once
+
+#include "esmm_gemm_shared.cuh"
+
+namespace esmm {
+
+constexpr int BM_WARPS = 12;                                // warps of the CTA that take part
+constexpr int BM_ROWS = 16;                                 // k per stage
+constexpr int BM_STEP = 8;                                  // k multiplied as one run of straight-line code
+constexpr int BM_PART = BM_ROWS * 128;                      // a stage's rows of one operand of one block
+constexpr int BM_SLOT_BYTES = 4 * BM_PART;                  // X of block 0, X of block 1, Y of block 0, Y of block 1
+constexpr int BM_SLOTS = 2;
+constexpr int BM_LIST = 512;                                // entries of a block's list (a ring)
+constexpr int BM_LIST_BYTES = BM_LIST * 2;
+constexpr int BM_WARP_BYTES = BM_SLOTS * BM_SLOT_BYTES + 2 * BM_LIST_BYTES;
+constexpr int BM_SMEM = BM_WARPS * BM_WARP_BYTES;
+constexpr int BM_TAIL = 6;                                  // of more than BM_WARPS items: 0 .. 12 measured, 4 - 6 best
+constexpr int BM_SAMPLES = 8;                               // tiles looked at to choose the mode
+
+// Pattern bytes of K blocks kb .. kb + 3 of one pattern row (null: no such row), zero past the end.  words: the row may be
+// read as 32-bit words.
+__device__ __forceinline__ unsigned pattern_word(const uint8_t *row, int kb, int nKB, bool words)
+{
+    if (row == nullptr || kb >= nKB) return 0u;
+    if (words) return *reinterpret_cast<const unsigned *>(row + kb);
+    unsigned v = 0u;
+    for (int j = 0; j < 4 && kb + j < nKB; ++j) v |= (unsigned)row[kb + j] << (8 * j);
+    return v;
+}
+
+// bits of the k of K blocks kb .. kb + 3 that are < K
+__device__ __forceinline__ unsigned inside_k(int kb, int K)
+{
+    const int left = K - kb * BK;
+    return left >= 32 ? 0xFFFFFFFFu : left <= 0 ? 0u : (1u << left) - 1u;
+}
+
+__device__ __forceinline__ const uint8_t *pattern_row(const uint8_t *pat, int row, int rows, int nKB)
+{
+    return row < rows ? pat + (size_t)row * nKB : nullptr;
+}
+
+// What one warp sees of a sample: a 128 x 128 tile over up to 128 of its K blocks.  (block, k) counts.
+struct TileStats {
+    int listed;      // k live for the tile as a whole
+    int slots;       // listed k times the tile's 32 x 32 blocks: what the tiled pipeline holds in shared memory
+    int work;        // (32 x 32 block, k) pairs that are live: what is multiplied
+    int rows64;      // (64 x 32 blocks, k) pairs with a live k: what the tiled pipeline's warps step through
+    int single;      // listed k in K blocks that are not live as a whole
+    int a_differ, b_differ;   // bits in which adjacent row blocks (column blocks) of a pair differ
+};
+
+template <typename Params>
+__device__ __forceinline__ TileStats tile_stats(const Params &p, int tm, int tn, int part, int lane)
+{
+    const uint8_t *ra[4], *rb[4];
+    int na = 0, nb = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        ra[i] = pattern_row(p.a_pat, tm * 4 + i, p.a_rows, p.nKB);
+        rb[i] = pattern_row(p.b_pat, tn * 4 + i, p.b_rows, p.nKB);
+        na += ra[i] != nullptr;
+        nb += rb[i] != nullptr;
+    }
+    TileStats s = {0, 0, 0, 0, 0, 0, 0};
+    // (one word per lane and row: a single round trip to memory)
+    const int span = (p.nKB + 3) >> 2, first = max(0, (span - 32) * part / (BM_SAMPLES - 1));
+    const int kb = 4 * (first + lane);
+    {
+        unsigned a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            a[i] = pattern_word(ra[i], kb, p.nKB, p.pat_words);
+            b[i] = pattern_word(rb[i], kb, p.nKB, p.pat_words);
+        }
+        const unsigned live = (a[0] | a[1] | a[2] | a[3]) & (b[0] | b[1] | b[2] | b[3]);
+        const int c = __popc(live);
+        s.listed += c;
+        const unsigned whole = __vcmpeq4(live, 0xFFFFFFFFu);
+        s.single += c - __popc(whole);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s.work += __popc(a[i] & b[j]);
+            s.rows64 += __popc((a[0] | a[1]) & b[j]) + __popc((a[2] | a[3]) & b[j]);
+        }
+        if (ra[1]) s.a_differ += __popc(a[0] ^ a[1]);
+        if (ra[3]) s.a_differ += __popc(a[2] ^ a[3]);
+        if (rb[1]) s.b_differ += __popc(b[0] ^ b[1]);
+        if (rb[3]) s.b_differ += __popc(b[2] ^ b[3]);
+    }
+    s.slots = s.listed * na * nb;
+    return s;
+}
+
+__device__ __forceinline__ int exclusive_scan(int v, int lane)
+{
+    int x = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(0xFFFFFFFFu, x, d);
+        if (lane >= d) x += t;
+    }
+    return x - v;
+}
+
+// Appends k0 + b for every set bit b of m to a list ring, from this lane's position q on.
+__device__ __forceinline__ void append_live(uint16_t *list, int q, unsigned m, int k0, int *status)
+{
+    while (m) {
+        const int bit = __ffs((int)m) - 1;
+        m &= m - 1u;
+        if (bounds_ok(q >= 0, status, 28)) list[q & (BM_LIST - 1)] = (uint16_t)(k0 + bit);   // checked build: site 28
+        ++q;
+    }
+}
+
+// A block's list of live k while its item is worked on: `list` is a ring; entries taken .. made - 1 are listed and not yet copied.
+struct LiveList {
+    uint16_t *list;
+    int made, taken;
+    __device__ __forceinline__ int pending() const { return made - taken; }
+};
+
+// BM_STEP steps of a stage: 8 x 8 outputs per thread, each half-warp on its own rows of X and Y.  Odd rows hold the upper half of
+// their 128 bytes first (see the copies).
+__device__ __forceinline__ void pair_steps(Acc &acc, const char *sx, const char *sy)
+{
+#pragma unroll
+    for (int r = 0; r < BM_STEP; ++r) {
+        const int lo = r * 128 + (r & 1) * 64, hi = r * 128 + 64 - (r & 1) * 64;
+        KFrag f;
+        f.at = *reinterpret_cast<const float4 *>(sx + lo);
+        f.ab = *reinterpret_cast<const float4 *>(sx + hi);
+        f.b0 = *reinterpret_cast<const float4 *>(sy + lo);
+        f.b1 = *reinterpret_cast<const float4 *>(sy + hi);
+        fma_top(acc, f);
+        fma_bottom(acc, f);
+    }
+}
+
+// BM_STEP k of a single block: 4 x 8 outputs per thread.  sx_odd: the lane's chunk of X in odd rows.
+__device__ __forceinline__ void single_steps(Acc &acc, const char *sx, const char *sx_odd, const char *sy)
+{
+#pragma unroll
+    for (int r = 0; r < BM_STEP; ++r) {
+        KFrag f;
+        f.at = *reinterpret_cast<const float4 *>(((r & 1) ? sx_odd : sx) + r * 128);
+        f.b0 = *reinterpret_cast<const float4 *>(sy + r * 128 + (r & 1) * 64);
+        f.b1 = *reinterpret_cast<const float4 *>(sy + r * 128 + 64 - (r & 1) * 64);
+        fma_top(acc, f);
+    }
+}
+
+__device__ __forceinline__ void fill_16(uint32_t dst, float v)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "f"(v) : "memory");
+}
+
+// One item: blocks x0 and x0 + 1 of X (TWO) or x0 alone, times block y of Y.
+template <bool TWO, typename Params>
+__device__ __forceinline__ void block_item(const Params &p, char *ring, int lane, bool wide_b, int x0, int y)
+{
+    LiveList l0, l1;
+    l0.list = reinterpret_cast<uint16_t *>(ring + BM_SLOTS * BM_SLOT_BYTES);
+    l1.list = l0.list + BM_LIST;
+    // every 4 consecutive lanes touch 2 chunks of X and 2 of Y (see the tiled pipeline)
+    const int half = lane >> 4, xg = (lane >> 1) & 3, yg = (lane & 1) | ((lane >> 2) & 2);   // pair: 4 x 4 lanes per block
+    const int lm = (lane >> 1) & 7, ln = (lane & 1) | ((lane >> 4) << 1);                    // single block: 8 x 4 lanes
+    // Copies: four lanes per row of the stage, eight rows at a time; a lane moves the 16-byte chunks c4 and c4 + 4 of its row.
+    // Rows are 128 bytes apart; odd rows have their two halves swapped, so that the eight rows of one copy instruction fall
+    // on all banks.
+    const int r8 = lane >> 2, c4 = lane & 3;
+    const uint32_t dst0 = smem_u32(ring) + (uint32_t)(r8 * 128 + c4 * 16 + (r8 & 1) * 64), dst1 = dst0 + 64 - (r8 & 1) * 128;
+    const unsigned n4 = (unsigned)p.N * 4u;                       // bytes of a row of B
+    const unsigned x_stride = wide_b ? n4 : TILE_M * 4u, y_stride = wide_b ? TILE_M * 4u : n4;
+
+                const uint8_t *px = (wide_b ? p.b_pat : p.a_pat) + (size_t)x0 * p.nKB;
+                const uint8_t *px1 = TWO ? px + p.nKB : nullptr;
+                const uint8_t *py = (wide_b ? p.a_pat : p.b_pat) + (size_t)y * p.nKB;
+                // 32 floats of packed A are contiguous within a panel of 128 rows; a row of B has N floats.  Chunks of B past its
+                // last column are not copied: whatever is multiplied there ends in columns of C that do not exist.
+                const int a_blk = wide_b ? y : x0, b_blk = wide_b ? x0 : y;
+                const char *a_src = reinterpret_cast<const char *>(p.a_packed + (size_t)(a_blk >> 2) * p.kp * TILE_M + (a_blk & 3) * 32);
+                const char *b_src = reinterpret_cast<const char *>(p.B + b_blk * 32);
+                const char *xs = (wide_b ? b_src : a_src) + c4 * 16, *ys = (wide_b ? a_src : b_src) + c4 * 16;
+                const int b_chunks = (p.N - b_blk * 32) >> 2;
+                const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);
+
+                Acc acc;
+                acc_clear(acc);
+
+                // The lane's pattern bits of the 128 K blocks kb0 .. (m0, m1: joint bits of either block; wy, w0, w1: the words of the
+                // 128 K blocks after them, on their way) and how many eighths of them are listed already.
+                int kb0 = -128, part = 0, live = 0;
+                unsigned m0 = 0u, m1 = 0u, wy = 0u, w0 = 0u, w1 = 0u;
+                auto load_words = [&](int kb) {
+                    wy = pattern_word(py, kb, p.nKB, p.pat_words) & inside_k(kb, p.K);
+                    w0 = pattern_word(px, kb, p.nKB, p.pat_words);
+                    w1 = pattern_word(px1, kb, p.nKB, p.pat_words);
+                };
+                auto next_words = [&]() {
+                    kb0 += 128;
+                    part = 0;
+                    m0 = w0 & wy;
+                    m1 = w1 & wy;
+                    live = __reduce_add_sync(0xFFFFFFFFu, __popc(m0) | (__popc(m1) << 16));   // (both counts in one word)
+                    if (kb0 + 128 < p.nKB) load_words(kb0 + 128 + 4 * lane);
+                };
+                load_words(4 * lane);
+                next_words();
+                l0.made = l0.taken = l1.made = l1.taken = 0;
+
+                // Lists further K blocks until each list holds a stage or there is no room: all 128 at once where they fit, or a
+                // quarter of them (then a lane takes one byte).
+                auto refill = [&]() {
+                    bool wrote = false;
+                    while (kb0 < p.nKB && (l0.pending() < BM_ROWS || (TWO && l1.pending() < BM_ROWS))) {
+                        const int room = BM_LIST - max(l0.pending(), l1.pending());
+                        unsigned a0 = m0, a1 = m1;
+                        int k0 = (kb0 + 4 * lane) * BK;
+                        if (part == 0 && max(live & 0xFFFF, live >> 16) <= room) {
+                            part = 4;
+                        } else {
+                            if (room < 32 * BK) break;
+                            const int from = part * 8 + (lane >> 2), sh = (lane & 3) * 8;
+                            a0 = (__shfl_sync(0xFFFFFFFFu, m0, from) >> sh) & 0xFFu;
+                            a1 = (__shfl_sync(0xFFFFFFFFu, m1, from) >> sh) & 0xFFu;
+                            k0 = (kb0 + part * 32 + lane) * BK;
+                            ++part;
+                        }
+                        const int c = __popc(a0) | (__popc(a1) << 16);
+                        const int before = exclusive_scan(c, lane);
+                        const int total = __shfl_sync(0xFFFFFFFFu, before + c, 31);
+                        append_live(l0.list, l0.made + (before & 0xFFFF), a0, k0, p.status);
+                        if (TWO) append_live(l1.list, l1.made + (before >> 16), a1, k0, p.status);
+                        l0.made += total & 0xFFFF;
+                        l1.made += total >> 16;
+                        wrote = true;
+                        if (part == 4) next_words();
+                    }
+                    if (wrote) __syncwarp();
+                };
+
+                uint32_t slot = 0;
+                int count = 0;                 // steps of the stage that is multiplied
+                bool same = false;             // both blocks have the same 16 k there: Y is held once
+                do {
+                    cp_async_wait_group<0>();
+                    __syncwarp();              // the stage is complete for all lanes, and the one before it read by all
+                    refill();
+                    // ---- copies of the next stage ----
+        const int d0 = min(BM_ROWS, l0.pending()), d1 = TWO ? min(BM_ROWS, l1.pending()) : 0;
+        const uint32_t to = BM_SLOT_BYTES - slot;
+        bool same_next = false;
+        if (!edge && d0 == BM_ROWS && (!TWO || d1 == BM_ROWS)) {
+            unsigned k0[BM_ROWS / 8], k1[BM_ROWS / 8];
+            same_next = TWO;
+#pragma unroll
+            for (int h = 0; h < BM_ROWS / 8; ++h) {
+                k0[h] = l0.list[(l0.taken + h * 8 + r8) & (BM_LIST - 1)];
+                k1[h] = TWO ? l1.list[(l1.taken + h * 8 + r8) & (BM_LIST - 1)] : 0;
+                if (TWO) same_next = __all_sync(0xFFFFFFFFu, k0[h] == k1[h]) && same_next;
+            }
+#pragma unroll
+            for (int h = 0; h < BM_ROWS / 8; ++h) {
+                const char *gx = xs + (size_t)k0[h] * x_stride, *gy = ys + (size_t)k0[h] * y_stride;
+                const uint32_t e0 = dst0 + to + h * 1024, e1 = dst1 + to + h * 1024;
+                cp_async_16(e0, gx, 16);
+                cp_async_16(e1, gx + 64, 16);
+                cp_async_16(e0 + 2 * BM_PART, gy, 16);
+                cp_async_16(e1 + 2 * BM_PART, gy + 64, 16);
+                if (TWO) {
+                    const char *gx1 = xs + (size_t)k1[h] * x_stride;
+                    cp_async_16(e0 + BM_PART, gx1 + 128, 16);
+                    cp_async_16(e1 + BM_PART, gx1 + 192, 16);
+                    if (!same_next) {
+                        const char *gy1 = ys + (size_t)k1[h] * y_stride;
+                        cp_async_16(e0 + 3 * BM_PART, gy1, 16);
+                        cp_async_16(e1 + 3 * BM_PART, gy1 + 64, 16);
+                    }
+                }
+            }
+        } else if (max(d0, d1) > 0) {
+            // Past the end of a list X = -0 and Y = +0: a multiply-add with them changes no accumulator, not even a zero's sign.
+            const int x_lim = wide_b ? b_chunks : 16, y_lim = wide_b ? 8 : b_chunks;
+#pragma unroll 1
+            for (int i = 0; i < 2 * (TWO ? 2 : 1) * (BM_ROWS / 8); ++i) {      // (row group, half of the row, block)
+                const int j = i & 1, row = ((i >> 1) & (BM_ROWS / 8 - 1)) * 8 + r8, blk = TWO ? i >> 2 : 0, ch = c4 + 4 * j;
+                const uint32_t e = (j ? dst1 : dst0) + to + (row - r8) * 128 + blk * BM_PART;
+                if (row < (blk ? d1 : d0)) {
+                    const size_t k = blk ? l1.list[(l1.taken + row) & (BM_LIST - 1)] : l0.list[(l0.taken + row) & (BM_LIST - 1)];
+                    if (blk * 8 + ch < x_lim) cp_async_16(e, xs + k * x_stride + blk * 128 + j * 64, 16);
+                    if (ch < y_lim) cp_async_16(e + 2 * BM_PART, ys + k * y_stride + j * 64, 16);
+                } else {
+                    fill_16(e, -0.0f);
+                    fill_16(e + 2 * BM_PART, 0.0f);
+                }
+            }
+        }
+        l0.taken += d0;
+        l1.taken += d1;
+        cp_async_commit();
+        // ---- the stage itself ----
+        const char *st = ring + slot;
+        if (TWO) {
+            const char *sx = st + half * BM_PART + xg * 16, *sy = st + (same ? 2 : 2 + half) * BM_PART + yg * 16;
+#pragma unroll 1
+            for (int r = 0; r < count; r += BM_STEP) pair_steps(acc, sx + r * 128, sy + r * 128);
+        } else {
+            const char *sx = st + lm * 16, *sx_odd = st + (lm ^ 4) * 16, *sy = st + 2 * BM_PART + ln * 16;
+#pragma unroll 1
+            for (int r = 0; r < count; r += BM_STEP) single_steps(acc, sx + r * 128, sx_odd + r * 128, sy + r * 128);
+        }
+        count = max(d0, d1);
+                    same = same_next;
+                    slot = to;
+                } while (count > 0);
+
+                // ---- C is overwritten (beta = 0) ----
+                // x values 4 * xv .. + 3 and, in a pair, + 16; y values 4 * yv .. + 3 and + 16, of block xb
+                const size_t c_floats = (size_t)p.M * p.N;
+                const int xb = x0 + (TWO ? half : 0), xv = TWO ? xg : lm, yv = TWO ? yg : ln;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {                       // the two groups of 4 x values
+                    if (q == 1 && !TWO) break;
+                    if (!wide_b) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int row = xb * 32 + q * 16 + xv * 4 + i, col = y * 32 + yv * 4;
+                            float v8[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) v8[j] = acc_get(acc, 2 * q + (i >> 1), i & 1, j);
+                            const size_t off = (size_t)row * p.N + col;
+                            if (row < p.M && col < p.N && bounds_ok(off + 4 <= c_floats, p.status, 29))
+                                *reinterpret_cast<float4 *>(p.C + off) = make_float4(v8[0], v8[1], v8[2], v8[3]);
+                            if (row < p.M && col + 16 < p.N && bounds_ok(off + 20 <= c_floats, p.status, 29))
+                                *reinterpret_cast<float4 *>(p.C + off + 16) = make_float4(v8[4], v8[5], v8[6], v8[7]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int row = y * 32 + yv * 4 + (j & 3) + 16 * (j >> 2), col = xb * 32 + q * 16 + xv * 4;
+                            const size_t off = (size_t)row * p.N + col;
+                            if (row < p.M && col < p.N && bounds_ok(off + 4 <= c_floats, p.status, 29))
+                                *reinterpret_cast<float4 *>(p.C + off) =
+                                    make_float4(acc_get(acc, 2 * q, 0, j), acc_get(acc, 2 * q, 1, j), acc_get(acc, 2 * q + 1, 0, j), acc_get(acc, 2 * q + 1, 1, j));
+                        }
+                    }
+                }
+}
+
+// All of a warp's share of block mode.  smem: the CTA's dynamic shared memory; next: the CTA's item counter (initially
+// BM_WARPS: a warp's first item is its own number).
+template <typename Params>
+__device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp, int lane, bool wide_b, int *next)
+{
+    char *ring = smem + warp * BM_WARP_BYTES;
+    // X spans pairs of blocks, Y single ones
+    const int x_blocks = wide_b ? p.b_rows : p.a_rows, y_blocks = wide_b ? p.a_rows : p.b_rows;
+    const int pairs_x = (x_blocks + 1) >> 1;
+    const int tiles_m = wide_b ? y_blocks : pairs_x, tiles_n = wide_b ? pairs_x : y_blocks;
+    const long items = (long)tiles_m * tiles_n;
+    const int mine = blockIdx.x < items ? (int)((items - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
+    const int tail = mine <= BM_WARPS ? mine : BM_TAIL, whole = mine - tail;   // the last `tail` items go as two single blocks each
+
+    for (int v = warp; v < whole + 2 * tail;) {
+        const int item = blockIdx.x + (v < whole ? v : whole + ((v - whole) >> 1)) * gridDim.x;
+        int tm, tn;
+        tile_coords(item, tiles_m, tiles_n, tm, tn, wide_b ? 32 : 16);
+        const int y = wide_b ? tm : tn, x0 = 2 * (wide_b ? tn : tm) + (v < whole ? 0 : (v - whole) & 1);
+        if (v < whole && x0 + 1 < x_blocks) block_item<true>(p, ring, lane, wide_b, x0, y);
+        else if (x0 < x_blocks) block_item<false>(p, ring, lane, wide_b, x0, y);
+        int nx = 0;
+        if (lane == 0) nx = atomicAdd(next, 1);
+        v = __shfl_sync(0xFFFFFFFFu, nx, 0);
+    }
+    cp_async_wait_group<0>();
+}
+
+}  // namespace esmm

@@ -46,11 +46,12 @@
 //
 // Every wait is bounded; a wait that expires raises the device status word and the CTA
 // leaves after waiting (bounded again) for its copies in flight.
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <mutex>
 
-#include "esmm_gemm_shared.cuh"
+#include "esmm_gemm_blocks.cuh"
 
 namespace esmm {
 
@@ -74,6 +75,12 @@ constexpr int P_CONSUMER_WARPS = 8;
 //     noted such tiles (see gemm_ab_packed_launch_form); esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins one.
 constexpr int P_TMA_WARP = P_CONSUMER_WARPS;                   // first producer warp
 constexpr int P_MAX_STAGES = 6;
+// Block mode (esmm_gemm_blocks.cuh) where at most this many sixteenths of what the tiled pipeline would hold in shared memory are
+// multiplied.  Measured at 4096^3, whole calls, pipeline / block mode: share 0.33 (32-granular, 0.5 / 0.5 of A's and B's
+// k live) 921 / 718 us, 0.44 (64-granular, 0.5 / 0.5) 730 / 695, 0.53 (32-granular, 1 / 0.5) 1414 / 1344, 0.64 (32-granular,
+// 0.8 / 0.8) 1900 / 1737, 0.67 (64-granular, 1 / 0.5) 1373 / 1346, 0.69 (64-granular, 0.8 / 0.8) 1675 / 1685, 0.83 (64-granular,
+// 0.9 / 0.9) 2050 / 2087, 1 (dense) 2130 / 2549.
+constexpr int BM_SIXTEENTHS = 11;
 
 // Optional timeline for tuning (build with -DESMM_TRACE): CTA 0 stamps %globaltimer at a few points
 // into a device array that esmm_trace_read copies out.  Not part of the product build or of the ABI.
@@ -108,8 +115,13 @@ struct PackedParams {
     int vec_patterns;  // K blocks per lane and load in the mask warp: 16, 4 (alignment permitting) or 0 = bytes
     int adaptive;      // 16-warp form: the CTA's first tile decides whether 3 or all 7 producer warps copy
     int *form_hint;    // host-mapped word, or null: CTA 0 notes whether its first tile wanted 7 producers
+    int block_mode;    // 1, 0: always, never; -1: as the sampled tiles say
+    int pat_words;     // pattern rows may be read as 32-bit words
+    int few_blocks;    // no more pairs of blocks than CTAs
     const uint8_t *a_pat;
     const uint8_t *b_pat;
+    const float *a_packed;
+    const float *B;
     float *C;
     int *status;
 };
@@ -125,7 +137,7 @@ constexpr int RUN_TILE = 0x100;
 constexpr int RUNS_LIKELY = 0x200;   // a listed tile whose stages may be whole runs of K blocks: the producers look for them
 
 struct PackedSmem {
-    uint32_t stage_off, krow_off, krow_stride, rmask_off, rmask_stride, wlist_off, bar_off, misc_off, total;
+    uint32_t stage_off, krow_off, krow_stride, rmask_off, rmask_stride, wlist_off, bar_off, misc_off, item_off, total;
 };
 
 __host__ __device__ inline PackedSmem packed_smem_layout(int stages, int cap)
@@ -147,58 +159,11 @@ __host__ __device__ inline PackedSmem packed_smem_layout(int stages, int cap)
     o += (2 * P_MAX_STAGES + 4) * 8;
     L.misc_off = o;   // nrows[2], abort, n_producers, runinfo[2]
     o += 32;
+    // block mode lays its warps' rings over all of this; its item counter is past them, or the last word of misc
+    L.item_off = L.misc_off >= BM_SMEM ? L.misc_off + 24 : BM_SMEM;
+    if (o < BM_SMEM + 16) o = BM_SMEM + 16;
     L.total = o;
     return L;
-}
-
-// One k of the tile for one thread: its 4 rows of the top block, 4 rows of the bottom block
-// and 2 x 4 columns are one 16-byte load each.
-struct KFrag {
-    float4 at, ab, b0, b1;
-};
-
-// WMB = 32-row blocks per consumer warp: 2 in the 128 x 128 tiling, 1 in the 64 x 128 tiling (where a
-// thread holds 4 x 8 outputs and the "bottom" half of everything below is compiled out).
-template <int WMB>
-__device__ __forceinline__ KFrag load_kfrag(const char *pa, const char *pb)
-{
-    KFrag f;
-    f.at = *reinterpret_cast<const float4 *>(pa);
-    if (WMB == 2) f.ab = *reinterpret_cast<const float4 *>(pa + 128);
-    f.b0 = *reinterpret_cast<const float4 *>(pb);
-    f.b1 = *reinterpret_cast<const float4 *>(pb + 64);
-    return f;
-}
-
-// The thread's 8 x 8 outputs are held as row pairs for the packed FP32 multiply-add of sm_100 (fma.rn.f32x2: two
-// independent IEEE FMAs per instruction, half the issue slots of scalar FFMA):
-//   c[p][j] = (c of row 2p, column j; c of row 2p + 1, column j)
-// so an FMA takes the row pair (a[2p], a[2p+1]) as it comes from shared memory and one column of B in both halves.  Row
-// pairs 0, 1 are the top 32-row block, 2, 3 the bottom one.  Every output still sees one FMA per live k, in ascending k.
-// The row pair is the outer loop, so that eight instructions in a row use the same pair: this loop alone, operands in
-// shared memory, reaches 67.6 TFLOP/s, which is what fma.rn.f32x2 does with no loads at all; 63.3 with the column as
-// the outer loop, and 62.4 with the columns kept as pairs too (diagonal and anti-diagonal of 2 x 2 blocks).
-struct Acc {
-    float2 c[4][8];
-};
-
-__device__ __forceinline__ void fma_pair_row(Acc &c, int p, float2 ar, const KFrag &f)
-{
-    const float b[8] = {f.b0.x, f.b0.y, f.b0.z, f.b0.w, f.b1.x, f.b1.y, f.b1.z, f.b1.w};
-#pragma unroll
-    for (int j = 0; j < 8; ++j) c.c[p][j] = __ffma2_rn(ar, make_float2(b[j], b[j]), c.c[p][j]);
-}
-
-__device__ __forceinline__ void fma_top(Acc &c, const KFrag &f)
-{
-    fma_pair_row(c, 0, make_float2(f.at.x, f.at.y), f);
-    fma_pair_row(c, 1, make_float2(f.at.z, f.at.w), f);
-}
-
-__device__ __forceinline__ void fma_bottom(Acc &c, const KFrag &f)
-{
-    fma_pair_row(c, 2, make_float2(f.ab.x, f.ab.y), f);
-    fma_pair_row(c, 3, make_float2(f.ab.z, f.ab.w), f);
 }
 
 // A stage whose 32 rows are all live for both row blocks: 16 rows of straight-line code per
@@ -465,6 +430,43 @@ __device__ __forceinline__ void tile_scan(const PackedParams &p, int tm, int tn,
     }
 }
 
+struct TileScan {
+    unsigned live_first;
+    bool uniform, full;
+    int live_total, live_small;
+};
+
+template <int RB>
+__device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm, int tn, int lane)
+{
+    TileScan s = {0u, true, true, 0, 0};
+    if (p.vec_patterns == 16) {
+        tile_scan<RB, 16>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
+    } else if (p.vec_patterns == 4) {
+        tile_scan<RB, 4>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
+    } else {
+        for (int kb0 = 0; kb0 < p.nKB; kb0 += 32) {
+            const int kb = kb0 + lane;
+            unsigned au = 0, bu = 0;
+            if (kb < p.nKB) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int mb = tm * RB + i, nb = tn * 4 + i;
+                    if (i < RB && mb < p.a_rows) au |= p.a_pat[(size_t)mb * p.nKB + kb];
+                    if (nb < p.b_rows) bu |= p.b_pat[(size_t)nb * p.nKB + kb];
+                }
+            }
+            const unsigned live = au & bu;
+            if (kb0 == 0) s.live_first = __shfl_sync(0xFFFFFFFFu, live, 0);
+            s.uniform = s.uniform && __all_sync(0xFFFFFFFFu, kb >= p.nKB || live == s.live_first);
+            s.full = false;   // the byte-wise path keeps the general listing
+            s.live_total += __reduce_add_sync(0xFFFFFFFFu, __popc(live));
+            s.live_small += __reduce_add_sync(0xFFFFFFFFu, __popc(live) <= p.brow_bits ? __popc(live) : 0);
+        }
+    }
+    return s;
+}
+
 // Second pass: the row list.  Lane l owns K blocks c0 + KPL l .. c0 + KPL l + KPL - 1 (consecutive lanes,
 // consecutive K); K blocks with more than whole_above live k are listed whole.  Returns the row count.
 template <int RB, int KPL>
@@ -541,6 +543,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
     // 4 or 8 consecutive live k (kk0 .. kk0 + c - 1), live for all of the tile's row and column blocks.  Such
     // a tile needs no row list: stage s is the 3-D box of K blocks 32 s / c .. and every stage is all-live.
     volatile int *runinfo = nrows + 4;
+    int *next_item = reinterpret_cast<int *>(smem + L.item_off);   // block mode's item counter
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
@@ -552,11 +555,70 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             mbar_init(lempty0 + 8 * b, P_CONSUMER_WARPS + P_TMA_WARPS);
         }
         *abort_flag = 0;
+        *next_item = BM_WARPS;
         fence_barrier_init();
         fence_proxy_async();
     }
     __syncthreads();
     grid_dependency_wait();   // (patterns and the packed copy of A come from the kernel before this one)
+
+    // The mode: every CTA looks at the same BM_SAMPLES samples, spread over the rows, the columns and K, so that all of them
+    // come to the same answer.  The mask warp scans the CTA's first tile meanwhile, which the pipeline starts with.
+    TileScan scan = {0u, true, true, 0, 0};
+    if (warp == P_MASK_WARP && (int)blockIdx.x < p.num_tiles) {
+        int tm, tn;
+        tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
+        scan = tile_scan_any<RB>(p, tm, tn, lane);
+    }
+    if (p.block_mode != 0) {
+        // two vectors per sample, where the consumers' lists will be
+        int4 *stats = reinterpret_cast<int4 *>(smem + L.wlist_off);
+        static_assert(2 * BM_SAMPLES * sizeof(int4) <= P_CONSUMER_WARPS * 2 * 96 && BM_SAMPLES <= P_CONSUMER_WARPS, "samples");
+        if (warp < BM_SAMPLES) {
+            const int panels = (p.a_rows + 3) >> 2;
+            const TileStats s = tile_stats(p, warp * panels / BM_SAMPLES, ((5 * warp + 2) & 7) * p.tiles_n / BM_SAMPLES, warp, lane);
+            int4 x, y;
+            x.x = __reduce_add_sync(0xFFFFFFFFu, s.slots);
+            x.y = __reduce_add_sync(0xFFFFFFFFu, s.work);
+            x.z = __reduce_add_sync(0xFFFFFFFFu, s.a_differ);
+            x.w = __reduce_add_sync(0xFFFFFFFFu, s.b_differ);
+            y.x = __reduce_add_sync(0xFFFFFFFFu, s.listed);
+            y.y = __reduce_add_sync(0xFFFFFFFFu, s.rows64);
+            y.z = __reduce_add_sync(0xFFFFFFFFu, s.single);
+            y.w = 0;
+            if (lane == 0) {
+                stats[warp] = x;
+                stats[BM_SAMPLES + warp] = y;
+            }
+        }
+        __syncthreads();
+        int slots = 0, work = 0, a_differ = 0, b_differ = 0;
+#pragma unroll
+        for (int i = 0; i < BM_SAMPLES; ++i) {
+            const int4 x = stats[i];
+            slots += x.x;
+            work += x.y;
+            a_differ += x.z;
+            b_differ += x.w;
+        }
+        const bool blocks = p.block_mode > 0 || 16 * work <= BM_SIXTEENTHS * slots;
+        if (blocks && blockIdx.x == 0 && threadIdx.x == 0 && p.form_hint != nullptr) {
+            // the note for the next launch (see gemm_ab_packed_launch_form)
+            int listed = 0, rows64 = 0, single = 0;
+            for (int i = 0; i < BM_SAMPLES; ++i) {
+                const int4 y = stats[BM_SAMPLES + i];
+                listed += y.x;
+                rows64 += y.y;
+                single += y.z;
+            }
+            *p.form_hint = p.few_blocks && 2 * single >= listed && rows64 <= 3 * listed ? 1 : 0;
+        }
+        __syncthreads();   // the samples have been read by all
+        if (blocks) {
+            if (warp < BM_WARPS) block_mode(p, smem, warp, lane, b_differ < a_differ, next_item);
+            return;
+        }
+    }
 
     bool ok = true;
     if (warp == 0) ESMM_STAMP(0);
@@ -569,40 +631,17 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
         int it = 0;
         for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++it) {
             const int buf = it & 1;
-            ok = mbar_wait(lempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag);
-            if (!ok) break;
             int tm, tn;
             tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
+            // A first pass over the tile's pattern bytes (the first tile's is done) decides the listing policy.
+            if (it > 0) scan = tile_scan_any<RB>(p, tm, tn, lane);
+            const unsigned live_first = scan.live_first;
+            const bool uniform = scan.uniform, full = scan.full;
+            const int live_total = scan.live_total, live_small = scan.live_small;
+            ok = mbar_wait(lempty0 + 8 * buf, ((it >> 1) & 1) ^ 1, abort_flag);
+            if (!ok) break;
             uint16_t *krow = reinterpret_cast<uint16_t *>(smem + L.krow_off + buf * L.krow_stride);
             uint8_t *rmask = reinterpret_cast<uint8_t *>(smem + L.rmask_off + buf * L.rmask_stride);
-            // A first pass over the tile's pattern bytes decides the listing policy.
-            unsigned live_first = 0;
-            bool uniform = true, full = true;
-            int live_total = 0, live_small = 0;
-            if (p.vec_patterns == 16) {
-                tile_scan<RB, 16>(p, tm, tn, lane, live_first, uniform, full, live_total, live_small);
-            } else if (p.vec_patterns == 4) {
-                tile_scan<RB, 4>(p, tm, tn, lane, live_first, uniform, full, live_total, live_small);
-            } else {
-                for (int kb0 = 0; kb0 < p.nKB; kb0 += 32) {
-                    const int kb = kb0 + lane;
-                    unsigned au = 0, bu = 0;
-                    if (kb < p.nKB) {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int mb = tm * RB + i, nb = tn * 4 + i;
-                            if (i < RB && mb < p.a_rows) au |= p.a_pat[(size_t)mb * p.nKB + kb];
-                            if (nb < p.b_rows) bu |= p.b_pat[(size_t)nb * p.nKB + kb];
-                        }
-                    }
-                    const unsigned live = au & bu;
-                    if (kb0 == 0) live_first = __shfl_sync(0xFFFFFFFFu, live, 0);
-                    uniform = uniform && __all_sync(0xFFFFFFFFu, kb >= p.nKB || live == live_first);
-                    full = false;   // the byte-wise path keeps the general listing
-                    live_total += __reduce_add_sync(0xFFFFFFFFu, __popc(live));
-                    live_small += __reduce_add_sync(0xFFFFFFFFu, __popc(live) <= p.brow_bits ? __popc(live) : 0);
-                }
-            }
             // uniform tile: list live k only.  Otherwise the policy is two numbers: K blocks with more than brow_bits
             // live k are listed whole, on tiles with at most row_density live k per K block on average; denser
             // tiles list every live K block whole.  With the producers fetching runs of consecutive rows as boxes,
@@ -858,10 +897,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             if (warp == 0) ESMM_STAMP(600 + 4 * it);
 
             Acc acc;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc.c[i][j] = make_float2(0.0f, 0.0f);
+            acc_clear(acc);
 
             // joint masks of a stage: bit r = row r is live for (top | bottom) block x my columns.  The
             // masks of the next stage are formed under the multiply-adds of the current one (the list's
@@ -927,7 +963,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
                     const int row = row0 + (i & 3) + 32 * (i >> 2);
                     float v[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = e == 0 ? acc.c[pr][j].x : acc.c[pr][j].y;
+                    for (int j = 0; j < 8; ++j) v[j] = acc_get(acc, pr, e, j);
                     if (row < p.M) {
                         float *c = p.C + (size_t)row * p.N + col0;
                         const size_t c_floats = (size_t)p.M * p.N, off = (size_t)row * p.N + col0;
@@ -1090,9 +1126,30 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     if (forced_vec == 0 || (forced_vec == 4 && p.vec_patterns >= 4) ||
         (forced_vec == 16 && p.nKB % 16 == 0 && (pat_bits & 15) == 0))
         p.vec_patterns = forced_vec;
+    p.pat_words = p.nKB % 4 == 0 && (pat_bits & 3) == 0;
     p.a_pat = d_a_pat;
     p.b_pat = d_b_pat;
+    p.a_packed = d_a_packed;
+    p.B = d_B;
     p.C = d_C;
+
+    // 3 = 12 warps; 7 = 16 warps, 7 producers copying; 0 = 16 warps, 3 or 7 copying as each CTA's first tile says;
+    // not set = 3 or 0 as the last launch on this device noted
+    int producer_warps = tuning_get("PRODUCER_WARPS", -1);
+    if (producer_warps != 3 && producer_warps != 7 && producer_warps != 0) {
+        producer_warps = 3;
+        if (follow_hint) {
+            const FormHint hint = form_hint_word(dev);
+            if (hint.host) {
+                p.form_hint = hint.device;
+                if (*hint.host != 0) producer_warps = 0;
+            }
+        }
+    }
+    const bool wide = producer_warps != 3;
+    p.adaptive = producer_warps == 0;
+    if (dev >= 0 && dev < 64) g_last_tiled_warps[dev].store(wide ? 16 : 12, std::memory_order_relaxed);
+    const int threads = (P_CONSUMER_WARPS + (wide ? 7 : 3) + 1) * 32;
 
     int stages = tuning_get("STAGES", P_MAX_STAGES);
     if (stages > P_MAX_STAGES) stages = P_MAX_STAGES;
@@ -1134,30 +1191,20 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     }
     if (st) return st;
 
+    // (in block mode a CTA has work as soon as there are pairs of blocks for it)
     int grid = tuning_get("GRID", sms);
-    if (grid > p.num_tiles) grid = p.num_tiles;
+    const long pairs = std::max((long)ceil_div(p.a_rows, 2) * p.b_rows, (long)p.a_rows * ceil_div(p.b_rows, 2));
+    // With no more pairs of blocks than SMs the pipeline's tiles would occupy an eighth of them or a quarter: block mode whatever
+    // the patterns (512^3 at half density: 20.8 us in the pipeline, 18.7 in block mode; with four times as many pairs, 1024^3,
+    // 33.3 and 37.4).
+    p.few_blocks = pairs <= grid;
+    p.block_mode = tuning_get("BLOCK_MODE", p.few_blocks ? 1 : -1);
+    if (grid > std::max((long)p.num_tiles, pairs)) grid = (int)std::max((long)p.num_tiles, pairs);
     if (grid < 1) grid = 1;
-    // 3 = 12 warps; 7 = 16 warps, 7 producers copying; 0 = 16 warps, 3 or 7 copying as each CTA's first tile says;
-    // not set = 3 or 0 as the last launch on this device noted
-    int producer_warps = tuning_get("PRODUCER_WARPS", -1);
-    if (producer_warps != 3 && producer_warps != 7 && producer_warps != 0) {
-        producer_warps = 3;
-        if (follow_hint) {
-            const FormHint hint = form_hint_word(dev);
-            if (hint.host) {
-                p.form_hint = hint.device;
-                if (*hint.host != 0) producer_warps = 0;
-            }
-        }
-    }
-    const bool wide = producer_warps != 3;
-    p.adaptive = producer_warps == 0;
-    if (dev >= 0 && dev < 64) g_last_tiled_warps[dev].store(wide ? 16 : 12, std::memory_order_relaxed);
     auto launch = [&](auto kernel, int threads) -> int {
         ESMM_CUDA_TRY(launch_dependent(kernel, dim3(grid), dim3(threads), L.total, stream, maps, p));
         return ESMM_OK;
     };
-    const int threads = (P_CONSUMER_WARPS + (wide ? 7 : 3) + 1) * 32;
     int lst;
     if (tile_rows == 64) lst = wide ? launch(esmm_joint_sgemm_packed_kernel<1, 7>, threads) : launch(esmm_joint_sgemm_packed_kernel<1, 3>, threads);
     else lst = wide ? launch(esmm_joint_sgemm_packed_kernel<2, 7>, threads) : launch(esmm_joint_sgemm_packed_kernel<2, 3>, threads);

@@ -40,6 +40,84 @@ __device__ __forceinline__ void fma8(float (&acc)[8], float a, const float4 &b0,
     acc[7] = fmaf(a, b1.w, acc[7]);
 }
 
+// One k of the tile for one thread: its 4 rows of the top block, 4 rows of the bottom block
+// and 2 x 4 columns are one 16-byte load each.
+struct KFrag {
+    float4 at, ab, b0, b1;
+};
+
+// WMB = 32-row blocks per consumer warp: 2 in the 128 x 128 tiling, 1 in the 64 x 128 tiling (where a
+// thread holds 4 x 8 outputs and the "bottom" half of everything below is compiled out).
+template <int WMB>
+__device__ __forceinline__ KFrag load_kfrag(const char *pa, const char *pb)
+{
+    KFrag f;
+    f.at = *reinterpret_cast<const float4 *>(pa);
+    if (WMB == 2) f.ab = *reinterpret_cast<const float4 *>(pa + 128);
+    f.b0 = *reinterpret_cast<const float4 *>(pb);
+    f.b1 = *reinterpret_cast<const float4 *>(pb + 64);
+    return f;
+}
+
+// The thread's 8 x 8 outputs are held as row pairs for the packed FP32 multiply-add of sm_100 (fma.rn.f32x2: two
+// independent IEEE FMAs per instruction, half the issue slots of scalar FFMA):
+//   c[p][j] = (c of row 2p, column j; c of row 2p + 1, column j)
+// so an FMA takes the row pair (a[2p], a[2p+1]) as it comes from shared memory and one column of B in both halves.  Row
+// pairs 0, 1 are the top 32-row block, 2, 3 the bottom one.  Every output still sees one FMA per live k, in ascending k.
+// The row pair is the outer loop, so that eight instructions in a row use the same pair: this loop alone, operands in
+// shared memory, reaches 67.6 TFLOP/s, which is what fma.rn.f32x2 does with no loads at all; 63.3 with the column as
+// the outer loop, and 62.4 with the columns kept as pairs too (diagonal and anti-diagonal of 2 x 2 blocks).
+struct Acc {
+    float2 c[4][8];
+};
+
+__device__ __forceinline__ void acc_clear(Acc &acc)
+{
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc.c[i][j] = make_float2(0.0f, 0.0f);
+}
+
+// row 2p (e = 0) or 2p + 1 (e = 1), column j
+__device__ __forceinline__ float acc_get(const Acc &acc, int p, int e, int j) { return e ? acc.c[p][j].y : acc.c[p][j].x; }
+
+__device__ __forceinline__ void fma_pair_row(Acc &c, int p, float2 ar, const KFrag &f)
+{
+    const float b[8] = {f.b0.x, f.b0.y, f.b0.z, f.b0.w, f.b1.x, f.b1.y, f.b1.z, f.b1.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c.c[p][j] = __ffma2_rn(ar, make_float2(b[j], b[j]), c.c[p][j]);
+}
+
+__device__ __forceinline__ void fma_top(Acc &c, const KFrag &f)
+{
+    fma_pair_row(c, 0, make_float2(f.at.x, f.at.y), f);
+    fma_pair_row(c, 1, make_float2(f.at.z, f.at.w), f);
+}
+
+__device__ __forceinline__ void fma_bottom(Acc &c, const KFrag &f)
+{
+    fma_pair_row(c, 2, make_float2(f.ab.x, f.ab.y), f);
+    fma_pair_row(c, 3, make_float2(f.ab.z, f.ab.w), f);
+}
+
+// 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros instead
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, int src_bytes)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_commit()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// returns when at most N of this thread's copy groups are still in flight
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 #endif  // __CUDACC__
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,

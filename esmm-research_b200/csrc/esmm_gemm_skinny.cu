@@ -68,24 +68,6 @@ struct SkinnyParams {
     int *status;
 };
 
-// 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros instead
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, int src_bytes)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit()
-{
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-// returns when at most N of this thread's copy groups are still in flight
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group()
-{
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 __device__ __forceinline__ int sk_scan(int v, int lane)
 {
 #pragma unroll

@@ -149,8 +149,8 @@ int esmm_preprocess_a_packed(const float *d_A, int M, int K, uint8_t *d_out, flo
 /*
  * Same contract as esmm_gemm_ab (32-row A patterns) with the packed copy in place of A, except that
  * the first call on a device sets aside one 64-byte word of host-mapped memory (kept for the life of
- * the process): every launch of the tiled kernel notes there whether its first tile was one of
- * scattered single rows, and the next launch on that device picks its launch shape (12 or 16 warps
+ * the process): every launch of the tiled kernel notes there whether its operands were of
+ * scattered single rows in a form that gains from it, and the next launch on that device picks its launch shape (12 or 16 warps
  * per CTA) by it, without waiting for anything.  The shapes differ in speed only, never in a bit of
  * C; esmm_tuning_set("PRODUCER_WARPS", ...) pins one.  No device memory is allocated.  Make the first
  * call on a device outside any stream capture (the set-up is not a stream operation).
@@ -229,7 +229,8 @@ int esmm_selftest_bounded_wait(unsigned budget_us, void *stream);
  * environment cannot change what the library does.  No counterpart in the reference, whose tile
  * shapes are compile-time template constants (include/runners.cuh:830-838).
  * Names: TILE_M (64 | 128), STAGES, BROW_BITS, ROW_DENSITY, FORCE_LISTED, NO_RUN_TILES, VEC_PATTERNS
- * (0 | 4 | 16), NO_SKINNY, SKINNY_ROWS (32), PRODUCER_WARPS (3 | 7 | 0: pins the tiled kernel's launch shape), NO_DEPENDENT_LAUNCH, GROUP_M, GRID, PACK (64 | 128), SWIZZLE, TF32_PAIR (0 | 128 | 256), TF32_SPLIT_LAST,
+ * (0 | 4 | 16), NO_SKINNY, SKINNY_ROWS (32), PRODUCER_WARPS (3 | 7 | 0: pins the tiled kernel's launch shape),
+ * BLOCK_MODE (0 | 1: pins the tiled kernel's way of working, see esmm_gemm_blocks.cuh), NO_DEPENDENT_LAUNCH, GROUP_M, GRID, PACK (64 | 128), SWIZZLE, TF32_PAIR (0 | 128 | 256), TF32_SPLIT_LAST,
  * TF32_DIRECT_STORES.  esmm_tuning_set returns ESMM_ERR_UNSUPPORTED for any other name;
  * esmm_tuning_reset returns every hook to "unset" (the library's own choice).
  */

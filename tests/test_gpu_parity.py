@@ -729,3 +729,46 @@ def test_multi_launcher_two_ranks_on_one_gpu(cuda, pkg, oracle_mod):
         L.esmm_multi_destroy(h)
     bad = (C.c_int * 2)(0, 99)
     assert L.esmm_multi_create(M, N, K, 2, bad, C.byref(h)) == pkg.ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("mode", [1, 0])
+def test_gemm_block_mode(cuda, pkg, oracle_mod, tuning, mode):
+    """The tiled kernel's two ways of working, pinned: every warp on its own pair of 32 x 32 blocks with its own list of live k
+    (1), and the tiled pipeline (0).  Granularities that pair row blocks, column blocks or neither; one block, odd numbers of
+    blocks, ragged edges; lists of no k, fewer than a stage, and longer than their ring; one block of a pair dead where the
+    other is dense; several items per warp; pattern rows that cannot be read as words; the deepest K."""
+    tuning("BLOCK_MODE", int(mode))
+    for M, N, K, pa, pb, ga, gb in [(33, 32, 8, 1.0, 1.0, 32, 32), (64, 4, 64, 1.0, 1.0, 32, 32), (128, 128, 1024, 0.0, 0.5, 32, 32),
+                                    (257, 260, 1000, 0.4, 0.4, 32, 32), (100, 132, 8 * 37, 0.3, 0.7, 32, 32), (96, 160, 76, 0.8, 0.8, 32, 32),
+                                    (320, 352, 4096, 0.7, 0.9, 32, 32), (256, 384, 2048, 0.5, 0.5, 64, 64), (160, 416, 2048, 0.4, 0.5, 32, 64),
+                                    (224, 160, 2048, 0.5, 0.4, 64, 32), (64, 96, 27488, 0.3, 0.3, 32, 32)]:
+        A, B = workloads.tile_random(M, N, K, pa, pb, seed=M + N + K, gran_a=ga, gran_b=gb)
+        check_all_paths(cuda, pkg, oracle_mod, A, B)
+    for pat in (0xFF, 0x0F, 0xA5, 0x80):
+        A, B = workloads.uniform_pattern(200, 160, 8 * 21, pat, seed=pat)
+        check_all_paths(cuda, pkg, oracle_mod, A, B)
+    A, B = workloads.tile_random(128, 128, 4096, 1.0, 1.0, seed=3)
+    A[:32] = 0.0                      # row blocks 0 and 2, column block 3: one of a pair dead or nearly so
+    A[64:96, 40:] = 0.0
+    B[:4000, 96:] = 0.0
+    check_all_paths(cuda, pkg, oracle_mod, A, B)
+    tuning("GRID", 2)
+    A, B = workloads.tile_random(256, 1024, 1024, 0.3, 0.5, seed=4, gran_a=32, gran_b=32)
+    check_all_paths(cuda, pkg, oracle_mod, A, B)
+
+
+@pytest.mark.parametrize("mode", [1, 0])
+def test_gemm_block_mode_infinities(cuda, pkg, oracle_mod, tuning, mode):
+    """Steps past the end of the shorter list of a pair change nothing: with infinities and NaN in one block's rows, and sums that
+    are -0, every output of both blocks has the oracle's bits."""
+    tuning("BLOCK_MODE", int(mode))
+    A, B = workloads.tile_random(128, 128, 512, 0.3, 0.4, seed=8, gran_a=32, gran_b=32)
+    A[5, np.flatnonzero(A[5])[:3]] = [np.inf, -np.inf, np.nan]
+    A[70] = np.where(A[70] != 0, np.float32(-1e-30), 0)
+    B[:, 100] = np.where(B[:, 100] != 0, np.float32(1e-30), 0)      # row 70, column 100: products that round to -0
+    d = Dev(cuda, pkg, A, B)
+    d.patterns()
+    got, _ = d.sgemm_joint()
+    want = oracle_mod.gemm_joint(A, B, oracle_mod.preprocess_a(A), oracle_mod.preprocess_b(B))
+    same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
+    assert same.all() and np.isnan(want).any()
