@@ -31,6 +31,8 @@
 // ascending k, as in the tiled pipeline: the results are the same bits.
 #pragma once
 
+#include <climits>
+
 #include "esmm_gemm_shared.cuh"
 
 namespace esmm {
@@ -46,6 +48,7 @@ constexpr int BM_LIST_BYTES = BM_LIST * 2;
 constexpr int BM_WARP_BYTES = BM_SLOTS * BM_SLOT_BYTES + 2 * BM_LIST_BYTES;
 constexpr int BM_SMEM = BM_WARPS * BM_WARP_BYTES;
 constexpr int BM_TAIL = 6;                                  // of more than BM_WARPS items: 0 .. 12 measured, 4 - 6 best
+constexpr int RM_KL = 8;                                    // row-major A: lanes of a 4-byte copy instruction on the k (4: 9 % slower, 16: 12 %)
 constexpr int BM_SAMPLES = 8;                               // tiles looked at to choose the mode
 
 // Pattern bytes of K blocks kb .. kb + 3 of one pattern row (null: no such row), zero past the end.  words: the row may be
@@ -66,9 +69,36 @@ __device__ __forceinline__ unsigned inside_k(int kb, int K)
     return left >= 32 ? 0xFFFFFFFFu : left <= 0 ? 0u : (1u << left) - 1u;
 }
 
-__device__ __forceinline__ const uint8_t *pattern_row(const uint8_t *pat, int row, int rows, int nKB)
+// The pattern rows of one 32-row (32-column) block: count rows from `first` on, whose OR is the block's pattern; none: no such block.
+struct PatternRows {
+    const uint8_t *first;
+    int count;
+};
+
+__device__ __forceinline__ unsigned pattern_word(const PatternRows &r, int kb, int nKB, bool words)
 {
-    return row < rows ? pat + (size_t)row * nKB : nullptr;
+    unsigned v = pattern_word(r.first, kb, nKB, words);
+    for (int t = 1; t < r.count; ++t) v |= pattern_word(r.first + (size_t)t * nKB, kb, nKB, words);
+    return v;
+}
+
+template <typename Params>
+__device__ __forceinline__ PatternRows b_pattern(const Params &p, int block)
+{
+    return {block < p.b_rows ? p.b_pat + (size_t)block * p.nKB : nullptr, 1};
+}
+
+// A's patterns have one row per 32 rows of A, or (ROW_MAJOR) one for every a_div blocks, or a_mul for each.
+template <bool ROW_MAJOR, typename Params>
+__device__ __forceinline__ PatternRows a_pattern(const Params &p, int block)
+{
+    if (block >= p.a_rows) return {nullptr, 1};
+    if constexpr (ROW_MAJOR) {
+        const int row = block / p.a_div * p.a_mul;
+        return {p.a_pat + (size_t)row * p.nKB, min(p.a_mul, p.a_pat_rows - row)};
+    } else {
+        return {p.a_pat + (size_t)block * p.nKB, 1};
+    }
 }
 
 // What one warp sees of a sample: a 128 x 128 tile over up to 128 of its K blocks.  (block, k) counts.
@@ -81,17 +111,17 @@ struct TileStats {
     int a_differ, b_differ;   // bits in which adjacent row blocks (column blocks) of a pair differ
 };
 
-template <typename Params>
+template <bool ROW_MAJOR, typename Params>
 __device__ __forceinline__ TileStats tile_stats(const Params &p, int tm, int tn, int part, int lane)
 {
-    const uint8_t *ra[4], *rb[4];
+    PatternRows ra[4], rb[4];
     int na = 0, nb = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        ra[i] = pattern_row(p.a_pat, tm * 4 + i, p.a_rows, p.nKB);
-        rb[i] = pattern_row(p.b_pat, tn * 4 + i, p.b_rows, p.nKB);
-        na += ra[i] != nullptr;
-        nb += rb[i] != nullptr;
+        ra[i] = a_pattern<ROW_MAJOR>(p, tm * 4 + i);
+        rb[i] = b_pattern(p, tn * 4 + i);
+        na += ra[i].first != nullptr;
+        nb += rb[i].first != nullptr;
     }
     TileStats s = {0, 0, 0, 0, 0, 0, 0};
     // (one word per lane and row: a single round trip to memory)
@@ -115,10 +145,10 @@ __device__ __forceinline__ TileStats tile_stats(const Params &p, int tm, int tn,
             for (int i = 0; i < 4; ++i) s.work += __popc(a[i] & b[j]);
             s.rows64 += __popc((a[0] | a[1]) & b[j]) + __popc((a[2] | a[3]) & b[j]);
         }
-        if (ra[1]) s.a_differ += __popc(a[0] ^ a[1]);
-        if (ra[3]) s.a_differ += __popc(a[2] ^ a[3]);
-        if (rb[1]) s.b_differ += __popc(b[0] ^ b[1]);
-        if (rb[3]) s.b_differ += __popc(b[2] ^ b[3]);
+        if (ra[1].first) s.a_differ += __popc(a[0] ^ a[1]);
+        if (ra[3].first) s.a_differ += __popc(a[2] ^ a[3]);
+        if (rb[1].first) s.b_differ += __popc(b[0] ^ b[1]);
+        if (rb[3].first) s.b_differ += __popc(b[2] ^ b[3]);
     }
     s.slots = s.listed * na * nb;
     return s;
@@ -183,13 +213,21 @@ __device__ __forceinline__ void single_steps(Acc &acc, const char *sx, const cha
     }
 }
 
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void fill_4(uint32_t dst, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory"); }
+
 __device__ __forceinline__ void fill_16(uint32_t dst, float v)
 {
     asm volatile("st.shared.v4.f32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "f"(v) : "memory");
 }
 
 // One item: blocks x0 and x0 + 1 of X (TWO) or x0 alone, times block y of Y.
-template <bool TWO, typename Params>
+// ROW_MAJOR: A is the caller's matrix instead of the k-major packed copy; 4-byte copies transpose it on the way.
+template <bool TWO, bool ROW_MAJOR, typename Params>
 __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane, bool wide_b, int x0, int y)
 {
     LiveList l0, l1;
@@ -206,126 +244,188 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     const unsigned n4 = (unsigned)p.N * 4u;                       // bytes of a row of B
     const unsigned x_stride = wide_b ? n4 : TILE_M * 4u, y_stride = wide_b ? TILE_M * 4u : n4;
 
-                const uint8_t *px = (wide_b ? p.b_pat : p.a_pat) + (size_t)x0 * p.nKB;
-                const uint8_t *px1 = TWO ? px + p.nKB : nullptr;
-                const uint8_t *py = (wide_b ? p.a_pat : p.b_pat) + (size_t)y * p.nKB;
-                // 32 floats of packed A are contiguous within a panel of 128 rows; a row of B has N floats.  Chunks of B past its
-                // last column are not copied: whatever is multiplied there ends in columns of C that do not exist.
-                const int a_blk = wide_b ? y : x0, b_blk = wide_b ? x0 : y;
-                const char *a_src = reinterpret_cast<const char *>(p.a_packed + (size_t)(a_blk >> 2) * p.kp * TILE_M + (a_blk & 3) * 32);
-                const char *b_src = reinterpret_cast<const char *>(p.B + b_blk * 32);
-                const char *xs = (wide_b ? b_src : a_src) + c4 * 16, *ys = (wide_b ? a_src : b_src) + c4 * 16;
-                const int b_chunks = (p.N - b_blk * 32) >> 2;
-                const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);
+    const PatternRows px = wide_b ? b_pattern(p, x0) : a_pattern<ROW_MAJOR>(p, x0);
+    const PatternRows px1 = !TWO ? PatternRows{nullptr, 1} : wide_b ? b_pattern(p, x0 + 1) : a_pattern<ROW_MAJOR>(p, x0 + 1);
+    const PatternRows py = wide_b ? a_pattern<ROW_MAJOR>(p, y) : b_pattern(p, y);
+    // 32 floats of packed A are contiguous within a panel of 128 rows; a row of B has N floats.  Chunks of B past its
+    // last column are not copied: whatever is multiplied there ends in columns of C that do not exist.
+    const int a_blk = wide_b ? y : x0, b_blk = wide_b ? x0 : y;
+    const char *a_src = nullptr;
+    if constexpr (!ROW_MAJOR) a_src = reinterpret_cast<const char *>(p.a_packed + (size_t)(a_blk >> 2) * p.kp * TILE_M + (a_blk & 3) * 32);
+    const char *b_src = reinterpret_cast<const char *>(p.B + b_blk * 32);
+    const char *xs = (wide_b ? b_src : a_src) + c4 * 16, *ys = (wide_b ? a_src : b_src) + c4 * 16;
+    const int b_chunks = (p.N - b_blk * 32) >> 2;
+    const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);
 
-                Acc acc;
-                acc_clear(acc);
+    Acc acc;
+    acc_clear(acc);
 
-                // The lane's pattern bits of the 128 K blocks kb0 .. (m0, m1: joint bits of either block; wy, w0, w1: the words of the
-                // 128 K blocks after them, on their way) and how many eighths of them are listed already.
-                int kb0 = -128, part = 0, live = 0;
-                unsigned m0 = 0u, m1 = 0u, wy = 0u, w0 = 0u, w1 = 0u;
-                auto load_words = [&](int kb) {
-                    wy = pattern_word(py, kb, p.nKB, p.pat_words) & inside_k(kb, p.K);
-                    w0 = pattern_word(px, kb, p.nKB, p.pat_words);
-                    w1 = pattern_word(px1, kb, p.nKB, p.pat_words);
-                };
-                auto next_words = [&]() {
-                    kb0 += 128;
-                    part = 0;
-                    m0 = w0 & wy;
-                    m1 = w1 & wy;
-                    live = __reduce_add_sync(0xFFFFFFFFu, __popc(m0) | (__popc(m1) << 16));   // (both counts in one word)
-                    if (kb0 + 128 < p.nKB) load_words(kb0 + 128 + 4 * lane);
-                };
-                load_words(4 * lane);
-                next_words();
-                l0.made = l0.taken = l1.made = l1.taken = 0;
+    // The lane's pattern bits of the 128 K blocks kb0 .. (m0, m1: joint bits of either block; wy, w0, w1: the words of the
+    // 128 K blocks after them, on their way) and how many quarters of them are listed already.
+    int kb0 = -128, part = 0, live = 0;
+    unsigned m0 = 0u, m1 = 0u, wy = 0u, w0 = 0u, w1 = 0u;
+    auto load_words = [&](int kb) {
+        wy = pattern_word(py, kb, p.nKB, p.pat_words) & inside_k(kb, p.K);
+        w0 = pattern_word(px, kb, p.nKB, p.pat_words);
+        w1 = pattern_word(px1, kb, p.nKB, p.pat_words);
+    };
+    auto next_words = [&]() {
+        kb0 += 128;
+        part = 0;
+        m0 = w0 & wy;
+        m1 = w1 & wy;
+        live = __reduce_add_sync(0xFFFFFFFFu, __popc(m0) | (__popc(m1) << 16));   // (both counts in one word)
+        if (kb0 + 128 < p.nKB) load_words(kb0 + 128 + 4 * lane);
+    };
+    load_words(4 * lane);
+    next_words();
+    l0.made = l0.taken = l1.made = l1.taken = 0;
+    int wrap0 = INT_MAX, wrap1 = INT_MAX;   // (ROW_MAJOR) list positions from which on an entry is k - 65536
 
-                // Lists further K blocks until each list holds a stage or there is no room: all 128 at once where they fit, or a
-                // quarter of them (then a lane takes one byte).
-                auto refill = [&]() {
-                    bool wrote = false;
-                    while (kb0 < p.nKB && (l0.pending() < BM_ROWS || (TWO && l1.pending() < BM_ROWS))) {
-                        const int room = BM_LIST - max(l0.pending(), l1.pending());
-                        unsigned a0 = m0, a1 = m1;
-                        int k0 = (kb0 + 4 * lane) * BK;
-                        if (part == 0 && max(live & 0xFFFF, live >> 16) <= room) {
-                            part = 4;
-                        } else {
-                            if (room < 32 * BK) break;
-                            const int from = part * 8 + (lane >> 2), sh = (lane & 3) * 8;
-                            a0 = (__shfl_sync(0xFFFFFFFFu, m0, from) >> sh) & 0xFFu;
-                            a1 = (__shfl_sync(0xFFFFFFFFu, m1, from) >> sh) & 0xFFu;
-                            k0 = (kb0 + part * 32 + lane) * BK;
-                            ++part;
-                        }
-                        const int c = __popc(a0) | (__popc(a1) << 16);
-                        const int before = exclusive_scan(c, lane);
-                        const int total = __shfl_sync(0xFFFFFFFFu, before + c, 31);
-                        append_live(l0.list, l0.made + (before & 0xFFFF), a0, k0, p.status);
-                        if (TWO) append_live(l1.list, l1.made + (before >> 16), a1, k0, p.status);
-                        l0.made += total & 0xFFFF;
-                        l1.made += total >> 16;
-                        wrote = true;
-                        if (part == 4) next_words();
-                    }
-                    if (wrote) __syncwarp();
-                };
+    // Lists further K blocks until each list holds a stage or there is no room: all 128 at once where they fit, or a
+    // quarter of them (then a lane takes one byte).
+    auto refill = [&]() {
+        bool wrote = false;
+        while (kb0 < p.nKB && (l0.pending() < BM_ROWS || (TWO && l1.pending() < BM_ROWS))) {
+            const int room = BM_LIST - max(l0.pending(), l1.pending());
+            unsigned a0 = m0, a1 = m1;
+            int k0 = (kb0 + 4 * lane) * BK;
+            if (part == 0 && max(live & 0xFFFF, live >> 16) <= room) {
+                part = 4;
+            } else {
+                if (room < 32 * BK) break;
+                const int from = part * 8 + (lane >> 2), sh = (lane & 3) * 8;
+                a0 = (__shfl_sync(0xFFFFFFFFu, m0, from) >> sh) & 0xFFu;
+                a1 = (__shfl_sync(0xFFFFFFFFu, m1, from) >> sh) & 0xFFu;
+                k0 = (kb0 + part * 32 + lane) * BK;
+                ++part;
+            }
+            const int c = __popc(a0) | (__popc(a1) << 16);
+            const int before = exclusive_scan(c, lane);
+            const int total = __shfl_sync(0xFFFFFFFFu, before + c, 31);
+            append_live(l0.list, l0.made + (before & 0xFFFF), a0, k0, p.status);
+            if (TWO) append_live(l1.list, l1.made + (before >> 16), a1, k0, p.status);
+            if (ROW_MAJOR && k0 >= 65536 && wrap0 == INT_MAX) wrap0 = l0.made, wrap1 = l1.made;
+            l0.made += total & 0xFFFF;
+            l1.made += total >> 16;
+            wrote = true;
+            if (part == 4) next_words();
+        }
+        if (wrote) __syncwarp();
+    };
 
-                uint32_t slot = 0;
-                int count = 0;                 // steps of the stage that is multiplied
-                bool same = false;             // both blocks have the same 16 k there: Y is held once
-                do {
-                    cp_async_wait_group<0>();
-                    __syncwarp();              // the stage is complete for all lanes, and the one before it read by all
-                    refill();
-                    // ---- copies of the next stage ----
+    uint32_t slot = 0;
+    int count = 0;                 // steps of the stage that is multiplied
+    bool same = false;             // both blocks have the same 16 k there: Y is held once
+    do {
+        cp_async_wait_group<0>();
+        __syncwarp();              // the stage is complete for all lanes, and the one before it read by all
+        refill();
+        // ---- copies of the next stage ----
         const int d0 = min(BM_ROWS, l0.pending()), d1 = TWO ? min(BM_ROWS, l1.pending()) : 0;
         const uint32_t to = BM_SLOT_BYTES - slot;
         bool same_next = false;
-        if (!edge && d0 == BM_ROWS && (!TWO || d1 == BM_ROWS)) {
-            unsigned k0[BM_ROWS / 8], k1[BM_ROWS / 8];
-            same_next = TWO;
+        if constexpr (ROW_MAJOR) {
+            const int r16 = lane & 15;
+            auto entry = [&](const LiveList &l, int wrap, int row, int d) {
+                const int pos = l.taken + row;
+                return row < d ? (unsigned)l.list[pos & (BM_LIST - 1)] + (pos >= wrap ? 65536u : 0u) : 0u;
+            };
+            same_next = TWO && d0 == BM_ROWS && d1 == BM_ROWS &&
+                        __all_sync(0xFFFFFFFFu, entry(l0, wrap0, r16, d0) == entry(l1, wrap1, r16, d1));
+            // B: Y of either block, or X
 #pragma unroll
             for (int h = 0; h < BM_ROWS / 8; ++h) {
-                k0[h] = l0.list[(l0.taken + h * 8 + r8) & (BM_LIST - 1)];
-                k1[h] = TWO ? l1.list[(l1.taken + h * 8 + r8) & (BM_LIST - 1)] : 0;
-                if (TWO) same_next = __all_sync(0xFFFFFFFFu, k0[h] == k1[h]) && same_next;
-            }
+                const int row = h * 8 + r8;
 #pragma unroll
-            for (int h = 0; h < BM_ROWS / 8; ++h) {
-                const char *gx = xs + (size_t)k0[h] * x_stride, *gy = ys + (size_t)k0[h] * y_stride;
-                const uint32_t e0 = dst0 + to + h * 1024, e1 = dst1 + to + h * 1024;
-                cp_async_16(e0, gx, 16);
-                cp_async_16(e1, gx + 64, 16);
-                cp_async_16(e0 + 2 * BM_PART, gy, 16);
-                cp_async_16(e1 + 2 * BM_PART, gy + 64, 16);
-                if (TWO) {
-                    const char *gx1 = xs + (size_t)k1[h] * x_stride;
-                    cp_async_16(e0 + BM_PART, gx1 + 128, 16);
-                    cp_async_16(e1 + BM_PART, gx1 + 192, 16);
-                    if (!same_next) {
-                        const char *gy1 = ys + (size_t)k1[h] * y_stride;
-                        cp_async_16(e0 + 3 * BM_PART, gy1, 16);
-                        cp_async_16(e1 + 3 * BM_PART, gy1 + 64, 16);
+                for (int blk = 0; blk < (TWO ? 2 : 1); ++blk) {
+                    const int d = blk ? d1 : d0;
+                    if (max(d0, d1) == 0 || (blk && !wide_b && same_next)) continue;
+                    const char *g = b_src + c4 * 16 + (size_t)entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d) * n4 + (wide_b ? blk * 128 : 0);
+                    const uint32_t part = (uint32_t)((wide_b ? 0 : 2) + blk) * BM_PART;
+                    const uint32_t e0 = dst0 + to + h * 1024 + part, e1 = dst1 + to + h * 1024 + part;
+                    if (row < d) {
+                        const int lim = b_chunks - (wide_b ? blk * 8 : 0);
+                        if (!edge || c4 < lim) cp_async_16(e0, g, 16);
+                        if (!edge || c4 + 4 < lim) cp_async_16(e1, g + 64, 16);
+                    } else {
+                        fill_16(e0, wide_b ? -0.0f : 0.0f);
+                        fill_16(e1, wide_b ? -0.0f : 0.0f);
                     }
                 }
             }
-        } else if (max(d0, d1) > 0) {
-            // Past the end of a list X = -0 and Y = +0: a multiply-add with them changes no accumulator, not even a zero's sign.
-            const int x_lim = wide_b ? b_chunks : 16, y_lim = wide_b ? 8 : b_chunks;
+            // A: X of either block, or Y.  RM_KL lanes on the k, 32 / RM_KL on the rows.
+            constexpr int RL = 32 / RM_KL, STEPS = 32 / RL;
+            const int kk = lane & (RM_KL - 1), rr = lane / RM_KL;
+#pragma unroll
+            for (int blk = 0; blk < (TWO ? 2 : 1); ++blk) {
+                const int d = blk ? d1 : d0;
+                if (max(d0, d1) == 0 || (blk && wide_b && same_next)) continue;
+                const int row0 = (a_blk + (wide_b ? 0 : blk)) * 32 + rr;
+                const uint32_t part = smem_u32(ring) + to + (uint32_t)((wide_b ? 2 : 0) + blk) * BM_PART + kk * 128 + rr * 4;
+                const uint32_t e0 = part + (kk & 1) * 64, e1 = part + 64 - (kk & 1) * 64;
+#pragma unroll
+                for (int g = 0; g < BM_ROWS / RM_KL; ++g) {
+                    const int row = g * RM_KL + kk;
+                    const float *src = p.A + (size_t)row0 * p.K + entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d);
+                    if (row < d) {
+#pragma unroll
+                        for (int q = 0; q < STEPS; ++q) {
+                            // (rows past the end of A: any row, what is multiplied there ends in rows of C that do not exist)
+                            const float *sq = row0 + q * RL < p.M ? src + (size_t)(q * RL) * p.K : p.A;
+                            cp_async_4((q < STEPS / 2 ? e0 : e1) + g * (RM_KL * 128) + (q & (STEPS / 2 - 1)) * (RL * 4), sq);
+                        }
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < STEPS; ++q)
+                            fill_4((q < STEPS / 2 ? e0 : e1) + g * (RM_KL * 128) + (q & (STEPS / 2 - 1)) * (RL * 4), wide_b ? 0.0f : -0.0f);
+                    }
+                }
+            }
+        } else {
+            if (!edge && d0 == BM_ROWS && (!TWO || d1 == BM_ROWS)) {
+                unsigned k0[BM_ROWS / 8], k1[BM_ROWS / 8];
+                same_next = TWO;
+#pragma unroll
+                for (int h = 0; h < BM_ROWS / 8; ++h) {
+                    k0[h] = l0.list[(l0.taken + h * 8 + r8) & (BM_LIST - 1)];
+                    k1[h] = TWO ? l1.list[(l1.taken + h * 8 + r8) & (BM_LIST - 1)] : 0;
+                    if (TWO) same_next = __all_sync(0xFFFFFFFFu, k0[h] == k1[h]) && same_next;
+                }
+#pragma unroll
+                for (int h = 0; h < BM_ROWS / 8; ++h) {
+                    const char *gx = xs + (size_t)k0[h] * x_stride, *gy = ys + (size_t)k0[h] * y_stride;
+                    const uint32_t e0 = dst0 + to + h * 1024, e1 = dst1 + to + h * 1024;
+                    cp_async_16(e0, gx, 16);
+                    cp_async_16(e1, gx + 64, 16);
+                    cp_async_16(e0 + 2 * BM_PART, gy, 16);
+                    cp_async_16(e1 + 2 * BM_PART, gy + 64, 16);
+                    if (TWO) {
+                        const char *gx1 = xs + (size_t)k1[h] * x_stride;
+                        cp_async_16(e0 + BM_PART, gx1 + 128, 16);
+                        cp_async_16(e1 + BM_PART, gx1 + 192, 16);
+                        if (!same_next) {
+                            const char *gy1 = ys + (size_t)k1[h] * y_stride;
+                            cp_async_16(e0 + 3 * BM_PART, gy1, 16);
+                            cp_async_16(e1 + 3 * BM_PART, gy1 + 64, 16);
+                        }
+                    }
+                }
+            } else if (max(d0, d1) > 0) {
+                // Past the end of a list X = -0 and Y = +0: a multiply-add with them changes no accumulator, not even a zero's sign.
+                const int x_lim = wide_b ? b_chunks : 16, y_lim = wide_b ? 8 : b_chunks;
 #pragma unroll 1
-            for (int i = 0; i < 2 * (TWO ? 2 : 1) * (BM_ROWS / 8); ++i) {      // (row group, half of the row, block)
-                const int j = i & 1, row = ((i >> 1) & (BM_ROWS / 8 - 1)) * 8 + r8, blk = TWO ? i >> 2 : 0, ch = c4 + 4 * j;
-                const uint32_t e = (j ? dst1 : dst0) + to + (row - r8) * 128 + blk * BM_PART;
-                if (row < (blk ? d1 : d0)) {
-                    const size_t k = blk ? l1.list[(l1.taken + row) & (BM_LIST - 1)] : l0.list[(l0.taken + row) & (BM_LIST - 1)];
-                    if (blk * 8 + ch < x_lim) cp_async_16(e, xs + k * x_stride + blk * 128 + j * 64, 16);
-                    if (ch < y_lim) cp_async_16(e + 2 * BM_PART, ys + k * y_stride + j * 64, 16);
-                } else {
-                    fill_16(e, -0.0f);
-                    fill_16(e + 2 * BM_PART, 0.0f);
+                for (int i = 0; i < 2 * (TWO ? 2 : 1) * (BM_ROWS / 8); ++i) {      // (row group, half of the row, block)
+                    const int j = i & 1, row = ((i >> 1) & (BM_ROWS / 8 - 1)) * 8 + r8, blk = TWO ? i >> 2 : 0, ch = c4 + 4 * j;
+                    const uint32_t e = (j ? dst1 : dst0) + to + (row - r8) * 128 + blk * BM_PART;
+                    if (row < (blk ? d1 : d0)) {
+                        const size_t k = blk ? l1.list[(l1.taken + row) & (BM_LIST - 1)] : l0.list[(l0.taken + row) & (BM_LIST - 1)];
+                        if (blk * 8 + ch < x_lim) cp_async_16(e, xs + k * x_stride + blk * 128 + j * 64, 16);
+                        if (ch < y_lim) cp_async_16(e + 2 * BM_PART, ys + k * y_stride + j * 64, 16);
+                    } else {
+                        fill_16(e, -0.0f);
+                        fill_16(e + 2 * BM_PART, 0.0f);
+                    }
                 }
             }
         }
@@ -344,46 +444,46 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
             for (int r = 0; r < count; r += BM_STEP) single_steps(acc, sx + r * 128, sx_odd + r * 128, sy + r * 128);
         }
         count = max(d0, d1);
-                    same = same_next;
-                    slot = to;
-                } while (count > 0);
+        same = same_next;
+        slot = to;
+    } while (count > 0);
 
-                // ---- C is overwritten (beta = 0) ----
-                // x values 4 * xv .. + 3 and, in a pair, + 16; y values 4 * yv .. + 3 and + 16, of block xb
-                const size_t c_floats = (size_t)p.M * p.N;
-                const int xb = x0 + (TWO ? half : 0), xv = TWO ? xg : lm, yv = TWO ? yg : ln;
+    // ---- C is overwritten (beta = 0) ----
+    // x values 4 * xv .. + 3 and, in a pair, + 16; y values 4 * yv .. + 3 and + 16, of block xb
+    const size_t c_floats = (size_t)p.M * p.N;
+    const int xb = x0 + (TWO ? half : 0), xv = TWO ? xg : lm, yv = TWO ? yg : ln;
 #pragma unroll
-                for (int q = 0; q < 2; ++q) {                       // the two groups of 4 x values
-                    if (q == 1 && !TWO) break;
-                    if (!wide_b) {
+    for (int q = 0; q < 2; ++q) {                       // the two groups of 4 x values
+        if (q == 1 && !TWO) break;
+        if (!wide_b) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int row = xb * 32 + q * 16 + xv * 4 + i, col = y * 32 + yv * 4;
-                            float v8[8];
+            for (int i = 0; i < 4; ++i) {
+                const int row = xb * 32 + q * 16 + xv * 4 + i, col = y * 32 + yv * 4;
+                float v8[8];
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) v8[j] = acc_get(acc, 2 * q + (i >> 1), i & 1, j);
-                            const size_t off = (size_t)row * p.N + col;
-                            if (row < p.M && col < p.N && bounds_ok(off + 4 <= c_floats, p.status, 29))
-                                *reinterpret_cast<float4 *>(p.C + off) = make_float4(v8[0], v8[1], v8[2], v8[3]);
-                            if (row < p.M && col + 16 < p.N && bounds_ok(off + 20 <= c_floats, p.status, 29))
-                                *reinterpret_cast<float4 *>(p.C + off + 16) = make_float4(v8[4], v8[5], v8[6], v8[7]);
-                        }
-                    } else {
+                for (int j = 0; j < 8; ++j) v8[j] = acc_get(acc, 2 * q + (i >> 1), i & 1, j);
+                const size_t off = (size_t)row * p.N + col;
+                if (row < p.M && col < p.N && bounds_ok(off + 4 <= c_floats, p.status, 29))
+                    *reinterpret_cast<float4 *>(p.C + off) = make_float4(v8[0], v8[1], v8[2], v8[3]);
+                if (row < p.M && col + 16 < p.N && bounds_ok(off + 20 <= c_floats, p.status, 29))
+                    *reinterpret_cast<float4 *>(p.C + off + 16) = make_float4(v8[4], v8[5], v8[6], v8[7]);
+            }
+        } else {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const int row = y * 32 + yv * 4 + (j & 3) + 16 * (j >> 2), col = xb * 32 + q * 16 + xv * 4;
-                            const size_t off = (size_t)row * p.N + col;
-                            if (row < p.M && col < p.N && bounds_ok(off + 4 <= c_floats, p.status, 29))
-                                *reinterpret_cast<float4 *>(p.C + off) =
-                                    make_float4(acc_get(acc, 2 * q, 0, j), acc_get(acc, 2 * q, 1, j), acc_get(acc, 2 * q + 1, 0, j), acc_get(acc, 2 * q + 1, 1, j));
-                        }
-                    }
-                }
+            for (int j = 0; j < 8; ++j) {
+                const int row = y * 32 + yv * 4 + (j & 3) + 16 * (j >> 2), col = xb * 32 + q * 16 + xv * 4;
+                const size_t off = (size_t)row * p.N + col;
+                if (row < p.M && col < p.N && bounds_ok(off + 4 <= c_floats, p.status, 29))
+                    *reinterpret_cast<float4 *>(p.C + off) =
+                        make_float4(acc_get(acc, 2 * q, 0, j), acc_get(acc, 2 * q, 1, j), acc_get(acc, 2 * q + 1, 0, j), acc_get(acc, 2 * q + 1, 1, j));
+            }
+        }
+    }
 }
 
 // All of a warp's share of block mode.  smem: the CTA's dynamic shared memory; next: the CTA's item counter (initially
 // BM_WARPS: a warp's first item is its own number).
-template <typename Params>
+template <bool ROW_MAJOR, typename Params>
 __device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp, int lane, bool wide_b, int *next)
 {
     char *ring = smem + warp * BM_WARP_BYTES;
@@ -400,8 +500,8 @@ __device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp
         int tm, tn;
         tile_coords(item, tiles_m, tiles_n, tm, tn, wide_b ? 32 : 16);
         const int y = wide_b ? tm : tn, x0 = 2 * (wide_b ? tn : tm) + (v < whole ? 0 : (v - whole) & 1);
-        if (v < whole && x0 + 1 < x_blocks) block_item<true>(p, ring, lane, wide_b, x0, y);
-        else if (x0 < x_blocks) block_item<false>(p, ring, lane, wide_b, x0, y);
+        if (v < whole && x0 + 1 < x_blocks) block_item<true, ROW_MAJOR>(p, ring, lane, wide_b, x0, y);
+        else if (x0 < x_blocks) block_item<false, ROW_MAJOR>(p, ring, lane, wide_b, x0, y);
         int nx = 0;
         if (lane == 0) nx = atomicAdd(next, 1);
         v = __shfl_sync(0xFFFFFFFFu, nx, 0);

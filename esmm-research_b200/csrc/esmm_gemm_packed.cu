@@ -81,6 +81,10 @@ constexpr int P_MAX_STAGES = 6;
 // 0.8 / 0.8) 1900 / 1737, 0.67 (64-granular, 1 / 0.5) 1373 / 1346, 0.69 (64-granular, 0.8 / 0.8) 1675 / 1685, 0.83 (64-granular,
 // 0.9 / 0.9) 2050 / 2087, 1 (dense) 2130 / 2549.
 constexpr int BM_SIXTEENTHS = 11;
+// The same for row-major A, where block mode has to transpose A for every pair of blocks: 2048^3, with the pattern pass, pipeline /
+// block mode: share 0.11 (32-granular, 0.2 / 0.2) 103 / 71 us; 4096^3 share 0.33 (32-granular, 0.5 / 0.5) 1484 / 1489;
+// 2048^3 share 0.44 (64-granular, 0.5 / 0.5) 159 / 189.
+constexpr int RM_SIXTEENTHS = 4;
 
 // Optional timeline for tuning (build with -DESMM_TRACE): CTA 0 stamps %globaltimer at a few points
 // into a device array that esmm_trace_read copies out.  Not part of the product build or of the ABI.
@@ -118,6 +122,9 @@ struct PackedParams {
     int block_mode;    // 1, 0: always, never; -1: as the sampled tiles say
     int pat_words;     // pattern rows may be read as 32-bit words
     int few_blocks;    // no more pairs of blocks than CTAs
+    // row-major A: 32-row block mb uses A pattern rows (mb / a_div) * a_mul + [0, a_mul) of a_pat_rows
+    int a_div, a_mul, a_pat_rows;
+    const float *A;
     const uint8_t *a_pat;
     const uint8_t *b_pat;
     const float *a_packed;
@@ -312,7 +319,7 @@ __device__ __forceinline__ int build_list(uint16_t *list, unsigned m, int lane, 
 // tile's RB 32-row blocks and four 32-column blocks: one 16-byte or 4-byte load per pattern row.  aw[j] /
 // bw[j] get the four bytes of K block kb0 + j (byte i = block i).  Long K takes 16 per lane; shorter K
 // takes 4, so that all lanes have work.
-template <int RB, int KPL>
+template <int RB, int KPL, bool RM>
 __device__ __forceinline__ void load_patterns(const PackedParams &p, int tm, int tn, int kb0, bool valid,
                                               unsigned (&aw)[KPL], unsigned (&bw)[KPL])
 {
@@ -323,13 +330,16 @@ __device__ __forceinline__ void load_patterns(const PackedParams &p, int tm, int
         const int mb = tm * RB + i, nb = tn * 4 + i;
 #pragma unroll
         for (int w = 0; w < W; ++w) ra[i][w] = rb[i][w] = 0u;
-        if (valid && i < RB && mb < p.a_rows && bounds_ok(kb0 >= 0 && kb0 + KPL <= p.nKB, p.status, 21)) {
-            const uint8_t *src = p.a_pat + (size_t)mb * p.nKB + kb0;
-            if (KPL == 16) {
-                const uint4 v = *reinterpret_cast<const uint4 *>(src);
-                ra[i][0] = v.x, ra[i][W > 1 ? 1 : 0] = v.y, ra[i][W > 2 ? 2 : 0] = v.z, ra[i][W > 3 ? 3 : 0] = v.w;
-            } else {
-                ra[i][0] = *reinterpret_cast<const unsigned *>(src);
+        const PatternRows pr = a_pattern<RM>(p, mb);
+        if (valid && i < RB && pr.first && bounds_ok(kb0 >= 0 && kb0 + KPL <= p.nKB, p.status, 21)) {
+            for (int j = 0; j < pr.count; ++j) {
+                const uint8_t *src = pr.first + (size_t)j * p.nKB + kb0;
+                if (KPL == 16) {
+                    const uint4 v = *reinterpret_cast<const uint4 *>(src);
+                    ra[i][0] |= v.x, ra[i][W > 1 ? 1 : 0] |= v.y, ra[i][W > 2 ? 2 : 0] |= v.z, ra[i][W > 3 ? 3 : 0] |= v.w;
+                } else {
+                    ra[i][0] |= *reinterpret_cast<const unsigned *>(src);
+                }
             }
         }
         if (valid && nb < p.b_rows && bounds_ok(kb0 >= 0 && kb0 + KPL <= p.nKB, p.status, 21)) {
@@ -404,14 +414,14 @@ __device__ __forceinline__ bool blocks_cover(unsigned aw, unsigned bw, unsigned 
     return ((aw & l4 & am) == (l4 & am)) && ((bw & l4) == l4);
 }
 
-template <int RB, int KPL>
+template <int RB, int KPL, bool RM>
 __device__ __forceinline__ void tile_scan(const PackedParams &p, int tm, int tn, int lane, unsigned &live_first,
                                           bool &uniform, bool &full, int &live_total, int &live_small)
 {
     for (int c0 = 0; c0 < p.nKB; c0 += 32 * KPL) {
         const int kb0 = c0 + KPL * lane;
         unsigned aw[KPL], bw[KPL];
-        load_patterns<RB, KPL>(p, tm, tn, kb0, kb0 < p.nKB, aw, bw);
+        load_patterns<RB, KPL, RM>(p, tm, tn, kb0, kb0 < p.nKB, aw, bw);
         if (c0 == 0) live_first = __shfl_sync(0xFFFFFFFFu, tile_live(aw[0], bw[0]), 0);
         bool same = true, cover = true;
         int cnt = 0, small = 0;
@@ -436,14 +446,24 @@ struct TileScan {
     int live_total, live_small;
 };
 
-template <int RB>
+template <bool RM>
+__device__ __forceinline__ unsigned a_byte(const PackedParams &p, int mb, int kb)
+{
+    const PatternRows pr = a_pattern<RM>(p, mb);
+    unsigned v = 0u;
+    if (pr.first)
+        for (int j = 0; j < pr.count; ++j) v |= pr.first[(size_t)j * p.nKB + kb];
+    return v;
+}
+
+template <int RB, bool RM>
 __device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm, int tn, int lane)
 {
     TileScan s = {0u, true, true, 0, 0};
     if (p.vec_patterns == 16) {
-        tile_scan<RB, 16>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
+        tile_scan<RB, 16, RM>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
     } else if (p.vec_patterns == 4) {
-        tile_scan<RB, 4>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
+        tile_scan<RB, 4, RM>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
     } else {
         for (int kb0 = 0; kb0 < p.nKB; kb0 += 32) {
             const int kb = kb0 + lane;
@@ -452,7 +472,7 @@ __device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm,
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int mb = tm * RB + i, nb = tn * 4 + i;
-                    if (i < RB && mb < p.a_rows) au |= p.a_pat[(size_t)mb * p.nKB + kb];
+                    if (i < RB) au |= a_byte<RM>(p, mb, kb);
                     if (nb < p.b_rows) bu |= p.b_pat[(size_t)nb * p.nKB + kb];
                 }
             }
@@ -469,7 +489,7 @@ __device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm,
 
 // Second pass: the row list.  Lane l owns K blocks c0 + KPL l .. c0 + KPL l + KPL - 1 (consecutive lanes,
 // consecutive K); K blocks with more than whole_above live k are listed whole.  Returns the row count.
-template <int RB, int KPL>
+template <int RB, int KPL, bool RM>
 __device__ __forceinline__ int tile_list(const PackedParams &p, int tm, int tn, int lane, int whole_above,
                                          uint16_t *krow, uint8_t *rmask)
 {
@@ -477,7 +497,7 @@ __device__ __forceinline__ int tile_list(const PackedParams &p, int tm, int tn, 
     for (int c0 = 0; c0 < p.nKB; c0 += 32 * KPL) {
         const int kb0 = c0 + KPL * lane;
         unsigned aw[KPL], bw[KPL];
-        load_patterns<RB, KPL>(p, tm, tn, kb0, kb0 < p.nKB, aw, bw);
+        load_patterns<RB, KPL, RM>(p, tm, tn, kb0, kb0 < p.nKB, aw, bw);
         unsigned rows[KPL];
         int c = 0;
 #pragma unroll
@@ -514,9 +534,12 @@ __device__ __noinline__ int listed_warp_rows(const uint8_t *rmask, int n, int la
     return __reduce_add_sync(0xFFFFFFFFu, warp_rows);
 }
 
-template <int WMB, int NPW>
-__global__ void __launch_bounds__((P_CONSUMER_WARPS + NPW + 1) * 32, 1)
-esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const PackedParams p)
+// RM: A is the caller's row-major matrix.  The producers then transpose the tile's rows of A with 4-byte copies, the rest is the same.
+// (Before, a kernel of its own fetched boxes of 128 rows x 8 k, multiplied with scalar FMAs and could not leave out dead k of A.
+// Kernel and pattern pass, before -> now: 2048^3 64-granular 0.5 / 0.5 237 -> 159 us, 32-granular 0.2 / 0.2 111 -> 71; 4096^3 dense
+// 2813 -> 2622, half 1855 -> 1322, quarter 1469 -> 687, eighth 855 -> 474; 16 x 11008 x 4096 MLP 146 -> 65.)
+template <int WMB, int NPW, bool RM>
+__device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const PackedParams &p)
 {
     static_assert(NPW == 3 || NPW == 7, "consumers, producers and the mask warp fill whole warp groups");
     constexpr int P_TMA_WARPS = NPW;
@@ -547,7 +570,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
-            mbar_init(full0 + 8 * s, 1);
+            mbar_init(full0 + 8 * s, RM ? 1 + 32 * P_TMA_WARPS : 1);
             mbar_init(empty0 + 8 * s, P_CONSUMER_WARPS);
         }
         for (int b = 0; b < 2; ++b) {
@@ -568,7 +591,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
     if (warp == P_MASK_WARP && (int)blockIdx.x < p.num_tiles) {
         int tm, tn;
         tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
-        scan = tile_scan_any<RB>(p, tm, tn, lane);
+        scan = tile_scan_any<RB, RM>(p, tm, tn, lane);
     }
     if (p.block_mode != 0) {
         // two vectors per sample, where the consumers' lists will be
@@ -576,7 +599,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
         static_assert(2 * BM_SAMPLES * sizeof(int4) <= P_CONSUMER_WARPS * 2 * 96 && BM_SAMPLES <= P_CONSUMER_WARPS, "samples");
         if (warp < BM_SAMPLES) {
             const int panels = (p.a_rows + 3) >> 2;
-            const TileStats s = tile_stats(p, warp * panels / BM_SAMPLES, ((5 * warp + 2) & 7) * p.tiles_n / BM_SAMPLES, warp, lane);
+            const TileStats s = tile_stats<RM>(p, warp * panels / BM_SAMPLES, ((5 * warp + 2) & 7) * p.tiles_n / BM_SAMPLES, warp, lane);
             int4 x, y;
             x.x = __reduce_add_sync(0xFFFFFFFFu, s.slots);
             x.y = __reduce_add_sync(0xFFFFFFFFu, s.work);
@@ -601,7 +624,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             a_differ += x.z;
             b_differ += x.w;
         }
-        const bool blocks = p.block_mode > 0 || 16 * work <= BM_SIXTEENTHS * slots;
+        const bool blocks = p.block_mode > 0 || 16 * work <= (RM ? RM_SIXTEENTHS : BM_SIXTEENTHS) * slots;
         if (blocks && blockIdx.x == 0 && threadIdx.x == 0 && p.form_hint != nullptr) {
             // the note for the next launch (see gemm_ab_packed_launch_form)
             int listed = 0, rows64 = 0, single = 0;
@@ -615,7 +638,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
         }
         __syncthreads();   // the samples have been read by all
         if (blocks) {
-            if (warp < BM_WARPS) block_mode(p, smem, warp, lane, b_differ < a_differ, next_item);
+            if (warp < BM_WARPS) block_mode<RM>(p, smem, warp, lane, RM ? b_differ <= a_differ : b_differ < a_differ, next_item);
             return;
         }
     }
@@ -634,7 +657,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             int tm, tn;
             tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
             // A first pass over the tile's pattern bytes (the first tile's is done) decides the listing policy.
-            if (it > 0) scan = tile_scan_any<RB>(p, tm, tn, lane);
+            if (it > 0) scan = tile_scan_any<RB, RM>(p, tm, tn, lane);
             const unsigned live_first = scan.live_first;
             const bool uniform = scan.uniform, full = scan.full;
             const int live_total = scan.live_total, live_small = scan.live_small;
@@ -663,9 +686,9 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             if (run_code) {
                 pos = p.nKB * __popc(live_first);
             } else if (p.vec_patterns == 16) {
-                pos = tile_list<RB, 16>(p, tm, tn, lane, whole_above, krow, rmask);
+                pos = tile_list<RB, 16, RM>(p, tm, tn, lane, whole_above, krow, rmask);
             } else if (p.vec_patterns == 4) {
-                pos = tile_list<RB, 4>(p, tm, tn, lane, whole_above, krow, rmask);
+                pos = tile_list<RB, 4, RM>(p, tm, tn, lane, whole_above, krow, rmask);
             } else {
                 for (int kb0 = 0; kb0 < p.nKB; kb0 += 32) {
                     const int kb = kb0 + lane;
@@ -674,7 +697,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const int mb = tm * RB + i, nb = tn * 4 + i;
-                            if (i < RB && mb < p.a_rows) aw |= (unsigned)p.a_pat[(size_t)mb * p.nKB + kb] << (8 * i);
+                            if (i < RB) aw |= a_byte<RM>(p, mb, kb) << (8 * i);
                             if (nb < p.b_rows) bw |= (unsigned)p.b_pat[(size_t)nb * p.nKB + kb] << (8 * i);
                         }
                     }
@@ -730,7 +753,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
         // count then goes negative for a moment, which it is allowed to, and the phase cannot complete
         // before producer 0's arrival.)
         const int q = warp - P_TMA_WARP;
-        if (q == 0 && lane < 16) tma_prefetch_descriptor(&maps.a_box[0] + lane);
+        if (q == 0 && lane < 16 && (!RM || lane >= 8)) tma_prefetch_descriptor(&maps.a_box[0] + lane);
         int slot = 0;
         uint32_t phase = 0;
         uint32_t issued_bits = 0, parity_bits = 0;  // per slot: ever issued / parity of last issue
@@ -758,7 +781,64 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             const int panel = WMB == 2 ? tm : tm >> 1;
             const int a_x = WMB == 2 ? 0 : (tm & 1) * TM_ROWS;
             const int a_row0 = panel * p.kp, b_col0 = tn * TILE_N;
-            if (run_code) {
+            if constexpr (RM) {
+                const int lc = run_code & 15, kk0 = (run_code >> 4) & 7;
+                for (int r0 = 0; r0 < n; r0 += ROWS_PER_STAGE) {
+                    const int cnt = min(ROWS_PER_STAGE, n - r0);
+                    int k = -1;                                    // of the stage's row `lane`
+                    if (run_code) k = (((r0 + lane) >> lc) << 3) + kk0 + (lane & ((1 << lc) - 1));
+                    else if (lane < cnt && bounds_ok(r0 + lane < p.cap, p.status, 27)) k = krow[r0 + lane];
+                    // B in boxes, as below
+                    const int k_prev = __shfl_up_sync(0xFFFFFFFFu, k, 1);
+                    const unsigned starts = __ballot_sync(0xFFFFFFFFu, lane < cnt && (lane == 0 || k != k_prev + 1));
+                    int box_log = -1;
+                    if (lane < cnt && !run_code) {
+                        const int first = 31 - __clz((int)(starts & (0xFFFFFFFFu >> (31 - lane))));
+                        const unsigned later = lane == 31 ? 0u : (starts >> (first + 1)) << (first + 1);
+                        const int len = (later ? __ffs((int)later) - 1 : cnt) - first, o = lane - first, full8 = len & ~7;
+                        if (o < full8) box_log = (o & 7) == 0 ? 3 : -1;
+                        else if ((len & 4) && o == full8) box_log = 2;
+                        else if ((len & 2) && o == full8 + (len & 4)) box_log = 1;
+                        else if ((len & 1) && o == len - 1) box_log = 0;
+                        if (((lane * P_TMA_WARPS) >> 5) != q) box_log = -1;
+                    }
+                    ok = mbar_wait(empty0 + 8 * slot, phase ^ 1, abort_flag);
+                    ok = __all_sync(0xFFFFFFFFu, ok);
+                    if (!ok) break;
+                    const uint32_t full = full0 + 8 * slot;
+                    const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * PSTAGE_BYTES;
+                    if (q == 0 && lane == 0) {
+                        mbar_arrive_expect_tx(full, (uint32_t)cnt * ROW_BYTES);
+                        if (run_code) tma_load_3d(s0 + STAGE_HALF_BYTES, &maps.b_run[lc], b_col0, kk0, r0 >> lc, full);
+                    }
+                    if (box_log >= 0) tma_load_2d(s0 + STAGE_HALF_BYTES + lane * ROW_BYTES, &maps.b_box[box_log], b_col0, k, full);
+                    // A: 4-byte copies, eight lanes on the k and four on the rows, so that neighbouring k of a row come as one
+                    // sector; row groups shared out among the producers.  Rows past the end of A, k past its width (in K
+                    // blocks listed whole) and past the end of the list: any element, never multiplied or never stored.
+                    // These copies are what bounds the form: 4096^3 dense 2622 us against 2144 with packed A.  (Four lanes
+                    // on the k, eight on the rows, fewer bank conflicts but half of each sector: 2753; seven producer
+                    // warps: 2793.)
+                    constexpr int KL = RM_KL, RL = 32 / KL;
+                    const int kk = lane & (KL - 1), rr = lane / KL;
+                    int kg[32 / KL];
+#pragma unroll
+                    for (int g = 0; g < 32 / KL; ++g) kg[g] = min(max(__shfl_sync(0xFFFFFFFFu, k, KL * g + kk), 0), p.K - 1);
+#pragma unroll 1
+                    for (int rg = q; rg < TM_ROWS / RL; rg += P_TMA_WARPS) {
+                        const float *row = p.A + (size_t)min(tm * TM_ROWS + rg * RL + rr, p.M - 1) * p.K;
+                        const uint32_t d = s0 + kk * A_ROW + (rg * RL + rr) * 4;
+#pragma unroll
+                        for (int g = 0; g < 32 / KL; ++g) cp_async_4(d + g * KL * A_ROW, row + kg[g]);
+                    }
+                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+                    issued_bits |= 1u << slot;
+                    parity_bits = (parity_bits & ~(1u << slot)) | (phase << slot);
+                    if (++slot == p.stages) {
+                        slot = 0;
+                        phase ^= 1;
+                    }
+                }
+            } else if (run_code) {
                 // a run tile: whole stages, each one box per operand, no row list
                 const int lc = run_code & 15, kk0 = (run_code >> 4) & 7;
                 for (int r0 = 0; r0 < n; r0 += ROWS_PER_STAGE) {
@@ -787,8 +867,8 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
                 }
             }
             // (the k of a stage's rows are read one stage ahead, under the copies of the stage before)
-            int k_next = !run_code && lane < n && bounds_ok(lane < p.cap, p.status, 27) ? (int)krow[lane] : -1;
-            for (int r0 = 0; r0 < n && !run_code; r0 += ROWS_PER_STAGE) {
+            int k_next = !RM && !run_code && lane < n && bounds_ok(lane < p.cap, p.status, 27) ? (int)krow[lane] : -1;
+            for (int r0 = 0; r0 < n && !RM && !run_code; r0 += ROWS_PER_STAGE) {
                 const int cnt = min(ROWS_PER_STAGE, n - r0);
                 const bool valid = lane < cnt;
                 if (it == 0 && q == 0 && r0 < 80 * ROWS_PER_STAGE) ESMM_STAMP(700 + 4 * (r0 / ROWS_PER_STAGE));
@@ -862,6 +942,7 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
             __syncwarp();
             if (lane == 0) mbar_arrive(lempty0 + 8 * buf);
         }
+        if (RM) cp_async_wait_group<0>();
         if (!ok && lane == 0) {
             // leave only after the copies already issued have landed (bounded)
             for (int s = 0; s < p.stages; ++s) {
@@ -982,6 +1063,20 @@ esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const Pa
     if (!ok && lane == 0) atomicExch(p.status, (int)ESMM_ERR_TIMEOUT);
 }
 
+template <int WMB, int NPW>
+__global__ void __launch_bounds__((P_CONSUMER_WARPS + NPW + 1) * 32, 1)
+esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const PackedParams p)
+{
+    tiled_sgemm<WMB, NPW, false>(maps, p);
+}
+
+template <int WMB>
+__global__ void __launch_bounds__((P_CONSUMER_WARPS + 4) * 32, 1)
+esmm_joint_sgemm_kernel(const __grid_constant__ PackedMaps maps, const PackedParams p)
+{
+    tiled_sgemm<WMB, 3, true>(maps, p);
+}
+
 #ifdef ESMM_TRACE
 extern "C" int esmm_trace_read(unsigned long long *host, int n)
 {
@@ -1029,7 +1124,7 @@ static FormHint form_hint_word(int dev)
     return words[dev];
 }
 
-// Once per device: the SM count, and the shared-memory allowance of all four forms of the kernel raised to the device's
+// Once per device: the SM count, and the shared-memory allowance of all forms of the kernel raised to the device's
 // maximum.  (Raising it also loads the forms' code, so that the first launch in the other shape does not pay for that.)
 static int prepare_device(int dev, int *sms)
 {
@@ -1045,6 +1140,8 @@ static int prepare_device(int dev, int *sms)
         ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_packed_kernel<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_packed_kernel<1, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_packed_kernel<2, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         sm_count[dev] = n;
     }
     *sms = sm_count[dev];
@@ -1072,6 +1169,9 @@ int gemm_ab_packed_launch(int M, int N, int K, const float *d_a_packed, const fl
 
 // follow_hint = false: the 12-warp form unless PRODUCER_WARPS says otherwise, and no host-mapped word (for the
 // entry point that may not allocate).
+static int tiled_launch(int M, int N, int K, const float *d_a_packed, const float *d_A, int a_tile_m, const float *d_B, float *d_C,
+                        const uint8_t *d_a_pat, const uint8_t *d_b_pat, cudaStream_t stream, bool follow_hint);
+
 int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, const float *d_B, float *d_C,
                                const uint8_t *d_a_pat, const uint8_t *d_b_pat, cudaStream_t stream, bool follow_hint)
 {
@@ -1080,7 +1180,28 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     if (((uintptr_t)d_a_packed | (uintptr_t)d_B | (uintptr_t)d_C) & 15) return ESMM_ERR_ALIGN;
     if (gemm_ab_skinny_applies(M, N, K))
         return gemm_ab_skinny_launch(M, N, K, d_a_packed, d_B, d_C, d_a_pat, d_b_pat, stream);
+    return tiled_launch(M, N, K, d_a_packed, nullptr, 32, d_B, d_C, d_a_pat, d_b_pat, stream, follow_hint);
+}
 
+constexpr int RM_MAX_KB = 8332;   // longest K taken with row-major A, in K blocks
+
+// Row-major A, A patterns with one row per a_tile_m rows.
+int gemm_ab_launch(int M, int N, int K, const float *d_A, const float *d_B, float *d_C,
+                   const uint8_t *d_a_pat, const uint8_t *d_b_pat, int a_tile_m, cudaStream_t stream)
+{
+    if (!d_A || !d_B || !d_C || !d_a_pat || !d_b_pat) return ESMM_ERR_NULL;
+    if (M <= 0 || N <= 0 || K <= 0 || (K & 3) || (N & 3)) return ESMM_ERR_SHAPE;
+    if (a_tile_m <= 0 || (a_tile_m < 32 ? (32 % a_tile_m) : (a_tile_m % 32))) return ESMM_ERR_UNSUPPORTED;
+    if (((uintptr_t)d_A | (uintptr_t)d_B | (uintptr_t)d_C) & 15) return ESMM_ERR_ALIGN;
+    if (ceil_div(K, BK) > RM_MAX_KB) return ESMM_ERR_TOO_LARGE;
+    return tiled_launch(M, N, K, nullptr, d_A, a_tile_m, d_B, d_C, d_a_pat, d_b_pat, stream, false);
+}
+
+// A packed (d_a_packed) or row-major (d_A, with a_tile_m).
+static int tiled_launch(int M, int N, int K, const float *d_a_packed, const float *d_A, int a_tile_m, const float *d_B, float *d_C,
+                        const uint8_t *d_a_pat, const uint8_t *d_b_pat, cudaStream_t stream, bool follow_hint)
+{
+    const bool row_major = d_a_packed == nullptr;
     PackedParams p;
     memset(&p, 0, sizeof p);
     p.M = M;
@@ -1088,8 +1209,15 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     p.K = K;
     p.nKB = ceil_div(K, BK);
     p.kp = p.nKB * BK;
-    if (p.kp > 65535) return ESMM_ERR_TOO_LARGE;  // row list entries are 16-bit k indices
+    if (p.kp > 65535 && !row_major) return ESMM_ERR_TOO_LARGE;  // row list entries are 16-bit k indices
     p.cap = ((p.kp + 31) & ~31) + 32;
+    // (row-major A with more k than the pipeline's row lists have room for: block mode, whose lists are rings)
+    const bool lists_fit = packed_smem_layout(2, p.cap).total <= SMEM_LIMIT;
+    if (row_major && !lists_fit) p.cap = 64;
+    p.A = d_A;
+    p.a_div = a_tile_m >= 32 ? a_tile_m / 32 : 1;
+    p.a_mul = a_tile_m >= 32 ? 1 : 32 / a_tile_m;
+    p.a_pat_rows = ceil_div(M, a_tile_m);
     p.a_rows = ceil_div(M, 32);
     p.b_rows = ceil_div(N, PAT_N);
     int dev = 0, sms = 0;
@@ -1136,7 +1264,9 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     // 3 = 12 warps; 7 = 16 warps, 7 producers copying; 0 = 16 warps, 3 or 7 copying as each CTA's first tile says;
     // not set = 3 or 0 as the last launch on this device noted
     int producer_warps = tuning_get("PRODUCER_WARPS", -1);
-    if (producer_warps != 3 && producer_warps != 7 && producer_warps != 0) {
+    if (row_major) {
+        producer_warps = 3;
+    } else if (producer_warps != 3 && producer_warps != 7 && producer_warps != 0) {
         producer_warps = 3;
         if (follow_hint) {
             const FormHint hint = form_hint_word(dev);
@@ -1148,7 +1278,7 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     }
     const bool wide = producer_warps != 3;
     p.adaptive = producer_warps == 0;
-    if (dev >= 0 && dev < 64) g_last_tiled_warps[dev].store(wide ? 16 : 12, std::memory_order_relaxed);
+    if (!row_major && dev >= 0 && dev < 64) g_last_tiled_warps[dev].store(wide ? 16 : 12, std::memory_order_relaxed);
     const int threads = (P_CONSUMER_WARPS + (wide ? 7 : 3) + 1) * 32;
 
     int stages = tuning_get("STAGES", P_MAX_STAGES);
@@ -1171,15 +1301,18 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     PackedMaps maps;
     const uint64_t a_rows_total = (uint64_t)panels * p.kp;
     int st = 0;
+    memset(&maps, 0, sizeof maps);
     for (int i = 0; i < 4 && !st; ++i) {
-        st = make_map_2d(&maps.a_box[i], d_a_packed, TILE_M, a_rows_total, tile_rows, 1u << i, CU_TENSOR_MAP_SWIZZLE_NONE,
+        if (!row_major)
+            st = make_map_2d(&maps.a_box[i], d_a_packed, TILE_M, a_rows_total, tile_rows, 1u << i, CU_TENSOR_MAP_SWIZZLE_NONE,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
         if (!st) st = make_map_2d(&maps.b_box[i], d_B, (uint64_t)N, (uint64_t)K, TILE_N, 1u << i, CU_TENSOR_MAP_SWIZZLE_NONE,
                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
     }
     for (int i = 0; i < 4 && !st; ++i) {
         const uint32_t c = 1u << i;
-        st = make_map_3d(&maps.a_run[i], d_a_packed, TILE_M, BK, (uint64_t)panels * p.nKB, (uint64_t)TILE_M * 4,
+        if (!row_major)
+            st = make_map_3d(&maps.a_run[i], d_a_packed, TILE_M, BK, (uint64_t)panels * p.nKB, (uint64_t)TILE_M * 4,
                          (uint64_t)TILE_M * 4 * BK, tile_rows, c, ROWS_PER_STAGE / c);
         if (!st) {
             if (p.b_runs_ok)
@@ -1199,6 +1332,7 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
     // 33.3 and 37.4).
     p.few_blocks = pairs <= grid;
     p.block_mode = tuning_get("BLOCK_MODE", p.few_blocks ? 1 : -1);
+    if (!lists_fit) p.block_mode = 1;
     if (grid > std::max((long)p.num_tiles, pairs)) grid = (int)std::max((long)p.num_tiles, pairs);
     if (grid < 1) grid = 1;
     auto launch = [&](auto kernel, int threads) -> int {
@@ -1206,7 +1340,8 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
         return ESMM_OK;
     };
     int lst;
-    if (tile_rows == 64) lst = wide ? launch(esmm_joint_sgemm_packed_kernel<1, 7>, threads) : launch(esmm_joint_sgemm_packed_kernel<1, 3>, threads);
+    if (row_major) lst = tile_rows == 64 ? launch(esmm_joint_sgemm_kernel<1>, threads) : launch(esmm_joint_sgemm_kernel<2>, threads);
+    else if (tile_rows == 64) lst = wide ? launch(esmm_joint_sgemm_packed_kernel<1, 7>, threads) : launch(esmm_joint_sgemm_packed_kernel<1, 3>, threads);
     else lst = wide ? launch(esmm_joint_sgemm_packed_kernel<2, 7>, threads) : launch(esmm_joint_sgemm_packed_kernel<2, 3>, threads);
     if (lst != ESMM_OK) return lst;
     ESMM_CUDA_TRY(cudaGetLastError());
@@ -1228,4 +1363,10 @@ extern "C" int esmm_gemm_ab_packed(int M, int N, int K, const float *d_a_packed,
                                    const uint8_t *d_a_pat, const uint8_t *d_b_pat, void *stream)
 {
     return esmm::gemm_ab_packed_launch(M, N, K, d_a_packed, d_B, d_C, d_a_pat, d_b_pat, (cudaStream_t)stream);
+}
+
+extern "C" int esmm_gemm_ab(int M, int N, int K, const float *d_A, const float *d_B, float *d_C,
+                            const uint8_t *d_a_pat, const uint8_t *d_b_pat, int a_tile_m, void *stream)
+{
+    return esmm::gemm_ab_launch(M, N, K, d_A, d_B, d_C, d_a_pat, d_b_pat, a_tile_m, (cudaStream_t)stream);
 }

@@ -772,3 +772,36 @@ def test_gemm_block_mode_infinities(cuda, pkg, oracle_mod, tuning, mode):
     want = oracle_mod.gemm_joint(A, B, oracle_mod.preprocess_a(A), oracle_mod.preprocess_b(B))
     same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
     assert same.all() and np.isnan(want).any()
+
+
+@pytest.mark.parametrize("mode", [None, 1, 0])
+@pytest.mark.parametrize("tile_m", [8, 16, 64, 128])
+def test_gemm_rowmajor_pattern_heights(cuda, pkg, oracle_mod, tuning, tile_m, mode):
+    """Row-major A whose patterns have one row per 8, 16, 64 or 128 rows: a 32-row block multiplies the OR of its pattern rows.
+    Ragged M, N and K; both ways of working and the rule's choice."""
+    if mode is not None:
+        tuning("BLOCK_MODE", int(mode))
+    for M, N, K, pat in [(300, 164, 76, None), (256, 384, 1024, None), (130, 260, 8 * 37, None), (256, 256, 512, 0x0F)]:
+        A, B = workloads.tile_random(M, N, K, 0.4, 0.5, seed=M + K, gran_a=32, gran_b=32) if pat is None else \
+            workloads.uniform_pattern(M, N, K, pat, seed=pat)
+        d = Dev(cuda, pkg, A, B)
+        d.patterns()
+        ap = cuda.empty((-(-M // tile_m), d.nKB), dtype=cuda.uint8, device="cuda")
+        pkg.preprocess_a(d.A.data_ptr(), M, K, ap.data_ptr(), tile_m=tile_m)
+        c = d.C()
+        pkg.gemm_ab(M, N, K, d.A.data_ptr(), d.B.data_ptr(), c.data_ptr(), ap.data_ptr(), d.bp.data_ptr(), tile_m)
+        pkg.device_status()
+        assert np.array_equal(c.cpu().numpy(), oracle_mod.gemm_joint(A, B)), (M, N, K)
+
+
+@pytest.mark.parametrize("K", [27488, 27496, 65536, 66656])
+def test_gemm_rowmajor_deepest_k(cuda, pkg, oracle_mod, K):
+    """Row-major A up to the deepest K that is taken: past what the pipeline's row lists hold (27488), and past the 16 bits of a
+    list entry; one K block more is refused."""
+    A, B = workloads.tile_random(40, 64, K, 0.3, 0.4, seed=K, gran_a=32, gran_b=32)
+    d = Dev(cuda, pkg, A, B)
+    d.patterns()
+    assert np.array_equal(d.gemm_rowmajor(), oracle_mod.gemm_joint(A, B))
+    if K == 66656:
+        assert pkg.lib().esmm_gemm_ab(40, 64, K + 8, d.A.data_ptr(), d.B.data_ptr(), d.C().data_ptr(), d.ap.data_ptr(),
+                                      d.bp.data_ptr(), 32, None) == pkg.ERR_TOO_LARGE
