@@ -206,6 +206,7 @@ esmm_tf32_split_pattern_kernel(const float *__restrict__ A, int M, int K, const 
                                float *__restrict__ hi, float *__restrict__ lo, uint8_t *__restrict__ a_pat,
                                const ZeroJob zj)
 {
+    grid_launch_dependents();   // the product kernel may be placed as SMs become free; it waits for this grid's end itself
     const int a_blocks = (M + 31) >> 5;
     if ((int)blockIdx.y >= a_blocks) {
         if (blockIdx.x != 0) return;
@@ -226,6 +227,9 @@ esmm_tf32_split_pattern_kernel(const float *__restrict__ A, int M, int K, const 
     const bool in_cols = col < Kc;                                // Kc is a multiple of 8: a float4 is in or out
     int4 k = make_int4(col, col + 1, col + 2, col + 3);
     if (klist != nullptr && in_cols) k = __ldg(reinterpret_cast<const int4 *>(klist + col));
+    // four kept columns that are neighbours and start on 16 bytes (all of them for patterns of 4 or 8 live k in a row) are
+    // one load
+    const bool run4 = k.x >= 0 && (k.x & 3) == 0 && k.y == k.x + 1 && k.z == k.x + 2 && k.w == k.x + 3;
     float4 v[16];
 #pragma unroll
     for (int rr = 0; rr < 16; ++rr) {
@@ -233,8 +237,8 @@ esmm_tf32_split_pattern_kernel(const float *__restrict__ A, int M, int K, const 
         v[rr] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (in_cols && row < M) {
             const float *a = A + (size_t)row * K;
-            if (klist == nullptr) {
-                v[rr] = __ldg(reinterpret_cast<const float4 *>(a + col));
+            if (run4) {
+                v[rr] = __ldg(reinterpret_cast<const float4 *>(a + k.x));
             } else {
                 v[rr].x = k.x >= 0 ? __ldg(a + k.x) : 0.0f;
                 v[rr].y = k.y >= 0 ? __ldg(a + k.y) : 0.0f;
@@ -374,6 +378,7 @@ esmm_joint_sgemm_tf32x3_kernel(const __grid_constant__ Tf32Maps maps, const Tf32
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();   // (A's parts and patterns come from the kernel before this one)
     const uint32_t tmem = *tmem_slot;
     const int nGroups = (p.nKB + T_GROUP_KB - 1) / T_GROUP_KB;
     bool ok = true;
@@ -696,6 +701,7 @@ esmm_joint_sgemm_tf32x3_pair_kernel(const __grid_constant__ Tf32PairMaps maps, c
     __syncthreads();
     cluster_sync_all();                          // both CTAs' barriers exist before anything remote touches them
     tc_fence_after();
+    grid_dependency_wait();                      // (A's parts and patterns, and the zeroed tiles of C, come from the kernel before)
     const uint32_t tmem = *tmem_slot;
     const int nGroups = (p.nKB + T_GROUP_KB - 1) / T_GROUP_KB;
     bool ok = true;
@@ -1149,16 +1155,16 @@ int esmm_sgemm_joint_tf32x3(int M, const float *d_A, const esmm_tf32x3_b *b, flo
         maps.b_hi = m_b_hi;
         maps.b_lo = m_b_lo;
         if (nb == 128)
-            esmm_joint_sgemm_tf32x3_pair_kernel<128><<<2 * pairs, PairCfg<128>::THREADS, smem, stream>>>(maps, p);
+            ESMM_CUDA_TRY(launch_dependent(esmm_joint_sgemm_tf32x3_pair_kernel<128>, dim3(2 * pairs), dim3(PairCfg<128>::THREADS), smem, stream, maps, p));
         else
-            esmm_joint_sgemm_tf32x3_pair_kernel<256><<<2 * pairs, PairCfg<256>::THREADS, smem, stream>>>(maps, p);
+            ESMM_CUDA_TRY(launch_dependent(esmm_joint_sgemm_tf32x3_pair_kernel<256>, dim3(2 * pairs), dim3(PairCfg<256>::THREADS), smem, stream, maps, p));
     } else {
         Tf32Maps maps;
         maps.a_hi = m_a_hi;
         maps.a_lo = m_a_lo;
         maps.b_hi = m_b_hi;
         maps.b_lo = m_b_lo;
-        esmm_joint_sgemm_tf32x3_kernel<<<std::min(sms, p.num_tiles), T_THREADS, smem, stream>>>(maps, p);
+        ESMM_CUDA_TRY(launch_dependent(esmm_joint_sgemm_tf32x3_kernel, dim3(std::min(sms, p.num_tiles)), dim3(T_THREADS), smem, stream, maps, p));
     }
     ESMM_CUDA_TRY(cudaGetLastError());
     return ESMM_OK;
