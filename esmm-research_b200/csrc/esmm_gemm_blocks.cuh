@@ -51,6 +51,13 @@ constexpr int BM_TAIL = 6;                                  // of more than BM_W
 constexpr int RM_KL = 8;                                    // row-major A: lanes of a 4-byte copy instruction on the k (4: 9 % slower, 16: 12 %)
 constexpr int BM_SAMPLES = 8;                               // tiles looked at to choose the mode
 
+// bits of the k of K blocks kb .. kb + 3 that are < K
+__device__ __forceinline__ unsigned inside_k(int kb, int K)
+{
+    const int left = K - kb * BK;
+    return left >= 32 ? 0xFFFFFFFFu : left <= 0 ? 0u : (1u << left) - 1u;
+}
+
 // Pattern bytes of K blocks kb .. kb + 3 of one pattern row (null: no such row), zero past the end.  words: the row may be
 // read as 32-bit words.
 __device__ __forceinline__ unsigned pattern_word(const uint8_t *row, int kb, int nKB, bool words)
@@ -58,15 +65,9 @@ __device__ __forceinline__ unsigned pattern_word(const uint8_t *row, int kb, int
     if (row == nullptr || kb >= nKB) return 0u;
     if (words) return *reinterpret_cast<const unsigned *>(row + kb);
     unsigned v = 0u;
-    for (int j = 0; j < 4 && kb + j < nKB; ++j) v |= (unsigned)row[kb + j] << (8 * j);
-    return v;
-}
-
-// bits of the k of K blocks kb .. kb + 3 that are < K
-__device__ __forceinline__ unsigned inside_k(int kb, int K)
-{
-    const int left = K - kb * BK;
-    return left >= 32 ? 0xFFFFFFFFu : left <= 0 ? 0u : (1u << left) - 1u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v |= (unsigned)row[min(kb + j, nKB - 1)] << (8 * j);   // (four loads in flight)
+    return v & inside_k(kb, nKB * BK);
 }
 
 // The pattern rows of one 32-row (32-column) block: count rows from `first` on, whose OR is the block's pattern; none: no such block.
@@ -255,7 +256,10 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     const char *b_src = reinterpret_cast<const char *>(p.B + b_blk * 32);
     const char *xs = (wide_b ? b_src : a_src) + c4 * 16, *ys = (wide_b ? a_src : b_src) + c4 * 16;
     const int b_chunks = (p.N - b_blk * 32) >> 2;
-    const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);
+    const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);   // (2330 x 932 x 5020 pruned MLP: 186 us with a slow path there, 138 with predicates)
+    const int x_chunks = wide_b ? b_chunks : 16, y_chunks = wide_b ? 8 : b_chunks;
+    const bool x_ok0 = c4 < x_chunks, x_ok1 = c4 + 4 < x_chunks, x_ok2 = c4 + 8 < x_chunks, x_ok3 = c4 + 12 < x_chunks;
+    const bool y_ok0 = c4 < y_chunks, y_ok1 = c4 + 4 < y_chunks;
 
     Acc acc;
     acc_clear(acc);
@@ -383,7 +387,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
                 }
             }
         } else {
-            if (!edge && d0 == BM_ROWS && (!TWO || d1 == BM_ROWS)) {
+            if (d0 == BM_ROWS && (!TWO || d1 == BM_ROWS)) {
                 unsigned k0[BM_ROWS / 8], k1[BM_ROWS / 8];
                 same_next = TWO;
 #pragma unroll
@@ -396,32 +400,31 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
                 for (int h = 0; h < BM_ROWS / 8; ++h) {
                     const char *gx = xs + (size_t)k0[h] * x_stride, *gy = ys + (size_t)k0[h] * y_stride;
                     const uint32_t e0 = dst0 + to + h * 1024, e1 = dst1 + to + h * 1024;
-                    cp_async_16(e0, gx, 16);
-                    cp_async_16(e1, gx + 64, 16);
-                    cp_async_16(e0 + 2 * BM_PART, gy, 16);
-                    cp_async_16(e1 + 2 * BM_PART, gy + 64, 16);
+                    if (x_ok0) cp_async_16(e0, gx, 16);
+                    if (x_ok1) cp_async_16(e1, gx + 64, 16);
+                    if (y_ok0) cp_async_16(e0 + 2 * BM_PART, gy, 16);
+                    if (y_ok1) cp_async_16(e1 + 2 * BM_PART, gy + 64, 16);
                     if (TWO) {
                         const char *gx1 = xs + (size_t)k1[h] * x_stride;
-                        cp_async_16(e0 + BM_PART, gx1 + 128, 16);
-                        cp_async_16(e1 + BM_PART, gx1 + 192, 16);
+                        if (x_ok2) cp_async_16(e0 + BM_PART, gx1 + 128, 16);
+                        if (x_ok3) cp_async_16(e1 + BM_PART, gx1 + 192, 16);
                         if (!same_next) {
                             const char *gy1 = ys + (size_t)k1[h] * y_stride;
-                            cp_async_16(e0 + 3 * BM_PART, gy1, 16);
-                            cp_async_16(e1 + 3 * BM_PART, gy1 + 64, 16);
+                            if (y_ok0) cp_async_16(e0 + 3 * BM_PART, gy1, 16);
+                            if (y_ok1) cp_async_16(e1 + 3 * BM_PART, gy1 + 64, 16);
                         }
                     }
                 }
             } else if (max(d0, d1) > 0) {
                 // Past the end of a list X = -0 and Y = +0: a multiply-add with them changes no accumulator, not even a zero's sign.
-                const int x_lim = wide_b ? b_chunks : 16, y_lim = wide_b ? 8 : b_chunks;
 #pragma unroll 1
                 for (int i = 0; i < 2 * (TWO ? 2 : 1) * (BM_ROWS / 8); ++i) {      // (row group, half of the row, block)
                     const int j = i & 1, row = ((i >> 1) & (BM_ROWS / 8 - 1)) * 8 + r8, blk = TWO ? i >> 2 : 0, ch = c4 + 4 * j;
                     const uint32_t e = (j ? dst1 : dst0) + to + (row - r8) * 128 + blk * BM_PART;
                     if (row < (blk ? d1 : d0)) {
                         const size_t k = blk ? l1.list[(l1.taken + row) & (BM_LIST - 1)] : l0.list[(l0.taken + row) & (BM_LIST - 1)];
-                        if (blk * 8 + ch < x_lim) cp_async_16(e, xs + k * x_stride + blk * 128 + j * 64, 16);
-                        if (ch < y_lim) cp_async_16(e + 2 * BM_PART, ys + k * y_stride + j * 64, 16);
+                        if (blk * 8 + ch < x_chunks) cp_async_16(e, xs + k * x_stride + blk * 128 + j * 64, 16);
+                        if (ch < y_chunks) cp_async_16(e + 2 * BM_PART, ys + k * y_stride + j * 64, 16);
                     } else {
                         fill_16(e, -0.0f);
                         fill_16(e + 2 * BM_PART, 0.0f);
@@ -493,7 +496,11 @@ __device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp
     const int tiles_m = wide_b ? y_blocks : pairs_x, tiles_n = wide_b ? pairs_x : y_blocks;
     const long items = (long)tiles_m * tiles_n;
     const int mine = blockIdx.x < items ? (int)((items - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
-    const int tail = mine <= BM_WARPS ? mine : BM_TAIL, whole = mine - tail;   // the last `tail` items go as two single blocks each
+    // The last `tail` items go as two single blocks each.  With at most 12 items it is what is over when every scheduler (SM
+    // sub-partition) has as many pairs as every other: of 8 items each has two pairs, where 16 single blocks on 12 warps would be
+    // four for some (3562 x 724 x 1336, 32-granular 0.67 / 0.35: 71.5 us with single blocks only, 59.5 now; 512 x 4096 x 4096 pruned
+    // MLP: 115.5 and 106).
+    const int tail = mine <= 4 ? mine : mine <= BM_WARPS ? (mine & 3) % 3 : BM_TAIL, whole = mine - tail;
 
     for (int v = warp; v < whole + 2 * tail;) {
         const int item = blockIdx.x + (v < whole ? v : whole + ((v - whole) >> 1)) * gridDim.x;

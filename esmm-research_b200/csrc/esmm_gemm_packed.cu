@@ -147,7 +147,7 @@ struct PackedSmem {
     uint32_t stage_off, krow_off, krow_stride, rmask_off, rmask_stride, wlist_off, bar_off, misc_off, item_off, total;
 };
 
-__host__ __device__ inline PackedSmem packed_smem_layout(int stages, int cap)
+__host__ __device__ inline PackedSmem packed_smem_layout(int stages, int cap, bool blocks)
 {
     PackedSmem L;
     uint32_t o = 0;
@@ -166,9 +166,13 @@ __host__ __device__ inline PackedSmem packed_smem_layout(int stages, int cap)
     o += (2 * P_MAX_STAGES + 4) * 8;
     L.misc_off = o;   // nrows[2], abort, n_producers, runinfo[2]
     o += 32;
-    // block mode lays its warps' rings over all of this; its item counter is past them, or the last word of misc
-    L.item_off = L.misc_off >= BM_SMEM ? L.misc_off + 24 : BM_SMEM;
-    if (o < BM_SMEM + 16) o = BM_SMEM + 16;
+    // block mode lays its warps' rings over all of this; its item counter is past them, or the seventh word of misc
+    if (L.misc_off >= (uint32_t)BM_SMEM) {
+        L.item_off = L.misc_off + 24;
+    } else {
+        L.item_off = o > (uint32_t)BM_SMEM ? o : (uint32_t)BM_SMEM;
+        if (blocks) o = L.item_off + 16;
+    }
     L.total = o;
     return L;
 }
@@ -446,13 +450,18 @@ struct TileScan {
     int live_total, live_small;
 };
 
+// K block kb's byte of the pattern of 32-row block mb, 0 past the last block
 template <bool RM>
 __device__ __forceinline__ unsigned a_byte(const PackedParams &p, int mb, int kb)
 {
-    const PatternRows pr = a_pattern<RM>(p, mb);
     unsigned v = 0u;
-    if (pr.first)
-        for (int j = 0; j < pr.count; ++j) v |= pr.first[(size_t)j * p.nKB + kb];
+    if constexpr (RM) {
+        const PatternRows pr = a_pattern<RM>(p, mb);
+        if (pr.first)
+            for (int j = 0; j < pr.count; ++j) v |= pr.first[(size_t)j * p.nKB + kb];
+    } else {
+        if (mb < p.a_rows) v = p.a_pat[(size_t)mb * p.nKB + kb];
+    }
     return v;
 }
 
@@ -538,7 +547,9 @@ __device__ __noinline__ int listed_warp_rows(const uint8_t *rmask, int n, int la
 // (Before, a kernel of its own fetched boxes of 128 rows x 8 k, multiplied with scalar FMAs and could not leave out dead k of A.
 // Kernel and pattern pass, before -> now: 2048^3 64-granular 0.5 / 0.5 237 -> 159 us, 32-granular 0.2 / 0.2 111 -> 71; 4096^3 dense
 // 2813 -> 2622, half 1855 -> 1322, quarter 1469 -> 687, eighth 855 -> 474; 16 x 11008 x 4096 MLP 146 -> 65.)
-template <int WMB, int NPW, bool RM>
+// BLOCKS: with block mode; without it for launches too short to look whether it would pay (the code is then that of the pipeline
+// alone: up to 1.3 us of a 15 us call).
+template <int WMB, int NPW, bool RM, bool BLOCKS>
 __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const PackedParams &p)
 {
     static_assert(NPW == 3 || NPW == 7, "consumers, producers and the mask warp fill whole warp groups");
@@ -550,7 +561,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
     constexpr int A_ROW = TM_ROWS * 4;                 // bytes of one k of the A tile in shared memory
     constexpr uint32_t STAGE_ROW_BYTES = A_ROW + ROW_BYTES;
     extern __shared__ __align__(1024) char smem[];
-    const PackedSmem L = packed_smem_layout(p.stages, p.cap);
+    const PackedSmem L = packed_smem_layout(p.stages, p.cap, BLOCKS);
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
@@ -578,7 +589,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             mbar_init(lempty0 + 8 * b, P_CONSUMER_WARPS + P_TMA_WARPS);
         }
         *abort_flag = 0;
-        *next_item = BM_WARPS;
+        if (BLOCKS) *next_item = BM_WARPS;   // (without block mode the launch has no memory there)
         fence_barrier_init();
         fence_proxy_async();
     }
@@ -593,7 +604,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
         tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
         scan = tile_scan_any<RB, RM>(p, tm, tn, lane);
     }
-    if (p.block_mode != 0) {
+    if (BLOCKS && p.block_mode != 0) {
         // two vectors per sample, where the consumers' lists will be
         int4 *stats = reinterpret_cast<int4 *>(smem + L.wlist_off);
         static_assert(2 * BM_SAMPLES * sizeof(int4) <= P_CONSUMER_WARPS * 2 * 96 && BM_SAMPLES <= P_CONSUMER_WARPS, "samples");
@@ -1063,18 +1074,18 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
     if (!ok && lane == 0) atomicExch(p.status, (int)ESMM_ERR_TIMEOUT);
 }
 
-template <int WMB, int NPW>
+template <int WMB, int NPW, bool BLOCKS>
 __global__ void __launch_bounds__((P_CONSUMER_WARPS + NPW + 1) * 32, 1)
 esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const PackedParams p)
 {
-    tiled_sgemm<WMB, NPW, false>(maps, p);
+    tiled_sgemm<WMB, NPW, false, BLOCKS>(maps, p);
 }
 
-template <int WMB>
+template <int WMB, bool BLOCKS>
 __global__ void __launch_bounds__((P_CONSUMER_WARPS + 4) * 32, 1)
 esmm_joint_sgemm_kernel(const __grid_constant__ PackedMaps maps, const PackedParams p)
 {
-    tiled_sgemm<WMB, 3, true>(maps, p);
+    tiled_sgemm<WMB, 3, true, BLOCKS>(maps, p);
 }
 
 #ifdef ESMM_TRACE
@@ -1134,14 +1145,21 @@ static int prepare_device(int dev, int *sms)
     std::lock_guard<std::mutex> lock(mu);
     if (!sm_count[dev]) {
         int n = 0, smem = 0;
+        auto allow_smem = [](auto kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
         ESMM_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
         ESMM_CUDA_TRY(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_packed_kernel<1, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_packed_kernel<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_packed_kernel<1, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_packed_kernel<2, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<1, 3, false>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<1, 3, true>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<1, 7, false>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<1, 7, true>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<2, 3, false>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<2, 3, true>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<2, 7, false>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_packed_kernel<2, 7, true>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_kernel<1, false>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_kernel<1, true>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_kernel<2, false>, smem));
+        ESMM_CUDA_TRY(allow_smem(esmm_joint_sgemm_kernel<2, true>, smem));
         sm_count[dev] = n;
     }
     *sms = sm_count[dev];
@@ -1212,7 +1230,7 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     if (p.kp > 65535 && !row_major) return ESMM_ERR_TOO_LARGE;  // row list entries are 16-bit k indices
     p.cap = ((p.kp + 31) & ~31) + 32;
     // (row-major A with more k than the pipeline's row lists have room for: block mode, whose lists are rings)
-    const bool lists_fit = packed_smem_layout(2, p.cap).total <= SMEM_LIMIT;
+    const bool lists_fit = packed_smem_layout(2, p.cap, false).total <= SMEM_LIMIT;
     if (row_major && !lists_fit) p.cap = 64;
     p.A = d_A;
     p.a_div = a_tile_m >= 32 ? a_tile_m / 32 : 1;
@@ -1281,11 +1299,22 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     if (!row_major && dev >= 0 && dev < 64) g_last_tiled_warps[dev].store(wide ? 16 : 12, std::memory_order_relaxed);
     const int threads = (P_CONSUMER_WARPS + (wide ? 7 : 3) + 1) * 32;
 
+    int grid = tuning_get("GRID", sms);
+    const long pairs = std::max((long)ceil_div(p.a_rows, 2) * p.b_rows, (long)p.a_rows * ceil_div(p.b_rows, 2));
+    p.few_blocks = pairs <= grid;
+    // The samples cost a launch a microsecond or two, which short ones do not win back: the pipeline, without looking, where an SM
+    // has fewer than 768 k of tiles to go through (58 x 7368 x 648: 15.2 us, 17.4 with the look; 2502 x 1112 x 456, 912 k of tiles
+    // per SM: 37.1 in the pipeline, 31.5 in block mode).
+    const long tile_rounds = (p.num_tiles + sms - 1) / sms;
+    p.block_mode = tuning_get("BLOCK_MODE", tile_rounds * p.kp < 768 ? 0 : -1);
+    if (!lists_fit) p.block_mode = 1;
+    const bool blocks = p.block_mode != 0;
+
     int stages = tuning_get("STAGES", P_MAX_STAGES);
     if (stages > P_MAX_STAGES) stages = P_MAX_STAGES;
     if (stages < 2) stages = 2;
-    while (stages > 2 && packed_smem_layout(stages, p.cap).total > SMEM_LIMIT) --stages;
-    const PackedSmem L = packed_smem_layout(stages, p.cap);
+    while (stages > 2 && packed_smem_layout(stages, p.cap, blocks).total > SMEM_LIMIT) --stages;
+    const PackedSmem L = packed_smem_layout(stages, p.cap, blocks);
     if (L.total > SMEM_LIMIT) return ESMM_ERR_TOO_LARGE;
     p.stages = stages;
 
@@ -1325,24 +1354,25 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     if (st) return st;
 
     // (in block mode a CTA has work as soon as there are pairs of blocks for it)
-    int grid = tuning_get("GRID", sms);
-    const long pairs = std::max((long)ceil_div(p.a_rows, 2) * p.b_rows, (long)p.a_rows * ceil_div(p.b_rows, 2));
-    // With no more pairs of blocks than SMs the pipeline's tiles would occupy an eighth of them or a quarter: block mode whatever
-    // the patterns (512^3 at half density: 20.8 us in the pipeline, 18.7 in block mode; with four times as many pairs, 1024^3,
-    // 33.3 and 37.4).
-    p.few_blocks = pairs <= grid;
-    p.block_mode = tuning_get("BLOCK_MODE", p.few_blocks ? 1 : -1);
-    if (!lists_fit) p.block_mode = 1;
-    if (grid > std::max((long)p.num_tiles, pairs)) grid = (int)std::max((long)p.num_tiles, pairs);
+    const long most = p.block_mode ? std::max((long)p.num_tiles, pairs) : (long)p.num_tiles;
+    if (grid > most) grid = (int)most;
     if (grid < 1) grid = 1;
     auto launch = [&](auto kernel, int threads) -> int {
         ESMM_CUDA_TRY(launch_dependent(kernel, dim3(grid), dim3(threads), L.total, stream, maps, p));
         return ESMM_OK;
     };
     int lst;
-    if (row_major) lst = tile_rows == 64 ? launch(esmm_joint_sgemm_kernel<1>, threads) : launch(esmm_joint_sgemm_kernel<2>, threads);
-    else if (tile_rows == 64) lst = wide ? launch(esmm_joint_sgemm_packed_kernel<1, 7>, threads) : launch(esmm_joint_sgemm_packed_kernel<1, 3>, threads);
-    else lst = wide ? launch(esmm_joint_sgemm_packed_kernel<2, 7>, threads) : launch(esmm_joint_sgemm_packed_kernel<2, 3>, threads);
+    auto pick = [&](auto with, auto without) { return blocks ? launch(with, threads) : launch(without, threads); };
+    if (row_major) {
+        lst = tile_rows == 64 ? pick(esmm_joint_sgemm_kernel<1, true>, esmm_joint_sgemm_kernel<1, false>)
+                              : pick(esmm_joint_sgemm_kernel<2, true>, esmm_joint_sgemm_kernel<2, false>);
+    } else if (tile_rows == 64) {
+        lst = wide ? pick(esmm_joint_sgemm_packed_kernel<1, 7, true>, esmm_joint_sgemm_packed_kernel<1, 7, false>)
+                   : pick(esmm_joint_sgemm_packed_kernel<1, 3, true>, esmm_joint_sgemm_packed_kernel<1, 3, false>);
+    } else {
+        lst = wide ? pick(esmm_joint_sgemm_packed_kernel<2, 7, true>, esmm_joint_sgemm_packed_kernel<2, 7, false>)
+                   : pick(esmm_joint_sgemm_packed_kernel<2, 3, true>, esmm_joint_sgemm_packed_kernel<2, 3, false>);
+    }
     if (lst != ESMM_OK) return lst;
     ESMM_CUDA_TRY(cudaGetLastError());
     return ESMM_OK;
