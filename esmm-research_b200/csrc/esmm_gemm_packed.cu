@@ -121,6 +121,7 @@ struct PackedParams {
     int *form_hint;    // host-mapped word, or null: CTA 0 notes whether its first tile wanted 7 producers
     int block_mode;    // 1, 0: always, never; -1: as the sampled tiles say
     int pat_words;     // pattern rows may be read as 32-bit words
+    unsigned last_bits;  // of the last K block's byte: the bits whose k is < K, in all four bytes of the word
     int few_blocks;    // no more pairs of blocks than CTAs
     // row-major A: 32-row block mb uses A pattern rows (mb / a_div) * a_mul + [0, a_mul) of a_pat_rows
     int a_div, a_mul, a_pat_rows;
@@ -319,6 +320,8 @@ __device__ __forceinline__ int build_list(uint16_t *list, unsigned m, int lane, 
 }
 
 // ---- mask warp helpers ---------------------------------------------------------------------------
+// (Row-major A: patterns come from the caller, who may have marked k past K live, in a dense product by 0xFF throughout.  Such k
+// are dropped here: there is no element of A to multiply, and the clamped address holds A[row][K - 1].)
 // Pattern bytes of KPL (16 or 4) consecutive K blocks kb0 .. kb0 + KPL - 1, all inside the matrix, for the
 // tile's RB 32-row blocks and four 32-column blocks: one 16-byte or 4-byte load per pattern row.  aw[j] /
 // bw[j] get the four bytes of K block kb0 + j (byte i = block i).  Long K takes 16 per lane; shorter K
@@ -368,6 +371,8 @@ __device__ __forceinline__ void load_patterns(const PackedParams &p, int tm, int
         aw[j] = a;
         bw[j] = b;
     }
+    // (nKB is a multiple of KPL here, so the last K block is some lane's last)
+    if (RM && kb0 + KPL == p.nKB) aw[KPL - 1] &= p.last_bits;
 }
 
 // k offsets of one K block that are live for the tile as a whole: (OR of the A bytes) & (OR of the B bytes)
@@ -450,7 +455,7 @@ struct TileScan {
     int live_total, live_small;
 };
 
-// K block kb's byte of the pattern of 32-row block mb, 0 past the last block
+// K block kb's byte of the pattern of 32-row block mb, 0 past the last block; with row-major A, without the bits of k past K
 template <bool RM>
 __device__ __forceinline__ unsigned a_byte(const PackedParams &p, int mb, int kb)
 {
@@ -459,6 +464,7 @@ __device__ __forceinline__ unsigned a_byte(const PackedParams &p, int mb, int kb
         const PatternRows pr = a_pattern<RM>(p, mb);
         if (pr.first)
             for (int j = 0; j < pr.count; ++j) v |= pr.first[(size_t)j * p.nKB + kb];
+        if (kb == p.nKB - 1) v &= p.last_bits & 0xFFu;
     } else {
         if (mb < p.a_rows) v = p.a_pat[(size_t)mb * p.nKB + kb];
     }
@@ -825,7 +831,8 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                     if (box_log >= 0) tma_load_2d(s0 + STAGE_HALF_BYTES + lane * ROW_BYTES, &maps.b_box[box_log], b_col0, k, full);
                     // A: 4-byte copies, eight lanes on the k and four on the rows, so that neighbouring k of a row come as one
                     // sector; row groups shared out among the producers.  Rows past the end of A, k past its width (in K
-                    // blocks listed whole) and past the end of the list: any element, never multiplied or never stored.
+                    // blocks listed whole; no mask has their bit) and past the end of the list: any element, never multiplied
+                    // or never stored.
                     // These copies are what bounds the form: 4096^3 dense 2622 us against 2144 with packed A.  (Four lanes
                     // on the k, eight on the rows, fewer bank conflicts but half of each sector: 2753; seven producer
                     // warps: 2793.)
@@ -1276,6 +1283,7 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
         (forced_vec == 16 && p.nKB % 16 == 0 && (pat_bits & 15) == 0))
         p.vec_patterns = forced_vec;
     p.pat_words = p.nKB % 4 == 0 && (pat_bits & 3) == 0;
+    p.last_bits = (K & 7) ? ((1u << (K & 7)) - 1u) * 0x01010101u : 0xFFFFFFFFu;
     p.a_pat = d_a_pat;
     p.b_pat = d_b_pat;
     p.a_packed = d_a_packed;

@@ -805,3 +805,48 @@ def test_gemm_rowmajor_deepest_k(cuda, pkg, oracle_mod, K):
     if K == 66656:
         assert pkg.lib().esmm_gemm_ab(40, 64, K + 8, d.A.data_ptr(), d.B.data_ptr(), d.C().data_ptr(), d.ap.data_ptr(),
                                       d.bp.data_ptr(), 32, None) == pkg.ERR_TOO_LARGE
+
+
+@pytest.mark.parametrize("mode", [1, 0, -1])
+@pytest.mark.parametrize("tile_m", [8, 32, 64])
+def test_gemm_rowmajor_pattern_bits_past_k(cuda, pkg, oracle_mod, tuning, tile_m, mode):
+    """Row-major A with K % 8 == 4 and patterns that mark k past K live (0xFF throughout): those k are not multiplied.  Infinities in
+    A's last column, which a product with anything past K would turn into NaN, and sums that are -0, which adding +0 would turn
+    into +0.  Pattern rows read by bytes (K = 76, 1028), words (1020) and 16 bytes (4092); both ways of working and the rule's choice."""
+    tuning("BLOCK_MODE", int(mode))
+    for M, N, K in [(40, 36, 76), (130, 132, 1020), (64, 128, 1028), (100, 64, 4092)]:
+        rng = np.random.default_rng(K)
+        A = rng.standard_normal((M, K), dtype=np.float32)
+        B = rng.standard_normal((K, N), dtype=np.float32)
+        A[3, K - 1], A[M - 1, K - 1] = np.inf, -np.inf
+        A[5], B[:, 7] = np.float32(-1e-30), np.float32(1e-30)      # row 5, column 7: products that round to -0
+        ap = np.full((-(-M // tile_m), -(-K // 8)), 0xFF, np.uint8)
+        bp = np.full((-(-N // 32), -(-K // 8)), 0xFF, np.uint8)
+        dA, dB, dap, dbp = (cuda.from_numpy(x).cuda() for x in (A, B, ap, bp))
+        c = cuda.full((M, N), float("nan"), device="cuda")
+        pkg.gemm_ab(M, N, K, dA.data_ptr(), dB.data_ptr(), c.data_ptr(), dap.data_ptr(), dbp.data_ptr(), tile_m)
+        pkg.device_status()
+        want = oracle_mod.gemm_joint(A, B, np.full((-(-M // 32), -(-K // 8)), 0xFF, np.uint8), bp)
+        got = c.cpu().numpy()
+        assert not np.isnan(want).any() and np.isinf(want).any() and np.signbit(want[5, 7]) and want[5, 7] == 0
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (M, N, K, mode)
+
+
+def test_run_kernel_prefix_pattern_past_k(cuda, pkg, oracle_mod, capfd):
+    """Id 14 fills A's and B's pattern arrays with constants, K's ragged end included: with K % 8 == 4 and infinities in the last
+    column of A, the product has the oracle's bits."""
+    M, N, K = 96, 132, 516
+    rng = np.random.default_rng(5)
+    A = rng.standard_normal((M, K), dtype=np.float32)
+    B = rng.standard_normal((K, N), dtype=np.float32)
+    A[::7, K - 1] = np.inf
+    dA, dB = cuda.from_numpy(A).cuda(), cuda.from_numpy(B).cuda()
+    dC = cuda.zeros((M, N), device="cuda")
+    passed, avg = C.c_int(0), C.c_float(0)
+    for pat, byte in ((b"11111111", 0xFF), (b"11101110", 0x3F)):
+        st = pkg.lib().esmm_run_kernel_pattern(14, M, N, K, dA.data_ptr(), dB.data_ptr(), dC.data_ptr(), None, None, 1, 0, 0,
+                                               None, pat, C.byref(passed), C.byref(avg))
+        assert st == 0 and passed.value == 1
+        want = oracle_mod.gemm_joint(A, B, np.full((M // 32, 65), byte, np.uint8), np.full((5, 65), 0xFF, np.uint8))
+        assert np.array_equal(dC.cpu().numpy().view(np.uint32), want.view(np.uint32)), pat
+    capfd.readouterr()
