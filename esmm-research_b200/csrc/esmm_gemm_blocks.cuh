@@ -37,16 +37,6 @@
 
 namespace esmm {
 
-constexpr int BM_WARPS = 12;                                // warps of the CTA that take part
-constexpr int BM_ROWS = 16;                                 // k per stage
-constexpr int BM_STEP = 8;                                  // k multiplied as one run of straight-line code
-constexpr int BM_PART = BM_ROWS * 128;                      // a stage's rows of one operand of one block
-constexpr int BM_SLOT_BYTES = 4 * BM_PART;                  // X of block 0, X of block 1, Y of block 0, Y of block 1
-constexpr int BM_SLOTS = 2;
-constexpr int BM_LIST = 512;                                // entries of a block's list (a ring)
-constexpr int BM_LIST_BYTES = BM_LIST * 2;
-constexpr int BM_WARP_BYTES = BM_SLOTS * BM_SLOT_BYTES + 2 * BM_LIST_BYTES;
-constexpr int BM_SMEM = BM_WARPS * BM_WARP_BYTES;
 constexpr int BM_TAIL = 6;                                  // of more than BM_WARPS items: 0 .. 12 measured, 4 - 6 best
 constexpr int RM_KL = 8;                                    // row-major A: lanes of a 4-byte copy instruction on the k (4: 9 % slower, 16: 12 %)
 constexpr int BM_SAMPLES = 8;                               // tiles looked at to choose the mode

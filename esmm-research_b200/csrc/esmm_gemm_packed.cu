@@ -55,11 +55,6 @@
 
 namespace esmm {
 
-constexpr int ROW_BYTES = TILE_N * 4;            // 512: one k of an operand tile
-constexpr int ROWS_PER_STAGE = 32;
-constexpr int STAGE_HALF_BYTES = ROWS_PER_STAGE * ROW_BYTES;   // 16384: A rows, then B rows
-constexpr int PSTAGE_BYTES = 2 * STAGE_HALF_BYTES;             // 32768
-constexpr int P_CONSUMER_WARPS = 8;
 // Issuing a copy costs the issuing warp about 50 cycles per copy, whatever the mechanism (2-D tensor copy of one row
 // or of an 8-row box, untiled bulk copy, or a warp-wide 16-byte cp.async per row: 3300 cycles for the 64 copies of a
 // row-by-row stage from one warp, 1270 from three, 970 from four - measured), and different warps issue in parallel.
@@ -74,7 +69,6 @@ constexpr int P_CONSUMER_WARPS = 8;
 //     dense and uniform patterns 0.5 % slower.  A launch takes this form when the launch before it on the device
 //     noted such tiles (see gemm_ab_packed_launch_form); esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins one.
 constexpr int P_TMA_WARP = P_CONSUMER_WARPS;                   // first producer warp
-constexpr int P_MAX_STAGES = 6;
 // Block mode (esmm_gemm_blocks.cuh) where at most this many sixteenths of what the tiled pipeline would hold in shared memory are
 // multiplied.  Measured at 4096^3, whole calls, pipeline / block mode: share 0.33 (32-granular, 0.5 / 0.5 of A's and B's
 // k live) 921 / 718 us, 0.44 (64-granular, 0.5 / 0.5) 730 / 695, 0.53 (32-granular, 1 / 0.5) 1414 / 1344, 0.64 (32-granular,
@@ -143,40 +137,6 @@ struct PackedMaps {
 
 constexpr int RUN_TILE = 0x100;
 constexpr int RUNS_LIKELY = 0x200;   // a listed tile whose stages may be whole runs of K blocks: the producers look for them
-
-struct PackedSmem {
-    uint32_t stage_off, krow_off, krow_stride, rmask_off, rmask_stride, wlist_off, bar_off, misc_off, item_off, total;
-};
-
-__host__ __device__ inline PackedSmem packed_smem_layout(int stages, int cap, bool blocks)
-{
-    PackedSmem L;
-    uint32_t o = 0;
-    L.stage_off = o;
-    o += (uint32_t)stages * PSTAGE_BYTES;
-    L.krow_off = o;   // two buffers: k index of every listed row
-    L.krow_stride = (uint32_t)cap * 2;
-    o += 2 * L.krow_stride;
-    L.rmask_off = o;  // two buffers: per row, bits 0-3 live row blocks, bits 4-7 live column blocks
-    L.rmask_stride = (uint32_t)cap;
-    o += 2 * L.rmask_stride;
-    o = (o + 15u) & ~15u;
-    L.wlist_off = o;  // per consumer warp: offsets of the live rows of its top and its bottom block
-    o += P_CONSUMER_WARPS * 2 * 96;  // two lists of WLIST_BYTES per warp
-    L.bar_off = o;    // full[P_MAX_STAGES], empty[P_MAX_STAGES], list_full[2], list_empty[2]
-    o += (2 * P_MAX_STAGES + 4) * 8;
-    L.misc_off = o;   // nrows[2], abort, n_producers, runinfo[2]
-    o += 32;
-    // block mode lays its warps' rings over all of this; its item counter is past them, or the seventh word of misc
-    if (L.misc_off >= (uint32_t)BM_SMEM) {
-        L.item_off = L.misc_off + 24;
-    } else {
-        L.item_off = o > (uint32_t)BM_SMEM ? o : (uint32_t)BM_SMEM;
-        if (blocks) o = L.item_off + 16;
-    }
-    L.total = o;
-    return L;
-}
 
 // A stage whose 32 rows are all live for both row blocks: 16 rows of straight-line code per
 // loop trip (measured: 4 rows 1 % slower than 8, 16 rows 1.6 % faster, 32 no better than 16),
@@ -583,7 +543,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
     // 4 or 8 consecutive live k (kk0 .. kk0 + c - 1), live for all of the tile's row and column blocks.  Such
     // a tile needs no row list: stage s is the 3-D box of K blocks 32 s / c .. and every stage is all-live.
     volatile int *runinfo = nrows + 4;
-    int *next_item = reinterpret_cast<int *>(smem + L.item_off);   // block mode's item counter
+    int *next_item = const_cast<int *>(nrows) + 6;   // block mode's item counter
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
@@ -595,7 +555,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             mbar_init(lempty0 + 8 * b, P_CONSUMER_WARPS + P_TMA_WARPS);
         }
         *abort_flag = 0;
-        if (BLOCKS) *next_item = BM_WARPS;   // (without block mode the launch has no memory there)
+        *next_item = BM_WARPS;
         fence_barrier_init();
         fence_proxy_async();
     }

@@ -5,13 +5,11 @@
 #include <cstdlib>
 
 #include "esmm_common.cuh"
+#include "esmm_tiled_layout.h"
 
 namespace esmm {
 
-constexpr int TILE_M = 128;
-constexpr int TILE_N = 128;
 constexpr int GROUP_M = 8;         // tile rows per raster group
-constexpr int SMEM_LIMIT = 232448; // 227 KB per CTA on sm_100
 
 #ifdef __CUDACC__
 // Tiles are walked in groups of `group_m` tile rows (GROUP_M unless the launch says otherwise), column by column

@@ -1,0 +1,70 @@
+// Sizes and shared-memory layout of the tiled kernel (esmm_gemm_packed.cu) and of its block mode (esmm_gemm_blocks.cuh).
+// Plain C++, so that the layout can be checked without a GPU.
+#pragma once
+
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define ESMM_HOST_DEVICE __host__ __device__
+#else
+#define ESMM_HOST_DEVICE
+#endif
+
+namespace esmm {
+
+constexpr int TILE_M = 128;
+constexpr int TILE_N = 128;
+constexpr int SMEM_LIMIT = 232448; // 227 KB per CTA on sm_100
+
+// ---- the pipeline ----
+constexpr int ROW_BYTES = TILE_N * 4;            // 512: one k of an operand tile
+constexpr int ROWS_PER_STAGE = 32;
+constexpr int STAGE_HALF_BYTES = ROWS_PER_STAGE * ROW_BYTES;   // 16384: A rows, then B rows
+constexpr int PSTAGE_BYTES = 2 * STAGE_HALF_BYTES;             // 32768
+constexpr int P_CONSUMER_WARPS = 8;
+constexpr int P_MAX_STAGES = 6;
+
+// ---- block mode ----
+constexpr int BM_WARPS = 12;                                // warps of the CTA that take part
+constexpr int BM_ROWS = 16;                                 // k per stage
+constexpr int BM_STEP = 8;                                  // k multiplied as one run of straight-line code
+constexpr int BM_PART = BM_ROWS * 128;                      // a stage's rows of one operand of one block
+constexpr int BM_SLOT_BYTES = 4 * BM_PART;                  // X of block 0, X of block 1, Y of block 0, Y of block 1
+constexpr int BM_SLOTS = 2;
+constexpr int BM_LIST = 512;                                // entries of a block's list (a ring)
+constexpr int BM_LIST_BYTES = BM_LIST * 2;
+constexpr int BM_WARP_BYTES = BM_SLOTS * BM_SLOT_BYTES + 2 * BM_LIST_BYTES;
+constexpr int BM_SMEM = BM_WARPS * BM_WARP_BYTES;           // the warps' rings and lists, from the start of shared memory
+
+struct PackedSmem {
+    uint32_t stage_off, krow_off, krow_stride, rmask_off, rmask_stride, wlist_off, bar_off, misc_off, total;
+};
+
+// blocks: the kernel has block mode.
+ESMM_HOST_DEVICE inline PackedSmem packed_smem_layout(int stages, int cap, bool blocks)
+{
+    PackedSmem L;
+    uint32_t o = 0;
+    L.stage_off = o;
+    o += (uint32_t)stages * PSTAGE_BYTES;
+    L.krow_off = o;   // two buffers: k index of every listed row
+    L.krow_stride = (uint32_t)cap * 2;
+    o += 2 * L.krow_stride;
+    L.rmask_off = o;  // two buffers: per row, bits 0-3 live row blocks, bits 4-7 live column blocks
+    L.rmask_stride = (uint32_t)cap;
+    o += 2 * L.rmask_stride;
+    o = (o + 15u) & ~15u;
+    L.wlist_off = o;  // per consumer warp: offsets of the live rows of its top and its bottom block
+    o += P_CONSUMER_WARPS * 2 * 96;  // two lists of WLIST_BYTES per warp
+    // Block mode lays its warps' rings over what is above, and over nothing below: the barriers' memory holds live mbarriers
+    // (which have to be invalidated before their memory may serve another use), and its item counter is in misc.
+    if (blocks && o < (uint32_t)BM_SMEM) o = BM_SMEM;
+    L.bar_off = o;    // full[P_MAX_STAGES], empty[P_MAX_STAGES], list_full[2], list_empty[2]
+    o += (2 * P_MAX_STAGES + 4) * 8;
+    L.misc_off = o;   // nrows[2], abort, n_producers, runinfo[2], next item
+    o += 32;
+    L.total = o;
+    return L;
+}
+
+}  // namespace esmm

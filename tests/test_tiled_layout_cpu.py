@@ -1,0 +1,68 @@
+"""CPU checks of what the tiled kernel's host and device sides share (csrc/esmm_tiled_layout.h), compiled with the host compiler, and of
+source rules that no GPU run can show without faulting."""
+import ctypes as C
+import os
+import re
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "esmm-research_b200", "csrc")
+
+SHIM = r"""
+#include "esmm_tiled_layout.h"
+using namespace esmm;
+extern "C" void layout(int stages, int cap, int blocks, unsigned *out)
+{
+    const PackedSmem L = packed_smem_layout(stages, cap, blocks != 0);
+    const unsigned v[] = {L.stage_off, L.krow_off, L.krow_stride, L.rmask_off, L.rmask_stride, L.wlist_off, L.bar_off, L.misc_off, L.total};
+    for (int i = 0; i < 9; ++i) out[i] = v[i];
+}
+extern "C" int constant(int i)
+{
+    const int v[] = {SMEM_LIMIT, BM_SMEM, PSTAGE_BYTES, P_MAX_STAGES, P_CONSUMER_WARPS};
+    return v[i];
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    d = tmp_path_factory.mktemp("layout")
+    src, so = d / "shim.cpp", d / "shim.so"
+    src.write_text(SHIM)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I" + CSRC, "-o", str(so), str(src)])
+    return C.CDLL(str(so))
+
+
+def test_shared_memory_layout(shim):
+    """For every ring depth and K: the regions follow one another, 16-byte (barriers: 8-byte) aligned; in a kernel with block mode
+    the barriers and what follows them lie past the rings that block mode lays over the rest, whose memory may not hold live
+    mbarriers; and block mode refuses no K that the pipeline alone takes."""
+    limit, bm_smem, stage, max_stages, warps = (shim.constant(i) for i in range(5))
+    out = (C.c_uint * 9)()
+    for stages in range(2, max_stages + 1):
+        for cap in list(range(64, 2048, 32)) + list(range(2048, 30000, 416)) + [27520, 27552]:
+            totals = {}
+            for blocks in (0, 1):
+                shim.layout(stages, cap, blocks, out)
+                st, krow, krow_stride, rmask, rmask_stride, wlist, bar, misc, total = out
+                assert st == 0 and krow >= stages * stage and krow_stride >= 2 * cap
+                assert rmask >= krow + 2 * krow_stride and rmask_stride >= cap
+                assert wlist >= rmask + 2 * rmask_stride and wlist % 16 == 0
+                assert bar >= wlist + warps * 2 * 96 and bar % 8 == 0
+                assert misc >= bar + (2 * max_stages + 4) * 8 and misc % 4 == 0 and total >= misc + 7 * 4
+                if blocks:
+                    assert bar >= bm_smem, (stages, cap)
+                totals[blocks] = total
+            assert (totals[0] <= limit) == (totals[1] <= limit), (stages, cap)
+
+
+def test_copies_that_signal_a_barrier_are_waited_for():
+    """Row-major producers' cp.async copies signal the stage's barrier and are never committed to a group, so waiting for committed
+    groups does not wait for them; a producer that leaves after a wait that ran out must wait for all of its copies."""
+    text = open(os.path.join(CSRC, "esmm_gemm_packed.cu")).read()
+    assert "cp.async.mbarrier.arrive.noinc" in text and "cp_async_commit" not in text
+    assert not re.search(r"cp_async_wait_group<", text)
+    assert re.search(r"if \(RM\) cp_async_wait_all\(\);", text)
