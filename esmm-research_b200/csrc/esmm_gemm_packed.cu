@@ -920,7 +920,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             __syncwarp();
             if (lane == 0) mbar_arrive(lempty0 + 8 * buf);
         }
-        if (RM) cp_async_wait_group<0>();
+        if (RM) cp_async_wait_all();   // (after a wait that ran out, copies may still be in flight)
         if (!ok && lane == 0) {
             // leave only after the copies already issued have landed (bounded)
             for (int s = 0; s < p.stages; ++s) {

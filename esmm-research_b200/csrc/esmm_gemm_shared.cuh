@@ -116,6 +116,12 @@ __device__ __forceinline__ void cp_async_wait_group()
 {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
+
+// returns when all of this thread's copies have landed, those too that belong to no committed group (the ones that signal a barrier)
+__device__ __forceinline__ void cp_async_wait_all()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
 #endif  // __CUDACC__
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
