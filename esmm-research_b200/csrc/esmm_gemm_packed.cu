@@ -601,7 +601,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             a_differ += x.z;
             b_differ += x.w;
         }
-        const bool blocks = p.block_mode > 0 || 16 * work <= (RM ? RM_SIXTEENTHS : BM_SIXTEENTHS) * slots;
+        const bool blocks = p.block_mode > 0 || block_mode_pays(work, slots, RM ? RM_SIXTEENTHS : BM_SIXTEENTHS);
         if (blocks && blockIdx.x == 0 && threadIdx.x == 0 && p.form_hint != nullptr) {
             // the note for the next launch (see gemm_ab_packed_launch_form)
             int listed = 0, rows64 = 0, single = 0;

@@ -19,6 +19,7 @@ extern "C" void layout(int stages, int cap, int blocks, unsigned *out)
     const unsigned v[] = {L.stage_off, L.krow_off, L.krow_stride, L.rmask_off, L.rmask_stride, L.wlist_off, L.bar_off, L.misc_off, L.total};
     for (int i = 0; i < 9; ++i) out[i] = v[i];
 }
+extern "C" int pays(int work, int slots, int sixteenths) { return block_mode_pays(work, slots, sixteenths); }
 extern "C" int constant(int i)
 {
     const int v[] = {SMEM_LIMIT, BM_SMEM, PSTAGE_BYTES, P_MAX_STAGES, P_CONSUMER_WARPS};
@@ -57,6 +58,19 @@ def test_shared_memory_layout(shim):
                     assert bar >= bm_smem, (stages, cap)
                 totals[blocks] = total
             assert (totals[0] <= limit) == (totals[1] <= limit), (stages, cap)
+
+
+def test_block_mode_rule(shim):
+    """Block mode where at most so many sixteenths of the sampled slots are live; never on samples that hold no live k at all (the
+    rest of the operands may be dense).  The largest counts, 8 samples of 1024 k and 16 blocks, stay inside 32 bits."""
+    for sixteenths in (4, 11):
+        assert not shim.pays(0, 0, sixteenths)
+        assert shim.pays(0, 16, sixteenths)
+        top = 8 * 1024 * 16
+        for slots in (16, 160, top):
+            assert shim.pays(slots * sixteenths // 16, slots, sixteenths)
+            assert not shim.pays(slots * sixteenths // 16 + 1, slots, sixteenths)
+            assert not shim.pays(slots, slots, sixteenths)
 
 
 def test_copies_that_signal_a_barrier_are_waited_for():
