@@ -92,7 +92,35 @@ __device__ __forceinline__ PatternRows a_pattern(const Params &p, int block)
     }
 }
 
-// What one warp sees of a sample: a 128 x 128 tile over up to 128 of its K blocks.  (block, k) counts.
+// A sample: one 32-bit word, four K blocks, of each pattern row of a 128 x 128 tile per lane; zero where there is no such block.
+struct SampleWords {
+    unsigned a[4], b[4];
+    int na, nb;      // row blocks, column blocks of the tile
+    bool differ;     // two row blocks, or two column blocks, are not the same
+};
+
+// Sample `part` of BM_SAMPLES: up to 128 K blocks of the tile, a single round trip to memory.
+template <bool ROW_MAJOR, typename Params>
+__device__ __forceinline__ SampleWords sample_words(const Params &p, int tm, int tn, int part, int lane)
+{
+    SampleWords s;
+    s.na = min(4, p.a_rows - tm * 4);
+    s.nb = min(4, p.b_rows - tn * 4);
+    const int span = (p.nKB + 3) >> 2, first = max(0, (span - 32) * part / (BM_SAMPLES - 1));
+    const int kb = 4 * (first + lane);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        s.a[i] = pattern_word(a_pattern<ROW_MAJOR>(p, tm * 4 + i), kb, p.nKB, p.pat_words);
+        s.b[i] = pattern_word(b_pattern(p, tn * 4 + i), kb, p.nKB, p.pat_words);
+    }
+    s.differ = false;
+#pragma unroll
+    for (int i = 1; i < 4; ++i)
+        s.differ = s.differ || (i < s.na && s.a[i] != s.a[0]) || (i < s.nb && s.b[i] != s.b[0]);
+    return s;
+}
+
+// What one lane counts in its words.  (block, k) counts.
 struct TileStats {
     int listed;      // k live for the tile as a whole
     int slots;       // listed k times the tile's 32 x 32 blocks: what the tiled pipeline holds in shared memory
@@ -102,46 +130,25 @@ struct TileStats {
     int a_differ, b_differ;   // bits in which adjacent row blocks (column blocks) of a pair differ
 };
 
-template <bool ROW_MAJOR, typename Params>
-__device__ __forceinline__ TileStats tile_stats(const Params &p, int tm, int tn, int part, int lane)
+__device__ __forceinline__ TileStats tile_stats(const SampleWords &w)
 {
-    PatternRows ra[4], rb[4];
-    int na = 0, nb = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        ra[i] = a_pattern<ROW_MAJOR>(p, tm * 4 + i);
-        rb[i] = b_pattern(p, tn * 4 + i);
-        na += ra[i].first != nullptr;
-        nb += rb[i].first != nullptr;
-    }
+    const unsigned(&a)[4] = w.a;
+    const unsigned(&b)[4] = w.b;
     TileStats s = {0, 0, 0, 0, 0, 0, 0};
-    // (one word per lane and row: a single round trip to memory)
-    const int span = (p.nKB + 3) >> 2, first = max(0, (span - 32) * part / (BM_SAMPLES - 1));
-    const int kb = 4 * (first + lane);
-    {
-        unsigned a[4], b[4];
+    const unsigned live = (a[0] | a[1] | a[2] | a[3]) & (b[0] | b[1] | b[2] | b[3]);
+    s.listed = __popc(live);
+    s.slots = s.listed * w.na * w.nb;
+    s.single = s.listed - __popc(__vcmpeq4(live, 0xFFFFFFFFu));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            a[i] = pattern_word(ra[i], kb, p.nKB, p.pat_words);
-            b[i] = pattern_word(rb[i], kb, p.nKB, p.pat_words);
-        }
-        const unsigned live = (a[0] | a[1] | a[2] | a[3]) & (b[0] | b[1] | b[2] | b[3]);
-        const int c = __popc(live);
-        s.listed += c;
-        const unsigned whole = __vcmpeq4(live, 0xFFFFFFFFu);
-        s.single += c - __popc(whole);
+    for (int j = 0; j < 4; ++j) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) s.work += __popc(a[i] & b[j]);
-            s.rows64 += __popc((a[0] | a[1]) & b[j]) + __popc((a[2] | a[3]) & b[j]);
-        }
-        if (ra[1].first) s.a_differ += __popc(a[0] ^ a[1]);
-        if (ra[3].first) s.a_differ += __popc(a[2] ^ a[3]);
-        if (rb[1].first) s.b_differ += __popc(b[0] ^ b[1]);
-        if (rb[3].first) s.b_differ += __popc(b[2] ^ b[3]);
+        for (int i = 0; i < 4; ++i) s.work += __popc(a[i] & b[j]);
+        s.rows64 += __popc((a[0] | a[1]) & b[j]) + __popc((a[2] | a[3]) & b[j]);
     }
-    s.slots = s.listed * na * nb;
+    if (w.na > 1) s.a_differ += __popc(a[0] ^ a[1]);
+    if (w.na > 3) s.a_differ += __popc(a[2] ^ a[3]);
+    if (w.nb > 1) s.b_differ += __popc(b[0] ^ b[1]);
+    if (w.nb > 3) s.b_differ += __popc(b[2] ^ b[3]);
     return s;
 }
 
