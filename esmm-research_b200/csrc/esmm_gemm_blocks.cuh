@@ -93,6 +93,7 @@ __device__ __forceinline__ PatternRows a_pattern(const Params &p, int block)
 }
 
 // A sample: one 32-bit word, four K blocks, of each pattern row of a 128 x 128 tile per lane; zero where there is no such block.
+// Pattern rows that may not be read as words: the first of the four K blocks only, where `whole` is not asked for.
 struct SampleWords {
     unsigned a[4], b[4];
     int na, nb;      // row blocks, column blocks of the tile
@@ -101,7 +102,7 @@ struct SampleWords {
 
 // Sample `part` of BM_SAMPLES: up to 128 K blocks of the tile, a single round trip to memory.
 template <bool ROW_MAJOR, typename Params>
-__device__ __forceinline__ SampleWords sample_words(const Params &p, int tm, int tn, int part, int lane)
+__device__ __forceinline__ SampleWords sample_words(const Params &p, int tm, int tn, int part, int lane, bool whole)
 {
     SampleWords s;
     s.na = min(4, p.a_rows - tm * 4);
@@ -110,8 +111,17 @@ __device__ __forceinline__ SampleWords sample_words(const Params &p, int tm, int
     const int kb = 4 * (first + lane);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        s.a[i] = pattern_word(a_pattern<ROW_MAJOR>(p, tm * 4 + i), kb, p.nKB, p.pat_words);
-        s.b[i] = pattern_word(b_pattern(p, tn * 4 + i), kb, p.nKB, p.pat_words);
+        const PatternRows ra = a_pattern<ROW_MAJOR>(p, tm * 4 + i), rb = b_pattern(p, tn * 4 + i);
+        if (p.pat_words || whole) {
+            s.a[i] = pattern_word(ra, kb, p.nKB, p.pat_words);
+            s.b[i] = pattern_word(rb, kb, p.nKB, p.pat_words);
+        } else {
+            s.a[i] = s.b[i] = 0u;
+            if (kb < p.nKB) {
+                for (int t = 0; ra.first && t < ra.count; ++t) s.a[i] |= ra.first[(size_t)t * p.nKB + kb];
+                if (rb.first) s.b[i] = rb.first[kb];
+            }
+        }
     }
     s.differ = false;
 #pragma unroll
