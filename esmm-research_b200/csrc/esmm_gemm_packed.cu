@@ -119,6 +119,7 @@ struct PackedParams {
     int few_blocks;    // no more pairs of blocks than CTAs
     // row-major A: 32-row block mb uses A pattern rows (mb / a_div) * a_mul + [0, a_mul) of a_pat_rows
     int a_div, a_mul, a_pat_rows;
+    int list_kb, lists;  // row-major A: K blocks per row list, row lists per tile
     const float *A;
     const uint8_t *a_pat;
     const uint8_t *b_pat;
@@ -384,14 +385,14 @@ __device__ __forceinline__ bool blocks_cover(unsigned aw, unsigned bw, unsigned 
 }
 
 template <int RB, int KPL, bool RM>
-__device__ __forceinline__ void tile_scan(const PackedParams &p, int tm, int tn, int lane, unsigned &live_first,
+__device__ __forceinline__ void tile_scan(const PackedParams &p, int tm, int tn, int kb_lo, int kb_hi, int lane, unsigned &live_first,
                                           bool &uniform, bool &full, int &live_total, int &live_small)
 {
-    for (int c0 = 0; c0 < p.nKB; c0 += 32 * KPL) {
+    for (int c0 = kb_lo; c0 < kb_hi; c0 += 32 * KPL) {
         const int kb0 = c0 + KPL * lane;
         unsigned aw[KPL], bw[KPL];
-        load_patterns<RB, KPL, RM>(p, tm, tn, kb0, kb0 < p.nKB, aw, bw);
-        if (c0 == 0) live_first = __shfl_sync(0xFFFFFFFFu, tile_live(aw[0], bw[0]), 0);
+        load_patterns<RB, KPL, RM>(p, tm, tn, kb0, kb0 < kb_hi, aw, bw);
+        if (c0 == kb_lo) live_first = __shfl_sync(0xFFFFFFFFu, tile_live(aw[0], bw[0]), 0);
         bool same = true, cover = true;
         int cnt = 0, small = 0;
 #pragma unroll
@@ -402,8 +403,8 @@ __device__ __forceinline__ void tile_scan(const PackedParams &p, int tm, int tn,
             cnt += __popc(live);
             small += __popc(live) <= p.brow_bits ? __popc(live) : 0;
         }
-        uniform = uniform && __all_sync(0xFFFFFFFFu, kb0 >= p.nKB || same);
-        full = full && __all_sync(0xFFFFFFFFu, kb0 >= p.nKB || cover);
+        uniform = uniform && __all_sync(0xFFFFFFFFu, kb0 >= kb_hi || same);
+        full = full && __all_sync(0xFFFFFFFFu, kb0 >= kb_hi || cover);
         live_total += __reduce_add_sync(0xFFFFFFFFu, cnt);
         live_small += __reduce_add_sync(0xFFFFFFFFu, small);
     }
@@ -432,18 +433,18 @@ __device__ __forceinline__ unsigned a_byte(const PackedParams &p, int mb, int kb
 }
 
 template <int RB, bool RM>
-__device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm, int tn, int lane)
+__device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm, int tn, int kb_lo, int kb_hi, int lane)
 {
     TileScan s = {0u, true, true, 0, 0};
     if (p.vec_patterns == 16) {
-        tile_scan<RB, 16, RM>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
+        tile_scan<RB, 16, RM>(p, tm, tn, kb_lo, kb_hi, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
     } else if (p.vec_patterns == 4) {
-        tile_scan<RB, 4, RM>(p, tm, tn, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
+        tile_scan<RB, 4, RM>(p, tm, tn, kb_lo, kb_hi, lane, s.live_first, s.uniform, s.full, s.live_total, s.live_small);
     } else {
-        for (int kb0 = 0; kb0 < p.nKB; kb0 += 32) {
+        for (int kb0 = kb_lo; kb0 < kb_hi; kb0 += 32) {
             const int kb = kb0 + lane;
             unsigned au = 0, bu = 0;
-            if (kb < p.nKB) {
+            if (kb < kb_hi) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int mb = tm * RB + i, nb = tn * 4 + i;
@@ -452,8 +453,8 @@ __device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm,
                 }
             }
             const unsigned live = au & bu;
-            if (kb0 == 0) s.live_first = __shfl_sync(0xFFFFFFFFu, live, 0);
-            s.uniform = s.uniform && __all_sync(0xFFFFFFFFu, kb >= p.nKB || live == s.live_first);
+            if (kb0 == kb_lo) s.live_first = __shfl_sync(0xFFFFFFFFu, live, 0);
+            s.uniform = s.uniform && __all_sync(0xFFFFFFFFu, kb >= kb_hi || live == s.live_first);
             s.full = false;   // the byte-wise path keeps the general listing
             s.live_total += __reduce_add_sync(0xFFFFFFFFu, __popc(live));
             s.live_small += __reduce_add_sync(0xFFFFFFFFu, __popc(live) <= p.brow_bits ? __popc(live) : 0);
@@ -464,15 +465,16 @@ __device__ __forceinline__ TileScan tile_scan_any(const PackedParams &p, int tm,
 
 // Second pass: the row list.  Lane l owns K blocks c0 + KPL l .. c0 + KPL l + KPL - 1 (consecutive lanes,
 // consecutive K); K blocks with more than whole_above live k are listed whole.  Returns the row count.
+// Rows are numbered from K block kb_lo's first on.
 template <int RB, int KPL, bool RM>
-__device__ __forceinline__ int tile_list(const PackedParams &p, int tm, int tn, int lane, int whole_above,
+__device__ __forceinline__ int tile_list(const PackedParams &p, int tm, int tn, int kb_lo, int kb_hi, int lane, int whole_above,
                                          uint16_t *krow, uint8_t *rmask)
 {
     int pos = 0;
-    for (int c0 = 0; c0 < p.nKB; c0 += 32 * KPL) {
+    for (int c0 = kb_lo; c0 < kb_hi; c0 += 32 * KPL) {
         const int kb0 = c0 + KPL * lane;
         unsigned aw[KPL], bw[KPL];
-        load_patterns<RB, KPL, RM>(p, tm, tn, kb0, kb0 < p.nKB, aw, bw);
+        load_patterns<RB, KPL, RM>(p, tm, tn, kb0, kb0 < kb_hi, aw, bw);
         unsigned rows[KPL];
         int c = 0;
 #pragma unroll
@@ -484,7 +486,7 @@ __device__ __forceinline__ int tile_list(const PackedParams &p, int tm, int tn, 
         const int incl = warp_inclusive_scan(c, lane);
         int q = pos + incl - c;
 #pragma unroll
-        for (int j = 0; j < KPL; ++j) q = append_rows(krow, rmask, q, kb0 + j, rows[j], aw[j], bw[j], p.cap, p.status);
+        for (int j = 0; j < KPL; ++j) q = append_rows(krow, rmask, q, kb0 - kb_lo + j, rows[j], aw[j], bw[j], p.cap, p.status);
         pos += __shfl_sync(0xFFFFFFFFu, incl, 31);
     }
     return pos;
@@ -507,6 +509,15 @@ __device__ __noinline__ int listed_warp_rows(const uint8_t *rmask, int n, int la
         warp_rows += na * __popc(b);
     }
     return __reduce_add_sync(0xFFFFFFFFu, warp_rows);
+}
+
+// The CTA's next row list: the tile's next one, or the first of its next tile.
+template <bool RM>
+__device__ __forceinline__ void next_list(const PackedParams &p, int &tile, int &list)
+{
+    if (RM && ++list < p.lists) return;
+    list = 0;
+    tile += gridDim.x;
 }
 
 // RM: A is the caller's row-major matrix.  The producers then transpose the tile's rows of A with 4-byte copies, the rest is the same.
@@ -568,7 +579,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
     if (warp == P_MASK_WARP && (int)blockIdx.x < p.num_tiles) {
         int tm, tn;
         tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
-        scan = tile_scan_any<RB, RM>(p, tm, tn, lane);
+        scan = tile_scan_any<RB, RM>(p, tm, tn, 0, RM ? p.list_kb : p.nKB, lane);
     }
     // Operands whose samples are the same in all row blocks and in all column blocks of their tiles (uniform patterns, dense ones)
     // are for the pipeline, at the price of one barrier and no counting (1024 x 1024 x 768 at half density 28.6 -> 26.7 us, as
@@ -635,13 +646,14 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
     if (warp == P_MASK_WARP) {
         if (P_REBALANCE_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ESMM_PROD_REGS));
         // ---------------- mask warp: the tile's list of live k rows ----------------
-        int it = 0;
-        for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++it) {
+        int it = 0, list = 0;
+        for (int tile = blockIdx.x; tile < p.num_tiles && ok; next_list<RM>(p, tile, list), ++it) {
             const int buf = it & 1;
+            const int kb_lo = RM ? list * p.list_kb : 0, kb_hi = RM ? min(kb_lo + p.list_kb, p.nKB) : p.nKB;
             int tm, tn;
             tile_coords(tile, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
-            // A first pass over the tile's pattern bytes (the first tile's is done) decides the listing policy.
-            if (it > 0) scan = tile_scan_any<RB, RM>(p, tm, tn, lane);
+            // A first pass over the list's pattern bytes (the first one's is done) decides the listing policy.
+            if (it > 0) scan = tile_scan_any<RB, RM>(p, tm, tn, kb_lo, kb_hi, lane);
             const unsigned live_first = scan.live_first;
             const bool uniform = scan.uniform, full = scan.full;
             const int live_total = scan.live_total, live_small = scan.live_small;
@@ -655,29 +667,29 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             // listing exactly the live k is best at every density measured (brow_bits 7, row_density 8: a K
             // block is then listed whole only when it is whole; 6 / 6 was 2-4 % slower on independent
             // 32-granular patterns at 0.5 / 0.5 and 0.3 / 0.7).
-            const int whole_above = uniform ? BK : (live_total <= p.row_density * p.nKB ? p.brow_bits : 0);
+            const int whole_above = uniform ? BK : (live_total <= p.row_density * (kb_hi - kb_lo) ? p.brow_bits : 0);
             // a run tile?  c = 1, 2, 4 or 8 consecutive live k, whole stages only, 3-D view of B valid
             int run_code = 0;
             {
                 const int c = __popc(live_first);
                 const int kk0 = __ffs((int)live_first) - 1;
                 if (uniform && full && live_first != 0u && (c & (c - 1)) == 0 &&
-                    (live_first >> kk0) == (1u << c) - 1u && (p.nKB * c) % ROWS_PER_STAGE == 0 && p.b_runs_ok &&
+                    (live_first >> kk0) == (1u << c) - 1u && ((kb_hi - kb_lo) * c) % ROWS_PER_STAGE == 0 && p.b_runs_ok &&
                     !p.force_listed && !p.no_run_tiles)
                     run_code = RUN_TILE | (31 - __clz(c)) | (kk0 << 4);
             }
             int pos = 0;
             if (run_code) {
-                pos = p.nKB * __popc(live_first);
+                pos = (kb_hi - kb_lo) * __popc(live_first);
             } else if (p.vec_patterns == 16) {
-                pos = tile_list<RB, 16, RM>(p, tm, tn, lane, whole_above, krow, rmask);
+                pos = tile_list<RB, 16, RM>(p, tm, tn, kb_lo, kb_hi, lane, whole_above, krow, rmask);
             } else if (p.vec_patterns == 4) {
-                pos = tile_list<RB, 4, RM>(p, tm, tn, lane, whole_above, krow, rmask);
+                pos = tile_list<RB, 4, RM>(p, tm, tn, kb_lo, kb_hi, lane, whole_above, krow, rmask);
             } else {
-                for (int kb0 = 0; kb0 < p.nKB; kb0 += 32) {
+                for (int kb0 = kb_lo; kb0 < kb_hi; kb0 += 32) {
                     const int kb = kb0 + lane;
                     unsigned aw = 0, bw = 0;  // byte i: pattern of the tile's i-th 32-row / 32-column block
-                    if (kb < p.nKB) {
+                    if (kb < kb_hi) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const int mb = tm * RB + i, nb = tn * 4 + i;
@@ -689,7 +701,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                     const unsigned rows = live == 0u ? 0u : (__popc(live) > whole_above ? 0xFFu : live);
                     const int c = __popc(rows);
                     const int incl = warp_inclusive_scan(c, lane);
-                    append_rows(krow, rmask, pos + incl - c, kb, rows, aw, bw, p.cap, p.status);
+                    append_rows(krow, rmask, pos + incl - c, kb - kb_lo, rows, aw, bw, p.cap, p.status);
                     pos += __shfl_sync(0xFFFFFFFFu, incl, 31);
                 }
             }
@@ -741,9 +753,9 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
         int slot = 0;
         uint32_t phase = 0;
         uint32_t issued_bits = 0, parity_bits = 0;  // per slot: ever issued / parity of last issue
-        int it = 0;
+        int it = 0, list = 0;
         int copying = P_TMA_WARPS;   // producer warps that share the copies out
-        for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++it) {
+        for (int tile = blockIdx.x; tile < p.num_tiles && ok; next_list<RM>(p, tile, list), ++it) {
             const int buf = it & 1;
             ok = NPW == 7 && q >= copying ? mbar_wait_idle(lfull0 + 8 * buf, (it >> 1) & 1, abort_flag)
                                           : mbar_wait(lfull0 + 8 * buf, (it >> 1) & 1, abort_flag);
@@ -767,6 +779,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             const int a_row0 = panel * p.kp, b_col0 = tn * TILE_N;
             if constexpr (RM) {
                 const int lc = run_code & 15, kk0 = (run_code >> 4) & 7;
+                const int k_lo = list * p.list_kb * BK;            // what the list's k are counted from
                 for (int r0 = 0; r0 < n; r0 += ROWS_PER_STAGE) {
                     const int cnt = min(ROWS_PER_STAGE, n - r0);
                     int k = -1;                                    // of the stage's row `lane`
@@ -793,9 +806,9 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                     const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * PSTAGE_BYTES;
                     if (q == 0 && lane == 0) {
                         mbar_arrive_expect_tx(full, (uint32_t)cnt * ROW_BYTES);
-                        if (run_code) tma_load_3d(s0 + STAGE_HALF_BYTES, &maps.b_run[lc], b_col0, kk0, r0 >> lc, full);
+                        if (run_code) tma_load_3d(s0 + STAGE_HALF_BYTES, &maps.b_run[lc], b_col0, kk0, list * p.list_kb + (r0 >> lc), full);
                     }
-                    if (box_log >= 0) tma_load_2d(s0 + STAGE_HALF_BYTES + lane * ROW_BYTES, &maps.b_box[box_log], b_col0, k, full);
+                    if (box_log >= 0) tma_load_2d(s0 + STAGE_HALF_BYTES + lane * ROW_BYTES, &maps.b_box[box_log], b_col0, k_lo + k, full);
                     // A: 4-byte copies, eight lanes on the k and four on the rows, so that neighbouring k of a row come as one
                     // sector; row groups shared out among the producers.  Rows past the end of A, k past its width (in K
                     // blocks listed whole; no mask has their bit) and past the end of the list: any element, never multiplied
@@ -807,7 +820,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                     const int kk = lane & (KL - 1), rr = lane / KL;
                     int kg[32 / KL];
 #pragma unroll
-                    for (int g = 0; g < 32 / KL; ++g) kg[g] = min(max(__shfl_sync(0xFFFFFFFFu, k, KL * g + kk), 0), p.K - 1);
+                    for (int g = 0; g < 32 / KL; ++g) kg[g] = min(k_lo + max(__shfl_sync(0xFFFFFFFFu, k, KL * g + kk), 0), p.K - 1);
 #pragma unroll 1
                     for (int rg = q; rg < TM_ROWS / RL; rg += P_TMA_WARPS) {
                         const float *row = p.A + (size_t)min(tm * TM_ROWS + rg * RL + rr, p.M - 1) * p.K;
@@ -950,8 +963,9 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
         uint16_t *wlist_b = wlist_t + WLIST_BYTES / 2;
         int slot = 0;
         uint32_t phase = 0;
-        int it = 0;
-        for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++it) {
+        int it = 0, list = 0;
+        Acc acc;
+        for (int tile = blockIdx.x; tile < p.num_tiles && ok; next_list<RM>(p, tile, list), ++it) {
             const int buf = it & 1;
             ok = mbar_wait(lfull0 + 8 * buf, (it >> 1) & 1, abort_flag);
             if (!ok) break;
@@ -962,8 +976,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             const bool run_tile = (runinfo[buf] & RUN_TILE) != 0;
             if (warp == 0) ESMM_STAMP(600 + 4 * it);
 
-            Acc acc;
-            acc_clear(acc);
+            if (!RM || list == 0) acc_clear(acc);
 
             // joint masks of a stage: bit r = row r is live for (top | bottom) block x my columns.  The
             // masks of the next stage are formed under the multiply-adds of the current one (the list's
@@ -1017,6 +1030,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
             __syncwarp();
             if (lane == 0) mbar_arrive(lempty0 + 8 * buf);
             if (warp == 0) ESMM_STAMP(601 + 4 * it);
+            if (RM && list + 1 < p.lists) continue;   // (the tile's sums go on through its next list)
 
             // epilogue: C is overwritten (beta = 0)
             const int row0 = tm * TM_ROWS + wm * 32 * WMB + lm * 4;
@@ -1179,6 +1193,11 @@ int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, con
 }
 
 constexpr int RM_MAX_KB = 8332;   // longest K taken with row-major A, in K blocks
+// Row-major A of more K blocks than RM_WHOLE_LIST_KB: a tile's rows are listed RM_LIST_KB K blocks at a time, its sums go on from
+// one list to the next.  Whole lists leave a ring of fewer than five stages from there on and no ring at all past K = 27488, where
+// block mode, whatever the operands, was the alternative.  Whole lists or block mode / lists in parts, kernel alone, 2048 x 2048 x K:
+// K = 12288 dense 2568 / 2577 us, 24576 dense 5148 / 5160 and 64-granular 0.5 / 0.5 2144 / 1945, 32768 dense 8497 / 5991.
+constexpr int RM_LIST_KB = 1024, RM_WHOLE_LIST_KB = 1390;
 
 // Row-major A, A patterns with one row per a_tile_m rows.
 int gemm_ab_launch(int M, int N, int K, const float *d_A, const float *d_B, float *d_C,
@@ -1206,9 +1225,13 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     p.kp = p.nKB * BK;
     if (p.kp > 65535 && !row_major) return ESMM_ERR_TOO_LARGE;  // row list entries are 16-bit k indices
     p.cap = ((p.kp + 31) & ~31) + 32;
-    // (row-major A with more k than the pipeline's row lists have room for: block mode, whose lists are rings)
-    const bool lists_fit = packed_smem_layout(2, p.cap, false).total <= SMEM_LIMIT;
-    if (row_major && !lists_fit) p.cap = 64;
+    p.list_kb = p.nKB;
+    p.lists = 1;
+    if (row_major && p.nKB > RM_WHOLE_LIST_KB) {
+        p.list_kb = RM_LIST_KB;
+        p.lists = ceil_div(p.nKB, RM_LIST_KB);
+        p.cap = RM_LIST_KB * BK + 32;
+    }
     p.A = d_A;
     p.a_div = a_tile_m >= 32 ? a_tile_m / 32 : 1;
     p.a_mul = a_tile_m >= 32 ? 1 : 32 / a_tile_m;
@@ -1285,7 +1308,6 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     // per SM: 37.1 in the pipeline, 31.5 in block mode).
     const long tile_rounds = (p.num_tiles + sms - 1) / sms;
     p.block_mode = tuning_get("BLOCK_MODE", tile_rounds * p.kp < 768 ? 0 : -1);
-    if (!lists_fit) p.block_mode = 1;
     const bool blocks = p.block_mode != 0;
 
     int stages = tuning_get("STAGES", P_MAX_STAGES);

@@ -832,6 +832,30 @@ def test_gemm_rowmajor_pattern_bits_past_k(cuda, pkg, oracle_mod, tuning, tile_m
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (M, N, K, mode)
 
 
+LONG_KB = 1390    # K blocks from which on (exclusive) row-major A's rows are listed in parts
+
+
+@pytest.mark.parametrize("mode", [1, 0, -1])
+def test_gemm_rowmajor_long_k(cuda, pkg, oracle_mod, tuning, mode):
+    """Row-major A whose rows are listed in several parts per tile: K blocks one more than a list holds, ragged ones, last parts of one
+    K block and of whole stages, pattern rows by bytes, words and 16 bytes, uniform (run tiles), dense, listed and empty parts,
+    several tiles per CTA; both ways of working and the rule's choice."""
+    tuning("BLOCK_MODE", int(mode))
+    for M, N, K, kind in [(130, 132, 8 * LONG_KB + 8, "tiles"), (40, 64, 8 * LONG_KB + 4, 0xFF), (64, 132, 8 * 2048, 0x0F),
+                          (64, 36, 8 * 2048 + 36, 0x81), (32, 128, 8 * 3072 + 512, "tiles"), (40, 64, 27488, 0xFF), (33, 32, 66652, 0x7F)]:
+        A, B = workloads.tile_random(M, N, K, 0.3, 0.6, seed=K, gran_a=32, gran_b=32) if kind == "tiles" else \
+            workloads.uniform_pattern(M, N, K, kind, seed=K)
+        d = Dev(cuda, pkg, A, B)
+        d.patterns()
+        assert np.array_equal(d.gemm_rowmajor(), oracle_mod.gemm_joint(A, B)), (M, N, K, kind)
+    tuning("GRID", 2)
+    A, B = workloads.tile_random(256, 260, 8 * 2100, 0.5, 0.5, seed=5, gran_a=32, gran_b=32)
+    A[:, 8 * 1024:8 * 2048] = 0.0            # the second part of every tile's list is empty
+    d = Dev(cuda, pkg, A, B)
+    d.patterns()
+    assert np.array_equal(d.gemm_rowmajor(), oracle_mod.gemm_joint(A, B))
+
+
 def test_run_kernel_prefix_pattern_past_k(cuda, pkg, oracle_mod, capfd):
     """Id 14 fills A's and B's pattern arrays with constants, K's ragged end included: with K % 8 == 4 and infinities in the last
     column of A, the product has the oracle's bits."""
