@@ -142,10 +142,11 @@ constexpr int RUNS_LIKELY = 0x200;   // a listed tile whose stages may be whole 
 // A stage whose 32 rows are all live for both row blocks: 16 rows of straight-line code per
 // loop trip (measured: 4 rows 1 % slower than 8, 16 rows 1.6 % faster, 32 no better than 16),
 // so that the compiler can issue the loads of a row under the multiply-adds of the row before.
-template <int WMB>
+// RM: row-major A, whose rows in a stage are 16 bytes further apart (see esmm_tiled_layout.h).
+template <int WMB, bool RM>
 __device__ __forceinline__ void dense_rows(Acc &acc, const char *sA, const char *sB)
 {
-    constexpr int A_ROW = 256 * WMB;   // bytes of one k of the A tile
+    constexpr int A_ROW = stage_a_row(WMB, RM);   // bytes of one k of the A tile
     // (Measured and dropped: a rolling prefetch across the loop's back edge; a non-blocking look at the next stage's
     // barrier under the last multiply-adds of this one, so that the wait at the stage change is skipped - no gain.)
 #ifndef ESMM_DENSE_UNROLL
@@ -181,11 +182,17 @@ __device__ __forceinline__ void dense_rows(Acc &acc, const char *sA, const char 
 // was 2-5 % slower on every workload.)
 enum { MODE_BOTH = 0, MODE_TOP = 1, MODE_BOTTOM = 2 };
 
-template <int MODE, int WMB>
+// What stands for a row in masks' walks and in lists: the byte offset in the stage's B rows, or (RM) a 32nd of it, of which the
+// offsets in either operand's rows are multiples.
+template <bool RM>
+constexpr int ROW_SHIFT = RM ? 4 : 9;
+
+template <int MODE, int WMB, bool RM>
 __device__ __forceinline__ KFrag load_entry(const char *sA, const char *sB, unsigned off)
 {
     KFrag f;
-    const unsigned a_off = WMB == 2 ? off : off >> 1;   // A rows are 512 or 256 bytes apart
+    const unsigned a_off = RM ? off * (stage_a_row(WMB, true) / 16) : WMB == 2 ? off : off >> 1;   // A rows are 512 or 256 bytes apart
+    if (RM) off *= ROW_BYTES / 16;
     if (MODE != MODE_BOTTOM) f.at = *reinterpret_cast<const float4 *>(sA + a_off);
     if (MODE != MODE_TOP) f.ab = *reinterpret_cast<const float4 *>(sA + a_off + 128);
     f.b0 = *reinterpret_cast<const float4 *>(sB + off);
@@ -200,37 +207,39 @@ __device__ __forceinline__ void fma_entry(Acc &acc, const KFrag &f)
     if (MODE != MODE_TOP) fma_bottom(acc, f);
 }
 
-// byte offset in the stage's B rows of the lowest live row of m, which is removed from m
+// the lowest live row of m, which is removed from m
+template <bool RM>
 __device__ __forceinline__ unsigned pop_row(unsigned &m)
 {
     const unsigned r = (unsigned)__ffs((int)m) - 1u;
     m &= m - 1u;
-    return r << 9;
+    return r << ROW_SHIFT<RM>;
 }
 
 // (128-row tiling only: in the 64-row tiling every stage that is not all-live takes the list.)
+template <bool RM>
 __device__ __forceinline__ void masked_rows_both(Acc &acc, const char *sA, const char *sB, unsigned m)
 {
     if (m == 0u) return;
-    KFrag f0 = load_entry<MODE_BOTH, 2>(sA, sB, pop_row(m)), f1;
+    KFrag f0 = load_entry<MODE_BOTH, 2, RM>(sA, sB, pop_row<RM>(m)), f1;
 #pragma unroll 1
     while (true) {
         if (m == 0u) {
             fma_entry<MODE_BOTH>(acc, f0);
             break;
         }
-        f1 = load_entry<MODE_BOTH, 2>(sA, sB, pop_row(m));
+        f1 = load_entry<MODE_BOTH, 2, RM>(sA, sB, pop_row<RM>(m));
         fma_entry<MODE_BOTH>(acc, f0);
         if (m == 0u) {
             fma_entry<MODE_BOTH>(acc, f1);
             break;
         }
-        f0 = load_entry<MODE_BOTH, 2>(sA, sB, pop_row(m));
+        f0 = load_entry<MODE_BOTH, 2, RM>(sA, sB, pop_row<RM>(m));
         fma_entry<MODE_BOTH>(acc, f1);
     }
 }
 
-// A list holds, ascending, the byte offset in the stage (row * 512, 16 bits) of every row that is
+// A list holds, ascending, an entry (row << ROW_SHIFT, 16 bits) for every row of the stage that is
 // live for one of the warp's blocks, padded with 8 zero entries so that look-ahead loads need no
 // bounds checks.
 constexpr int WLIST_ENTRIES = ROWS_PER_STAGE + 8;
@@ -244,22 +253,22 @@ __device__ __forceinline__ unsigned entry_of(const uint2 &w, int j)
 }
 
 // Two rows per step, the next pair loaded before the current pair is multiplied.
-template <int MODE, int WMB>
+template <int MODE, int WMB, bool RM>
 __device__ __forceinline__ void listed_rows(Acc &acc, const char *sA, const char *sB, const uint16_t *list, int cnt)
 {
     const int n4 = cnt & ~3;
     uint2 ew = *reinterpret_cast<const uint2 *>(list);   // entries 0..3
-    KFrag f0 = load_entry<MODE, WMB>(sA, sB, entry_of(ew, 0));
-    KFrag f1 = load_entry<MODE, WMB>(sA, sB, entry_of(ew, 1));
+    KFrag f0 = load_entry<MODE, WMB, RM>(sA, sB, entry_of(ew, 0));
+    KFrag f1 = load_entry<MODE, WMB, RM>(sA, sB, entry_of(ew, 1));
 #pragma unroll 1
     for (int i = 0; i < n4; i += 4) {
-        const KFrag g0 = load_entry<MODE, WMB>(sA, sB, entry_of(ew, 2));
-        const KFrag g1 = load_entry<MODE, WMB>(sA, sB, entry_of(ew, 3));
+        const KFrag g0 = load_entry<MODE, WMB, RM>(sA, sB, entry_of(ew, 2));
+        const KFrag g1 = load_entry<MODE, WMB, RM>(sA, sB, entry_of(ew, 3));
         fma_entry<MODE>(acc, f0);
         fma_entry<MODE>(acc, f1);
         ew = *reinterpret_cast<const uint2 *>(list + i + 4);   // padded: always readable
-        f0 = load_entry<MODE, WMB>(sA, sB, entry_of(ew, 0));
-        f1 = load_entry<MODE, WMB>(sA, sB, entry_of(ew, 1));
+        f0 = load_entry<MODE, WMB, RM>(sA, sB, entry_of(ew, 0));
+        f1 = load_entry<MODE, WMB, RM>(sA, sB, entry_of(ew, 1));
         fma_entry<MODE>(acc, g0);
         fma_entry<MODE>(acc, g1);
     }
@@ -267,15 +276,16 @@ __device__ __forceinline__ void listed_rows(Acc &acc, const char *sA, const char
     const int rem = cnt - n4;
     if (rem >= 1) fma_entry<MODE>(acc, f0);
     if (rem >= 2) fma_entry<MODE>(acc, f1);
-    if (rem == 3) fma_entry<MODE>(acc, load_entry<MODE, WMB>(sA, sB, entry_of(ew, 2)));
+    if (rem == 3) fma_entry<MODE>(acc, load_entry<MODE, WMB, RM>(sA, sB, entry_of(ew, 2)));
 }
 
 // Lanes write the list of the rows whose bit is set in `m`; returns the count.
+template <bool RM>
 __device__ __forceinline__ int build_list(uint16_t *list, unsigned m, int lane, int *status)
 {
     const int cnt = __popc(m);
     const int mine = __popc(m & ((1u << lane) - 1u));
-    if (((m >> lane) & 1u) && bounds_ok(mine < WLIST_ENTRIES, status, 25)) list[mine] = (uint16_t)(lane << 9);
+    if (((m >> lane) & 1u) && bounds_ok(mine < WLIST_ENTRIES, status, 25)) list[mine] = (uint16_t)(lane << ROW_SHIFT<RM>);
     if (lane < 8 && bounds_ok(cnt + lane < WLIST_ENTRIES, status, 25)) list[cnt + lane] = 0;
     return cnt;
 }
@@ -535,10 +545,11 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
     constexpr bool P_REBALANCE_REGS = NPW == 7;
     constexpr int TM_ROWS = 64 * WMB;                  // rows of a tile of C: 128 or 64
     constexpr int RB = 2 * WMB;                        // 32-row blocks per tile
-    constexpr int A_ROW = TM_ROWS * 4;                 // bytes of one k of the A tile in shared memory
-    constexpr uint32_t STAGE_ROW_BYTES = A_ROW + ROW_BYTES;
+    constexpr int A_ROW = stage_a_row(WMB, RM);        // bytes of one k of the A tile in shared memory
+    constexpr uint32_t STAGE_ROW_BYTES = TM_ROWS * 4 + ROW_BYTES;
+    constexpr int STAGE_A_BYTES = RM ? RM_STAGE_A_BYTES : STAGE_HALF_BYTES, STAGE_BYTES = STAGE_A_BYTES + STAGE_HALF_BYTES;
     extern __shared__ __align__(1024) char smem[];
-    const PackedSmem L = packed_smem_layout(p.stages, p.cap, BLOCKS);
+    const PackedSmem L = packed_smem_layout(p.stages, STAGE_BYTES, p.cap, BLOCKS);
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
@@ -803,19 +814,20 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                     ok = __all_sync(0xFFFFFFFFu, ok);
                     if (!ok) break;
                     const uint32_t full = full0 + 8 * slot;
-                    const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * PSTAGE_BYTES;
+                    const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * STAGE_BYTES;
                     if (q == 0 && lane == 0) {
                         mbar_arrive_expect_tx(full, (uint32_t)cnt * ROW_BYTES);
-                        if (run_code) tma_load_3d(s0 + STAGE_HALF_BYTES, &maps.b_run[lc], b_col0, kk0, list * p.list_kb + (r0 >> lc), full);
+                        if (run_code) tma_load_3d(s0 + STAGE_A_BYTES, &maps.b_run[lc], b_col0, kk0, list * p.list_kb + (r0 >> lc), full);
                     }
-                    if (box_log >= 0) tma_load_2d(s0 + STAGE_HALF_BYTES + lane * ROW_BYTES, &maps.b_box[box_log], b_col0, k_lo + k, full);
+                    if (box_log >= 0) tma_load_2d(s0 + STAGE_A_BYTES + lane * ROW_BYTES, &maps.b_box[box_log], b_col0, k_lo + k, full);
                     // A: 4-byte copies, eight lanes on the k and four on the rows, so that neighbouring k of a row come as one
                     // sector; row groups shared out among the producers.  Rows past the end of A, k past its width (in K
                     // blocks listed whole; no mask has their bit) and past the end of the list: any element, never multiplied
                     // or never stored.
-                    // These copies are what bounds the form: 4096^3 dense 2622 us against 2144 with packed A.  (Four lanes
-                    // on the k, eight on the rows, fewer bank conflicts but half of each sector: 2753; seven producer
-                    // warps: 2793.)
+                    // What bounds the form: these copies go through the banks the consumers load from, one pass per sector since a
+                    // stage's rows of A are 16 bytes further apart.  Kernel alone, before that -> now (packed A: 2144): 4096^3 dense
+                    // 2621 -> 2387 us, 64-granular 0.5 / 0.5 977 -> 874; 2048 x 2048 x 1000 dense 233 -> 199.  (Rows in place and their
+                    // 16-byte chunks exchanged instead: 4096^3 dense 2445, then with 16 lanes on the k 2501, with 32 2642.)
                     constexpr int KL = RM_KL, RL = 32 / KL;
                     const int kk = lane & (KL - 1), rr = lane / KL;
                     int kg[32 / KL];
@@ -848,10 +860,10 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                     const uint32_t full = full0 + 8 * slot;
                     if (q == 0 && lane == 0) {
                         mbar_arrive_expect_tx(full, (uint32_t)ROWS_PER_STAGE * STAGE_ROW_BYTES);
-                        const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * PSTAGE_BYTES;
+                        const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * STAGE_BYTES;
                         const int kb0 = r0 >> lc;
                         tma_load_3d(s0, &maps.a_run[lc], a_x, kk0, panel * p.nKB + kb0, full);
-                        tma_load_3d(s0 + STAGE_HALF_BYTES, &maps.b_run[lc], b_col0, kk0, kb0, full);
+                        tma_load_3d(s0 + STAGE_A_BYTES, &maps.b_run[lc], b_col0, kk0, kb0, full);
                     }
                     if (q == 0) {
                         issued_bits |= 1u << slot;
@@ -913,9 +925,9 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                 if (it == 0 && q == 0 && r0 < 80 * ROWS_PER_STAGE) ESMM_STAMP(702 + 4 * (r0 / ROWS_PER_STAGE));
                 {
                     const uint32_t full = full0 + 8 * slot;
-                    const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * PSTAGE_BYTES;
+                    const uint32_t s0 = smem_u32(smem + L.stage_off) + (uint32_t)slot * STAGE_BYTES;
                     const uint32_t sa = s0 + lane * A_ROW;
-                    const uint32_t sb = s0 + STAGE_HALF_BYTES + lane * ROW_BYTES;
+                    const uint32_t sb = s0 + STAGE_A_BYTES + lane * ROW_BYTES;
                     if (run >= 0) {
                         if (q == 0 && lane == 0) {
                             tma_load_3d(sa, &maps.a_run[run], a_x, kk0, panel * p.nKB + kb0, full);
@@ -957,7 +969,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
         const int lm = (lane >> 1) & 7;                       // group of 4 rows within a 32-row block
         const int ln = (lane & 1) | ((lane >> 4) << 1);       // 16-byte column chunk
         const uint32_t a_thr = (uint32_t)(wm * 32 * WMB + lm * 4) * 4;                // within a row of A
-        const uint32_t b_thr = STAGE_HALF_BYTES + (uint32_t)(wn * 32 + ln * 4) * 4;  // within a row of B
+        const uint32_t b_thr = STAGE_A_BYTES + (uint32_t)(wn * 32 + ln * 4) * 4;  // within a row of B
         const int t_shift = WMB * wm, b_shift = 4 + wn;
         uint16_t *wlist_t = reinterpret_cast<uint16_t *>(smem + L.wlist_off + warp * 2 * WLIST_BYTES);
         uint16_t *wlist_b = wlist_t + WLIST_BYTES / 2;
@@ -994,29 +1006,29 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                 // in the 64-row tiling a row feeds 16 two-wide FMAs, as in the half modes: lists there too
                 int cnt_t = 0, cnt_b = 0;
                 if (WMB == 1 ? !dense : jt != jb) {
-                    cnt_t = build_list(wlist_t, jt, lane, p.status);
-                    if (WMB == 2) cnt_b = build_list(wlist_b, jb, lane, p.status);
+                    cnt_t = build_list<RM>(wlist_t, jt, lane, p.status);
+                    if (WMB == 2) cnt_b = build_list<RM>(wlist_b, jb, lane, p.status);
                     __syncwarp();
                 }
                 ok = mbar_wait(full0 + 8 * slot, phase, abort_flag);
                 if (!ok) break;
-                if (!bounds_ok(slot >= 0 && slot < p.stages && L.stage_off + (uint32_t)(slot + 1) * PSTAGE_BYTES <= L.krow_off,
+                if (!bounds_ok(slot >= 0 && slot < p.stages && L.stage_off + (uint32_t)(slot + 1) * STAGE_BYTES <= L.krow_off,
                                p.status, 24)) {
                     ok = false;   // a stage outside the ring: leave through the time-out path rather than read it
                     break;
                 }
-                const char *sA = smem + L.stage_off + (size_t)slot * PSTAGE_BYTES + a_thr;
-                const char *sB = smem + L.stage_off + (size_t)slot * PSTAGE_BYTES + b_thr;
+                const char *sA = smem + L.stage_off + (size_t)slot * STAGE_BYTES + a_thr;
+                const char *sB = smem + L.stage_off + (size_t)slot * STAGE_BYTES + b_thr;
                 if (warp == 0 && it == 0) ESMM_STAMP(10 + r0 / ROWS_PER_STAGE);
                 if (dense) {
-                    dense_rows<WMB>(acc, sA, sB);
+                    dense_rows<WMB, RM>(acc, sA, sB);
                 } else if (WMB == 1) {
-                    listed_rows<MODE_TOP, 1>(acc, sA, sB, wlist_t, cnt_t);
+                    listed_rows<MODE_TOP, 1, RM>(acc, sA, sB, wlist_t, cnt_t);
                 } else if (jt == jb) {
-                    masked_rows_both(acc, sA, sB, jt);
+                    masked_rows_both<RM>(acc, sA, sB, jt);
                 } else {
-                    listed_rows<MODE_TOP, 2>(acc, sA, sB, wlist_t, cnt_t);
-                    listed_rows<MODE_BOTTOM, 2>(acc, sA, sB, wlist_b, cnt_b);
+                    listed_rows<MODE_TOP, 2, RM>(acc, sA, sB, wlist_t, cnt_t);
+                    listed_rows<MODE_BOTTOM, 2, RM>(acc, sA, sB, wlist_b, cnt_b);
                 }
                 if (warp == 0 && it == 0) ESMM_STAMP(200 + r0 / ROWS_PER_STAGE);
                 __syncwarp();
@@ -1197,7 +1209,7 @@ constexpr int RM_MAX_KB = 8332;   // longest K taken with row-major A, in K bloc
 // one list to the next.  Whole lists leave a ring of fewer than five stages from there on and no ring at all past K = 27488, where
 // block mode, whatever the operands, was the alternative.  Whole lists or block mode / lists in parts, kernel alone, 2048 x 2048 x K:
 // K = 12288 dense 2568 / 2577 us, 24576 dense 5148 / 5160 and 64-granular 0.5 / 0.5 2144 / 1945, 32768 dense 8497 / 5991.
-constexpr int RM_LIST_KB = 1024, RM_WHOLE_LIST_KB = 1390;
+constexpr int RM_LIST_KB = 1024, RM_WHOLE_LIST_KB = 1336;
 
 // Row-major A, A patterns with one row per a_tile_m rows.
 int gemm_ab_launch(int M, int N, int K, const float *d_A, const float *d_B, float *d_C,
@@ -1313,8 +1325,9 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     int stages = tuning_get("STAGES", P_MAX_STAGES);
     if (stages > P_MAX_STAGES) stages = P_MAX_STAGES;
     if (stages < 2) stages = 2;
-    while (stages > 2 && packed_smem_layout(stages, p.cap, blocks).total > SMEM_LIMIT) --stages;
-    const PackedSmem L = packed_smem_layout(stages, p.cap, blocks);
+    const int stage_bytes = row_major ? RM_STAGE_A_BYTES + STAGE_HALF_BYTES : PSTAGE_BYTES;
+    while (stages > 2 && packed_smem_layout(stages, stage_bytes, p.cap, blocks).total > SMEM_LIMIT) --stages;
+    const PackedSmem L = packed_smem_layout(stages, stage_bytes, p.cap, blocks);
     if (L.total > SMEM_LIMIT) return ESMM_ERR_TOO_LARGE;
     p.stages = stages;
 

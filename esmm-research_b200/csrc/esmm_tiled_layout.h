@@ -21,6 +21,12 @@ constexpr int ROW_BYTES = TILE_N * 4;            // 512: one k of an operand til
 constexpr int ROWS_PER_STAGE = 32;
 constexpr int STAGE_HALF_BYTES = ROWS_PER_STAGE * ROW_BYTES;   // 16384: A rows, then B rows
 constexpr int PSTAGE_BYTES = 2 * STAGE_HALF_BYTES;             // 32768
+// Row-major A: the rows of A in a stage are 16 bytes further apart, so that the producers' 4-byte copies of eight k of four rows of
+// A fall on all 32 banks.  (At 512 or 256 bytes they all fall on four, and every copied sector takes eight passes: 4096^3 dense 2621
+// us, 2387 with the rows apart.)
+ESMM_HOST_DEVICE constexpr int stage_a_row(int wmb, bool row_major) { return 256 * wmb + (row_major ? 16 : 0); }
+constexpr int RM_STAGE_A_BYTES = ROWS_PER_STAGE * stage_a_row(2, true);   // 16896; B's rows after them start on 128 bytes, as the copy engine needs
+static_assert(RM_STAGE_A_BYTES % 128 == 0, "B's rows in a stage");
 constexpr int P_CONSUMER_WARPS = 8;
 constexpr int P_MAX_STAGES = 6;
 
@@ -50,12 +56,12 @@ struct PackedSmem {
 };
 
 // blocks: the kernel has block mode.
-ESMM_HOST_DEVICE inline PackedSmem packed_smem_layout(int stages, int cap, bool blocks)
+ESMM_HOST_DEVICE inline PackedSmem packed_smem_layout(int stages, int stage_bytes, int cap, bool blocks)
 {
     PackedSmem L;
     uint32_t o = 0;
     L.stage_off = o;
-    o += (uint32_t)stages * PSTAGE_BYTES;
+    o += (uint32_t)stages * stage_bytes;
     L.krow_off = o;   // two buffers: k index of every listed row
     L.krow_stride = (uint32_t)cap * 2;
     o += 2 * L.krow_stride;

@@ -832,7 +832,7 @@ def test_gemm_rowmajor_pattern_bits_past_k(cuda, pkg, oracle_mod, tuning, tile_m
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (M, N, K, mode)
 
 
-LONG_KB = 1390    # K blocks from which on (exclusive) row-major A's rows are listed in parts
+LONG_KB = 1336    # K blocks from which on (exclusive) row-major A's rows are listed in parts
 
 
 @pytest.mark.parametrize("mode", [1, 0, -1])

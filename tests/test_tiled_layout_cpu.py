@@ -13,16 +13,16 @@ CSRC = os.path.join(ROOT, "esmm-research_b200", "csrc")
 SHIM = r"""
 #include "esmm_tiled_layout.h"
 using namespace esmm;
-extern "C" void layout(int stages, int cap, int blocks, unsigned *out)
+extern "C" void layout(int stages, int stage_bytes, int cap, int blocks, unsigned *out)
 {
-    const PackedSmem L = packed_smem_layout(stages, cap, blocks != 0);
+    const PackedSmem L = packed_smem_layout(stages, stage_bytes, cap, blocks != 0);
     const unsigned v[] = {L.stage_off, L.krow_off, L.krow_stride, L.rmask_off, L.rmask_stride, L.wlist_off, L.bar_off, L.misc_off, L.total};
     for (int i = 0; i < 9; ++i) out[i] = v[i];
 }
 extern "C" int pays(int work, int slots, int sixteenths) { return block_mode_pays(work, slots, sixteenths); }
 extern "C" int constant(int i)
 {
-    const int v[] = {SMEM_LIMIT, BM_SMEM, PSTAGE_BYTES, P_MAX_STAGES, P_CONSUMER_WARPS};
+    const int v[] = {SMEM_LIMIT, BM_SMEM, PSTAGE_BYTES, P_MAX_STAGES, P_CONSUMER_WARPS, RM_STAGE_A_BYTES + STAGE_HALF_BYTES};
     return v[i];
 }
 """
@@ -41,23 +41,24 @@ def test_shared_memory_layout(shim):
     """For every ring depth and K: the regions follow one another, 16-byte (barriers: 8-byte) aligned; in a kernel with block mode
     the barriers and what follows them lie past the rings that block mode lays over the rest, whose memory may not hold live
     mbarriers; and block mode refuses no K that the pipeline alone takes."""
-    limit, bm_smem, stage, max_stages, warps = (shim.constant(i) for i in range(5))
+    limit, bm_smem, packed_stage, max_stages, warps, rm_stage = (shim.constant(i) for i in range(6))
     out = (C.c_uint * 9)()
-    for stages in range(2, max_stages + 1):
-        for cap in list(range(64, 2048, 32)) + list(range(2048, 30000, 416)) + [27520, 27552]:
-            totals = {}
-            for blocks in (0, 1):
-                shim.layout(stages, cap, blocks, out)
-                st, krow, krow_stride, rmask, rmask_stride, wlist, bar, misc, total = out
-                assert st == 0 and krow >= stages * stage and krow_stride >= 2 * cap
-                assert rmask >= krow + 2 * krow_stride and rmask_stride >= cap
-                assert wlist >= rmask + 2 * rmask_stride and wlist % 16 == 0
-                assert bar >= wlist + warps * 2 * 96 and bar % 8 == 0
-                assert misc >= bar + (2 * max_stages + 4) * 8 and misc % 4 == 0 and total >= misc + 7 * 4
-                if blocks:
-                    assert bar >= bm_smem, (stages, cap)
-                totals[blocks] = total
-            assert (totals[0] <= limit) == (totals[1] <= limit), (stages, cap)
+    for stage in (packed_stage, rm_stage):
+        for stages in range(2, max_stages + 1):
+            for cap in list(range(64, 2048, 32)) + list(range(2048, 30000, 416)) + [27520, 27552]:
+                totals = {}
+                for blocks in (0, 1):
+                    shim.layout(stages, stage, cap, blocks, out)
+                    st, krow, krow_stride, rmask, rmask_stride, wlist, bar, misc, total = out
+                    assert st == 0 and stage % 128 == 0 and krow >= stages * stage and krow_stride >= 2 * cap
+                    assert rmask >= krow + 2 * krow_stride and rmask_stride >= cap
+                    assert wlist >= rmask + 2 * rmask_stride and wlist % 16 == 0
+                    assert bar >= wlist + warps * 2 * 96 and bar % 8 == 0
+                    assert misc >= bar + (2 * max_stages + 4) * 8 and misc % 4 == 0 and total >= misc + 7 * 4
+                    if blocks:
+                        assert bar >= bm_smem, (stages, cap)
+                    totals[blocks] = total
+                assert (totals[0] <= limit) == (totals[1] <= limit), (stages, cap)
 
 
 def test_block_mode_rule(shim):
