@@ -1,4 +1,4 @@
-// Pieces shared by the two joint-sparse GEMM kernels (row-major A and packed A).
+// Pieces shared by the joint-sparse GEMM kernels: tiled (packed and row-major A), its block mode, and the strip kernel.
 #pragma once
 
 #include <cstdio>
@@ -24,18 +24,6 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
     const int r = tile - group * per_group;
     tm = first_m + r % gsize;
     tn = r / gsize;
-}
-
-__device__ __forceinline__ void fma8(float (&acc)[8], float a, const float4 &b0, const float4 &b1)
-{
-    acc[0] = fmaf(a, b0.x, acc[0]);
-    acc[1] = fmaf(a, b0.y, acc[1]);
-    acc[2] = fmaf(a, b0.z, acc[2]);
-    acc[3] = fmaf(a, b0.w, acc[3]);
-    acc[4] = fmaf(a, b1.x, acc[4]);
-    acc[5] = fmaf(a, b1.y, acc[5]);
-    acc[6] = fmaf(a, b1.z, acc[6]);
-    acc[7] = fmaf(a, b1.w, acc[7]);
 }
 
 // One k of the tile for one thread: its 4 rows of the top block, 4 rows of the bottom block
