@@ -50,9 +50,10 @@ __device__ __forceinline__ unsigned inside_k(int kb, int K)
 
 // Pattern bytes of K blocks kb .. kb + 3 of one pattern row (null: no such row), zero past the end.  words: the row may be
 // read as 32-bit words.
-__device__ __forceinline__ unsigned pattern_word(const uint8_t *row, int kb, int nKB, bool words)
+__device__ __forceinline__ unsigned pattern_word(const uint8_t *row, int kb, int nKB, bool words, int *status)
 {
     if (row == nullptr || kb >= nKB) return 0u;
+    if (!bounds_ok(kb >= 0 && (!words || (kb + 4 <= nKB && ((uintptr_t)(row + kb) & 3) == 0)), status, 36)) return 0u;   // checked build: site 36
     if (words) return *reinterpret_cast<const unsigned *>(row + kb);
     unsigned v = 0u;
 #pragma unroll
@@ -66,10 +67,10 @@ struct PatternRows {
     int count;
 };
 
-__device__ __forceinline__ unsigned pattern_word(const PatternRows &r, int kb, int nKB, bool words)
+__device__ __forceinline__ unsigned pattern_word(const PatternRows &r, int kb, int nKB, bool words, int *status)
 {
-    unsigned v = pattern_word(r.first, kb, nKB, words);
-    for (int t = 1; t < r.count; ++t) v |= pattern_word(r.first + (size_t)t * nKB, kb, nKB, words);
+    unsigned v = pattern_word(r.first, kb, nKB, words, status);
+    for (int t = 1; t < r.count; ++t) v |= pattern_word(r.first + (size_t)t * nKB, kb, nKB, words, status);
     return v;
 }
 
@@ -113,8 +114,8 @@ __device__ __forceinline__ SampleWords sample_words(const Params &p, int tm, int
     for (int i = 0; i < 4; ++i) {
         const PatternRows ra = a_pattern<ROW_MAJOR>(p, tm * 4 + i), rb = b_pattern(p, tn * 4 + i);
         if (p.pat_words || whole) {
-            s.a[i] = pattern_word(ra, kb, p.nKB, p.pat_words);
-            s.b[i] = pattern_word(rb, kb, p.nKB, p.pat_words);
+            s.a[i] = pattern_word(ra, kb, p.nKB, p.pat_words, p.status);
+            s.b[i] = pattern_word(rb, kb, p.nKB, p.pat_words, p.status);
         } else {
             s.a[i] = s.b[i] = 0u;
             if (kb < p.nKB) {
@@ -173,13 +174,13 @@ __device__ __forceinline__ int exclusive_scan(int v, int lane)
     return x - v;
 }
 
-// Appends k0 + b for every set bit b of m to a list ring, from this lane's position q on.
-__device__ __forceinline__ void append_live(uint16_t *list, int q, unsigned m, int k0, int *status)
+// Appends k0 + b for every set bit b of m to a list ring, from this lane's position q on; the entries before `taken` are done with.
+__device__ __forceinline__ void append_live(uint16_t *list, int q, int taken, unsigned m, int k0, int *status)
 {
     while (m) {
         const int bit = __ffs((int)m) - 1;
         m &= m - 1u;
-        if (bounds_ok(q >= 0, status, 28)) list[q & (BM_LIST - 1)] = (uint16_t)(k0 + bit);   // checked build: site 28
+        if (bounds_ok(q >= taken && q - taken < BM_LIST, status, 28)) list[q & (BM_LIST - 1)] = (uint16_t)(k0 + bit);   // checked build: site 28
         ++q;
     }
 }
@@ -220,6 +221,10 @@ __device__ __forceinline__ void single_steps(Acc &acc, const char *sx, const cha
         fma_top(acc, f);
     }
 }
+
+// Whether a listed k is inside the operands; row-major A and B end at K, packed A at the K blocks' end (checked build: site 37).
+template <typename Params>
+__device__ __forceinline__ bool k_ok(const Params &p, size_t k) { return bounds_ok(k < (size_t)p.K, p.status, 37); }
 
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src)
 {
@@ -276,9 +281,9 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     int kb0 = -128, part = 0, live = 0;
     unsigned m0 = 0u, m1 = 0u, wy = 0u, w0 = 0u, w1 = 0u;
     auto load_words = [&](int kb) {
-        wy = pattern_word(py, kb, p.nKB, p.pat_words) & inside_k(kb, p.K);
-        w0 = pattern_word(px, kb, p.nKB, p.pat_words);
-        w1 = pattern_word(px1, kb, p.nKB, p.pat_words);
+        wy = pattern_word(py, kb, p.nKB, p.pat_words, p.status) & inside_k(kb, p.K);
+        w0 = pattern_word(px, kb, p.nKB, p.pat_words, p.status);
+        w1 = pattern_word(px1, kb, p.nKB, p.pat_words, p.status);
     };
     auto next_words = [&]() {
         kb0 += 128;
@@ -314,8 +319,8 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
             const int c = __popc(a0) | (__popc(a1) << 16);
             const int before = exclusive_scan(c, lane);
             const int total = __shfl_sync(0xFFFFFFFFu, before + c, 31);
-            append_live(l0.list, l0.made + (before & 0xFFFF), a0, k0, p.status);
-            if (TWO) append_live(l1.list, l1.made + (before >> 16), a1, k0, p.status);
+            append_live(l0.list, l0.made + (before & 0xFFFF), l0.taken, a0, k0, p.status);
+            if (TWO) append_live(l1.list, l1.made + (before >> 16), l1.taken, a1, k0, p.status);
             if (ROW_MAJOR && k0 >= 65536 && wrap0 == INT_MAX) wrap0 = l0.made, wrap1 = l1.made;
             l0.made += total & 0xFFFF;
             l1.made += total >> 16;
@@ -355,7 +360,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
                     const char *g = b_src + c4 * 16 + (size_t)entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d) * n4 + (wide_b ? blk * 128 : 0);
                     const uint32_t part = (uint32_t)((wide_b ? 0 : 2) + blk) * BM_PART;
                     const uint32_t e0 = dst0 + to + h * 1024 + part, e1 = dst1 + to + h * 1024 + part;
-                    if (row < d) {
+                    if (row < d && k_ok(p, entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d))) {
                         const int lim = b_chunks - (wide_b ? blk * 8 : 0);
                         if (!edge || c4 < lim) cp_async_16(e0, g, 16);
                         if (!edge || c4 + 4 < lim) cp_async_16(e1, g + 64, 16);
@@ -379,7 +384,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
                 for (int g = 0; g < BM_ROWS / RM_KL; ++g) {
                     const int row = g * RM_KL + kk;
                     const float *src = p.A + (size_t)row0 * p.K + entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d);
-                    if (row < d) {
+                    if (row < d && k_ok(p, entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d))) {
 #pragma unroll
                         for (int q = 0; q < STEPS; ++q) {
                             // (rows past the end of A: any row, what is multiplied there ends in rows of C that do not exist)
@@ -407,6 +412,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
                 for (int h = 0; h < BM_ROWS / 8; ++h) {
                     const char *gx = xs + (size_t)k0[h] * x_stride, *gy = ys + (size_t)k0[h] * y_stride;
                     const uint32_t e0 = dst0 + to + h * 1024, e1 = dst1 + to + h * 1024;
+                    if (!k_ok(p, k0[h]) || (TWO && !k_ok(p, k1[h]))) continue;
                     if (x_ok0) cp_async_16(e0, gx, 16);
                     if (x_ok1) cp_async_16(e1, gx + 64, 16);
                     if (y_ok0) cp_async_16(e0 + 2 * BM_PART, gy, 16);
@@ -430,6 +436,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
                     const uint32_t e = (j ? dst1 : dst0) + to + (row - r8) * 128 + blk * BM_PART;
                     if (row < (blk ? d1 : d0)) {
                         const size_t k = blk ? l1.list[(l1.taken + row) & (BM_LIST - 1)] : l0.list[(l0.taken + row) & (BM_LIST - 1)];
+                        if (!k_ok(p, k)) continue;
                         if (blk * 8 + ch < x_chunks) cp_async_16(e, xs + k * x_stride + blk * 128 + j * 64, 16);
                         if (ch < y_chunks) cp_async_16(e + 2 * BM_PART, ys + k * y_stride + j * 64, 16);
                     } else {

@@ -105,12 +105,16 @@ def test_guarded_buffers_and_bounds_checks(cuda, pkg, libs, oracle_mod, which, M
 
 @pytest.mark.parametrize("which", ["checked", "product"])
 @pytest.mark.parametrize("hook,value", [(b"PRODUCER_WARPS", 0), (b"PRODUCER_WARPS", 7)])
-def test_guarded_buffers_sixteen_warp_form(cuda, pkg, libs, oracle_mod, which, hook, value):
+@pytest.mark.parametrize("mode", [None, 0])
+def test_guarded_buffers_sixteen_warp_form(cuda, pkg, libs, oracle_mod, which, hook, value, mode):
     """The 16-warp launch shape of the tiled kernel, pinned (its per-CTA choice of copying producers, and all 7 copying),
-    on scattered, ragged and block-dense shapes: same guards, no bounds report, the oracle's bits."""
+    on scattered, ragged and block-dense shapes, in the pipeline (mode 0) and as the rule says (which sends some of them to block
+    mode): same guards, no bounds report, the oracle's bits."""
     t, L = cuda, libs[which]
     assert L.esmm_tuning_set(hook, value) == 0
     try:
+        if mode is not None:
+            assert L.esmm_tuning_set(b"BLOCK_MODE", mode) == 0
         for M, N, K, pA, pB in [(512, 384, 1024, 0.2, 0.2), (257, 260, 1000, 0.4, 0.4), (100, 132, 8 * 37, 0.3, 0.7),
                                 (200, 64, 64, 1.0, 1.0), (64, 512, 8 * 1025, 0.1, 0.5)]:
             A, B = workloads.tile_random(M, N, K, pA, pB, seed=M + N + K, gran_a=32, gran_b=32)
@@ -125,6 +129,37 @@ def test_guarded_buffers_sixteen_warp_form(cuda, pkg, libs, oracle_mod, which, h
             assert bp.intact() and c.intact() and ws.intact(), (M, N, K)
             got = c.view(t.float32, (M, N)).cpu().numpy()
             assert not np.isnan(got).any() and np.array_equal(got, oracle_mod.gemm_joint(A, B)), (M, N, K)
+    finally:
+        L.esmm_tuning_reset()
+
+
+@pytest.mark.parametrize("which", ["checked", "product"])
+@pytest.mark.parametrize("mode", [1, 0])
+def test_guarded_buffers_on_one_cta(cuda, pkg, libs, oracle_mod, which, mode):
+    """Packed and row-major A on one CTA: block mode (1), whose raw copies no tensor map bounds, with pairs of blocks and lists that wrap
+    around, and the pipeline (0) with several tiles and row-major lists in parts.  Ragged sizes, pattern rows read by bytes and by
+    words; same guards, no bounds report, the oracle's bits."""
+    t, L = cuda, libs[which]
+    assert L.esmm_tuning_set(b"BLOCK_MODE", mode) == 0 and L.esmm_tuning_set(b"GRID", 1) == 0
+    try:
+        for M, N, K, pA, pB, ga, gb in [(257, 260, 1000, 0.4, 0.4, 32, 32), (100, 132, 8 * 37, 0.3, 0.7, 32, 64), (160, 292, 76, 0.8, 0.8, 64, 32),
+                                        (292, 160, 2052, 0.9, 0.8, 32, 32), (200, 132, 11008, 0.3, 0.3, 64, 32)]:
+            A, B = workloads.tile_random(M, N, K, pA, pB, seed=M + N + K, gran_a=ga, gran_b=gb)
+            dA, dB = read_only(t, A), read_only(t, B)
+            ap = Guarded(t, -(-M // 32) * -(-K // 8))
+            bp = Guarded(t, -(-N // 32) * -(-K // 8))
+            c1, c2 = Guarded(t, M * N * 4, fill=0xFF), Guarded(t, M * N * 4, fill=0xFF)
+            ws = Guarded(t, int(L.esmm_sgemm_joint_workspace_bytes(M, K)), fill=0xFF)
+            assert L.esmm_preprocess_a(dA.data_ptr(), M, K, 32, ap.ptr, None) == 0
+            assert L.esmm_preprocess_b(dB.data_ptr(), K, N, bp.ptr, None) == 0
+            assert L.esmm_gemm_ab(M, N, K, dA.data_ptr(), dB.data_ptr(), c1.ptr, ap.ptr, bp.ptr, 32, None) == 0
+            assert L.esmm_sgemm_joint(M, N, K, dA.data_ptr(), dB.data_ptr(), c2.ptr, bp.ptr, ws.ptr, None) == 0
+            st = L.esmm_device_status(None)
+            assert st == 0, (st, L.esmm_last_cuda_error())
+            assert all(g.intact() for g in (ap, bp, c1, c2, ws)), (M, N, K)
+            want = oracle_mod.gemm_joint(A, B)
+            for g in (c1, c2):
+                assert np.array_equal(g.view(t.float32, (M, N)).cpu().numpy(), want), (M, N, K)
     finally:
         L.esmm_tuning_reset()
 
