@@ -58,6 +58,12 @@ class Dev:
         return c.cpu().numpy(), ws[:n].reshape(self.ap.shape).cpu().numpy()
 
 
+def pin_mode(tuning, mode):
+    """BLOCK_MODE: 0 = the pipeline, 1 = block mode, -1 = the rule in a kernel that has both, None = the library's choice."""
+    if mode is not None:
+        tuning("BLOCK_MODE", int(mode))
+
+
 def check_all_paths(cuda, pkg, oracle_mod, A, B, expect_bits=True):
     d = Dev(cuda, pkg, A, B)
     ap, bp = d.patterns()
@@ -209,22 +215,29 @@ def test_gemm_llm_mlp_shapes(cuda, pkg, oracle_mod):
         check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
-def test_gemm_long_k_multi_tile_per_cta(cuda, pkg, oracle_mod, tuning):
-    """2048 K blocks (the reference kernel stops at 1024) and several tiles per CTA."""
+@pytest.mark.parametrize("mode", [None, 0])
+def test_gemm_long_k_multi_tile_per_cta(cuda, pkg, oracle_mod, tuning, mode):
+    """2048 K blocks (the reference kernel stops at 1024) and several tiles per CTA, in the pipeline (mode 0) and as the rule says."""
+    pin_mode(tuning, mode)
     tuning("GRID", 3)
     A, B = workloads.tile_random(256, 512, 16384, 0.15, 0.5, seed=4)
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
+@pytest.mark.parametrize("mode", [None, 0])
 @pytest.mark.parametrize("stages", [2, 3])
-def test_gemm_shallow_ring(cuda, pkg, oracle_mod, tuning, stages):
+def test_gemm_shallow_ring(cuda, pkg, oracle_mod, tuning, stages, mode):
+    """A ring of two or three stages, in the pipeline (mode 0) and as the rule says."""
+    pin_mode(tuning, mode)
     tuning("STAGES", int(stages))
     A, B = workloads.tile_random(256, 256, 1024, 0.5, 0.5, seed=11)
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
+@pytest.mark.parametrize("mode", [None, 0])
 @pytest.mark.parametrize("brow", [0, 1, 8])
-def test_gemm_row_fetch_policies(cuda, pkg, oracle_mod, tuning, brow):
+def test_gemm_row_fetch_policies(cuda, pkg, oracle_mod, tuning, brow, mode):
+    pin_mode(tuning, mode)
     tuning("BROW_BITS", int(brow))
     A, B = workloads.tile_random(256, 256, 512, 0.3, 0.4, seed=12, gran_a=32, gran_b=32)
     check_all_paths(cuda, pkg, oracle_mod, A, B)
@@ -232,11 +245,13 @@ def test_gemm_row_fetch_policies(cuda, pkg, oracle_mod, tuning, brow):
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
+@pytest.mark.parametrize("mode", [None, 0])
 @pytest.mark.parametrize("rows", [64, 128])
-def test_gemm_both_tile_heights(cuda, pkg, oracle_mod, tuning, rows):
+def test_gemm_both_tile_heights(cuda, pkg, oracle_mod, tuning, rows, mode):
     """The packed kernel tiles C in 128 x 128 or, where that fills the GPU better, 64 x 128 (a 64-row tile is
     one half of a 128-row panel of packed A).  Both tilings, forced, on uniform, random, ragged and small-M
-    inputs: same bits as the oracle."""
+    inputs: same bits as the oracle, in the pipeline (mode 0) and as the rule says."""
+    pin_mode(tuning, mode)
     tuning("TILE_M", int(rows))
     for pat in (0xFF, 0x0F, 0x01, 0x24):
         A, B = workloads.uniform_pattern(384, 256, 512, pat, seed=pat)
@@ -255,13 +270,16 @@ def test_gemm_both_tile_heights(cuda, pkg, oracle_mod, tuning, rows):
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
+@pytest.mark.parametrize("mode", [None, 0])
 @pytest.mark.parametrize("producers", [7, 0, 3])
 @pytest.mark.parametrize("rows", [128, 64])
-def test_gemm_producer_warp_forms(cuda, pkg, oracle_mod, tuning, rows, producers):
+def test_gemm_producer_warp_forms(cuda, pkg, oracle_mod, tuning, rows, producers, mode):
     """The launch shapes of the tiled kernel, each pinned with esmm_tuning_set("PRODUCER_WARPS", v): 7 = the 16-warp
     form (registers moved between warp groups with setmaxnreg) with all 7 producer warps copying, 0 = the same form
     where each CTA's first tile decides between 3 and 7, 3 = the 12-warp form.  Run tiles, row-by-row stages, boxes
-    of 1 / 2 / 4 / 8 consecutive rows, ragged edges, both tile heights - the same bits as the oracle in every shape."""
+    of 1 / 2 / 4 / 8 consecutive rows, ragged edges, both tile heights - the same bits as the oracle in every shape, in the
+    pipeline (mode 0) and as the rule says (which sends the sparse ones to block mode)."""
+    pin_mode(tuning, mode)
     tuning("PRODUCER_WARPS", int(producers))
     tuning("TILE_M", int(rows))
     for pat in (0xFF, 0x0F, 0x01):
@@ -689,14 +707,18 @@ def test_bounded_wait_reports_timeout_and_context_survives(cuda, pkg, oracle_mod
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
-def test_gemm_mask_builder_paths_agree(cuda, pkg, oracle_mod, tuning):
+@pytest.mark.parametrize("mode", [None, 0])
+def test_gemm_mask_builder_paths_agree(cuda, pkg, oracle_mod, tuning, mode):
     """The tile's row list is built from 16-byte pattern loads (long K), 4-byte loads (shorter K) or byte
-    by byte (pattern rows that are not a multiple of 4 bytes); all must give the same C."""
+    by byte (pattern rows that are not a multiple of 4 bytes); all must give the same C, in the pipeline (mode 0), which builds the
+    list, and as the rule says."""
     A, B = workloads.tile_random(256, 384, 8192 + 128, 0.3, 0.5, seed=17, gran_a=32, gran_b=32)  # 1040 K blocks
-    for mode in ("0", "4", "16"):
-        tuning("VEC_PATTERNS", int(mode))
+    for kpl in ("0", "4", "16"):
+        pin_mode(tuning, mode)
+        tuning("VEC_PATTERNS", int(kpl))
         check_all_paths(cuda, pkg, oracle_mod, A, B)
     tuning.reset()
+    pin_mode(tuning, mode)
     A, B = workloads.tile_random(256, 256, 8 * 37, 0.5, 0.5, seed=18, gran_a=32, gran_b=32)      # 37 K blocks: bytes
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
@@ -757,30 +779,110 @@ def test_gemm_block_mode(cuda, pkg, oracle_mod, tuning, mode):
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
+@pytest.mark.parametrize("grid", [None, 1])
 @pytest.mark.parametrize("mode", [1, 0])
-def test_gemm_block_mode_infinities(cuda, pkg, oracle_mod, tuning, mode):
+def test_gemm_block_mode_infinities(cuda, pkg, oracle_mod, tuning, mode, grid):
     """Steps past the end of the shorter list of a pair change nothing: with infinities and NaN in one block's rows, and sums that
-    are -0, every output of both blocks has the oracle's bits."""
+    are -0, every output of both blocks has the oracle's bits.  On one CTA all eight items are pairs; on a CTA each they are single
+    blocks.  Row-major and packed A, and B's blocks agreeing in pairs more often than A's and the other way round."""
     tuning("BLOCK_MODE", int(mode))
-    A, B = workloads.tile_random(128, 128, 512, 0.3, 0.4, seed=8, gran_a=32, gran_b=32)
+    if grid:
+        tuning("GRID", grid)
+    for ga, gb in [(32, 64), (64, 32)]:
+        infinities_case(cuda, pkg, oracle_mod, ga, gb)
+
+
+def infinities_case(cuda, pkg, oracle_mod, ga, gb):
+    A, B = workloads.tile_random(128, 128, 512, 0.3, 0.4, seed=8, gran_a=ga, gran_b=gb)
     A[5, np.flatnonzero(A[5])[:3]] = [np.inf, -np.inf, np.nan]
+    A[9, np.flatnonzero(A[9])[:30]] = np.resize(np.float32([np.inf, -np.inf, np.nan]), 30)
     A[70] = np.where(A[70] != 0, np.float32(-1e-30), 0)
     B[:, 100] = np.where(B[:, 100] != 0, np.float32(1e-30), 0)      # row 70, column 100: products that round to -0
     d = Dev(cuda, pkg, A, B)
     d.patterns()
-    got, _ = d.sgemm_joint()
     want = oracle_mod.gemm_joint(A, B, oracle_mod.preprocess_a(A), oracle_mod.preprocess_b(B))
-    same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
-    assert same.all() and np.isnan(want).any()
+    assert np.isnan(want).any() and want[70, 100] == 0 and np.signbit(want[70, 100])
+    for got in (d.sgemm_joint()[0], d.gemm_rowmajor()):
+        same = (got.view(np.uint32) == want.view(np.uint32)) | (np.isnan(got) & np.isnan(want))
+        assert same.all(), (ga, gb)
 
 
-@pytest.mark.parametrize("mode", [None, 1, 0])
+@pytest.mark.parametrize("ga,gb", [(32, 64), (64, 32), (32, 32)])
+def test_gemm_block_mode_pairs(cuda, pkg, oracle_mod, tuning, ga, gb):
+    """Block mode on one or two CTAs, so that nearly all items are pairs of blocks (with the launch's own grid these sizes have few
+    items per CTA, which go as single blocks): pairs of row blocks (gran_a 64) and of column blocks (gran_b 64), ragged M, N and K,
+    odd numbers of blocks, pattern rows read by bytes and words, one block of a pair dead where the other is dense."""
+    tuning("BLOCK_MODE", 1)
+    for grid in (1, 2):
+        tuning("GRID", grid)
+        for M, N, K, pa, pb in [(257, 260, 1000, 0.4, 0.4), (100, 132, 8 * 37, 0.3, 0.7), (160, 292, 76, 0.8, 0.8),
+                                (292, 160, 1028, 0.5, 0.3), (320, 352, 1024, 0.7, 0.9), (128, 256, 2048, 0.05, 0.05)]:
+            A, B = workloads.tile_random(M, N, K, pa, pb, seed=M + N + K, gran_a=ga, gran_b=gb)
+            check_all_paths(cuda, pkg, oracle_mod, A, B)
+        A, B = workloads.tile_random(192, 228, 4096, 1.0, 1.0, seed=3)
+        A[:32] = 0.0                      # row blocks 0 and 2, column blocks 1 and 3: one of a pair dead or nearly so
+        A[64:96, 40:] = 0.0
+        B[:4000, 96:128] = 0.0
+        B[100:, 32:64] = 0.0
+        check_all_paths(cuda, pkg, oracle_mod, A, B)
+
+
+@pytest.mark.parametrize("K", [27488, 66656])
+def test_gemm_block_mode_pairs_deepest_k(cuda, pkg, oracle_mod, tuning, K):
+    """Nine items of pairs on one CTA at the deepest K of packed A and of row-major A (list entries past 16 bits), lists that
+    wrap around their rings many times, and B's and A's blocks alike in pairs."""
+    tuning("BLOCK_MODE", 1)
+    tuning("GRID", 1)
+    for ga, gb in [(32, 64), (64, 32)]:
+        A, B = workloads.tile_random(160, 100, K, 0.3, 0.4, seed=K, gran_a=ga, gran_b=gb)
+        d = Dev(cuda, pkg, A, B)
+        d.patterns()
+        want = oracle_mod.gemm_joint(A, B)
+        assert np.array_equal(d.gemm_rowmajor(), want)
+        if K == 27488:
+            assert np.array_equal(d.sgemm_joint()[0], want)
+
+
+def live_share(oracle_mod, A, B):
+    """Share of the (32 x 32 block, k) slots the pipeline would hold for 128 x 128 tiles that are live, over all tiles."""
+    ap = np.unpackbits(oracle_mod.preprocess_a(A), axis=1, bitorder="little").astype(np.int64)
+    bp = np.unpackbits(oracle_mod.preprocess_b(B), axis=1, bitorder="little").astype(np.int64)
+    work = slots = 0
+    for i in range(0, len(ap), 4):
+        for j in range(0, len(bp), 4):
+            a, b = ap[i:i + 4], bp[j:j + 4]
+            work += int((a.sum(0) * b.sum(0)).sum())
+            slots += int((a.any(0) & b.any(0)).sum()) * len(a) * len(b)
+    return work / slots
+
+
+@pytest.mark.parametrize("rows", [128, 64])
+@pytest.mark.parametrize("producers", [3, 0, 7])
+def test_gemm_pipeline_of_kernels_with_block_mode(cuda, pkg, oracle_mod, tuning, rows, producers):
+    """The kernels that have both ways of working (BLOCK_MODE -1), on operands that the rule sends to the pipeline: scattered live k
+    that are the same in all blocks (nothing to count), and blocks that differ, at shares above either limit.  Ragged sizes, listed
+    rows, several tiles per CTA, both tile heights and launch shapes."""
+    tuning("BLOCK_MODE", -1)
+    tuning("TILE_M", rows)
+    tuning("PRODUCER_WARPS", producers)
+    for M, N, K, p, gran in [(257, 260, 1000, 0.4, 2048), (100, 132, 8 * 37, 0.5, 2048), (130, 132, 1028, 0.3, 2048),
+                             (384, 256, 2048, 0.2, 2048), (257, 260, 1000, 0.97, 32), (200, 292, 76, 0.97, 32), (192, 132, 2048, 0.95, 32)]:
+        A, B = workloads.tile_random(M, N, K, p, p, seed=M + K, gran_a=gran, gran_b=gran)
+        assert live_share(oracle_mod, A, B) > 0.75
+        check_all_paths(cuda, pkg, oracle_mod, A, B)
+    tuning("GRID", 2)
+    A, B = workloads.tile_random(300, 420, 1200, 0.96, 0.96, seed=6, gran_a=32, gran_b=32)
+    check_all_paths(cuda, pkg, oracle_mod, A, B)
+
+
+@pytest.mark.parametrize("mode,grid", [(None, None), (1, None), (1, 1), (0, None), (0, 1)])
 @pytest.mark.parametrize("tile_m", [8, 16, 64, 128])
-def test_gemm_rowmajor_pattern_heights(cuda, pkg, oracle_mod, tuning, tile_m, mode):
+def test_gemm_rowmajor_pattern_heights(cuda, pkg, oracle_mod, tuning, tile_m, mode, grid):
     """Row-major A whose patterns have one row per 8, 16, 64 or 128 rows: a 32-row block multiplies the OR of its pattern rows.
-    Ragged M, N and K; both ways of working and the rule's choice."""
-    if mode is not None:
-        tuning("BLOCK_MODE", int(mode))
+    Ragged M, N and K; both ways of working and the rule's choice, and all of it on one CTA (pairs of blocks, several tiles)."""
+    pin_mode(tuning, mode)
+    if grid:
+        tuning("GRID", grid)
     for M, N, K, pat in [(300, 164, 76, None), (256, 384, 1024, None), (130, 260, 8 * 37, None), (256, 256, 512, 0x0F)]:
         A, B = workloads.tile_random(M, N, K, 0.4, 0.5, seed=M + K, gran_a=32, gran_b=32) if pat is None else \
             workloads.uniform_pattern(M, N, K, pat, seed=pat)
