@@ -112,7 +112,8 @@ struct PackedParams {
     int no_run_tiles;  // tuning aid: build the row list even for tiles that need none
     int vec_patterns;  // K blocks per lane and load in the mask warp: 16, 4 (alignment permitting) or 0 = bytes
     int adaptive;      // 16-warp form: the CTA's first tile decides whether 3 or all 7 producer warps copy
-    int *form_hint;    // host-mapped word, or null: CTA 0 notes whether its first tile wanted 7 producers
+    int *form_hint;    // host-mapped word, or null: CTA 0 notes whether its first tile wanted 7 producers ...
+    int form_known;    // ... where that is not what the host read there
     int block_mode;    // 1, 0: always, never; -1: as the sampled tiles say
     int pat_words;     // pattern rows may be read as 32-bit words
     unsigned last_bits;  // of the last K block's byte: the bits whose k is < K, in all four bytes of the word
@@ -640,7 +641,8 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                 rows64 += y.y;
                 single += y.z;
             }
-            *p.form_hint = p.few_blocks && 2 * single >= listed && rows64 <= 3 * listed ? 1 : 0;
+            const int note = p.few_blocks && 2 * single >= listed && rows64 <= 3 * listed ? 1 : 0;
+            if (note != p.form_known) *p.form_hint = note;
         }
         __syncthreads();   // the samples have been read by all
         if (blocks) {
@@ -740,7 +742,7 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                 if (lane == 0) {
                     *n_producers = !p.adaptive || wants7 ? 7 : 3;
                     // (either form computes the same C; the note only steers the shape of the next launch)
-                    if (blockIdx.x == 0 && p.form_hint != nullptr) *p.form_hint = wants7 ? 1 : 0;
+                    if (blockIdx.x == 0 && p.form_hint != nullptr && (wants7 ? 1 : 0) != p.form_known) *p.form_hint = wants7 ? 1 : 0;
                 }
             }
             if (lane == 0) {
@@ -1103,10 +1105,12 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
 // The launch shape follows the operands: the 16-warp form pays on tiles of scattered single rows and costs about
 // half a percent elsewhere, and which kind the operands are is known on the device only.  So CTA 0 of every
 // launch notes what its first tile would have wanted in a word of host-mapped memory (one per device, set up at
-// the first launch), and the next launch on that device reads the word, without waiting for anything: repeated
+// the first launch) where the word said otherwise when the host launched it (the launch's end waits for the store across PCIe: 512 x
+// 1024 x 704 32-granular 0.2 / 0.2 16.4 us with a note every time, 14.4 now), and the next launch on that device reads the word, without waiting for anything: repeated
 // products of like operands - what a benchmark loop or a layer with fixed weights issues - get the right
 // shape from the second call on, and a stale or missing note only costs that difference.  The results are
-// bit-identical in both shapes.  esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins the shape instead.  (Operands of that kind that are
+// bit-identical in both shapes.  esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins the shape instead.  (Scattered rows
+// reach the pipeline in launches too short to look at the samples: 512 x 1024 x 704 as above 16.4 us with 12 warps.  Operands of that kind that are
 // large enough to be looked at go to block mode now, where twelve warps work in either shape and the 12-warp form is the faster
 // one or as fast; there the note is set only with no more pairs of blocks than CTAs, where both take the same time: 512 x 1024 x
 // 2048 at 0.3 / 0.3 25.3 and 24.9 us.)
@@ -1303,7 +1307,8 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
             const FormHint hint = form_hint_word(dev);
             if (hint.host) {
                 p.form_hint = hint.device;
-                if (*hint.host != 0) producer_warps = 0;
+                p.form_known = *hint.host != 0 ? 1 : 0;
+                if (p.form_known) producer_warps = 0;
             }
         }
     }

@@ -149,7 +149,7 @@ int esmm_preprocess_a_packed(const float *d_A, int M, int K, uint8_t *d_out, flo
 /*
  * Same contract as esmm_gemm_ab (32-row A patterns) with the packed copy in place of A, except that
  * the first call on a device sets aside one 64-byte word of host-mapped memory (kept for the life of
- * the process): every launch of the tiled kernel notes there whether its operands were of
+ * the process): every launch of the tiled kernel notes there, where that is news, whether its operands were of
  * scattered single rows in a form that gains from it, and the next launch on that device picks its launch shape (12 or 16 warps
  * per CTA) by it, without waiting for anything.  The shapes differ in speed only, never in a bit of
  * C; esmm_tuning_set("PRODUCER_WARPS", ...) pins one.  No device memory is allocated.  Make the first
