@@ -522,6 +522,71 @@ __device__ __noinline__ int listed_warp_rows(const uint8_t *rmask, int n, int la
     return __reduce_add_sync(0xFFFFFFFFu, warp_rows);
 }
 
+// Which way of working the launch takes: the same answer in every CTA.  All warps of the CTA call this; scratch: shared memory for the
+// samples, free again on return.  (A call rather than inline code: it runs once per CTA, and what follows gets better registers: pruned
+// MLP 2048 x 11008 x 4096 765 -> 748 us, 1000 x 1508 x 2012 at 0.5 / 0.5 59.4 -> 57.4, 4096^3 dense 2165 -> 2148.  Block mode as a call
+// spills: 866, 67.6, 2170.)
+enum { MODE_PIPELINE, MODE_BLOCKS, MODE_BLOCKS_WIDE_B };
+
+template <bool RM>
+__device__ __noinline__ int choose_mode(const PackedParams &p, char *scratch, int warp, int lane)
+{
+    // Operands whose samples are the same in all row blocks and in all column blocks of their tiles (uniform patterns, dense ones)
+    // are for the pipeline, at the price of one barrier and no counting (1024 x 1024 x 768 at half density 28.6 -> 26.7 us, as
+    // without the look; 1024^3 33.0 -> 32.8; pattern rows read byte by byte: 1126 x 776 x 840 at a quarter 24.6 -> 22.6).
+    SampleWords words;
+    words.differ = false;
+    const int sample_m = warp * ((p.a_rows + 3) >> 2) / BM_SAMPLES, sample_n = ((5 * warp + 2) & 7) * p.tiles_n / BM_SAMPLES;
+    if (warp < BM_SAMPLES) words = sample_words<RM>(p, sample_m, sample_n, warp, lane, false);
+    if (!__syncthreads_or(words.differ) && p.block_mode <= 0) return MODE_PIPELINE;
+    // two vectors per sample
+    int4 *stats = reinterpret_cast<int4 *>(scratch);
+    static_assert(2 * BM_SAMPLES * sizeof(int4) <= P_CONSUMER_WARPS * 2 * 96 && BM_SAMPLES <= P_CONSUMER_WARPS, "samples");
+    if (warp < BM_SAMPLES) {
+        if (!p.pat_words) words = sample_words<RM>(p, sample_m, sample_n, warp, lane, true);
+        const TileStats s = tile_stats(words);
+        int4 x, y;
+        x.x = __reduce_add_sync(0xFFFFFFFFu, s.slots);
+        x.y = __reduce_add_sync(0xFFFFFFFFu, s.work);
+        x.z = __reduce_add_sync(0xFFFFFFFFu, s.a_differ);
+        x.w = __reduce_add_sync(0xFFFFFFFFu, s.b_differ);
+        y.x = __reduce_add_sync(0xFFFFFFFFu, s.listed);
+        y.y = __reduce_add_sync(0xFFFFFFFFu, s.rows64);
+        y.z = __reduce_add_sync(0xFFFFFFFFu, s.single);
+        y.w = 0;
+        if (lane == 0) {
+            stats[warp] = x;
+            stats[BM_SAMPLES + warp] = y;
+        }
+    }
+    __syncthreads();
+    int slots = 0, work = 0, a_differ = 0, b_differ = 0;
+#pragma unroll
+    for (int i = 0; i < BM_SAMPLES; ++i) {
+        const int4 x = stats[i];
+        slots += x.x;
+        work += x.y;
+        a_differ += x.z;
+        b_differ += x.w;
+    }
+    const bool blocks = p.block_mode > 0 || block_mode_pays(work, slots, RM ? RM_SIXTEENTHS : BM_SIXTEENTHS);
+    if (blocks && blockIdx.x == 0 && threadIdx.x == 0 && p.form_hint != nullptr) {
+        // the note for the next launch (see gemm_ab_packed_launch_form)
+        int listed = 0, rows64 = 0, single = 0;
+        for (int i = 0; i < BM_SAMPLES; ++i) {
+            const int4 y = stats[BM_SAMPLES + i];
+            listed += y.x;
+            rows64 += y.y;
+            single += y.z;
+        }
+        const int note = p.few_blocks && 2 * single >= listed && rows64 <= 3 * listed ? 1 : 0;
+        if (note != p.form_known) *p.form_hint = note;
+    }
+    __syncthreads();   // the samples have been read by all
+    if (!blocks) return MODE_PIPELINE;
+    return (RM ? b_differ <= a_differ : b_differ < a_differ) ? MODE_BLOCKS_WIDE_B : MODE_BLOCKS;
+}
+
 // The CTA's next row list: the tile's next one, or the first of its next tile.
 template <bool RM>
 __device__ __forceinline__ void next_list(const PackedParams &p, int &tile, int &list)
@@ -593,60 +658,10 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
         tile_coords(blockIdx.x, p.tiles_m, p.tiles_n, tm, tn, p.group_m);
         scan = tile_scan_any<RB, RM>(p, tm, tn, 0, RM ? p.list_kb : p.nKB, lane);
     }
-    // Operands whose samples are the same in all row blocks and in all column blocks of their tiles (uniform patterns, dense ones)
-    // are for the pipeline, at the price of one barrier and no counting (1024 x 1024 x 768 at half density 28.6 -> 26.7 us, as
-    // without the look; 1024^3 33.0 -> 32.8; pattern rows read byte by byte: 1126 x 776 x 840 at a quarter 24.6 -> 22.6).
-    SampleWords words;
-    words.differ = false;
-    const int sample_m = warp * ((p.a_rows + 3) >> 2) / BM_SAMPLES, sample_n = ((5 * warp + 2) & 7) * p.tiles_n / BM_SAMPLES;
-    if (BLOCKS && warp < BM_SAMPLES) words = sample_words<RM>(p, sample_m, sample_n, warp, lane, false);
-    if (BLOCKS && p.block_mode != 0 && (__syncthreads_or(words.differ) || p.block_mode > 0)) {
-        // two vectors per sample, where the consumers' lists will be
-        int4 *stats = reinterpret_cast<int4 *>(smem + L.wlist_off);
-        static_assert(2 * BM_SAMPLES * sizeof(int4) <= P_CONSUMER_WARPS * 2 * 96 && BM_SAMPLES <= P_CONSUMER_WARPS, "samples");
-        if (warp < BM_SAMPLES) {
-            if (!p.pat_words) words = sample_words<RM>(p, sample_m, sample_n, warp, lane, true);
-            const TileStats s = tile_stats(words);
-            int4 x, y;
-            x.x = __reduce_add_sync(0xFFFFFFFFu, s.slots);
-            x.y = __reduce_add_sync(0xFFFFFFFFu, s.work);
-            x.z = __reduce_add_sync(0xFFFFFFFFu, s.a_differ);
-            x.w = __reduce_add_sync(0xFFFFFFFFu, s.b_differ);
-            y.x = __reduce_add_sync(0xFFFFFFFFu, s.listed);
-            y.y = __reduce_add_sync(0xFFFFFFFFu, s.rows64);
-            y.z = __reduce_add_sync(0xFFFFFFFFu, s.single);
-            y.w = 0;
-            if (lane == 0) {
-                stats[warp] = x;
-                stats[BM_SAMPLES + warp] = y;
-            }
-        }
-        __syncthreads();
-        int slots = 0, work = 0, a_differ = 0, b_differ = 0;
-#pragma unroll
-        for (int i = 0; i < BM_SAMPLES; ++i) {
-            const int4 x = stats[i];
-            slots += x.x;
-            work += x.y;
-            a_differ += x.z;
-            b_differ += x.w;
-        }
-        const bool blocks = p.block_mode > 0 || block_mode_pays(work, slots, RM ? RM_SIXTEENTHS : BM_SIXTEENTHS);
-        if (blocks && blockIdx.x == 0 && threadIdx.x == 0 && p.form_hint != nullptr) {
-            // the note for the next launch (see gemm_ab_packed_launch_form)
-            int listed = 0, rows64 = 0, single = 0;
-            for (int i = 0; i < BM_SAMPLES; ++i) {
-                const int4 y = stats[BM_SAMPLES + i];
-                listed += y.x;
-                rows64 += y.y;
-                single += y.z;
-            }
-            const int note = p.few_blocks && 2 * single >= listed && rows64 <= 3 * listed ? 1 : 0;
-            if (note != p.form_known) *p.form_hint = note;
-        }
-        __syncthreads();   // the samples have been read by all
-        if (blocks) {
-            if (warp < BM_WARPS) block_mode<RM>(p, smem, warp, lane, RM ? b_differ <= a_differ : b_differ < a_differ, next_item);
+    if (BLOCKS && p.block_mode != 0) {
+        const int mode = choose_mode<RM>(p, smem + L.wlist_off, warp, lane);
+        if (mode != MODE_PIPELINE) {
+            if (warp < BM_WARPS) block_mode<RM>(p, smem, warp, lane, mode == MODE_BLOCKS_WIDE_B, next_item);
             return;
         }
     }
@@ -1078,14 +1093,14 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
 
 template <int WMB, int NPW, bool BLOCKS>
 __global__ void __launch_bounds__((P_CONSUMER_WARPS + NPW + 1) * 32, 1)
-esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const PackedParams p)
+esmm_joint_sgemm_packed_kernel(const __grid_constant__ PackedMaps maps, const __grid_constant__ PackedParams p)
 {
     tiled_sgemm<WMB, NPW, false, BLOCKS>(maps, p);
 }
 
 template <int WMB, bool BLOCKS>
 __global__ void __launch_bounds__((P_CONSUMER_WARPS + 4) * 32, 1)
-esmm_joint_sgemm_kernel(const __grid_constant__ PackedMaps maps, const PackedParams p)
+esmm_joint_sgemm_kernel(const __grid_constant__ PackedMaps maps, const __grid_constant__ PackedParams p)
 {
     tiled_sgemm<WMB, 3, true, BLOCKS>(maps, p);
 }
