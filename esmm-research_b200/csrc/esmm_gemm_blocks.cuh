@@ -19,11 +19,12 @@
 //   * the warps of a CTA draw items from a counter in shared memory; the last ones come as single blocks spread over the whole
 //     warp, so that the warps finish together (a problem with few blocks consists of nothing else).
 //
-// What bounds it: the FMA pipe, 74 % busy where the lists are long (the pipeline on dense tiles: 76 %); what is lost goes to the
+// What bounds it: the FMA pipe (ncu, sm__pipe_fma_cycles_active of the launch: 71 % at 4096^3 64-granular 0.5 / 0.5, 58 % at 32-granular
+// 0.2 / 0.2; the pipeline on dense tiles 88 %); what is lost goes to the
 // copies, which take issue slots and shared-memory bandwidth from the same warps (without them, a probe, 12 % faster at long
 // lists, 6 % at short ones), and to the listing.  Measured, whole calls, the tiled pipeline before -> block mode: 2048 x 11008 x 4096
-// pruned MLP 1016 -> 739 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 167 and at 0.5 / 0.5 921 -> 718,
-// 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 59.7.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 / 0.5 824),
+// pruned MLP 1016 -> 748 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 167 and at 0.5 / 0.5 921 -> 718,
+// 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 57.4.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 / 0.5 824),
 // 8 k per stage (971), lists made for all of K before the first copy (762), rows past a list's end skipped in a second code
 // path instead of multiplied by zeros (752: the accumulators are then moved between registers at every stage).
 //

@@ -75,9 +75,9 @@ constexpr int P_TMA_WARP = P_CONSUMER_WARPS;                   // first producer
 // 0.8 / 0.8) 1900 / 1737, 0.67 (64-granular, 1 / 0.5) 1373 / 1346, 0.69 (64-granular, 0.8 / 0.8) 1675 / 1685, 0.83 (64-granular,
 // 0.9 / 0.9) 2050 / 2087, 1 (dense) 2130 / 2549.
 constexpr int BM_SIXTEENTHS = 11;
-// The same for row-major A, where block mode has to transpose A for every pair of blocks: 2048^3, with the pattern pass, pipeline /
-// block mode: share 0.11 (32-granular, 0.2 / 0.2) 103 / 71 us; 4096^3 share 0.33 (32-granular, 0.5 / 0.5) 1484 / 1489;
-// 2048^3 share 0.44 (64-granular, 0.5 / 0.5) 159 / 189.
+// The same for row-major A, where block mode has to transpose A for every pair of blocks: kernel alone, pipeline / block mode, share 0.11
+// (32-granular, 0.2 / 0.2) 2048^3 83 / 71 us, 4096^3 455 / 437; share 0.16 (0.3 / 0.3) 123 / 113, 724 / 686; share 0.33 (0.5 / 0.5) 4096^3
+// 1194 / 1402; share 0.44 (64-granular, 0.5 / 0.5) 2048^3 147 / 178.
 constexpr int RM_SIXTEENTHS = 4;
 
 // Optional timeline for tuning (build with -DESMM_TRACE): CTA 0 stamps %globaltimer at a few points
@@ -598,8 +598,8 @@ __device__ __forceinline__ void next_list(const PackedParams &p, int &tile, int 
 
 // RM: A is the caller's row-major matrix.  The producers then transpose the tile's rows of A with 4-byte copies, the rest is the same.
 // (Before, a kernel of its own fetched boxes of 128 rows x 8 k, multiplied with scalar FMAs and could not leave out dead k of A.
-// Kernel and pattern pass, before -> now: 2048^3 64-granular 0.5 / 0.5 237 -> 159 us, 32-granular 0.2 / 0.2 111 -> 71; 4096^3 dense
-// 2813 -> 2622, half 1855 -> 1322, quarter 1469 -> 687, eighth 855 -> 474; 16 x 11008 x 4096 MLP 146 -> 65.)
+// Kernel alone, before -> now: 2048^3 64-granular 0.5 / 0.5 232 -> 149 us, 32-granular 0.2 / 0.2 106 -> 72; 4096^3 dense 2806 -> 2387, half
+// 1844 -> 1210; 2048 x 2048 x 1000 dense 210 -> 199.)
 // BLOCKS: with block mode; without it for launches too short to look whether it would pay (the code is then that of the pipeline
 // alone: up to 1.3 us of a 15 us call).
 template <int WMB, int NPW, bool RM, bool BLOCKS>
@@ -1335,7 +1335,7 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     int grid = tuning_get("GRID", sms);
     const long pairs = std::max((long)ceil_div(p.a_rows, 2) * p.b_rows, (long)p.a_rows * ceil_div(p.b_rows, 2));
     p.few_blocks = pairs <= grid;
-    // The samples cost a launch a microsecond or two, which short ones do not win back: the pipeline, without looking, where an SM
+    // Where blocks differ the samples cost a launch a microsecond or two, which short ones do not win back: the pipeline, without looking, where an SM
     // has fewer than 768 k of tiles to go through (58 x 7368 x 648: 15.2 us, 17.4 with the look; 2502 x 1112 x 456, 912 k of tiles
     // per SM: 37.1 in the pipeline, 31.5 in block mode).
     const long tile_rounds = (p.num_tiles + sms - 1) / sms;
