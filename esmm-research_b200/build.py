@@ -19,9 +19,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo"] + ARCH
 
 LIB_SRCS = [os.path.join(HERE, "csrc", f) for f in
-            ("esmm_gemm_packed.cu", "esmm_gemm_skinny.cu", "esmm_preprocess.cu", "esmm_api.cu", "esmm_noalloc.cu",
+            ("esmm_gemm_packed.cu", "esmm_gemm_rowmajor.cu", "esmm_gemm_skinny.cu", "esmm_preprocess.cu", "esmm_api.cu", "esmm_noalloc.cu",
              "esmm_cusparse.cu", "esmm_gemm_tf32.cu", "esmm_host.cu", "esmm_multi.cu")]
-LIB_DEPS = LIB_SRCS + [os.path.join(HERE, "csrc", "esmm_common.cuh"), os.path.join(HERE, "csrc", "esmm_gemm_shared.cuh"), os.path.join(HERE, "csrc", "esmm_gemm_blocks.cuh"),
+LIB_DEPS = LIB_SRCS + [os.path.join(HERE, "csrc", "esmm_common.cuh"), os.path.join(HERE, "csrc", "esmm_gemm_shared.cuh"), os.path.join(HERE, "csrc", "esmm_gemm_tiled.cuh"), os.path.join(HERE, "csrc", "esmm_gemm_blocks.cuh"),
                        os.path.join(HERE, "csrc", "esmm_tiled_layout.h"), os.path.join(ROOT, "include", "esmm.h")]
 EXE_SRCS = [os.path.join(HERE, "driver.cu")]
 EXE_DEPS = EXE_SRCS + [os.path.join(ROOT, "include", h) for h in ("runners.cuh", "utils.cuh", "esmm.h")]

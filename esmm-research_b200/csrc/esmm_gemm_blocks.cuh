@@ -1,7 +1,7 @@
 // Block mode of the packed joint-sparse SGEMM: every warp of the CTA works on its own blocks of C, with its own list of live k
 // and its own copies.
 //
-// The tiled pipeline (esmm_gemm_packed.cu) fetches every k that is live for any part of a 128 x 128 tile and moves in steps
+// The tiled pipeline (esmm_gemm_tiled.cuh) fetches every k that is live for any part of a 128 x 128 tile and moves in steps
 // of 32 such rows, eight warps together.  On operands whose 32-row and 32-column blocks are zero in different places most of
 // a fetched row is of no use to most of the warps, and a step lasts as long as its busiest warp.  Here nothing is shared:
 //

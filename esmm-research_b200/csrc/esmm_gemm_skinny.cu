@@ -1,6 +1,6 @@
 // Joint-sparse FP32 SGEMM for sm_100a, few rows: M <= 32 (one 32-row pattern block of A).
 //
-// Same arithmetic as the packed kernel (esmm_gemm_packed.cu) and as esmm_ab_optimized_v3 of the
+// Same arithmetic as the packed kernel (esmm_gemm_tiled.cuh) and as esmm_ab_optimized_v3 of the
 // reference (src/kernels/esmm_ab_optimized_v3.cu:157, 183-203): for every output one FMA chain in
 // ascending k over the k whose joint bit is set.  With a single row block of A the large kernel has
 // M / 128 x N / 128 = N / 128 tiles, runs half of its consumer warps on rows that do not exist and

@@ -1,4 +1,4 @@
-// Sizes and shared-memory layout of the tiled kernel (esmm_gemm_packed.cu) and of its block mode (esmm_gemm_blocks.cuh).
+// Sizes and shared-memory layout of the tiled kernel (esmm_gemm_tiled.cuh) and of its block mode (esmm_gemm_blocks.cuh).
 // Plain C++, so that the layout can be checked without a GPU.
 #pragma once
 

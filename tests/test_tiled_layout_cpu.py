@@ -77,7 +77,7 @@ def test_block_mode_rule(shim):
 def test_copies_that_signal_a_barrier_are_waited_for():
     """Row-major producers' cp.async copies signal the stage's barrier and are never committed to a group, so waiting for committed
     groups does not wait for them; a producer that leaves after a wait that ran out must wait for all of its copies."""
-    text = open(os.path.join(CSRC, "esmm_gemm_packed.cu")).read()
+    text = open(os.path.join(CSRC, "esmm_gemm_tiled.cuh")).read()
     assert "cp.async.mbarrier.arrive.noinc" in text and "cp_async_commit" not in text
     assert not re.search(r"cp_async_wait_group<", text)
     assert re.search(r"if \(RM\) cp_async_wait_all\(\);", text)
