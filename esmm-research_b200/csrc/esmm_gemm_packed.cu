@@ -30,15 +30,15 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
 // The launch shape follows the operands: the 16-warp form pays on tiles of scattered single rows and costs about
 // half a percent elsewhere, and which kind the operands are is known on the device only.  So CTA 0 of every
 // launch notes what its first tile would have wanted in a word of host-mapped memory (one per device, set up at
-// the first launch) where the word said otherwise when the host launched it (the launch's end waits for the store across PCIe: 512 x
-// 1024 x 704 32-granular 0.2 / 0.2 16.4 us with a note every time, 14.4 now), and the next launch on that device reads the word, without waiting for anything: repeated
-// products of like operands - what a benchmark loop or a layer with fixed weights issues - get the right
-// shape from the second call on, and a stale or missing note only costs that difference.  The results are
-// bit-identical in both shapes.  esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins the shape instead.  (Scattered rows
-// reach the pipeline in launches too short to look at the samples: 512 x 1024 x 704 as above 16.4 us with 12 warps.  Operands of that kind that are
-// large enough to be looked at go to block mode now, where twelve warps work in either shape and the 12-warp form is the faster
-// one or as fast; there the note is set only with no more pairs of blocks than CTAs, where both take the same time: 512 x 1024 x
-// 2048 at 0.3 / 0.3 25.3 and 24.9 us.)
+// the first launch) where the word said otherwise when the host launched it (a launch's end waits for the store across
+// PCIe: 512 x 1024 x 704, 32-granular 0.2 / 0.2, 16.4 us with a note every time, 14.4 now), and the next launch on that
+// device reads the word, without waiting for anything: repeated products of like operands - what a benchmark loop or a
+// layer with fixed weights issues - get the right shape from the second call on, and a stale or missing note only costs
+// that difference.  The results are bit-identical in both shapes.  esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins the
+// shape instead.  (Scattered rows reach the pipeline in launches too short to look at the samples.  Larger operands of that
+// kind go to block mode, where twelve warps work in either shape and the 12-warp form is the faster one or as fast; there
+// the note is set only with no more pairs of blocks than CTAs, where both take the same time: 512 x 1024 x 2048 at 0.3 / 0.3
+// 25.3 and 24.9 us.)
 static std::atomic<int> g_last_tiled_warps[64];   // per device: warps per CTA of the last launch of the tiled kernel
 
 struct FormHint {

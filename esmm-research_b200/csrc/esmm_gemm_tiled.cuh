@@ -63,8 +63,8 @@ namespace esmm {
 //     consumers raise their allowance to 160 and the two warp groups of producers / mask warp lower theirs to 96
 //     (setmaxnreg).  Each CTA's first tile decides whether all 7 copy (tiles of scattered single rows with little
 //     work per consumer warp: a stage is then posted every 0.92 us instead of 1.19) or 3 do and 4 sleep.  Measured
-//     at 4096^3 against the 12-warp form: independent 32-granular patterns at 0.2 / 0.2 0.369 -> 0.322 ms, but
-//     dense and uniform patterns 0.5 % slower.  A launch takes this form when the launch before it on the device
+//     against the 12-warp form: 512 x 1024 x 704, 32-granular patterns at 0.2 / 0.2 16.4 -> 14.4 us (larger operands of
+//     this kind take block mode), but dense and uniform patterns 0.5 % slower.  A launch takes this form when the launch before it on the device
 //     noted such tiles (see gemm_ab_packed_launch_form); esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins one.
 constexpr int P_TMA_WARP = P_CONSUMER_WARPS;                   // first producer warp
 // Block mode (esmm_gemm_blocks.cuh) where at most this many sixteenths of what the tiled pipeline would hold in shared memory are
