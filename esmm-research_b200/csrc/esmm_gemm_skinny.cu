@@ -10,26 +10,26 @@
 //     pattern block of B, so its live k are a_pat[0][kb] & b_pat[strip][kb]: every listed row is live
 //     for the whole CTA, there are no per-warp masks and no index lists in the inner loop;
 //   * all threads first build the strip's list of live k (pattern bytes read as 32-bit words); then stages of
-//     32 rows travel through a ring as 16-byte asynchronous copies (cp.async, one commit group per stage): per
-//     row 128 bytes of B and 128 bytes of packed A (rows 0-31 of the first panel), or only 64 bytes of A (rows
-//     0-15) when M <= 16 - the 16-row variant moves and multiplies half as much of A;
-//   * four warps, one per SM sub-partition, hold ROWS rows x 8 columns each, (ROWS / 8) rows x 2 columns per
-//     thread, as 2 x 2 blocks of two-wide FMAs (fma.rn.f32x2) like the packed kernel.  The operands of four rows
-//     are loaded (volatile, so that they stay put) one batch ahead of the multiply-adds that use them, two
-//     register sets in ping-pong: without that the compiler sank every load to its first use and a row cost a
-//     shared-memory round trip (36 cycles per row and warp measured; 26 with the batches).
+//     64 k travel through a ring of four as 16-byte asynchronous copies: per k 128 bytes of B and 32, 64 or 128 bytes of
+//     packed A (rows 0-7, 0-15 or 0-31 of the first panel: as many as M needs);
+//   * two warps copy, a stage each in turn, two or four multiply.  A stage's barrier takes an arrival of every copying lane when its
+//     copies have landed (cp.async.mbarrier.arrive.noinc); the multiplying warps hand the slot back.  No warp does both: copies in the
+//     multiplying warps' own instruction stream, with a barrier of the whole CTA per 32 k, were what the kernel before spent most
+//     of its time on (the call below: FMA pipe 22 % active);
+//   * a multiplying thread holds 4 x 4, 4 x 2 or 2 x 2 outputs as row pairs times one broadcast column.  The operands of four k
+//     are loaded (volatile, so that they stay put) one batch ahead of the multiply-adds that use them, two register sets in
+//     ping-pong, over the stages' borders too;
+//   * co-resident strips start their roles at different warps (by %warpid), so that the multiplying warps of an SM's two or three strips
+//     lie on different SM sub-partitions: with every strip's on the same one the call below takes 39 us.
 //
-// Measured on M = 16, N = 11008, K = 4096 (819 live k per strip, 344 CTAs on 148 SMs), kernel alone, back to back:
-// 24.8 us (35.5 us before the 16-row variant and the batched loads; tiled kernel 49 us; cuBLAS 110 us).  What is
-// left: an SM holds 2 or 3 strips, i.e. 8-12 warps, and every asynchronous-copy or shared-load instruction costs its
-// warp tens of cycles of issue whatever its width (a warp-wide 16-byte cp.async: about 26 cycles, measured), so the
-// row rate is set by the number of such instructions, not by bytes.  Variants measured and dropped: a tensor-copy
-// producer warp with two computing warps, a cp.async producer warp with four, one warp per strip with 8 x 4 outputs per
-// thread (33-45 us, before batching); two warps per strip, 16 columns and (ROWS / 8) x 4 outputs per thread each, with
-// private rings and no barrier in the main loop (28.2 us at M = 16, 49.3 us at M = 32: twice the copy instructions per
-// warp) or on one shared ring (28.9 / 37.4 us).
-// The only waits are cp.async.wait_group and __syncthreads with a trip count common to all threads: no flag or
-// barrier that another agent has to signal, nothing that can wait forever.
+// What bounds it: a multiplying warp is alone on its SM sub-partition, so its loads' issue and its multiply-adds add up: 13 cycles a k for
+// 4 x 2 outputs (8 of multiply-adds) with no copies and no barriers at all, 15 with them; on SMs with three strips shared memory (7.5 of
+// its wavefronts per strip and k).  Measured, whole calls, the kernel before -> this one: M = 16, N = 11008, K = 4096 pruned MLP (819 live k
+// per strip, 344 strips) 28.5 -> 22.5 us; M = 8 28.4 -> 16.4; M = 1 19.4 -> 12.7; M = 32 34.1 -> 29.0; dense, N = 4096, K = 4096,
+// M = 16 61.5 -> 36.2; dense, N = 11008, M = 1 100.5 -> 50.5; N = 512, K = 16384, M = 6 148 -> 72.  Also measured (same inputs as the
+// first): stages of 32 k 10-20 % slower, of 128 in a ring of two as fast, k of a batch 2 or 8 and three batches ahead as fast, 4 x 4 outputs
+// by one multiplying warp 39 us, counters in shared memory with release / acquire instead of barriers 3-5 % slower.
+// Every wait is bounded: a wait that runs out raises the abort flag, nothing is stored and the status word tells.
 #include <cstring>
 
 #include "esmm_gemm_shared.cuh"
@@ -38,25 +38,12 @@ namespace esmm {
 
 constexpr int SK_COLS = 32;                     // columns of a strip = one B pattern block
 constexpr int SK_ROWS = 32;                     // rows of C handled (M <= 32)
-constexpr int SK_STAGE_ROWS = 32;               // k per stage
-constexpr int SK_ROW_BYTES = 128;               // one k of either operand in shared memory
-constexpr int SK_STAGES = 6;
-constexpr int SK_WARPS = 4;                      // one per SM sub-partition
-constexpr int SK_THREADS = SK_WARPS * 32;
+constexpr int SK_STAGE_ROWS = 64;               // k per stage
+constexpr int SK_ROW_BYTES = 128;               // one k of B in shared memory
+constexpr int SK_STAGES = 4;                    // (a power of two)
 constexpr int SK_MAX_KP = 16384;                // longest K the row list is sized for
-
-// Optional timeline for tuning (build with -DESMM_TRACE), as in the packed kernel.
-#ifdef ESMM_TRACE
-__device__ unsigned long long g_sk_trace[1024];
-#define SK_STAMP(idx)                                                                                \
-    do {                                                                                             \
-        if (blockIdx.x == 0 && (threadIdx.x & 31) == 0 && (idx) < 1024) g_sk_trace[(idx)] = global_timer_ns();     \
-    } while (0)
-#else
-#define SK_STAMP(idx) \
-    do {              \
-    } while (0)
-#endif
+constexpr int SK_BATCH = 4;                     // k per register set of operands
+constexpr int SK_SETS = 2;                      // register sets
 
 struct SkinnyParams {
     int M, N, K, nKB, kp, cap;
@@ -78,32 +65,60 @@ __device__ __forceinline__ int sk_scan(int v, int lane)
     return v;
 }
 
-// ROWS = 32: rows 0-31 of the first panel (any M <= 32).  ROWS = 16 (M <= 16): only rows 0-15 are fetched and
-// multiplied - half the shared-memory traffic of A and half the multiply-adds.
-template <int ROWS>
-__global__ void __launch_bounds__(SK_THREADS)
+// (one group of copies per stage and lane)
+__device__ __forceinline__ void sk_copies_arrive(uint32_t bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool on)
+{
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %1, 0;\n@p mbarrier.arrive.shared::cta.b64 _, [%0];\n}" ::"r"(bar), "r"((int)on) : "memory");
+}
+
+// Shared memory: ring | list (u16 x cap) | warp sums | full and empty barriers, abort flag
+__host__ __device__ constexpr int sk_stage_bytes(int rows) { return SK_STAGE_ROWS * (rows * 4 + SK_ROW_BYTES); }
+__host__ __device__ constexpr size_t sk_list_off(int rows) { return (size_t)SK_STAGES * sk_stage_bytes(rows); }
+__host__ __device__ constexpr size_t sk_sum_off(int rows, int cap) { return sk_list_off(rows) + (((size_t)cap * 2 + 15) & ~(size_t)15); }
+__host__ __device__ constexpr size_t sk_bar_off(int rows, int cap) { return sk_sum_off(rows, cap) + 32; }
+__host__ __device__ constexpr size_t sk_smem(int rows, int cap) { return sk_bar_off(rows, cap) + 2 * SK_STAGES * 8 + 16; }
+
+// ROWS: rows of C that are fetched and multiplied, 8, 16 or 32.  CW: warps that multiply, PW: warps that copy.  RT: rows per thread.
+template <int ROWS, int CW, int PW, int RT>
+__global__ void __launch_bounds__((CW + PW) * 32)
 esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
 {
     constexpr int A_ROW_BYTES = ROWS * 4;                           // one k of A in shared memory
-    constexpr int A_CHUNKS = A_ROW_BYTES / 16;                      // 16-byte pieces per A row
     constexpr int A_HALF = SK_STAGE_ROWS * A_ROW_BYTES;             // A rows, then B rows
-    constexpr int STAGE_BYTES = A_HALF + SK_STAGE_ROWS * SK_ROW_BYTES;
-    constexpr int BATCH = 4;                                        // rows per register set of operands
+    constexpr int STAGE_BYTES = sk_stage_bytes(ROWS);
+    constexpr int SK_WARPS = CW + PW, SK_THREADS = SK_WARPS * 32;
+    static_assert(SK_WARPS < 8, "warp sums");
     extern __shared__ __align__(1024) char smem[];
-    // layout: ring | krow (u16 x cap) | warp sums
-    uint16_t *krow = reinterpret_cast<uint16_t *>(smem + SK_STAGES * STAGE_BYTES);
-    volatile int *wsum = reinterpret_cast<volatile int *>(smem + SK_STAGES * STAGE_BYTES + ((p.cap * 2 + 15) & ~15));
+    uint16_t *krow = reinterpret_cast<uint16_t *>(smem + sk_list_off(ROWS));
+    volatile int *wsum = reinterpret_cast<volatile int *>(smem + sk_sum_off(ROWS, p.cap));
+    const uint32_t full0 = smem_u32(smem + sk_bar_off(ROWS, p.cap)), empty0 = full0 + SK_STAGES * 8;
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + sk_bar_off(ROWS, p.cap) + 2 * SK_STAGES * 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int strip = blockIdx.x;
-    SK_STAMP(0);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SK_STAGES; ++s) {
+            mbar_init(full0 + 8 * s, 32);         // a copying warp's lanes, when their copies have landed
+            mbar_init(empty0 + 8 * s, CW);
+        }
+        *abort_flag = 0;
+        unsigned place;                           // of the CTA among those on its SM
+        asm volatile("mov.u32 %0, %%warpid;" : "=r"(place));
+        wsum[SK_WARPS] = (int)place / SK_WARPS;
+    }
     grid_dependency_wait();   // (the A patterns and the packed copy come from the kernel before this one)
 
+    int n = 0;
     // ---------------- the strip's list of live k ----------------
     // Thread t owns the K blocks t * per .. t * per + per - 1 (consecutive threads, ascending k; per a multiple
     // of 4 so that a thread's pattern bytes are whole 32-bit words where the arrays allow): count, prefix over
     // the CTA, write.
     {
-        constexpr int MAX_WORDS = SK_MAX_KP / BK / SK_THREADS / 4;   // 4 words of 4 K blocks per thread at most
+        constexpr int MAX_WORDS = ((SK_MAX_KP / BK + SK_THREADS - 1) / SK_THREADS + 3) / 4;   // 4 words of 4 K blocks per thread at most
         const uint8_t *bp = p.b_pat + (size_t)strip * p.nKB;
         const int per = ((p.nKB + SK_THREADS - 1) / SK_THREADS + 3) & ~3;
         const int kb_lo = min((int)threadIdx.x * per, p.nKB), kb_hi = min(kb_lo + per, p.nKB);
@@ -128,147 +143,198 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
         if (lane == 31) wsum[warp] = incl;
         __syncthreads();
         int q = incl - c;
-        for (int w = 0; w < warp; ++w) q += wsum[w];
+#pragma unroll
+        for (int w = 0; w < SK_WARPS; ++w) {
+            if (w < warp) q += wsum[w];
+            n += wsum[w];
+        }
 #pragma unroll
         for (int w = 0; w < MAX_WORDS; ++w) {
             unsigned v = live[w];
-            while (v) {
-                const int bit = __ffs((int)v) - 1;                   // bit 8 j + kk: K block kb_lo + 4 w + j, offset kk
-                if (bounds_ok(q < p.cap, p.status, 30)) krow[q] = (uint16_t)((kb_lo + 4 * w) * BK + bit);   // checked build: site 30
+            int e = q + __popc(v);
+            const int k0 = (kb_lo + 4 * w) * BK, qn = e;
+            while (v) {                                              // from both ends of the word
+                const int lo = __ffs((int)v) - 1, hi = 31 - __clz((int)v);   // bit 8 j + kk: K block kb_lo + 4 w + j, offset kk
+                --e;
+                if (bounds_ok(q < p.cap, p.status, 30)) krow[q] = (uint16_t)(k0 + lo);   // checked build: site 30
+                if (bounds_ok(e < p.cap, p.status, 30)) krow[e] = (uint16_t)(k0 + hi);
                 ++q;
-                v &= v - 1u;
+                v &= ~((1u << lo) | (1u << hi));
             }
+            q = qn;
         }
+        // (the rest of the last stage: copied like the others, never multiplied)
+        for (int pad = n + (int)threadIdx.x; pad < ((n + SK_STAGE_ROWS - 1) & ~(SK_STAGE_ROWS - 1)); pad += SK_THREADS)
+            if (bounds_ok(pad < p.cap, p.status, 30)) krow[pad] = 0;
         __syncthreads();
     }
-    int n = 0;
-#pragma unroll
-    for (int w = 0; w < SK_WARPS; ++w) n += wsum[w];
     const int num_stages = (n + SK_STAGE_ROWS - 1) / SK_STAGE_ROWS;
-    SK_STAMP(1);
+    const int col0 = strip * SK_COLS;
+    // the warps' roles: strips that share an SM have their multiplying warps on different SM sub-partitions
+    const int role = (warp + wsum[SK_WARPS] * CW) % SK_WARPS;
+    bool ok = true;
 
-    // ---------------- copies: every thread moves up to 4 of a stage's sixteen-byte pieces ----------------
-    // (Rows of 128 bytes are too short for the tensor copy engine, which spends about as long on a row of
-    // 128 bytes as on one of 512: measured, one row per ~17 cycles per SM.)
-    const int col0 = strip * SK_COLS, chunk = threadIdx.x & 7, sub = threadIdx.x >> 3;   // sub: 0 .. 15
-    const bool col_ok = col0 + chunk * 4 < p.N;
-    auto issue = [&](int stage) {
-        if (stage < num_stages) {
-            const int r0 = stage * SK_STAGE_ROWS, cnt = min(SK_STAGE_ROWS, n - r0);
-            const uint32_t s0 = smem_u32(smem) + (uint32_t)(stage % SK_STAGES) * STAGE_BYTES + (uint32_t)chunk * 16;
+    if (role >= CW) {
+        // ---------------- copies: a warp takes every PW-th stage ----------------
+        // 32 rows at a time.  B: 8 lanes per row, 4 rows an instruction, rows 8 apart, so that a lane's 8 list entries are one load;
+        // A likewise.  (Rows of 128 bytes are too short for the tensor copy engine: about 57 cycles of issue per copy and warp.)
+        constexpr int A_LANES = ROWS / 4, A_N = A_LANES;            // lanes per row of A; instructions per 32 rows
+        const int b_row = (lane >> 3) * 8, b_chunk = lane & 7;
+        const int a_row = lane / A_LANES * A_N, a_chunk = lane % A_LANES;
+        const bool col_ok = col0 + b_chunk * 4 < p.N;
+        const char *b_src = reinterpret_cast<const char *>(col_ok ? p.B + col0 + b_chunk * 4 : p.B);
+        const char *a_src = reinterpret_cast<const char *>(p.a_packed + a_chunk * 4);
+        const unsigned n4 = col_ok ? (unsigned)p.N * 4u : 0u;
+        const uint32_t dst_a = smem_u32(smem) + (uint32_t)(a_row * A_ROW_BYTES + a_chunk * 16);
+        const uint32_t dst_b = smem_u32(smem) + (uint32_t)(A_HALF + b_row * SK_ROW_BYTES + b_chunk * 16);
+        for (int s = role - CW; s < num_stages; s += PW) {
+            const int slot = s & (SK_STAGES - 1);
+            if (!bounds_ok((s + 1) * SK_STAGE_ROWS <= p.cap, p.status, 31)) break;
+            ok = mbar_wait(empty0 + 8 * slot, ((s / SK_STAGES) & 1) ^ 1, abort_flag);
+            if (!ok) break;
 #pragma unroll
-            for (int i = 0; i < SK_STAGE_ROWS / 16; ++i) {
-                const int r = i * 16 + sub;
-                if (r < cnt && bounds_ok(r0 + r < p.cap, p.status, 31)) {
-                    const int k = krow[r0 + r];
-                    if (!bounds_ok(k >= 0 && k < p.kp, p.status, 32)) continue;   // site 32: a k outside the packed panel / B
-                    if (chunk < A_CHUNKS)
-                        cp_async_16(s0 + r * A_ROW_BYTES, p.a_packed + (size_t)k * TILE_M + chunk * 4, 16);
-                    const bool b_ok = col_ok && k < p.K;   // outside B: zero fill
-                    cp_async_16(s0 + A_HALF + r * SK_ROW_BYTES, b_ok ? p.B + (size_t)k * p.N + col0 + chunk * 4 : p.B,
-                                b_ok ? 16 : 0);
+            for (int h = 0; h < SK_STAGE_ROWS / 32; ++h) {
+                const uint32_t s_off = (uint32_t)slot * STAGE_BYTES;
+                const uint16_t *list = krow + s * SK_STAGE_ROWS + h * 32;
+                const uint4 bk = *reinterpret_cast<const uint4 *>(list + b_row);
+                unsigned ka[8];
+                const unsigned kb[8] = {bk.x & 0xFFFFu, bk.x >> 16, bk.y & 0xFFFFu, bk.y >> 16, bk.z & 0xFFFFu, bk.z >> 16, bk.w & 0xFFFFu, bk.w >> 16};
+                if (A_N == 8) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) ka[j] = kb[j];
+                } else if (A_N == 4) {
+                    const uint2 v = *reinterpret_cast<const uint2 *>(list + a_row);
+                    ka[0] = v.x & 0xFFFFu, ka[1] = v.x >> 16, ka[2] = v.y & 0xFFFFu, ka[3] = v.y >> 16;
+                } else {
+                    const unsigned v = *reinterpret_cast<const unsigned *>(list + a_row);
+                    ka[0] = v & 0xFFFFu, ka[1] = v >> 16;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (!bounds_ok(kb[j] < (unsigned)p.kp, p.status, 32)) continue;   // site 32: a k outside the packed panel / B
+                    const bool in = kb[j] < (unsigned)p.K;                            // past B's last row: zeros
+                    cp_async_16(dst_b + s_off + (h * 32 + j) * SK_ROW_BYTES, b_src + (size_t)(in ? kb[j] : 0u) * n4, in ? 16 : 0);
+                }
+#pragma unroll
+                for (int j = 0; j < A_N; ++j) {
+                    if (!bounds_ok(ka[j] < (unsigned)p.kp, p.status, 32)) continue;
+                    cp_async_16(dst_a + s_off + (h * 32 + j) * A_ROW_BYTES, a_src + (size_t)ka[j] * (TILE_M * 4), 16);
+                }
+            }
+            sk_copies_arrive(full0 + 8 * slot);
+        }
+        cp_async_wait_all();      // nothing of this thread is in flight when it leaves
+    } else {
+        // ---------------- multiplying warps: WROWS rows x WCOLS columns each, 4 rows x CT columns per thread ----------------
+        constexpr int WROWS = ROWS < 16 ? ROWS : 16, ROW_SPLIT = ROWS / WROWS, WCOLS = SK_COLS * ROW_SPLIT / CW;
+        constexpr int RG = WROWS / RT, CG = 32 / RG, CT = WCOLS / CG;     // groups of lanes on the rows, on the columns
+        static_assert(CT == 2 || CT == 4, "columns per thread");
+        static_assert(RT == 2 || RT == 4, "rows per thread");
+        // every 4 consecutive lanes touch 2 row groups x 2 column groups (few distinct bytes per load)
+        const int rg = RG == 4 ? ((lane >> 1) & 1) | ((lane >> 4) << 1) : ((lane >> 1) & 1) | ((lane >> 3) << 1);
+        const int cg = RG == 4 ? (lane & 1) | (((lane >> 2) & 3) << 1) : (lane & 1) | (((lane >> 2) & 1) << 1);
+        static_assert(RG == 4 || RG == 8, "lanes");
+        const int row0 = (role % ROW_SPLIT) * WROWS + rg * RT, colw = (role / ROW_SPLIT) * WCOLS + cg * CT;
+        const uint32_t tA = smem_u32(smem) + row0 * 4, tB = smem_u32(smem) + A_HALF + colw * 4;
+        // c[pr][j] = rows 2 pr, 2 pr + 1 of column j
+        float2 c[RT / 2][CT];
+#pragma unroll
+        for (int i = 0; i < RT / 2; ++i)
+#pragma unroll
+            for (int j = 0; j < CT; ++j) c[i][j] = make_float2(0.0f, 0.0f);
+
+        // Operands of SK_BATCH consecutive k of a stage.  The next batch is loaded before the current one is multiplied (two
+        // register sets, ping-pong), across the stages' borders too, so that a load has a whole batch of multiply-adds to land
+        // under; the loads are volatile so that they stay where they are written.
+        struct Ops {
+            float2 a[SK_BATCH][RT / 2];
+            float b[SK_BATCH][CT];
+        };
+        auto load_rows = [&](Ops &o, uint32_t s_off, int r) {
+#pragma unroll
+            for (int i = 0; i < SK_BATCH; ++i) {
+                const uint32_t pa = tA + s_off + (uint32_t)((r + i) * A_ROW_BYTES), pb = tB + s_off + (uint32_t)((r + i) * SK_ROW_BYTES);
+                if constexpr (RT == 4)
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(o.a[i][0].x), "=f"(o.a[i][0].y), "=f"(o.a[i][RT / 2 - 1].x), "=f"(o.a[i][RT / 2 - 1].y) : "r"(pa));
+                else
+                    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(o.a[i][0].x), "=f"(o.a[i][0].y) : "r"(pa));
+                if constexpr (CT == 4)
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(o.b[i][0]), "=f"(o.b[i][1]), "=f"(o.b[i][2]), "=f"(o.b[i][3]) : "r"(pb));
+                else
+                    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(o.b[i][0]), "=f"(o.b[i][1]) : "r"(pb));
+            }
+        };
+        auto fma_rows = [&](const Ops &o, int count) {
+#pragma unroll
+            for (int i = 0; i < SK_BATCH; ++i)
+                if (i < count) {
+#pragma unroll
+                    for (int pr = 0; pr < RT / 2; ++pr)
+#pragma unroll
+                        for (int j = 0; j < CT; ++j) c[pr][j] = __ffma2_rn(o.a[i][pr], make_float2(o.b[i][j], o.b[i][j]), c[pr][j]);
+                }
+        };
+
+        constexpr int BATCHES = SK_STAGE_ROWS / SK_BATCH, AHEAD = SK_SETS - 1;
+        static_assert(BATCHES % SK_SETS == 0, "a stage's first batch is in set 0");
+        Ops o[SK_SETS];
+        if (num_stages > 0) {
+            ok = mbar_wait(full0, 0, abort_flag);
+            if (ok) {
+#pragma unroll
+                for (int b = 0; b < AHEAD; ++b) load_rows(o[b], 0, b * SK_BATCH);
+            }
+        }
+        // (after a wait that ran out the sums are worthless and not stored; the loop goes on, as the waits no longer do)
+        for (int s = 0; s < num_stages; ++s) {
+            const int slot = s & (SK_STAGES - 1), cnt = n - s * SK_STAGE_ROWS;
+            const uint32_t s_off = (uint32_t)slot * STAGE_BYTES;
+            if (cnt > SK_STAGE_ROWS) {
+                const int next = (s + 1) & (SK_STAGES - 1);
+                const uint32_t next_bar = full0 + 8 * next, next_phase = ((s + 1) / SK_STAGES) & 1;
+                bool ready = false;
+#pragma unroll
+                for (int b = 0; b < BATCHES; ++b) {
+                    if (b + AHEAD < BATCHES) {
+                        load_rows(o[(b + AHEAD) % SK_SETS], s_off, (b + AHEAD) * SK_BATCH);
+                    } else {
+                        if (b + AHEAD == BATCHES && !ready) ok = ok && mbar_wait(next_bar, next_phase, abort_flag);
+                        load_rows(o[(b + AHEAD) % SK_SETS], (uint32_t)next * STAGE_BYTES, (b + AHEAD - BATCHES) * SK_BATCH);
+                    }
+                    if (b == BATCHES - 4) ready = mbar_test_wait(next_bar, next_phase);   // (its answer comes under the multiply-adds)
+                    fma_rows(o[b % SK_SETS], SK_BATCH);
+                }
+                __syncwarp();
+                mbar_arrive_if(empty0 + 8 * slot, lane == 0);
+            } else {
+                // the last stage (batches loaded past its last row are in bounds and never multiplied)
+#pragma unroll
+                for (int b = 0; b < BATCHES; ++b) {
+                    if (b * SK_BATCH >= cnt) break;
+                    if (b + AHEAD < BATCHES) load_rows(o[(b + AHEAD) % SK_SETS], s_off, (b + AHEAD) * SK_BATCH);
+                    fma_rows(o[b % SK_SETS], cnt - b * SK_BATCH);
                 }
             }
         }
-        cp_async_commit();   // one group per stage, empty past the end: the wait below counts groups
-    };
-
-    // ---------------- per warp ROWS rows x 8 columns; per thread (ROWS / 8) rows x 2 columns ----------------
-    // every 4 consecutive lanes touch 2 row groups x 2 column pairs (few distinct bytes per load)
-    const int rg = ((lane >> 1) & 3) | ((lane >> 4) << 2);       // group of ROWS / 8 consecutive rows
-    const int cp = (lane & 1) | (((lane >> 3) & 1) << 1);        // pair of columns within the warp's 8
-    const uint32_t tA = smem_u32(smem) + rg * (ROWS / 2);
-    const uint32_t tB = smem_u32(smem) + A_HALF + warp * 32 + cp * 8;
-    // rows 2p, 2p+1 x the column pair: diag[p] = (c[2p][0], c[2p+1][1]), anti[p] = (c[2p][1], c[2p+1][0])
-    constexpr int RP = ROWS / 16;                                 // row pairs per thread
-    float2 diag[RP], anti[RP];
+        // C is overwritten (beta = 0)
+        const int col = col0 + colw;
 #pragma unroll
-    for (int i = 0; i < RP; ++i) diag[i] = anti[i] = make_float2(0.0f, 0.0f);
-
-    // Operands of BATCH consecutive rows of a stage.  The loop below loads the next batch before it multiplies
-    // the current one (two register sets, ping-pong), so that a load has a whole batch of multiply-adds to land
-    // under; the loads are volatile so that they stay where they are written.
-    struct Ops {
-        float2 a[BATCH][RP], b[BATCH];
-    };
-    auto load_rows = [&](Ops &o, uint32_t sA, uint32_t sB, int r) {
+        for (int e = 0; e < RT; ++e) {
+            const int r = row0 + e;
+            float v[CT];
 #pragma unroll
-        for (int i = 0; i < BATCH; ++i) {
-            const uint32_t pa = sA + (uint32_t)((r + i) * A_ROW_BYTES), pb = sB + (uint32_t)((r + i) * SK_ROW_BYTES);
-            if (RP == 2)
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                             : "=f"(o.a[i][0].x), "=f"(o.a[i][0].y), "=f"(o.a[i][RP - 1].x), "=f"(o.a[i][RP - 1].y) : "r"(pa));
-            else
-                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(o.a[i][0].x), "=f"(o.a[i][0].y) : "r"(pa));
-            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(o.b[i].x), "=f"(o.b[i].y) : "r"(pb));
-        }
-    };
-    auto fma_rows = [&](const Ops &o, int count) {
-#pragma unroll
-        for (int i = 0; i < BATCH; ++i) {
-            if (i < count) {
-                const float2 bs = make_float2(o.b[i].y, o.b[i].x);
-#pragma unroll
-                for (int pr = 0; pr < RP; ++pr) {
-                    diag[pr] = __ffma2_rn(o.a[i][pr], o.b[i], diag[pr]);
-                    anti[pr] = __ffma2_rn(o.a[i][pr], bs, anti[pr]);
-                }
+            for (int j = 0; j < CT; ++j) v[j] = (e & 1) ? c[e >> 1][j].y : c[e >> 1][j].x;
+            if (ok && r < p.M && col < p.N && bounds_ok((size_t)r * p.N + col + CT <= (size_t)p.M * p.N, p.status, 33)) {
+                float *dst = p.C + (size_t)r * p.N + col;
+                if constexpr (CT == 4) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+                else *reinterpret_cast<float2 *>(dst) = make_float2(v[0], v[1]);
             }
         }
-    };
-
-#pragma unroll
-    for (int s = 0; s < SK_STAGES - 1; ++s) issue(s);
-    for (int s = 0; s < num_stages; ++s) {
-        cp_async_wait_group<SK_STAGES - 2>();   // this thread's pieces of stage s have landed ...
-        __syncthreads();                        // ... everybody's have, and stage s - 1 has been read by all
-        issue(s + SK_STAGES - 1);               // into the slot of stage s - 1
-        if (warp == 0) SK_STAMP(10 + s);
-        const int cnt = min(SK_STAGE_ROWS, n - s * SK_STAGE_ROWS);
-        const uint32_t sA = tA + (uint32_t)(s % SK_STAGES) * STAGE_BYTES;
-        const uint32_t sB = tB + (uint32_t)(s % SK_STAGES) * STAGE_BYTES;
-        // (a batch loaded past the stage's last row reads the next slot or the row list: in bounds, never multiplied)
-        Ops x, y;
-        load_rows(x, sA, sB, 0);
-        if (cnt == SK_STAGE_ROWS) {
-#pragma unroll 1
-            for (int r = 0; r < SK_STAGE_ROWS; r += 2 * BATCH) {
-                load_rows(y, sA, sB, r + BATCH);
-                fma_rows(x, BATCH);
-                load_rows(x, sA, sB, r + 2 * BATCH);
-                fma_rows(y, BATCH);
-            }
-        } else {
-#pragma unroll 1
-            for (int r = 0; r < cnt; r += BATCH) {
-                fma_rows(x, min(BATCH, cnt - r));
-                load_rows(x, sA, sB, r + BATCH);
-            }
-        }
-        if (warp == 0) SK_STAMP(200 + s);
     }
-    cp_async_wait_group<0>();   // nothing of this thread is in flight when it leaves
-    SK_STAMP(5);
-
-    // C is overwritten (beta = 0); un-scramble the 2 x 2 blocks into rows
-    const int col = strip * SK_COLS + warp * 8 + cp * 2;
-#pragma unroll
-    for (int pr = 0; pr < RP; ++pr)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int r = rg * (ROWS / 8) + 2 * pr + e;
-            const float2 v = e == 0 ? make_float2(diag[pr].x, anti[pr].x) : make_float2(anti[pr].y, diag[pr].y);
-            if (r < p.M && col < p.N && bounds_ok((size_t)r * p.N + col + 2 <= (size_t)p.M * p.N, p.status, 33))
-                *reinterpret_cast<float2 *>(p.C + (size_t)r * p.N + col) = v;
-        }
+    if (!ok && lane == 0) atomicExch(p.status, (int)ESMM_ERR_TIMEOUT);
 }
-
-#ifdef ESMM_TRACE
-extern "C" int esmm_sk_trace_read(unsigned long long *host, int n)
-{
-    return (int)cudaMemcpyFromSymbol(host, g_sk_trace, sizeof(unsigned long long) * (n < 1024 ? n : 1024));
-}
-#endif
 
 // Whether the few-rows kernel takes a problem (otherwise the packed kernel does).
 bool gemm_ab_skinny_applies(int M, int N, int K)
@@ -287,7 +353,7 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
     p.K = K;
     p.nKB = ceil_div(K, BK);
     p.kp = p.nKB * BK;
-    p.cap = p.kp + 32;
+    p.cap = p.kp + SK_STAGE_ROWS;
     p.a_pat = d_a_pat;
     p.b_pat = d_b_pat;
     p.a_packed = d_a_packed;
@@ -295,21 +361,26 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
     p.C = d_C;
     p.status = device_status_ptr();
     if (!p.status) return ESMM_ERR_CUDA;
-    const bool rows16 = M <= 16 && tuning_get("SKINNY_ROWS", 0) != 32;
-    // ring, row list, one int per warp
-    const size_t stage_bytes = (size_t)SK_STAGE_ROWS * ((rows16 ? 16 : 32) * 4 + SK_ROW_BYTES);
-    const size_t smem = (size_t)SK_STAGES * stage_bytes + ((p.cap * 2 + 15) & ~15) + (SK_WARPS * 4 + 15) / 16 * 16;
-    if (rows16) {
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_skinny_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
-        ESMM_CUDA_TRY(launch_dependent(esmm_joint_sgemm_skinny_kernel<16>, dim3(ceil_div(N, SK_COLS)), dim3(SK_THREADS), smem, stream, p));
-    } else {
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_joint_sgemm_skinny_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
-        ESMM_CUDA_TRY(launch_dependent(esmm_joint_sgemm_skinny_kernel<32>, dim3(ceil_div(N, SK_COLS)), dim3(SK_THREADS), smem, stream, p));
-    }
-    ESMM_CUDA_TRY(cudaGetLastError());
-    return ESMM_OK;
+    int dev = 0, sms = 0;
+    ESMM_CUDA_TRY(cudaGetDevice(&dev));
+    ESMM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int strips = ceil_div(N, SK_COLS), forced = tuning_get("SKINNY_ROWS", 0);
+    const int rows = M > 16 || forced == 32 ? 32 : M > 8 || forced == 16 ? 16 : 8;
+    auto launch = [&](auto kernel, int r, int warps) -> int {
+        const size_t smem = sk_smem(r, p.cap);
+        ESMM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ESMM_CUDA_TRY(launch_dependent(kernel, dim3(strips), dim3(warps * 32), smem, stream, p));
+        ESMM_CUDA_TRY(cudaGetLastError());
+        return ESMM_OK;
+    };
+    // Four multiplying warps where an SM has one or two strips; with three, shared memory bounds the kernel and two warps, which
+    // load less of A, are faster.  The multiplying part alone, us, two / four warps, K = 4096: M = 16 dense, one strip per SM 31.1 / 28.6;
+    // M = 16 pruned MLP, SMs with two strips 9.2 / 8.6, with three 9.9 / 11.6; M = 32 one strip 10.3 / 7.6, two 14.2 / 11.7, three 14.9 / 16.2.
+    const bool spread = strips <= 2 * sms;
+    if (rows == 8) return launch(esmm_joint_sgemm_skinny_kernel<8, 2, 2, 2>, 8, 4);
+    if (rows == 16)
+        return spread ? launch(esmm_joint_sgemm_skinny_kernel<16, 4, 2, 2>, 16, 6) : launch(esmm_joint_sgemm_skinny_kernel<16, 2, 2, 4>, 16, 4);
+    return spread ? launch(esmm_joint_sgemm_skinny_kernel<32, 4, 2, 4>, 32, 6) : launch(esmm_joint_sgemm_skinny_kernel<32, 2, 2, 4>, 32, 4);
 }
 
 }  // namespace esmm

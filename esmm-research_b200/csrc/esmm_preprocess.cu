@@ -366,8 +366,20 @@ int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, flo
         long blocks = (tasks + PACK_WARPS - 1) / PACK_WARPS;
         const long cap = (long)sms * 6 * 8;
         if (blocks > cap) blocks = cap;
-        esmm_preprocess_a_pack64_kernel<<<(unsigned)blocks, PACK_WARPS * 32, smem, stream>>>(
-            d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)blocks);
+        cfg.blockDim = dim3(PACK_WARPS * 32);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        // Few rows: the strip kernel's CTAs are placed while this kernel ends, and an SM whose shared memory is carved out for less
+        // than they need takes none of them until it has (M = 16, K = 4096: 344 strips on 132 of 148 SMs).  Not for large A: with
+        // so little left of L1 4096^2 is packed more slowly (whole call at 32-granular 0.2 / 0.2 167 -> 175 us).
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[0].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+        cfg.attrs = attr;
+        cfg.numAttrs = nMB == 1 ? 1 : 0;
+        ESMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, esmm_preprocess_a_pack64_kernel, d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status));
         ESMM_CUDA_TRY(cudaGetLastError());
         return ESMM_OK;
     }

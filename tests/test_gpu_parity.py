@@ -976,3 +976,28 @@ def test_run_kernel_prefix_pattern_past_k(cuda, pkg, oracle_mod, capfd):
         want = oracle_mod.gemm_joint(A, B, np.full((M // 32, 65), byte, np.uint8), np.full((5, 65), 0xFF, np.uint8))
         assert np.array_equal(dC.cpu().numpy().view(np.uint32), want.view(np.uint32)), pat
     capfd.readouterr()
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("N", [128, 1000, 9472, 9476])
+def test_gemm_strip_kernel_variants(cuda, pkg, oracle_mod, M, N):
+    """Every variant of the strip kernel (8, 16 and 32 rows; two and four multiplying warps, the line between them at two strips per
+    SM of 148), lists around the borders of its stages of 64 k and of its ring of four, a ragged last strip and a last K block of four
+    k: the oracle's bits."""
+    for live, K in [(0, 8), (1, 12), (63, 68), (64, 64), (65, 132), (128, 260), (255, 256), (257, 1028), (640, 2048)]:
+        rng = np.random.default_rng(live + K + M + N)
+        A = rng.standard_normal((M, K), dtype=np.float32)
+        B = rng.standard_normal((K, N), dtype=np.float32)
+        keep = np.zeros(K, bool)
+        keep[rng.choice(K, live, replace=False)] = True
+        A[:, ~keep] = 0.0
+        B[::3, 32:64] = 0.0                                  # one strip with a shorter list than the others
+        dA, dB = cuda.from_numpy(A).cuda(), cuda.from_numpy(B).cuda()
+        bp = cuda.empty((-(-N // 32), -(-K // 8)), dtype=cuda.uint8, device="cuda")
+        pkg.preprocess_b(dB.data_ptr(), K, N, bp.data_ptr())
+        ws = cuda.full((pkg.sgemm_joint_workspace_bytes(M, K),), 0xFF, dtype=cuda.uint8, device="cuda")
+        C_ = cuda.full((M, N), float("nan"), device="cuda")
+        pkg.sgemm_joint(M, N, K, dA.data_ptr(), dB.data_ptr(), C_.data_ptr(), bp.data_ptr(), ws.data_ptr())
+        pkg.device_status()
+        want = oracle_mod.gemm_joint(A, B)
+        assert np.array_equal(C_.cpu().numpy().view(np.uint32), want.view(np.uint32)), (M, N, live, K)
