@@ -22,21 +22,28 @@ __device__ __forceinline__ unsigned nz4(const float4 &v)
     return nz(v.x) | (nz(v.y) << 1) | (nz(v.z) << 2) | (nz(v.w) << 3);
 }
 
-// One warp owns tile_m rows x 128 columns (16 K blocks).  Lane l reads columns 4l..4l+3 of
+// SPLIT = 1: one warp owns tile_m rows x 128 columns (16 K blocks).  Lane l reads columns 4l..4l+3 of
 // every row (one 512-byte request per row per warp), ORs the nonzero bits of its 4 columns
 // over the rows in registers, then pairs of lanes join their nibbles into a pattern byte.
+// SPLIT = PRE_WARPS: the CTA's four warps share the rows, eight in turn, and join their nibbles in shared memory.  A warp waits for
+// memory once per eight rows, and on a small A there is little else to do meanwhile: 2048^2 at tile_m 128
+// 12.4 -> 6.2 us, at 64 8.3 -> 4.6, 1024^2 at 32 6.2 -> 4.6.
 // Needs K % 4 == 0 and a 16-byte aligned A.
+constexpr int PRE_WARPS = PRE_THREADS / 32;
+
+template <int SPLIT>
 __global__ void __launch_bounds__(PRE_THREADS)
 esmm_preprocess_a_patterns_kernel(const float *__restrict__ A, int M, int K, int tile_m, int nMB,
                                   int nKB, int k_chunks, uint8_t *__restrict__ out, int *status)
 {
+    grid_launch_dependents();   // (as in the packing kernel below)
     // checked build, sites 10 (loads of A) and 11 (pattern stores)
     const size_t a_floats = (size_t)M * K, out_bytes = (size_t)nMB * nKB;
-    const int lane = threadIdx.x & 31;
-    const long warps_total = (long)gridDim.x * (PRE_THREADS / 32);
+    __shared__ uint8_t nibs[PRE_WARPS][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part = SPLIT > 1 ? warp : 0;
+    const long step = SPLIT > 1 ? gridDim.x : (long)gridDim.x * PRE_WARPS;
     const long tasks = (long)nMB * k_chunks;
-    for (long task = (long)blockIdx.x * (PRE_THREADS / 32) + (threadIdx.x >> 5); task < tasks;
-         task += warps_total) {
+    for (long task = SPLIT > 1 ? blockIdx.x : (long)blockIdx.x * PRE_WARPS + warp; task < tasks; task += step) {
         const int mb = (int)(task / k_chunks);
         const int kc = (int)(task - (long)mb * k_chunks);
         const int col = kc * 128 + lane * 4;
@@ -45,8 +52,8 @@ esmm_preprocess_a_patterns_kernel(const float *__restrict__ A, int M, int K, int
             const int row0 = mb * tile_m;
             const int rows = min(tile_m, M - row0);
             const float *src = A + (size_t)row0 * K + col;
-            int r = 0;
-            for (; r + 8 <= rows; r += 8) {
+            int r = 8 * part;
+            for (; r + 8 <= rows; r += 8 * SPLIT) {
                 float4 v[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
@@ -57,13 +64,21 @@ esmm_preprocess_a_patterns_kernel(const float *__restrict__ A, int M, int K, int
 #pragma unroll
                 for (int u = 0; u < 8; ++u) nib |= nz4(v[u]);
             }
-            for (; r < rows; ++r)
+            for (const int end = min(rows, r + 8); r < end; ++r)   // (a group of fewer than eight rows; of the warps one at most has it)
                 if (bounds_ok((size_t)(row0 + r) * K + col + 4 <= a_floats, status, 10))
                     nib |= nz4(__ldg(reinterpret_cast<const float4 *>(src + (size_t)r * K)));
         }
+        if (SPLIT > 1) {
+            nibs[warp][lane] = (uint8_t)nib;
+            __syncthreads();
+            if (warp == 0)
+#pragma unroll
+                for (int w = 1; w < PRE_WARPS; ++w) nib |= nibs[w][lane];
+            __syncthreads();
+        }
         const unsigned other = __shfl_xor_sync(0xFFFFFFFFu, nib, 1);
         const int kb = kc * 16 + (lane >> 1);
-        if (!(lane & 1) && kb < nKB && bounds_ok((size_t)mb * nKB + kb < out_bytes, status, 11))
+        if (part == 0 && !(lane & 1) && kb < nKB && bounds_ok((size_t)mb * nKB + kb < out_bytes, status, 11))
             out[(size_t)mb * nKB + kb] = (uint8_t)(nib | (other << 4));
     }
 }
@@ -327,11 +342,14 @@ int preprocess_a_launch(const float *d_A, int M, int K, int tile_m, uint8_t *d_o
         const long tasks = (long)nMB * k_chunks;
         const int sms = sm_count();
         if (sms <= 0) return record_cuda_error_text("no CUDA device");
-        long blocks = (tasks + PRE_THREADS / 32 - 1) / (PRE_THREADS / 32);
+        // Four warps to a task where a warp each would leave the GPU's 64 warps per SM unfilled: 6000^2 (8836 tasks) 27.0 -> 24.6 us,
+        // 4096^2 8.3 either way.
+        const bool split = tile_m >= 8 * PRE_WARPS && tasks < (long)sms * 64;
+        long blocks = split ? tasks : (tasks + PRE_WARPS - 1) / PRE_WARPS;
         const long cap = (long)sms * 16 * 4;
         if (blocks > cap) blocks = cap;
-        esmm_preprocess_a_patterns_kernel<<<(unsigned)blocks, PRE_THREADS, 0, stream>>>(
-            d_A, M, K, tile_m, nMB, nKB, k_chunks, d_out, status);
+        const auto kernel = split ? esmm_preprocess_a_patterns_kernel<PRE_WARPS> : esmm_preprocess_a_patterns_kernel<1>;
+        kernel<<<(unsigned)blocks, PRE_THREADS, 0, stream>>>(d_A, M, K, tile_m, nMB, nKB, k_chunks, d_out, status);
     } else {
         const long total = (long)nMB * nKB;
         esmm_preprocess_a_patterns_generic_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(

@@ -1001,3 +1001,21 @@ def test_gemm_strip_kernel_variants(cuda, pkg, oracle_mod, M, N):
         pkg.device_status()
         want = oracle_mod.gemm_joint(A, B)
         assert np.array_equal(C_.cpu().numpy().view(np.uint32), want.view(np.uint32)), (M, N, live, K)
+
+
+@pytest.mark.parametrize("tile_m", [8, 31, 32, 33, 64, 96, 128])
+def test_preprocess_a_rows_shared_by_warps(cuda, pkg, oracle_mod, tile_m):
+    """A's patterns with a task's rows in one warp (tile_m below 32) and shared by four, eight in turn: blocks that end inside a group of
+    eight, a warp with no rows, a last task past K, a single nonzero in the last row of a block."""
+    for M, K in [(1, 4), (tile_m, 128), (tile_m + 1, 132), (2 * tile_m - 1, 516), (5 * tile_m + 13, 1000)]:
+        A = np.zeros((M, K), np.float32)
+        rng = np.random.default_rng(M + K)
+        A[rng.integers(0, M, 40), rng.integers(0, K, 40)] = 1.0
+        A[M - 1, K - 1] = -0.0
+        A[min(M, tile_m) - 1, 0] = 1e-45
+        dA = cuda.from_numpy(A).cuda()
+        want = oracle_mod.preprocess_a(A, tile_m)
+        out = cuda.full(want.shape, 0xEE, dtype=cuda.uint8, device="cuda")
+        pkg.preprocess_a(dA.data_ptr(), M, K, out.data_ptr(), tile_m)
+        pkg.device_status()
+        assert np.array_equal(out.cpu().numpy(), want), (M, K)
