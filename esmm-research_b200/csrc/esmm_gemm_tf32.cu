@@ -202,11 +202,12 @@ struct ZeroJob {
 };
 
 __global__ void __launch_bounds__(256)
-esmm_tf32_split_pattern_kernel(const float *__restrict__ A, int M, int K, const int *__restrict__ klist, int Kc,
+esmm_tf32_split_pattern_kernel(const float *A, int M, int K, const int *__restrict__ klist, int Kc,
                                float *__restrict__ hi, float *__restrict__ lo, uint8_t *__restrict__ a_pat,
                                const ZeroJob zj)
 {
     grid_launch_dependents();   // the product kernel may be placed as SMs become free; it waits for this grid's end itself
+    grid_dependency_wait();     // (launched as a dependent in its turn, as the packing kernel is; A through coherent loads)
     const int a_blocks = (M + 31) >> 5;
     if ((int)blockIdx.y >= a_blocks) {
         if (blockIdx.x != 0) return;
@@ -238,12 +239,12 @@ esmm_tf32_split_pattern_kernel(const float *__restrict__ A, int M, int K, const 
         if (in_cols && row < M) {
             const float *a = A + (size_t)row * K;
             if (run4) {
-                v[rr] = __ldg(reinterpret_cast<const float4 *>(a + k.x));
+                v[rr] = __ldca(reinterpret_cast<const float4 *>(a + k.x));
             } else {
-                v[rr].x = k.x >= 0 ? __ldg(a + k.x) : 0.0f;
-                v[rr].y = k.y >= 0 ? __ldg(a + k.y) : 0.0f;
-                v[rr].z = k.z >= 0 ? __ldg(a + k.z) : 0.0f;
-                v[rr].w = k.w >= 0 ? __ldg(a + k.w) : 0.0f;
+                v[rr].x = k.x >= 0 ? __ldca(a + k.x) : 0.0f;
+                v[rr].y = k.y >= 0 ? __ldca(a + k.y) : 0.0f;
+                v[rr].z = k.z >= 0 ? __ldca(a + k.z) : 0.0f;
+                v[rr].w = k.w >= 0 ? __ldca(a + k.w) : 0.0f;
             }
         }
     }
@@ -1145,8 +1146,7 @@ int esmm_sgemm_joint_tf32x3(int M, const float *d_A, const esmm_tf32x3_b *b, flo
 
     {
         dim3 grid((unsigned)ceil_div(Kc, 512), (unsigned)(ceil_div(M, 32) + 8 * zj.count));
-        esmm_tf32_split_pattern_kernel<<<grid, 256, 0, stream>>>(d_A, M, K, b->d_klist, Kc, a_hi, a_lo, a_pat, zj);
-        ESMM_CUDA_TRY(cudaGetLastError());
+        ESMM_CUDA_TRY(launch_dependent(esmm_tf32_split_pattern_kernel, grid, dim3(256), 0, stream, d_A, M, K, b->d_klist, Kc, a_hi, a_lo, a_pat, zj));
     }
     if (nb) {
         Tf32PairMaps maps;

@@ -33,10 +33,11 @@ constexpr int PRE_WARPS = PRE_THREADS / 32;
 
 template <int SPLIT>
 __global__ void __launch_bounds__(PRE_THREADS)
-esmm_preprocess_a_patterns_kernel(const float *__restrict__ A, int M, int K, int tile_m, int nMB,
+esmm_preprocess_a_patterns_kernel(const float *A, int M, int K, int tile_m, int nMB,
                                   int nKB, int k_chunks, uint8_t *__restrict__ out, int *status)
 {
-    grid_launch_dependents();   // (as in the packing kernel below)
+    grid_launch_dependents();   // (both as in the packing kernel below)
+    grid_dependency_wait();
     // checked build, sites 10 (loads of A) and 11 (pattern stores)
     const size_t a_floats = (size_t)M * K, out_bytes = (size_t)nMB * nKB;
     __shared__ uint8_t nibs[PRE_WARPS][32];
@@ -59,14 +60,14 @@ esmm_preprocess_a_patterns_kernel(const float *__restrict__ A, int M, int K, int
                 for (int u = 0; u < 8; ++u) {
                     v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (bounds_ok((size_t)(row0 + r + u) * K + col + 4 <= a_floats, status, 10))
-                        v[u] = __ldg(reinterpret_cast<const float4 *>(src + (size_t)(r + u) * K));
+                        v[u] = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)(r + u) * K));
                 }
 #pragma unroll
                 for (int u = 0; u < 8; ++u) nib |= nz4(v[u]);
             }
             for (const int end = min(rows, r + 8); r < end; ++r)   // (a group of fewer than eight rows; of the warps one at most has it)
                 if (bounds_ok((size_t)(row0 + r) * K + col + 4 <= a_floats, status, 10))
-                    nib |= nz4(__ldg(reinterpret_cast<const float4 *>(src + (size_t)r * K)));
+                    nib |= nz4(__ldcg(reinterpret_cast<const float4 *>(src + (size_t)r * K)));
         }
         if (SPLIT > 1) {
             nibs[warp][lane] = (uint8_t)nib;
@@ -166,14 +167,17 @@ esmm_preprocess_a_pack_kernel(const float *__restrict__ A, int M, int K, int nMB
 constexpr int PACK64_SMEM_PER_WARP = 64 * 32 * 4;  // 8 KB
 
 __global__ void __launch_bounds__(PACK_WARPS * 32)
-esmm_preprocess_a_pack64_kernel(const float *__restrict__ A, int M, int K, int nMB, int nKB, int k_chunks,
+esmm_preprocess_a_pack64_kernel(const float *A, int M, int K, int nMB, int nKB, int k_chunks,
                                 uint8_t *__restrict__ out, float *__restrict__ packed, int *status)
 {
     // The product kernel, launched as a dependent of this one, may be placed where SMs become free once every CTA of this
-    // grid has got here; it waits for this grid's end itself.  (This kernel is launched the ordinary way: launched as a
-    // dependent of the product kernel before it, it made a loop of calls 0.2 % slower - its early CTAs and those of the
-    // next product kernel then wait on SMs the running grid could use.)
+    // grid has got here; it waits for this grid's end itself.
     grid_launch_dependents();
+    // This kernel is a dependent launch too, of whatever was before it: it is launched as that ends rather than after, which takes 2 us off
+    // every call of a train of them (1000 x 1508 x 2012 57.4 -> 55.2 us, 1024^3 at half density 32.9 -> 30.9).  The product kernels don't
+    // call it early: strips placed beside those of the call before are 15-100 % slower.  Nothing of A is read before the wait, and what is
+    // read goes past L1, which may have been filled while A was written.
+    grid_dependency_wait();
     // checked build, sites 10 (loads of A), 11 (pattern stores), 12 (stores into the packed copy), 13 (the warp's tile)
     const size_t a_floats = (size_t)M * K, out_bytes = (size_t)nMB * nKB;
     const size_t packed_floats = (size_t)((M + 127) / 128) * nKB * BK * 128;
@@ -196,7 +200,7 @@ esmm_preprocess_a_pack64_kernel(const float *__restrict__ A, int M, int K, int n
             const int r = 2 * i + h;
             v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (col_ok && row0 + r < M && bounds_ok((size_t)(row0 + r) * K + col + 4 <= a_floats, status, 10))
-                v[i] = __ldg(reinterpret_cast<const float4 *>(src + (size_t)r * K));
+                v[i] = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)r * K));
         }
         unsigned nib = 0;
 #pragma unroll
@@ -349,7 +353,7 @@ int preprocess_a_launch(const float *d_A, int M, int K, int tile_m, uint8_t *d_o
         const long cap = (long)sms * 16 * 4;
         if (blocks > cap) blocks = cap;
         const auto kernel = split ? esmm_preprocess_a_patterns_kernel<PRE_WARPS> : esmm_preprocess_a_patterns_kernel<1>;
-        kernel<<<(unsigned)blocks, PRE_THREADS, 0, stream>>>(d_A, M, K, tile_m, nMB, nKB, k_chunks, d_out, status);
+        ESMM_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)blocks), dim3(PRE_THREADS), 0, stream, d_A, M, K, tile_m, nMB, nKB, k_chunks, d_out, status));
     } else {
         const long total = (long)nMB * nKB;
         esmm_preprocess_a_patterns_generic_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(
@@ -392,11 +396,18 @@ int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, flo
         // Few rows: the strip kernel's CTAs are placed while this kernel ends, and an SM whose shared memory is carved out for less
         // than they need takes none of them until it has (M = 16, K = 4096: 344 strips on 132 of 148 SMs).  Not for large A: with
         // so little left of L1 4096^2 is packed more slowly (whole call at 32-granular 0.2 / 0.2 167 -> 175 us).
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-        attr[0].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+        cudaLaunchAttribute attr[2];
+        int attrs = 0;
+        if (!tuning_get("NO_DEPENDENT_LAUNCH", 0)) {
+            attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+        }
+        if (nMB == 1) {
+            attr[attrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+            attr[attrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+        }
         cfg.attrs = attr;
-        cfg.numAttrs = nMB == 1 ? 1 : 0;
+        cfg.numAttrs = attrs;
         ESMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, esmm_preprocess_a_pack64_kernel, d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status));
         ESMM_CUDA_TRY(cudaGetLastError());
         return ESMM_OK;

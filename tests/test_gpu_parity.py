@@ -1019,3 +1019,74 @@ def test_preprocess_a_rows_shared_by_warps(cuda, pkg, oracle_mod, tile_m):
         pkg.preprocess_a(dA.data_ptr(), M, K, out.data_ptr(), tile_m)
         pkg.device_status()
         assert np.array_equal(out.cpu().numpy(), want), (M, K)
+
+
+@pytest.mark.parametrize("M", [16, 512])
+@pytest.mark.parametrize("captured", [False, True])
+def test_calls_wait_for_what_is_before_them(cuda, pkg, M, captured):
+    """The packing, pattern and splitting kernels are launched as dependents of whatever is before them in the stream, and read A only
+    once that is complete: trains of calls whose A a kernel or a copy has just written and whose C is read right after, on one stream
+    and after the join of two, eager and in a replayed graph, give the bits of calls that are each waited for."""
+    N, K, rounds = 768, 2048, 6
+    gen = cuda.Generator(device="cuda")
+    gen.manual_seed(7)
+    B = cuda.randn((K, N), generator=gen, device="cuda")
+    B.view(K, N // 32, 32).mul_((cuda.rand((K, N // 32, 1), generator=gen, device="cuda") < 0.5).float())
+    src = []
+    for _ in range(rounds):
+        x = cuda.randn((M, K), generator=gen, device="cuda")
+        src.append(x.mul_((cuda.rand((1, K), generator=gen, device="cuda") < 0.5).float()))
+    nkb = K // 8
+    bp = cuda.empty((N // 32, nkb), dtype=cuda.uint8, device="cuda")
+    pkg.preprocess_b(B.data_ptr(), K, N, bp.data_ptr())
+    cuda.cuda.synchronize()
+    handle = pkg.Tf32x3B(B.data_ptr(), K, N)
+    A, ap = cuda.empty((M, K), device="cuda"), cuda.empty((-(-M // 32), nkb), dtype=cuda.uint8, device="cuda")
+    ws = cuda.empty(pkg.sgemm_joint_workspace_bytes(M, K), dtype=cuda.uint8, device="cuda")
+    ws2 = cuda.empty(pkg.tf32x3_workspace_bytes(M, K), dtype=cuda.uint8, device="cuda")
+    C_ = cuda.empty((M, N), device="cuda")
+    out = [[cuda.empty((M, N), device="cuda") for _ in range(3)] for _ in range(rounds)]
+    side = cuda.cuda.Stream()
+
+    def train(wait):
+        for i in range(rounds):
+            cur = cuda.cuda.current_stream()
+            if i % 3 == 0:
+                A.copy_(src[i])                                       # a copy
+            elif i % 3 == 1:
+                cuda.mul(src[i], 1.0, out=A)                          # a kernel
+            else:                                                     # a kernel on another stream
+                side.wait_stream(cur)
+                with cuda.cuda.stream(side):
+                    cuda.mul(src[i], 1.0, out=A)
+                cur.wait_stream(side)
+            st = cur.cuda_stream
+            pkg.sgemm_joint(M, N, K, A.data_ptr(), B.data_ptr(), C_.data_ptr(), bp.data_ptr(), ws.data_ptr(), st)
+            out[i][0].copy_(C_)
+            pkg.preprocess_a(A.data_ptr(), M, K, ap.data_ptr(), 32, st)
+            pkg.gemm_ab(M, N, K, A.data_ptr(), B.data_ptr(), C_.data_ptr(), ap.data_ptr(), bp.data_ptr(), 32, st)
+            cuda.mul(C_, 1.0, out=out[i][1])
+            pkg.sgemm_joint_tf32x3(M, A.data_ptr(), handle, C_.data_ptr(), ws2.data_ptr(), st)
+            out[i][2].copy_(C_)
+            if wait:
+                cuda.cuda.synchronize()
+
+    train(True)
+    want = [[x.clone() for x in row] for row in out]
+    assert not cuda.equal(want[0][0], want[1][0])
+    run = lambda: train(False)
+    if captured:
+        graph = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(graph):
+            train(False)
+        run = graph.replay
+    for _ in range(5):
+        for row in out:
+            for x in row:
+                x.fill_(float("nan"))
+        run()
+        cuda.cuda.synchronize()
+        assert all(cuda.equal(x, w) for row, wrow in zip(out, want) for x, w in zip(row, wrow))
+    pkg.device_status()
+    if captured:
+        del graph
