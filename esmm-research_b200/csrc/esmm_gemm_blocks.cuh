@@ -19,14 +19,18 @@
 //   * the warps of a CTA draw items from a counter in shared memory; the last ones come as single blocks spread over the whole
 //     warp, so that the warps finish together (a problem with few blocks consists of nothing else).
 //
-// What bounds it: the FMA pipe (ncu, sm__pipe_fma_cycles_active of the launch: 71 % at 4096^3 64-granular 0.5 / 0.5, 58 % at 32-granular
-// 0.2 / 0.2; the pipeline on dense tiles 88 %); what is lost goes to the
-// copies, which take issue slots and shared-memory bandwidth from the same warps (without them, a probe, 12 % faster at long
-// lists, 6 % at short ones), and to the listing.  Measured, whole calls, the tiled pipeline before -> block mode: 2048 x 11008 x 4096
-// pruned MLP 1016 -> 748 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 167 and at 0.5 / 0.5 921 -> 718,
-// 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 57.4.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 / 0.5 824),
-// 8 k per stage (971), lists made for all of K before the first copy (762), rows past a list's end skipped in a second code
-// path instead of multiplied by zeros (752: the accumulators are then moved between registers at every stage).
+// What bounds it: the FMA pipe together with everything else that is issued.  A stage (16 steps) is 512 two-wide FMAs and 64 loads; where it
+// took 210 instructions more for copies, addresses and lists, a scheduler's three warps got through one in 1310 cycles each, 1113 being
+// what the FMAs need: every one of the others costs about 0.7 cycles of it, wherever it stands.  So they are kept few: one load per list
+// for a lane's entries, one instruction per address, no predicates where all of B's blocks are whole, one list for blocks that agree.
+// The rest is lost to the end of a launch (3-4 % between SMs, whose items differ, 2 % inside them).  Measured, whole calls, the tiled pipeline before ->
+// block mode: 2048 x 11008 x 4096 pruned MLP 1016 -> 724 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 164 and at
+// 0.5 / 0.5 921 -> 718, 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 50.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 /
+// 0.5 824), 8 k per stage (971), lists made for all of K before the first copy (762), rows past a list's end skipped in a second code
+// path instead of multiplied by zeros (752: the accumulators are then moved between registers at every stage); eight warps that multiply
+// and four that list and copy for them (pruned MLP 1129: a warp alone on its scheduler's spare slots takes 2000 cycles for a stage's 250
+// instructions), the copies among the multiply-adds and an item's first stage under the last of the one before (823-875: 470 M
+// instructions instead of 411 M).
 //
 // There is no barrier between warps and nothing to wait for but a warp's own copies.  Every output sees one FMA per live k, in
 // ascending k, as in the tiled pipeline: the results are the same bits.
@@ -192,13 +196,14 @@ struct LiveList {
     __device__ __forceinline__ int pending() const { return made - taken; }
 };
 
-// BM_STEP steps of a stage: 8 x 8 outputs per thread, each half-warp on its own rows of X and Y.  Odd rows hold the upper half of
-// their 128 bytes first (see the copies).
+// BM_STEP steps of a stage: 8 x 8 outputs per thread, each half-warp on its own rows of X and Y.  SWAP: odd rows hold the upper half
+// of their 128 bytes first (see the copies).
+template <bool SWAP>
 __device__ __forceinline__ void pair_steps(Acc &acc, const char *sx, const char *sy)
 {
 #pragma unroll
     for (int r = 0; r < BM_STEP; ++r) {
-        const int lo = r * 128 + (r & 1) * 64, hi = r * 128 + 64 - (r & 1) * 64;
+        const int lo = r * 128 + (SWAP ? (r & 1) * 64 : 0), hi = r * 128 + 64 - (SWAP ? (r & 1) * 64 : 0);
         KFrag f;
         f.at = *reinterpret_cast<const float4 *>(sx + lo);
         f.ab = *reinterpret_cast<const float4 *>(sx + hi);
@@ -209,7 +214,7 @@ __device__ __forceinline__ void pair_steps(Acc &acc, const char *sx, const char 
     }
 }
 
-// BM_STEP k of a single block: 4 x 8 outputs per thread.  sx_odd: the lane's chunk of X in odd rows.
+// BM_STEP k of a single block: 4 x 8 outputs per thread.  Odd rows hold their upper half first; sx_odd: the lane's chunk of X in them.
 __device__ __forceinline__ void single_steps(Acc &acc, const char *sx, const char *sx_odd, const char *sy)
 {
 #pragma unroll
@@ -231,6 +236,21 @@ __device__ __forceinline__ void cp_async_4(uint32_t dst, const void *src)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
+// dst <- 16 bytes at row + OFFSET
+template <int OFFSET>
+__device__ __forceinline__ void copy_16(uint32_t dst, const char *row)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1+%2], 16;" ::"r"(dst), "l"(row), "n"(OFFSET) : "memory");
+}
+
+// base + k * stride in one instruction (of the multiply-adds' pipe, where the compiler takes two)
+__device__ __forceinline__ const char *row_of(const char *base, unsigned k, unsigned stride)
+{
+    const char *r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(k), "r"(stride), "l"(base));
+    return r;
+}
+
 __device__ __forceinline__ void fill_4(uint32_t dst, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory"); }
 
 __device__ __forceinline__ void fill_16(uint32_t dst, float v)
@@ -240,7 +260,8 @@ __device__ __forceinline__ void fill_16(uint32_t dst, float v)
 
 // One item: blocks x0 and x0 + 1 of X (TWO) or x0 alone, times block y of Y.
 // ROW_MAJOR: A is the caller's matrix instead of the k-major packed copy; 4-byte copies transpose it on the way.
-template <bool TWO, bool ROW_MAJOR, typename Params>
+// EDGE: blocks of B may be cut off by its last column.  AGREE: X's blocks had the same patterns in pairs wherever samples were taken.
+template <bool TWO, bool ROW_MAJOR, bool EDGE, bool AGREE, typename Params>
 __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane, bool wide_b, int x0, int y)
 {
     LiveList l0, l1;
@@ -249,9 +270,13 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     // every 4 consecutive lanes touch 2 chunks of X and 2 of Y (see the tiled pipeline)
     const int half = lane >> 4, xg = (lane >> 1) & 3, yg = (lane & 1) | ((lane >> 2) & 2);   // pair: 4 x 4 lanes per block
     const int lm = (lane >> 1) & 7, ln = (lane & 1) | ((lane >> 4) << 1);                    // single block: 8 x 4 lanes
-    // Copies: four lanes per row of the stage, eight rows at a time; a lane moves the 16-byte chunks c4 and c4 + 4 of its row.
-    // Rows are 128 bytes apart; odd rows have their two halves swapped, so that the eight rows of one copy instruction fall
-    // on all banks.
+    // Copies of a pair from packed A: eight lanes per row, a lane's rows are 4 r4 .. 4 r4 + 3, so that its list entries are one load and the
+    // rows of one copy instruction are whole (80 bytes a clock and SM arrive so at most, 64 in the other order).
+    const int r4 = lane >> 3, c8 = lane & 7;
+    const uint32_t dst = smem_u32(ring) + (uint32_t)(r4 * 512 + c8 * 16);
+    // Single blocks, and all with row-major A: four lanes per row of the stage, eight rows at a time; a lane moves the 16-byte chunks c4
+    // and c4 + 4 of its row.  Rows are 128 bytes apart; odd rows have their two halves swapped, so that the eight rows of one copy
+    // instruction fall on all banks.  (Fewer addresses: 100 x 6000 x 3000, single blocks only, 54.7 us so, 56.6 in the order above.)
     const int r8 = lane >> 2, c4 = lane & 3;
     const uint32_t dst0 = smem_u32(ring) + (uint32_t)(r8 * 128 + c4 * 16 + (r8 & 1) * 64), dst1 = dst0 + 64 - (r8 & 1) * 128;
     const unsigned n4 = (unsigned)p.N * 4u;                       // bytes of a row of B
@@ -266,12 +291,11 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     const char *a_src = nullptr;
     if constexpr (!ROW_MAJOR) a_src = reinterpret_cast<const char *>(p.a_packed + (size_t)(a_blk >> 2) * p.kp * TILE_M + (a_blk & 3) * 32);
     const char *b_src = reinterpret_cast<const char *>(p.B + b_blk * 32);
-    const char *xs = (wide_b ? b_src : a_src) + c4 * 16, *ys = (wide_b ? a_src : b_src) + c4 * 16;
+    const char *xs = (wide_b ? b_src : a_src) + c8 * 16, *ys = (wide_b ? a_src : b_src) + c8 * 16;
     const int b_chunks = (p.N - b_blk * 32) >> 2;
-    const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);   // (2330 x 932 x 5020 pruned MLP: 186 us with a slow path there, 138 with predicates)
+    const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);
     const int x_chunks = wide_b ? b_chunks : 16, y_chunks = wide_b ? 8 : b_chunks;
-    const bool x_ok0 = c4 < x_chunks, x_ok1 = c4 + 4 < x_chunks, x_ok2 = c4 + 8 < x_chunks, x_ok3 = c4 + 12 < x_chunks;
-    const bool y_ok0 = c4 < y_chunks, y_ok1 = c4 + 4 < y_chunks;
+    const bool x_ok0 = c8 < x_chunks, x_ok1 = c8 + 8 < x_chunks, y_ok = c8 < y_chunks;
 
     Acc acc;
     acc_clear(acc);
@@ -279,6 +303,10 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     // The lane's pattern bits of the 128 K blocks kb0 .. (m0, m1: joint bits of either block; wy, w0, w1: the words of the
     // 128 K blocks after them, on their way) and how many quarters of them are listed already.
     int kb0 = -128, part = 0, live = 0;
+    // A list that holds less than a stage gives nothing as long as more of it is to come (the other list may be full and keep it from being
+    // refilled), so that a full stage's entries start at a multiple of BM_ROWS.
+    int taken_mask = BM_ROWS;
+    static_assert((BM_ROWS & (BM_ROWS - 1)) == 0, "mask");
     unsigned m0 = 0u, m1 = 0u, wy = 0u, w0 = 0u, w1 = 0u;
     auto load_words = [&](int kb) {
         wy = pattern_word(py, kb, p.nKB, p.pat_words, p.status) & inside_k(kb, p.K);
@@ -287,6 +315,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     };
     auto next_words = [&]() {
         kb0 += 128;
+        if (kb0 >= p.nKB) taken_mask = 2 * BM_ROWS - 1;
         part = 0;
         m0 = w0 & wy;
         m1 = w1 & wy;
@@ -296,6 +325,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     load_words(4 * lane);
     next_words();
     l0.made = l0.taken = l1.made = l1.taken = 0;
+    bool one_list = TWO && AGREE;   // so far both blocks have the same live k: list 0 stands for both
     int wrap0 = INT_MAX, wrap1 = INT_MAX;   // (ROW_MAJOR) list positions from which on an entry is k - 65536
 
     // Lists further K blocks until each list holds a stage or there is no room: all 128 at once where they fit, or a
@@ -319,8 +349,13 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
             const int c = __popc(a0) | (__popc(a1) << 16);
             const int before = exclusive_scan(c, lane);
             const int total = __shfl_sync(0xFFFFFFFFu, before + c, 31);
+            if (one_list && !__all_sync(0xFFFFFFFFu, a0 == a1)) {   // from here on a list each
+                one_list = false;
+                __syncwarp();
+                for (int i = l0.taken + lane; i < l0.made; i += 32) l1.list[i & (BM_LIST - 1)] = l0.list[i & (BM_LIST - 1)];
+            }
             append_live(l0.list, l0.made + (before & 0xFFFF), l0.taken, a0, k0, p.status);
-            if (TWO) append_live(l1.list, l1.made + (before >> 16), l1.taken, a1, k0, p.status);
+            if (TWO && !one_list) append_live(l1.list, l1.made + (before >> 16), l1.taken, a1, k0, p.status);
             if (ROW_MAJOR && k0 >= 65536 && wrap0 == INT_MAX) wrap0 = l0.made, wrap1 = l1.made;
             l0.made += total & 0xFFFF;
             l1.made += total >> 16;
@@ -338,7 +373,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
         __syncwarp();              // the stage is complete for all lanes, and the one before it read by all
         refill();
         // ---- copies of the next stage ----
-        const int d0 = min(BM_ROWS, l0.pending()), d1 = TWO ? min(BM_ROWS, l1.pending()) : 0;
+        const int d0 = min(BM_ROWS, l0.pending()) & taken_mask, d1 = TWO ? min(BM_ROWS, l1.pending()) & taken_mask : 0;
         const uint32_t to = BM_SLOT_BYTES - slot;
         bool same_next = false;
         if constexpr (ROW_MAJOR) {
@@ -399,46 +434,63 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
                 }
             }
         } else {
-            if (d0 == BM_ROWS && (!TWO || d1 == BM_ROWS)) {
-                unsigned k0[BM_ROWS / 8], k1[BM_ROWS / 8];
-                same_next = TWO;
+            if (!TWO && d0 == BM_ROWS) {
+                const uint16_t *entry = l0.list + (l0.taken & (BM_LIST - 1)) + r8;
+                const unsigned k[2] = {entry[0], entry[8]};
+                const char *xs4 = xs - c8 * 16 + c4 * 16, *ys4 = ys - c8 * 16 + c4 * 16;
 #pragma unroll
-                for (int h = 0; h < BM_ROWS / 8; ++h) {
-                    k0[h] = l0.list[(l0.taken + h * 8 + r8) & (BM_LIST - 1)];
-                    k1[h] = TWO ? l1.list[(l1.taken + h * 8 + r8) & (BM_LIST - 1)] : 0;
-                    if (TWO) same_next = __all_sync(0xFFFFFFFFu, k0[h] == k1[h]) && same_next;
-                }
-#pragma unroll
-                for (int h = 0; h < BM_ROWS / 8; ++h) {
-                    const char *gx = xs + (size_t)k0[h] * x_stride, *gy = ys + (size_t)k0[h] * y_stride;
+                for (int h = 0; h < 2; ++h) {
+                    if (!k_ok(p, k[h])) continue;
+                    const char *gx = row_of(xs4, k[h], x_stride), *gy = row_of(ys4, k[h], y_stride);
                     const uint32_t e0 = dst0 + to + h * 1024, e1 = dst1 + to + h * 1024;
-                    if (!k_ok(p, k0[h]) || (TWO && !k_ok(p, k1[h]))) continue;
-                    if (x_ok0) cp_async_16(e0, gx, 16);
-                    if (x_ok1) cp_async_16(e1, gx + 64, 16);
-                    if (y_ok0) cp_async_16(e0 + 2 * BM_PART, gy, 16);
-                    if (y_ok1) cp_async_16(e1 + 2 * BM_PART, gy + 64, 16);
-                    if (TWO) {
-                        const char *gx1 = xs + (size_t)k1[h] * x_stride;
-                        if (x_ok2) cp_async_16(e0 + BM_PART, gx1 + 128, 16);
-                        if (x_ok3) cp_async_16(e1 + BM_PART, gx1 + 192, 16);
-                        if (!same_next) {
-                            const char *gy1 = ys + (size_t)k1[h] * y_stride;
-                            if (y_ok0) cp_async_16(e0 + 3 * BM_PART, gy1, 16);
-                            if (y_ok1) cp_async_16(e1 + 3 * BM_PART, gy1 + 64, 16);
-                        }
+                    if (!EDGE || c4 < x_chunks) copy_16<0>(e0, gx);
+                    if (!EDGE || c4 + 4 < x_chunks) copy_16<64>(e1, gx);
+                    if (!EDGE || c4 < y_chunks) copy_16<0>(e0 + 2 * BM_PART, gy);
+                    if (!EDGE || c4 + 4 < y_chunks) copy_16<64>(e1 + 2 * BM_PART, gy);
+                }
+            } else if (TWO && d0 == BM_ROWS && d1 == BM_ROWS) {
+                const uint2 v0 = *reinterpret_cast<const uint2 *>(l0.list + (l0.taken & (BM_LIST - 1)) + r4 * 4);
+                uint2 v1 = v0;
+                same_next = true;
+                if (!one_list) {
+                    v1 = *reinterpret_cast<const uint2 *>(l1.list + (l1.taken & (BM_LIST - 1)) + r4 * 4);
+                    same_next = __all_sync(0xFFFFFFFFu, v0.x == v1.x && v0.y == v1.y);
+                }
+                if (same_next) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const unsigned w0 = j & 2 ? v0.y : v0.x, k0 = j & 1 ? w0 >> 16 : w0 & 0xFFFFu;
+                        const uint32_t e = dst + to + j * 128;
+                        if (!k_ok(p, k0)) continue;
+                        const char *gx = row_of(xs, k0, x_stride), *gy = row_of(ys, k0, y_stride);
+                        if (!EDGE || x_ok0) copy_16<0>(e, gx);
+                        if (!EDGE || y_ok) copy_16<0>(e + 2 * BM_PART, gy);
+                        if (!EDGE || x_ok1) copy_16<128>(e + BM_PART, gx);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const unsigned w0 = j & 2 ? v0.y : v0.x, w1 = j & 2 ? v1.y : v1.x;
+                        const unsigned k0 = j & 1 ? w0 >> 16 : w0 & 0xFFFFu, k1 = j & 1 ? w1 >> 16 : w1 & 0xFFFFu;
+                        const uint32_t e = dst + to + j * 128;
+                        if (!k_ok(p, k0) || !k_ok(p, k1)) continue;
+                        if (!EDGE || x_ok0) copy_16<0>(e, row_of(xs, k0, x_stride));
+                        if (!EDGE || y_ok) copy_16<0>(e + 2 * BM_PART, row_of(ys, k0, y_stride));
+                        if (!EDGE || x_ok1) copy_16<128>(e + BM_PART, row_of(xs, k1, x_stride));
+                        if (!EDGE || y_ok) copy_16<0>(e + 3 * BM_PART, row_of(ys, k1, y_stride));
                     }
                 }
             } else if (max(d0, d1) > 0) {
                 // Past the end of a list X = -0 and Y = +0: a multiply-add with them changes no accumulator, not even a zero's sign.
 #pragma unroll 1
-                for (int i = 0; i < 2 * (TWO ? 2 : 1) * (BM_ROWS / 8); ++i) {      // (row group, half of the row, block)
-                    const int j = i & 1, row = ((i >> 1) & (BM_ROWS / 8 - 1)) * 8 + r8, blk = TWO ? i >> 2 : 0, ch = c4 + 4 * j;
-                    const uint32_t e = (j ? dst1 : dst0) + to + (row - r8) * 128 + blk * BM_PART;
+                for (int i = 0; i < (TWO ? 8 : 4); ++i) {      // (row of four, block)
+                    const int j = i & 3, row = r4 * 4 + j, blk = TWO ? i >> 2 : 0;
+                    const uint32_t e = (TWO || !(row & 1) ? dst : dst ^ 64u) + to + j * 128 + blk * BM_PART;
                     if (row < (blk ? d1 : d0)) {
-                        const size_t k = blk ? l1.list[(l1.taken + row) & (BM_LIST - 1)] : l0.list[(l0.taken + row) & (BM_LIST - 1)];
+                        const size_t k = blk && !one_list ? l1.list[(l1.taken + row) & (BM_LIST - 1)] : l0.list[(l0.taken + row) & (BM_LIST - 1)];
                         if (!k_ok(p, k)) continue;
-                        if (blk * 8 + ch < x_chunks) cp_async_16(e, xs + k * x_stride + blk * 128 + j * 64, 16);
-                        if (ch < y_chunks) cp_async_16(e + 2 * BM_PART, ys + k * y_stride + j * 64, 16);
+                        if (blk ? x_ok1 : x_ok0) copy_16<0>(e, xs + k * x_stride + blk * 128);
+                        if (y_ok) copy_16<0>(e + 2 * BM_PART, ys + k * y_stride);
                     } else {
                         fill_16(e, -0.0f);
                         fill_16(e + 2 * BM_PART, 0.0f);
@@ -454,7 +506,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
         if (TWO) {
             const char *sx = st + half * BM_PART + xg * 16, *sy = st + (same ? 2 : 2 + half) * BM_PART + yg * 16;
 #pragma unroll 1
-            for (int r = 0; r < count; r += BM_STEP) pair_steps(acc, sx + r * 128, sy + r * 128);
+            for (int r = 0; r < count; r += BM_STEP) pair_steps<ROW_MAJOR>(acc, sx + r * 128, sy + r * 128);
         } else {
             const char *sx = st + lm * 16, *sx_odd = st + (lm ^ 4) * 16, *sy = st + 2 * BM_PART + ln * 16;
 #pragma unroll 1
@@ -500,7 +552,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
 
 // All of a warp's share of block mode.  smem: the CTA's dynamic shared memory; next: the CTA's item counter (initially
 // BM_WARPS: a warp's first item is its own number).
-template <bool ROW_MAJOR, typename Params>
+template <bool ROW_MAJOR, bool EDGE, bool AGREE, typename Params>
 __device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp, int lane, bool wide_b, int *next)
 {
     char *ring = smem + warp * BM_WARP_BYTES;
@@ -523,8 +575,8 @@ __device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp
         int tm, tn;
         tile_coords(item, tiles_m, tiles_n, tm, tn, wide_b ? 32 : 16);
         const int y = wide_b ? tm : tn, x0 = 2 * (wide_b ? tn : tm) + (v < whole ? 0 : (v - whole) & 1);
-        if (v < whole && x0 + 1 < x_blocks) block_item<true, ROW_MAJOR>(p, ring, lane, wide_b, x0, y);
-        else if (x0 < x_blocks) block_item<false, ROW_MAJOR>(p, ring, lane, wide_b, x0, y);
+        if (v < whole && x0 + 1 < x_blocks) block_item<true, ROW_MAJOR, EDGE, AGREE>(p, ring, lane, wide_b, x0, y);
+        else if (x0 < x_blocks) block_item<false, ROW_MAJOR, EDGE, AGREE>(p, ring, lane, wide_b, x0, y);
         int nx = 0;
         if (lane == 0) nx = atomicAdd(next, 1);
         v = __shfl_sync(0xFFFFFFFFu, nx, 0);

@@ -524,7 +524,7 @@ __device__ __noinline__ int listed_warp_rows(const uint8_t *rmask, int n, int la
 // samples, free again on return.  (A call rather than inline code: it runs once per CTA, and what follows gets better registers: pruned
 // MLP 2048 x 11008 x 4096 765 -> 748 us, 1000 x 1508 x 2012 at 0.5 / 0.5 59.4 -> 57.4, 4096^3 dense 2165 -> 2148.  Block mode as a call
 // spills: 866, 67.6, 2170.)
-enum { MODE_PIPELINE, MODE_BLOCKS, MODE_BLOCKS_WIDE_B };
+enum { MODE_PIPELINE = 0, MODE_BLOCKS = 1, MODE_BLOCKS_WIDE_B = 2, MODE_BLOCKS_AGREE = 4 };
 
 template <bool RM>
 __device__ __noinline__ int choose_mode(const PackedParams &p, char *scratch, int warp, int lane)
@@ -582,7 +582,8 @@ __device__ __noinline__ int choose_mode(const PackedParams &p, char *scratch, in
     }
     __syncthreads();   // the samples have been read by all
     if (!blocks) return MODE_PIPELINE;
-    return (RM ? b_differ <= a_differ : b_differ < a_differ) ? MODE_BLOCKS_WIDE_B : MODE_BLOCKS;
+    const bool wide_b = RM ? b_differ <= a_differ : b_differ < a_differ;
+    return MODE_BLOCKS | (wide_b ? MODE_BLOCKS_WIDE_B : 0) | ((wide_b ? b_differ : a_differ) == 0 ? MODE_BLOCKS_AGREE : 0);
 }
 
 // The CTA's next row list: the tile's next one, or the first of its next tile.
@@ -659,7 +660,17 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
     if (BLOCKS && p.block_mode != 0) {
         const int mode = choose_mode<RM>(p, smem + L.wlist_off, warp, lane);
         if (mode != MODE_PIPELINE) {
-            if (warp < BM_WARPS) block_mode<RM>(p, smem, warp, lane, mode == MODE_BLOCKS_WIDE_B, next_item);
+            if (warp < BM_WARPS) {
+                // The code of a whole launch, so that no two kinds of it compete for the instruction cache (items at N's edge alone
+                // with predicates of their own: 2330 x 932 x 5020 128 -> 136 us).  Column blocks all whole: copies without predicates;
+                // blocks that agree in pairs, where samples were taken: one list for both until they differ.  Without / with: pruned MLP
+                // 2048 x 11008 x 4096 744 -> 724, 4096^3 64-granular 0.5 / 0.5 692 -> 674 us, 32-granular 0.2 / 0.2 164 either way (165 with one
+                // list until they differ, which is at once).
+                const bool wide_b = (mode & MODE_BLOCKS_WIDE_B) != 0;
+                if (RM || (p.N & 63)) block_mode<RM, true, false>(p, smem, warp, lane, wide_b, next_item);
+                else if (mode & MODE_BLOCKS_AGREE) block_mode<RM, RM, !RM>(p, smem, warp, lane, wide_b, next_item);
+                else block_mode<RM, RM, false>(p, smem, warp, lane, wide_b, next_item);
+            }
             return;
         }
     }

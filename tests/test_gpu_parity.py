@@ -1090,3 +1090,42 @@ def test_calls_wait_for_what_is_before_them(cuda, pkg, M, captured):
     pkg.device_status()
     if captured:
         del graph
+
+
+@pytest.mark.parametrize("kind", ["agree", "part", "sparse_second", "sparse_first"])
+@pytest.mark.parametrize("swap", [False, True])
+@pytest.mark.parametrize("N", [192, 256, 228])
+def test_gemm_block_mode_pair_lists(cuda, pkg, oracle_mod, tuning, kind, swap, N):
+    """Pairs of blocks with one list for both: patterns that agree in pairs everywhere; that agree where samples are taken and part
+    ways after a stretch that is already listed; and a dense block beside one with a few live k, whose list the other's keeps from
+    being refilled in time, so that it gives nothing for some stages (stages start at multiples of 16 entries).  Blocks of B whole
+    (N a multiple of 64) or cut off; the pairs on A's side and (swap) on B's.  All on one CTA: twelve or more items, most of them pairs."""
+    tuning("BLOCK_MODE", 1)
+    tuning("GRID", 1)
+    M, K = 256, 6004
+    rng = np.random.default_rng(len(kind) + N)
+    A = rng.standard_normal((M, K), dtype=np.float32)
+    B = rng.standard_normal((K, N), dtype=np.float32)
+    paired = (B.T if swap else A)                                  # the operand whose blocks come in pairs, [64-wide][K]
+    other = (A if swap else B.T)
+    for o in range(0, other.shape[0], 32):
+        other[o:o + 32, rng.random(K) < 0.3] = 0.0
+    for o in range(0, paired.shape[0], 64):
+        if kind in ("agree", "part"):
+            dead = rng.random(K) < 0.5
+            paired[o:o + 64, dead] = 0.0
+            if kind == "part" and o == 0:                          # the first pair alone, past the middle of K
+                more = np.arange(K) > 3500 + 8 * rng.integers(0, 100)
+                paired[o + 32:o + 64, more & (rng.random(K) < 0.5)] = 0.0
+        else:
+            lo, hi = (o + 32, o + 64) if kind == "sparse_second" else (o, o + 32)
+            paired[lo:hi, rng.random(K) < 0.98] = 0.0
+    dA, dB = cuda.from_numpy(A).cuda(), cuda.from_numpy(np.ascontiguousarray(B)).cuda()
+    bp = cuda.empty((-(-N // 32), -(-K // 8)), dtype=cuda.uint8, device="cuda")
+    pkg.preprocess_b(dB.data_ptr(), K, N, bp.data_ptr())
+    ws = cuda.full((pkg.sgemm_joint_workspace_bytes(M, K),), 0xFF, dtype=cuda.uint8, device="cuda")
+    C_ = cuda.full((M, N), float("nan"), device="cuda")
+    pkg.sgemm_joint(M, N, K, dA.data_ptr(), dB.data_ptr(), C_.data_ptr(), bp.data_ptr(), ws.data_ptr())
+    pkg.device_status()
+    want = oracle_mod.gemm_joint(A, np.ascontiguousarray(B))
+    assert np.array_equal(C_.cpu().numpy().view(np.uint32), want.view(np.uint32))
