@@ -502,7 +502,7 @@ def run_ours(args) -> None:
     # the packed copy) over the launch-train time, against the measured copy bandwidth
     pre_bytes_sum = sum(4.0 * M * K + ap_bytes + 4.0 * M * K * v["joint_density"] for v in sweep.values())
     roofline_pre = {
-        "kernel": "esmm_preprocess_a_pack64_kernel", "bound": "hbm", "achieved": pre_bytes_sum / (pre_ms_sum * 1e-3) / 1e9,
+        "kernel": "esmm_preprocess_a_pack32_kernel", "bound": "hbm", "achieved": pre_bytes_sum / (pre_ms_sum * 1e-3) / 1e9,
         "peak": hbm_peak, "unit": "GB/s", "frac": pre_bytes_sum / (pre_ms_sum * 1e-3) / 1e9 / hbm_peak,
         "peak_source": "MEASURED_PEAKS.json hbm_gbs (of %s)" % hbm_src, "bytes_per_step": pre_bytes_sum,
         "launches_per_step": len(cases), "traffic": None, "share_of_step": pre_ms_sum / (gemm_ms_sum + pre_ms_sum),

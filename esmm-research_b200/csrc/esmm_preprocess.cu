@@ -85,89 +85,25 @@ esmm_preprocess_a_patterns_kernel(const float *A, int M, int K, int tile_m, int 
 }
 
 // Pattern scan fused with the re-layout the packed GEMM variant reads: besides the pattern
-// bytes the warp writes its 32 rows x 128 columns transposed into
+// bytes the warp writes its 32 rows x 32 columns transposed into
 //   packed[((tile * nKB + kb) * 8 + k) * 128 + row_in_tile],   tile = row / 128,
 // i.e. k-major rows of 128 floats per 128-row tile, so that one K block of a tile is 4 KB of
-// contiguous memory.  The transpose goes through a skewed shared-memory tile (conflict-free
-// both ways).  A k whose pattern bit is clear for the warp's 32-row block is not written: the
+// contiguous memory.  A k whose pattern bit is clear for the warp's 32-row block is not written: the
 // GEMM never multiplies it, so whatever the buffer holds there is harmless.
+//
+// Lane = (row r4 of four, column group cq of eight): lane loads rows 4 i + r4, columns 4 cq .. 4 cq + 3.  All rows of a column are OR-ed as
+// bit patterns before the one test for zero (without the sign bit), and one reduction over the warp gives the 32 live bits, which
+// are the block's four pattern bytes as they stand.  The transpose goes through shared memory 16 bytes at a time, chunk cq of row r at
+// position cq ^ (r & 7), so that neither the stores (eight lanes a row) nor the loads (a lane a row) meet a bank twice; four stores
+// of 128 bytes per chunk follow, of live columns only.
+// What bounds it: HBM.  In a train of calls 4096^2 takes 11.4 us with a fifth of the columns live, 16.2 with half and 21.8 with all (12.3, 15.4
+// and 20.5 us of bytes at the measured copy bandwidth); 32 x 64 columns per warp with every element's own test, store and load through shared
+// memory, 1280 instructions per task where these two have 320, took 15.2, 18.5 and 22.3 and had 16 warps per SM for these 32.
 constexpr int PACK_WARPS = 4;
-constexpr int PACK_SMEM_PER_WARP = 128 * 32 * 4;  // 16 KB
+constexpr int PACK_COLS = 32;
 
 __global__ void __launch_bounds__(PACK_WARPS * 32)
-esmm_preprocess_a_pack_kernel(const float *__restrict__ A, int M, int K, int nMB, int nKB, int k_chunks,
-                              uint8_t *__restrict__ out, float *__restrict__ packed, int *status)
-{
-    // checked build, sites 10 (loads of A), 11 (pattern stores), 12 (stores into the packed copy), 13 (the warp's tile)
-    const size_t a_floats = (size_t)M * K, out_bytes = (size_t)nMB * nKB;
-    const size_t packed_floats = (size_t)((M + 127) / 128) * nKB * BK * 128;
-    extern __shared__ __align__(16) float pack_smem[];
-    float *tile = pack_smem + (threadIdx.x >> 5) * (PACK_SMEM_PER_WARP / 4);
-    const int lane = threadIdx.x & 31;
-    const long warps_total = (long)gridDim.x * PACK_WARPS;
-    const long tasks = (long)nMB * k_chunks;
-    for (long task = (long)blockIdx.x * PACK_WARPS + (threadIdx.x >> 5); task < tasks; task += warps_total) {
-        const int mb = (int)(task / k_chunks);
-        const int kc = (int)(task - (long)mb * k_chunks);
-        const int col = kc * 128 + lane * 4;
-        const bool col_ok = col < K;
-        const int row0 = mb * 32;
-        const float *src = A + (size_t)row0 * K + col;
-        unsigned nib = 0;
-        // all 32 rows of the lane's 4 columns are requested before anything is consumed: 16 KB in
-        // flight per warp, which is what keeps HBM busy at the occupancy the 16 KB tile allows
-        float4 v[32];
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-            v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (col_ok && row0 + r < M && bounds_ok((size_t)(row0 + r) * K + col + 4 <= a_floats, status, 10))
-                v[r] = __ldg(reinterpret_cast<const float4 *>(src + (size_t)r * K));
-        }
-#pragma unroll
-        for (int r = 0; r < 32; ++r) nib |= nz4(v[r]);
-        // live columns of the chunk: bit l of liveq[q] says column 4 l + q has a nonzero
-        unsigned liveq[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) liveq[q] = __ballot_sync(0xFFFFFFFFu, (nib >> q) & 1u);
-        // Only live columns go through the tile.  (This also makes every store depend on all 32
-        // loads, so the loads are all in flight together.)
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-            // element (r, c) lives at c * 32 + ((r + (c >> 2)) & 31); here c >> 2 == lane
-            const int pos = (r + lane) & 31;
-            if (!bounds_ok((lane * 4 + 3) * 32 + pos < PACK_SMEM_PER_WARP / 4, status, 13)) continue;
-            if (nib & 1u) tile[(lane * 4 + 0) * 32 + pos] = v[r].x;
-            if (nib & 2u) tile[(lane * 4 + 1) * 32 + pos] = v[r].y;
-            if (nib & 4u) tile[(lane * 4 + 2) * 32 + pos] = v[r].z;
-            if (nib & 8u) tile[(lane * 4 + 3) * 32 + pos] = v[r].w;
-        }
-        const unsigned other = __shfl_xor_sync(0xFFFFFFFFu, nib, 1);
-        const int kb_lane = kc * 16 + (lane >> 1);
-        if (!(lane & 1) && kb_lane < nKB && bounds_ok((size_t)mb * nKB + kb_lane < out_bytes, status, 11))
-            out[(size_t)mb * nKB + kb_lane] = (uint8_t)(nib | (other << 4));
-        __syncwarp();
-        const size_t dst0 = (size_t)(mb >> 2) * nKB * BK * 128 + (mb & 3) * 32 + lane;
-        float *dst = packed + dst0;
-#pragma unroll 8
-        for (int c = 0; c < 128; ++c) {
-            const int k = kc * 128 + c;  // global k = kb * 8 + kk
-            if (((liveq[c & 3] >> (c >> 2)) & 1u) && k < nKB * BK &&
-                bounds_ok(dst0 + (size_t)k * 128 < packed_floats, status, 12))
-                dst[(size_t)k * 128] = tile[c * 32 + ((lane + (c >> 2)) & 31)];
-        }
-        __syncwarp();
-    }
-}
-
-// The same with half the task (the default; ESMM_PACK=128 selects the kernel above): 32 rows x 64 columns per warp (8 KB in flight and 8 KB of shared
-// memory per warp instead of 16, half the registers), so that more warps are resident and the tail of
-// the grid is shorter.  Lane = (row parity h, column group cl): lane loads rows 2 i + h, columns
-// 4 cl .. 4 cl + 3.  Element (r, c) of the tile lives at c * 32 + ((r + 2 (c >> 2)) & 31): both the
-// stores (lanes differ in 2 cl + h) and the k-major loads (lanes differ in r) are conflict-free.
-constexpr int PACK64_SMEM_PER_WARP = 64 * 32 * 4;  // 8 KB
-
-__global__ void __launch_bounds__(PACK_WARPS * 32)
-esmm_preprocess_a_pack64_kernel(const float *A, int M, int K, int nMB, int nKB, int k_chunks,
+esmm_preprocess_a_pack32_kernel(const float *A, int M, int K, int nMB, int nKB, int k_chunks,
                                 uint8_t *__restrict__ out, float *__restrict__ packed, int *status)
 {
     // The product kernel, launched as a dependent of this one, may be placed where SMs become free once every CTA of this
@@ -178,62 +114,63 @@ esmm_preprocess_a_pack64_kernel(const float *A, int M, int K, int nMB, int nKB, 
     // call it early: strips placed beside those of the call before are 15-100 % slower.  Nothing of A is read before the wait, and what is
     // read goes past L1, which may have been filled while A was written.
     grid_dependency_wait();
-    // checked build, sites 10 (loads of A), 11 (pattern stores), 12 (stores into the packed copy), 13 (the warp's tile)
+    // checked build, sites 10 (loads of A), 11 (pattern stores), 12 (stores into the packed copy)
     const size_t a_floats = (size_t)M * K, out_bytes = (size_t)nMB * nKB;
     const size_t packed_floats = (size_t)((M + 127) / 128) * nKB * BK * 128;
-    extern __shared__ __align__(16) float pack_smem[];
-    float *tile = pack_smem + (threadIdx.x >> 5) * (PACK64_SMEM_PER_WARP / 4);
-    const int lane = threadIdx.x & 31;
-    const int h = lane >> 4, cl = lane & 15;
+    __shared__ __align__(16) float4 pack_smem[PACK_WARPS][32 * PACK_COLS / 4];
+    float4 *tile = pack_smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, r4 = lane >> 3, cq = lane & 7;
     const long warps_total = (long)gridDim.x * PACK_WARPS;
     const long tasks = (long)nMB * k_chunks;
     for (long task = (long)blockIdx.x * PACK_WARPS + (threadIdx.x >> 5); task < tasks; task += warps_total) {
         const int mb = (int)(task / k_chunks);
         const int kc = (int)(task - (long)mb * k_chunks);
-        const int col = kc * 64 + cl * 4;
-        const bool col_ok = col < K;
+        const int col = kc * PACK_COLS + cq * 4;
         const int row0 = mb * 32;
-        const float *src = A + (size_t)row0 * K + col;
-        float4 v[16];
+        const float *src = A + (size_t)(row0 + r4) * K + col;
+        float4 v[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int r = 2 * i + h;
+        for (int i = 0; i < 8; ++i) {
+            const int row = row0 + 4 * i + r4;
             v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (col_ok && row0 + r < M && bounds_ok((size_t)(row0 + r) * K + col + 4 <= a_floats, status, 10))
-                v[i] = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)r * K));
+            if (col < K && row < M && bounds_ok((size_t)row * K + col + 4 <= a_floats, status, 10))
+                v[i] = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)(4 * i) * K));
         }
-        unsigned nib = 0;
+        unsigned any[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-        for (int i = 0; i < 16; ++i) nib |= nz4(v[i]);
-        nib |= __shfl_xor_sync(0xFFFFFFFFu, nib, 16);           // both row parities
-        // live columns of the chunk: bit cl of liveq[q] says column 4 cl + q has a nonzero
-        unsigned liveq[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) liveq[q] = __ballot_sync(0xFFFFFFFFu, (nib >> q) & 1u);
-        // only live columns go through the tile (and every store depends on all the loads, which keeps
-        // them in flight together)
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int pos = (2 * i + h + 2 * cl) & 31;
-            if (!bounds_ok((cl * 4 + 3) * 32 + pos < PACK64_SMEM_PER_WARP / 4, status, 13)) continue;
-            if (nib & 1u) tile[(cl * 4 + 0) * 32 + pos] = v[i].x;
-            if (nib & 2u) tile[(cl * 4 + 1) * 32 + pos] = v[i].y;
-            if (nib & 4u) tile[(cl * 4 + 2) * 32 + pos] = v[i].z;
-            if (nib & 8u) tile[(cl * 4 + 3) * 32 + pos] = v[i].w;
+        for (int i = 0; i < 8; ++i) {
+            any[0] |= __float_as_uint(v[i].x);
+            any[1] |= __float_as_uint(v[i].y);
+            any[2] |= __float_as_uint(v[i].z);
+            any[3] |= __float_as_uint(v[i].w);
+            tile[(4 * i + r4) * 8 + (cq ^ ((4 * i + r4) & 7))] = v[i];
         }
-        const unsigned other = __shfl_xor_sync(0xFFFFFFFFu, nib, 1);
-        const int kb_lane = kc * 8 + (cl >> 1);
-        if (h == 0 && !(cl & 1) && kb_lane < nKB && bounds_ok((size_t)mb * nKB + kb_lane < out_bytes, status, 11))
-            out[(size_t)mb * nKB + kb_lane] = (uint8_t)(nib | (other << 4));
+        unsigned nib = 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) nib |= (any[q] << 1) != 0u ? 1u << q : 0u;
+        const unsigned live = __reduce_or_sync(0xFFFFFFFFu, nib << (4 * cq));   // bit c: column c of the 32
+        if (lane == 0) {
+            uint8_t *bytes = out + (size_t)mb * nKB + kc * 4;
+            if (kc * 4 + 4 <= nKB && (reinterpret_cast<uintptr_t>(bytes) & 3) == 0) {
+                if (bounds_ok((size_t)mb * nKB + kc * 4 + 4 <= out_bytes, status, 11)) *reinterpret_cast<unsigned *>(bytes) = live;
+            } else {
+                for (int j = 0; j < 4; ++j)
+                    if (kc * 4 + j < nKB && bounds_ok((size_t)mb * nKB + kc * 4 + j < out_bytes, status, 11)) bytes[j] = (uint8_t)(live >> (8 * j));
+            }
+        }
         __syncwarp();
-        const size_t dst0 = (size_t)(mb >> 2) * nKB * BK * 128 + (mb & 3) * 32 + lane;
+        // (a live column is inside A)
+        const size_t dst0 = ((size_t)(mb >> 2) * nKB * BK + kc * PACK_COLS) * 128 + (mb & 3) * 32 + lane;
         float *dst = packed + dst0;
-#pragma unroll 8
-        for (int c = 0; c < 64; ++c) {
-            const int k = kc * 64 + c;  // global k = kb * 8 + kk
-            if (((liveq[c & 3] >> (c >> 2)) & 1u) && k < nKB * BK &&
-                bounds_ok(dst0 + (size_t)k * 128 < packed_floats, status, 12))
-                dst[(size_t)k * 128] = tile[c * 32 + ((lane + 2 * (c >> 2)) & 31)];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (!((live >> (4 * j)) & 0xFu)) continue;
+            const float4 x = tile[lane * 8 + (j ^ (lane & 7))];
+            if (!bounds_ok(dst0 + (size_t)(4 * j + 3) * 128 < packed_floats, status, 12)) continue;
+            if ((live >> (4 * j)) & 1u) dst[(4 * j + 0) * 128] = x.x;
+            if ((live >> (4 * j)) & 2u) dst[(4 * j + 1) * 128] = x.y;
+            if ((live >> (4 * j)) & 4u) dst[(4 * j + 2) * 128] = x.z;
+            if ((live >> (4 * j)) & 8u) dst[(4 * j + 3) * 128] = x.w;
         }
         __syncwarp();
     }
@@ -373,61 +310,30 @@ int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, flo
     const int sms = sm_count();
     if (sms <= 0) return record_cuda_error_text("no CUDA device");
     int *status = kCheckedBuild ? device_status_ptr() : nullptr;
-    if (tuning_get("PACK", 64) == 64) {
-        const int k_chunks = ceil_div(K, 64);
-        const long tasks = (long)nMB * k_chunks;
-        static bool attr64_set[64] = {false};
-        int dev = 0;
-        ESMM_CUDA_TRY(cudaGetDevice(&dev));
-        const int smem = PACK_WARPS * PACK64_SMEM_PER_WARP;
-        if (dev >= 0 && dev < 64 && !attr64_set[dev]) {
-            ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_preprocess_a_pack64_kernel,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            attr64_set[dev] = true;
-        }
-        long blocks = (tasks + PACK_WARPS - 1) / PACK_WARPS;
-        const long cap = (long)sms * 6 * 8;
-        if (blocks > cap) blocks = cap;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)blocks);
-        cfg.blockDim = dim3(PACK_WARPS * 32);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        // Few rows: the strip kernel's CTAs are placed while this kernel ends, and an SM whose shared memory is carved out for less
-        // than they need takes none of them until it has (M = 16, K = 4096: 344 strips on 132 of 148 SMs).  Not for large A: with
-        // so little left of L1 4096^2 is packed more slowly (whole call at 32-granular 0.2 / 0.2 167 -> 175 us).
-        cudaLaunchAttribute attr[2];
-        int attrs = 0;
-        if (!tuning_get("NO_DEPENDENT_LAUNCH", 0)) {
-            attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
-        }
-        if (nMB == 1) {
-            attr[attrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-            attr[attrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
-        }
-        cfg.attrs = attr;
-        cfg.numAttrs = attrs;
-        ESMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, esmm_preprocess_a_pack64_kernel, d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status));
-        ESMM_CUDA_TRY(cudaGetLastError());
-        return ESMM_OK;
-    }
-    const int k_chunks = ceil_div(K, 128);
+    const int k_chunks = ceil_div(K, PACK_COLS);
     const long tasks = (long)nMB * k_chunks;
-    static bool attr_set[64] = {false};
-    int dev = 0;
-    ESMM_CUDA_TRY(cudaGetDevice(&dev));
-    const int smem = PACK_WARPS * PACK_SMEM_PER_WARP;
-    if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(esmm_preprocess_a_pack_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr_set[dev] = true;
-    }
     long blocks = (tasks + PACK_WARPS - 1) / PACK_WARPS;
-    const long cap = (long)sms * 3 * 8;
+    const long cap = (long)sms * 8 * 8;
     if (blocks > cap) blocks = cap;
-    esmm_preprocess_a_pack_kernel<<<(unsigned)blocks, PACK_WARPS * 32, smem, stream>>>(
-        d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(PACK_WARPS * 32);
+    cfg.stream = stream;
+    // Few rows: the strip kernel's CTAs are placed while this kernel ends, and an SM whose shared memory is carved out for less
+    // than they need takes none of them until it has (M = 16, K = 4096: 344 strips on 132 of 148 SMs).
+    cudaLaunchAttribute attr[2];
+    int attrs = 0;
+    if (!tuning_get("NO_DEPENDENT_LAUNCH", 0)) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (nMB == 1) {
+        attr[attrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[attrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = attrs;
+    ESMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, esmm_preprocess_a_pack32_kernel, d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status));
     ESMM_CUDA_TRY(cudaGetLastError());
     return ESMM_OK;
 }

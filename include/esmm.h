@@ -229,9 +229,9 @@ int esmm_selftest_bounded_wait(unsigned budget_us, void *stream);
  * environment cannot change what the library does.  No counterpart in the reference, whose tile
  * shapes are compile-time template constants (include/runners.cuh:830-838).
  * Names: TILE_M (64 | 128), STAGES, BROW_BITS, ROW_DENSITY, FORCE_LISTED, NO_RUN_TILES, VEC_PATTERNS
- * (0 | 4 | 16), NO_SKINNY, SKINNY_ROWS (32), PRODUCER_WARPS (3 | 7 | 0: pins the tiled kernel's launch shape),
- * BLOCK_MODE (0 | 1: pins the tiled kernel's way of working, see esmm_gemm_blocks.cuh; -1: its own rule, also in short launches), NO_DEPENDENT_LAUNCH, GROUP_M, GRID, PACK (64 | 128), TF32_PAIR (0 | 128 | 256), TF32_SPLIT_LAST,
- * TF32_DIRECT_STORES, and SWIZZLE, which is accepted and without effect (the kernel it was for is gone).  esmm_tuning_set returns ESMM_ERR_UNSUPPORTED for any other name;
+ * (0 | 4 | 16), NO_SKINNY, SKINNY_ROWS (16 | 32), PRODUCER_WARPS (3 | 7 | 0: pins the tiled kernel's launch shape),
+ * BLOCK_MODE (0 | 1: pins the tiled kernel's way of working, see esmm_gemm_blocks.cuh; -1: its own rule, also in short launches), NO_DEPENDENT_LAUNCH, GROUP_M, GRID, TF32_PAIR (0 | 128 | 256), TF32_SPLIT_LAST,
+ * TF32_DIRECT_STORES, and SWIZZLE and PACK, which are accepted and without effect (the kernels they were for are gone).  esmm_tuning_set returns ESMM_ERR_UNSUPPORTED for any other name;
  * esmm_tuning_reset returns every hook to "unset" (the library's own choice).
  */
 int esmm_tuning_set(const char *name, int value);

@@ -1129,3 +1129,35 @@ def test_gemm_block_mode_pair_lists(cuda, pkg, oracle_mod, tuning, kind, swap, N
     pkg.device_status()
     want = oracle_mod.gemm_joint(A, np.ascontiguousarray(B))
     assert np.array_equal(C_.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("M,K", [(1, 4), (31, 28), (32, 32), (33, 36), (129, 100), (64, 1000), (200, 516), (40, 2048)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_packing_kernel_edges(cuda, pkg, oracle_mod, M, K, shift):
+    """The packing kernel's 32 x 32 tasks at the edges of A: pattern bytes as words and (a row of K blocks that is no multiple of four,
+    an array that starts at an odd address) one by one, -0 and denormals, the packed copy of every live k, zeros in rows past the last, and
+    nothing written for a dead k."""
+    nkb, panels = -(-K // 8), -(-M // 128)
+    rng = np.random.default_rng(M * K)
+    A = rng.standard_normal((M, K), dtype=np.float32)
+    for r in range(0, M, 32):
+        A[r:r + 32, rng.random(K) < 0.5] = 0.0
+    A[M - 1, 0], A[0, K - 1], A[M // 2, K // 2] = -0.0, 1e-45, -1e-45
+    dA = cuda.from_numpy(A).cuda()
+    want = oracle_mod.preprocess_a(A)
+    raw = cuda.full((want.size + 2,), 0xEE, dtype=cuda.uint8, device="cuda")
+    mark = 123.25
+    packed = cuda.full((panels, nkb * 8, 128), mark, device="cuda")
+    pkg.preprocess_a_packed(dA.data_ptr(), M, K, raw.data_ptr() + shift, packed.data_ptr())
+    pkg.device_status()
+    got = raw.cpu().numpy()
+    assert np.array_equal(got[shift:shift + want.size].reshape(want.shape), want)
+    assert (np.delete(got, np.s_[shift:shift + want.size]) == 0xEE).all()
+    live = np.unpackbits(want, axis=1, bitorder="little").astype(bool)      # [row block][k]
+    full = np.zeros((panels * 128, nkb * 8), np.float32)
+    full[:M, :K] = A
+    expect = np.full((panels, nkb * 8, 128), mark, np.float32)
+    for mb in range(live.shape[0]):
+        rows = slice((mb % 4) * 32, (mb % 4) * 32 + 32)
+        expect[mb // 4, live[mb], rows] = full[mb * 32:mb * 32 + 32, live[mb]].T
+    assert np.array_equal(packed.cpu().numpy().view(np.uint32), expect.view(np.uint32))
