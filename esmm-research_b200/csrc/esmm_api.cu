@@ -23,7 +23,8 @@ int gemm_ab_packed_launch(int M, int N, int K, const float *d_a_packed, const fl
 int gemm_ab_packed_prepare();
 int preprocess_a_launch(const float *d_A, int M, int K, int tile_m, uint8_t *d_out, cudaStream_t stream);
 int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, float *d_packed,
-                             cudaStream_t stream);
+                             cudaStream_t stream, bool beside);
+bool gemm_ab_skinny_applies(int M, int N, int K);
 int preprocess_b_launch(const float *d_B, int K, int N, uint8_t *d_out, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------
@@ -53,6 +54,7 @@ static const char *const kTuningNames[] = {"TILE_M", "STAGES", "BROW_BITS", "ROW
 constexpr int kTuningCount = (int)(sizeof kTuningNames / sizeof kTuningNames[0]);
 static std::atomic<int> g_tuning_value[kTuningCount];
 static std::atomic<bool> g_tuning_set[kTuningCount];
+static std::atomic<bool> g_tuning_any;   // one is set: without, no name is looked up
 
 static int tuning_index(const char *name)
 {
@@ -64,8 +66,18 @@ static int tuning_index(const char *name)
 
 int tuning_get(const char *name, int dflt)
 {
+    if (!g_tuning_any.load(std::memory_order_acquire)) return dflt;
     const int i = tuning_index(name);
     return (i >= 0 && g_tuning_set[i].load(std::memory_order_acquire)) ? g_tuning_value[i].load() : dflt;
+}
+
+bool tiled_kernel_tuned()
+{
+    if (!g_tuning_any.load(std::memory_order_acquire)) return false;
+    for (const char *name : {"TILE_M", "STAGES", "BROW_BITS", "ROW_DENSITY", "FORCE_LISTED", "NO_RUN_TILES", "VEC_PATTERNS", "PRODUCER_WARPS",
+                             "BLOCK_MODE", "GROUP_M", "GRID"})
+        if (g_tuning_set[tuning_index(name)].load(std::memory_order_acquire)) return true;
+    return false;
 }
 
 __device__ int g_esmm_device_status;
@@ -302,12 +314,14 @@ int esmm_tuning_set(const char *name, int value)
     if (i < 0) return ESMM_ERR_UNSUPPORTED;
     esmm::g_tuning_value[i].store(value);
     esmm::g_tuning_set[i].store(true, std::memory_order_release);
+    esmm::g_tuning_any.store(true, std::memory_order_release);
     return ESMM_OK;
 }
 
 void esmm_tuning_reset(void)
 {
     for (int i = 0; i < esmm::kTuningCount; ++i) esmm::g_tuning_set[i].store(false, std::memory_order_release);
+    esmm::g_tuning_any.store(false, std::memory_order_release);
 }
 
 int esmm_pattern_from_string(const char *s)
@@ -348,7 +362,7 @@ int esmm_sgemm_joint(int M, int N, int K, const float *d_A, const float *d_B, fl
     if ((uintptr_t)d_workspace & 255) return ESMM_ERR_ALIGN;
     uint8_t *a_pat = static_cast<uint8_t *>(d_workspace);
     float *a_packed = reinterpret_cast<float *>(a_pat + pattern_region_bytes(M, K));
-    int st = esmm::preprocess_a_pack_launch(d_A, M, K, a_pat, a_packed, (cudaStream_t)stream);
+    int st = esmm::preprocess_a_pack_launch(d_A, M, K, a_pat, a_packed, (cudaStream_t)stream, esmm::gemm_ab_skinny_applies(M, N, K));
     if (st != ESMM_OK) return st;
     return esmm::gemm_ab_packed_launch(M, N, K, a_packed, d_B, d_C, a_pat, d_b_pat, (cudaStream_t)stream);
 }
@@ -509,7 +523,7 @@ int esmm_plan_submit(esmm_plan *pl, const float *h_A, float *h_C)
         ESMM_CUDA_TRY(cudaStreamWaitEvent(s_run, pl->down[c], 0));
         uint8_t *apat = pl->d_a_pat + (size_t)(r0 / 32) * nKB;
         float *apacked = pl->d_a_packed + (size_t)r0 * nKB * esmm::BK;  // r0 is a multiple of 128
-        int st = esmm::preprocess_a_pack_launch(pl->d_A + a_off, r1 - r0, K, apat, apacked, s_run);
+        int st = esmm::preprocess_a_pack_launch(pl->d_A + a_off, r1 - r0, K, apat, apacked, s_run, esmm::gemm_ab_skinny_applies(r1 - r0, N, K));
         if (st != ESMM_OK) return st;
         st = esmm::gemm_ab_packed_launch(r1 - r0, N, K, apacked, pl->d_B, pl->d_C + c_off, apat, pl->d_b_pat,
                                          s_run);
@@ -893,7 +907,7 @@ int esmm_run_kernel_pattern(int kernel_id, int rows, int cols, int inners, float
                         st = esmm_preprocess_b(d_B, inners, cols, d_bp, 0);
                     }
                 }
-                if (st == ESMM_OK) st = esmm::preprocess_a_pack_launch(d_A, rows, inners, d_ap, d_packed, 0);
+                if (st == ESMM_OK) st = esmm::preprocess_a_pack_launch(d_A, rows, inners, d_ap, d_packed, 0, rows <= 32);
                 if (st == ESMM_OK)
                     st = esmm::gemm_ab_packed_launch(rows, cols, inners, d_packed, d_B, d_C, d_ap, d_bp, 0);
                 cudaDeviceSynchronize();
@@ -905,7 +919,7 @@ int esmm_run_kernel_pattern(int kernel_id, int rows, int cols, int inners, float
             st = esmm_preprocess_ab(d_A, d_B, rows, cols, inners, a_tile, d_b_pat_cached, &meta);
             if (st != ESMM_OK) break;
             if (d_packed) {
-                st = esmm::preprocess_a_pack_launch(d_A, rows, inners, meta.d_a_patterns, d_packed, 0);
+                st = esmm::preprocess_a_pack_launch(d_A, rows, inners, meta.d_a_patterns, d_packed, 0, rows <= 32);
                 if (st == ESMM_OK)
                     st = esmm::gemm_ab_packed_launch(rows, cols, inners, d_packed, d_B, d_C, meta.d_a_patterns,
                                                      meta.d_b_patterns, 0);

@@ -27,6 +27,7 @@ int record_cuda_error_text(const char *text);
 // Tuning and test hooks (esmm_tuning_set): the value set for `name`, else `dflt`.  Nothing is read
 // from the process environment.
 int tuning_get(const char *name, int dflt);
+bool tiled_kernel_tuned();   // whether a hook of the tiled kernel is set: then problems that have a choice take that kernel
 
 // Device status word shared by all kernels of the library (0 = ok).
 int *device_status_ptr();  // device address, valid after the first call on the current device

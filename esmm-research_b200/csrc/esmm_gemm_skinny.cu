@@ -1,35 +1,39 @@
-// Joint-sparse FP32 SGEMM for sm_100a, few rows: M <= 32 (one 32-row pattern block of A).
+// Joint-sparse FP32 SGEMM for sm_100a, few rows: the strip kernel, for M <= 32 (one 32-row pattern block of A) and for problems of a
+// few row blocks that have too few tiles for the GPU.
 //
-// Same arithmetic as the packed kernel (esmm_gemm_tiled.cuh) and as esmm_ab_optimized_v3 of the
-// reference (src/kernels/esmm_ab_optimized_v3.cu:157, 183-203): for every output one FMA chain in
-// ascending k over the k whose joint bit is set.  With a single row block of A the large kernel has
-// M / 128 x N / 128 = N / 128 tiles, runs half of its consumer warps on rows that do not exist and
-// leaves a third of the SMs idle (N = 11008: 86 tiles).  Here the work is cut the other way:
+// Same arithmetic as the packed kernel (esmm_gemm_tiled.cuh) and as esmm_ab_optimized_v3 of the reference
+// (src/kernels/esmm_ab_optimized_v3.cu:157, 183-203): for every output one FMA chain in ascending k over the k whose joint bit is set.
+// With a single row block of A the large kernel has M / 128 x N / 128 = N / 128 tiles, runs half of its consumer warps on rows that do
+// not exist and leaves a third of the SMs idle (N = 11008: 86 tiles).  Here the work is cut the other way:
 //
-//   * one CTA per 32-column strip of C (N / 32 CTAs, several resident per SM).  A strip is exactly one
-//     pattern block of B, so its live k are a_pat[0][kb] & b_pat[strip][kb]: every listed row is live
-//     for the whole CTA, there are no per-warp masks and no index lists in the inner loop;
-//   * all threads first build the strip's list of live k (pattern bytes read as 32-bit words); then stages of
-//     64 k travel through a ring of four as 16-byte asynchronous copies: per k 128 bytes of B and 32, 64 or 128 bytes of
-//     packed A (rows 0-7, 0-15 or 0-31 of the first panel: as many as M needs);
+//   * one CTA per row block and 32-column strip of C (N / 32 of them per row block, several resident per SM).  That is exactly one
+//     pattern block of A and one of B, so its live k are a_pat[rb][kb] & b_pat[strip][kb]: every listed row is live for the whole CTA,
+//     there are no per-warp masks and no index lists in the inner loop;
+//   * all threads first build the strip's list of live k (pattern bytes read as 32-bit words); then stages of 64 k travel through a
+//     ring of four (three or two, where K is long and an SM has room for more strips so) as 16-byte asynchronous copies: per k 128
+//     bytes of B and 32, 64 or 128 bytes of packed A (8, 16 or 32 of the block's rows: as many as M needs);
 //   * two warps copy, a stage each in turn, two or four multiply.  A stage's barrier takes an arrival of every copying lane when its
 //     copies have landed (cp.async.mbarrier.arrive.noinc); the multiplying warps hand the slot back.  No warp does both: copies in the
-//     multiplying warps' own instruction stream, with a barrier of the whole CTA per 32 k, were what the kernel before spent most
-//     of its time on (the call below: FMA pipe 22 % active);
-//   * a multiplying thread holds 4 x 4, 4 x 2 or 2 x 2 outputs as row pairs times one broadcast column.  The operands of four k
-//     are loaded (volatile, so that they stay put) one batch ahead of the multiply-adds that use them, two register sets in
-//     ping-pong, over the stages' borders too;
-//   * co-resident strips start their roles at different warps (by %warpid), so that the multiplying warps of an SM's two or three strips
-//     lie on different SM sub-partitions: with every strip's on the same one the call below takes 39 us.
+//     multiplying warps' own instruction stream, with a barrier of the whole CTA per 32 k, were what the kernel before spent most of
+//     its time on (the first call below: FMA pipe 22 % active);
+//   * a multiplying thread holds 4 x 4, 4 x 2 or 2 x 2 outputs as row pairs times one broadcast column.  The operands of four k are
+//     loaded (volatile, so that they stay put) one batch ahead of the multiply-adds that use them, two register sets in ping-pong,
+//     over the stages' borders too;
+//   * the multiplying warps of an SM's strips lie on different SM sub-partitions.  The hardware starts a CTA's first warp on any of
+//     the four, so a CTA with two multiplying warps takes its turn from a counter per SM and places them by its own %warpid (without:
+//     K = 4096 dense, 32 rows, three and four strips per SM 13-20 % slower on average and up to twice as long where all fall
+//     together).
 //
-// What bounds it: a multiplying warp is alone on its SM sub-partition, so its loads' issue and its multiply-adds add up: 13 cycles a k for
-// 4 x 2 outputs (8 of multiply-adds) with no copies and no barriers at all, 15 with them; on SMs with three strips shared memory (7.5 of
-// its wavefronts per strip and k).  Measured, whole calls, the kernel before -> this one: M = 16, N = 11008, K = 4096 pruned MLP (819 live k
-// per strip, 344 strips) 28.5 -> 22.5 us; M = 8 28.4 -> 16.4; M = 1 19.4 -> 12.7; M = 32 34.1 -> 29.0; dense, N = 4096, K = 4096,
-// M = 16 61.5 -> 36.2; dense, N = 11008, M = 1 100.5 -> 50.5; N = 512, K = 16384, M = 6 148 -> 72.  Also measured (same inputs as the
-// first): stages of 32 k 10-20 % slower, of 128 in a ring of two as fast, k of a batch 2 or 8 and three batches ahead as fast, 4 x 4 outputs
-// by one multiplying warp 39 us, counters in shared memory with release / acquire instead of barriers 3-5 % slower.
-// Every wait is bounded: a wait that runs out raises the abort flag, nothing is stored and the status word tells.
+// What bounds it: a multiplying warp is alone or nearly so on its SM sub-partition, so its loads' issue and its multiply-adds add up:
+// 13 cycles a k for 4 x 2 outputs (8 of multiply-adds) with no copies and no barriers at all, 15 with them; on SMs with three or more
+// strips shared memory (10 of its wavefronts per strip of 32 rows and k, 7.5 of 16).  Measured, whole calls, the kernel before -> this
+// one: M = 16, N = 11008, K = 4096 pruned MLP (819 live k per strip, 344 strips) 28.5 -> 19.3 us; M = 8 28.4 -> 14.1; M = 1 19.4 ->
+// 10.6; M = 32 34.1 -> 27.3; dense, N = 4096, K = 4096, M = 16 61.5 -> 33.5; dense, N = 11008, M = 1 100.5 -> 47.4; N = 512, K =
+// 16384, M = 6 148 -> 70.  Also measured: stages of 32 k 10-20 % slower, of 128 in a ring of two as fast, k of a batch 2 or 8 and
+// three batches ahead as fast, counters in shared memory with release / acquire instead of barriers 3-5 % slower; lanes past B's last
+// column that all copy the matrix's first bytes instead of others of their row: N = 300, 32 row blocks 118 us instead of 61. Every
+// wait is bounded: a wait that runs out raises the abort flag, nothing is stored and the status word tells.
+#include <algorithm>
 #include <cstring>
 
 #include "esmm_gemm_shared.cuh"
@@ -37,23 +41,36 @@
 namespace esmm {
 
 constexpr int SK_COLS = 32;                     // columns of a strip = one B pattern block
-constexpr int SK_ROWS = 32;                     // rows of C handled (M <= 32)
+constexpr int SK_ROWS = 32;                     // rows of a row block = one A pattern block
 constexpr int SK_STAGE_ROWS = 64;               // k per stage
 constexpr int SK_ROW_BYTES = 128;               // one k of B in shared memory
-constexpr int SK_STAGES = 4;                    // (a power of two)
+constexpr int SK_MAX_STAGES = 4;                // of the ring; two at least
 constexpr int SK_MAX_KP = 16384;                // longest K the row list is sized for
 constexpr int SK_BATCH = 4;                     // k per register set of operands
 constexpr int SK_SETS = 2;                      // register sets
 
+// Whose turn it is, per SM: the CTAs of two multiplying warps that an SM gets one after the other have them on different SM
+// sub-partitions.  (A hint: whatever the counters hold, every CTA has its two.)
+constexpr int SK_TURNS = 256;
+__device__ unsigned g_sk_turn[SK_TURNS];
+
 struct SkinnyParams {
     int M, N, K, nKB, kp, cap;
-    const uint8_t *a_pat;   // row block 0 of the A patterns
+    int row_blocks, stages;
+    const uint8_t *a_pat;
     const uint8_t *b_pat;
-    const float *a_packed;  // [k][128]: rows 0-31 of the first panel are read
+    const float *a_packed;  // [panel][k][128]: a quarter of a panel's rows are read
     const float *B;
     float *C;
     int *status;
 };
+
+// bits of the k of K blocks kb .. kb + 3 that are < K (a pattern may mark more of a ragged last K block live: there is no B for them)
+__device__ __forceinline__ unsigned sk_inside(int kb, int K)
+{
+    const int left = K - kb * BK;
+    return left >= 32 ? 0xFFFFFFFFu : left <= 0 ? 0u : (1u << left) - 1u;
+}
 
 __device__ __forceinline__ int sk_scan(int v, int lane)
 {
@@ -63,6 +80,11 @@ __device__ __forceinline__ int sk_scan(int v, int lane)
         if (lane >= d) v += t;
     }
     return v;
+}
+
+__device__ __forceinline__ void sk_copy_16(uint32_t dst, const char *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
 // (one group of copies per stage and lane)
@@ -78,10 +100,14 @@ __device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool on)
 
 // Shared memory: ring | list (u16 x cap) | warp sums | full and empty barriers, abort flag
 __host__ __device__ constexpr int sk_stage_bytes(int rows) { return SK_STAGE_ROWS * (rows * 4 + SK_ROW_BYTES); }
-__host__ __device__ constexpr size_t sk_list_off(int rows) { return (size_t)SK_STAGES * sk_stage_bytes(rows); }
-__host__ __device__ constexpr size_t sk_sum_off(int rows, int cap) { return sk_list_off(rows) + (((size_t)cap * 2 + 15) & ~(size_t)15); }
-__host__ __device__ constexpr size_t sk_bar_off(int rows, int cap) { return sk_sum_off(rows, cap) + 32; }
-__host__ __device__ constexpr size_t sk_smem(int rows, int cap) { return sk_bar_off(rows, cap) + 2 * SK_STAGES * 8 + 16; }
+__host__ __device__ constexpr size_t sk_sum_off(int rows, int stages, int cap)
+{
+    return (size_t)stages * sk_stage_bytes(rows) + (((size_t)cap * 2 + 15) & ~(size_t)15);
+}
+__host__ __device__ constexpr size_t sk_smem(int rows, int stages, int cap)
+{
+    return sk_sum_off(rows, stages, cap) + 32 + 2 * SK_MAX_STAGES * 8 + 16;
+}
 
 // ROWS: rows of C that are fetched and multiplied, 8, 16 or 32.  CW: warps that multiply, PW: warps that copy.  RT: rows per thread.
 template <int ROWS, int CW, int PW, int RT>
@@ -92,23 +118,28 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
     constexpr int A_HALF = SK_STAGE_ROWS * A_ROW_BYTES;             // A rows, then B rows
     constexpr int STAGE_BYTES = sk_stage_bytes(ROWS);
     constexpr int SK_WARPS = CW + PW, SK_THREADS = SK_WARPS * 32;
-    static_assert(SK_WARPS < 8, "warp sums");
+    static_assert(SK_WARPS < 8 && (CW == 2 ? SK_WARPS == 4 : CW == 4), "warp sums; roles");
     extern __shared__ __align__(1024) char smem[];
-    uint16_t *krow = reinterpret_cast<uint16_t *>(smem + sk_list_off(ROWS));
-    volatile int *wsum = reinterpret_cast<volatile int *>(smem + sk_sum_off(ROWS, p.cap));
-    const uint32_t full0 = smem_u32(smem + sk_bar_off(ROWS, p.cap)), empty0 = full0 + SK_STAGES * 8;
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + sk_bar_off(ROWS, p.cap) + 2 * SK_STAGES * 8);
+    uint16_t *krow = reinterpret_cast<uint16_t *>(smem + (size_t)p.stages * STAGE_BYTES);
+    char *rest = smem + sk_sum_off(ROWS, p.stages, p.cap);
+    volatile int *wsum = reinterpret_cast<volatile int *>(rest);
+    const uint32_t full0 = smem_u32(rest + 32), empty0 = full0 + SK_MAX_STAGES * 8;
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(rest + 32 + 2 * SK_MAX_STAGES * 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int strip = blockIdx.x;
+    const int strip = blockIdx.x / p.row_blocks, rb = blockIdx.x - strip * p.row_blocks;
+    const uint8_t *a_pat = p.a_pat + (size_t)rb * p.nKB;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < SK_STAGES; ++s) {
+        for (int s = 0; s < SK_MAX_STAGES; ++s) {
             mbar_init(full0 + 8 * s, 32);         // a copying warp's lanes, when their copies have landed
             mbar_init(empty0 + 8 * s, CW);
         }
         *abort_flag = 0;
-        unsigned place;                           // of the CTA among those on its SM
-        asm volatile("mov.u32 %0, %%warpid;" : "=r"(place));
-        wsum[SK_WARPS] = (int)place / SK_WARPS;
+        if (CW == 2) {
+            unsigned sm, slot;
+            asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+            asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+            wsum[SK_WARPS] = (int)(slot + 2u * atomicAdd(&g_sk_turn[sm % SK_TURNS], 1u)) & 3;
+        }
     }
     grid_dependency_wait();   // (the A patterns and the packed copy come from the kernel before this one)
 
@@ -122,7 +153,7 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
         const uint8_t *bp = p.b_pat + (size_t)strip * p.nKB;
         const int per = ((p.nKB + SK_THREADS - 1) / SK_THREADS + 3) & ~3;
         const int kb_lo = min((int)threadIdx.x * per, p.nKB), kb_hi = min(kb_lo + per, p.nKB);
-        const bool words = (p.nKB & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.a_pat) | reinterpret_cast<uintptr_t>(bp)) & 3) == 0;
+        const bool words = (p.nKB & 3) == 0 && ((reinterpret_cast<uintptr_t>(a_pat) | reinterpret_cast<uintptr_t>(bp)) & 3) == 0;
         unsigned live[MAX_WORDS];
         int c = 0;
 #pragma unroll
@@ -131,11 +162,12 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
             unsigned v = 0u;
             if (kb < kb_hi) {
                 if (words) {
-                    v = *reinterpret_cast<const unsigned *>(p.a_pat + kb) & *reinterpret_cast<const unsigned *>(bp + kb);
+                    v = *reinterpret_cast<const unsigned *>(a_pat + kb) & *reinterpret_cast<const unsigned *>(bp + kb);
                 } else {
-                    for (int j = 0; j < 4 && kb + j < kb_hi; ++j) v |= (unsigned)(p.a_pat[kb + j] & bp[kb + j]) << (8 * j);
+                    for (int j = 0; j < 4 && kb + j < kb_hi; ++j) v |= (unsigned)(a_pat[kb + j] & bp[kb + j]) << (8 * j);
                 }
             }
+            v &= sk_inside(kb, p.K);
             live[w] = v;
             c += __popc(v);
         }
@@ -171,7 +203,7 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
     const int num_stages = (n + SK_STAGE_ROWS - 1) / SK_STAGE_ROWS;
     const int col0 = strip * SK_COLS;
     // the warps' roles: strips that share an SM have their multiplying warps on different SM sub-partitions
-    const int role = (warp + wsum[SK_WARPS] * CW) % SK_WARPS;
+    const int role = CW == 2 ? (warp + wsum[SK_WARPS]) & 3 : warp;
     bool ok = true;
 
     if (role >= CW) {
@@ -181,16 +213,22 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
         constexpr int A_LANES = ROWS / 4, A_N = A_LANES;            // lanes per row of A; instructions per 32 rows
         const int b_row = (lane >> 3) * 8, b_chunk = lane & 7;
         const int a_row = lane / A_LANES * A_N, a_chunk = lane % A_LANES;
-        const bool col_ok = col0 + b_chunk * 4 < p.N;
-        const char *b_src = reinterpret_cast<const char *>(col_ok ? p.B + col0 + b_chunk * 4 : p.B);
-        const char *a_src = reinterpret_cast<const char *>(p.a_packed + a_chunk * 4);
-        const unsigned n4 = col_ok ? (unsigned)p.N * 4u : 0u;
+        // (columns past B's last one: another chunk of the same row; what is multiplied there is not stored)
+        const char *b_src = reinterpret_cast<const char *>(p.B + col0 + (col0 + b_chunk * 4 < p.N ? b_chunk * 4 : 0));
+        const char *a_src = reinterpret_cast<const char *>(p.a_packed + (size_t)(rb >> 2) * p.kp * TILE_M + (rb & 3) * 32 + a_chunk * 4);
+        const unsigned n4 = (unsigned)p.N * 4u;
         const uint32_t dst_a = smem_u32(smem) + (uint32_t)(a_row * A_ROW_BYTES + a_chunk * 16);
         const uint32_t dst_b = smem_u32(smem) + (uint32_t)(A_HALF + b_row * SK_ROW_BYTES + b_chunk * 16);
-        for (int s = role - CW; s < num_stages; s += PW) {
-            const int slot = s & (SK_STAGES - 1);
+        int slot = role - CW;
+        uint32_t phase = 1u;                                        // of the slot's empty barrier that the warp waits for
+        static_assert(PW <= 2, "a warp's first slot and its steps along the ring");
+        for (int s = role - CW; s < num_stages; s += PW, slot += PW) {
+            if (slot >= p.stages) {
+                slot -= p.stages;
+                phase ^= 1u;
+            }
             if (!bounds_ok((s + 1) * SK_STAGE_ROWS <= p.cap, p.status, 31)) break;
-            ok = mbar_wait(empty0 + 8 * slot, ((s / SK_STAGES) & 1) ^ 1, abort_flag);
+            ok = mbar_wait(empty0 + 8 * slot, phase, abort_flag);
             if (!ok) break;
 #pragma unroll
             for (int h = 0; h < SK_STAGE_ROWS / 32; ++h) {
@@ -211,14 +249,13 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    if (!bounds_ok(kb[j] < (unsigned)p.kp, p.status, 32)) continue;   // site 32: a k outside the packed panel / B
-                    const bool in = kb[j] < (unsigned)p.K;                            // past B's last row: zeros
-                    cp_async_16(dst_b + s_off + (h * 32 + j) * SK_ROW_BYTES, b_src + (size_t)(in ? kb[j] : 0u) * n4, in ? 16 : 0);
+                    if (!bounds_ok(kb[j] < (unsigned)p.K, p.status, 32)) continue;   // site 32: a k outside B / the packed panel
+                    sk_copy_16(dst_b + s_off + (h * 32 + j) * SK_ROW_BYTES, b_src + (size_t)kb[j] * n4);
                 }
 #pragma unroll
                 for (int j = 0; j < A_N; ++j) {
                     if (!bounds_ok(ka[j] < (unsigned)p.kp, p.status, 32)) continue;
-                    cp_async_16(dst_a + s_off + (h * 32 + j) * A_ROW_BYTES, a_src + (size_t)ka[j] * (TILE_M * 4), 16);
+                    sk_copy_16(dst_a + s_off + (h * 32 + j) * A_ROW_BYTES, a_src + (size_t)ka[j] * (TILE_M * 4));
                 }
             }
             sk_copies_arrive(full0 + 8 * slot);
@@ -288,12 +325,15 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
             }
         }
         // (after a wait that ran out the sums are worthless and not stored; the loop goes on, as the waits no longer do)
+        int slot = 0;
+        uint32_t phase = 0u;
         for (int s = 0; s < num_stages; ++s) {
-            const int slot = s & (SK_STAGES - 1), cnt = n - s * SK_STAGE_ROWS;
+            const int cnt = n - s * SK_STAGE_ROWS;
             const uint32_t s_off = (uint32_t)slot * STAGE_BYTES;
             if (cnt > SK_STAGE_ROWS) {
-                const int next = (s + 1) & (SK_STAGES - 1);
-                const uint32_t next_bar = full0 + 8 * next, next_phase = ((s + 1) / SK_STAGES) & 1;
+                const bool wrap = slot + 1 == p.stages;
+                const int next = wrap ? 0 : slot + 1;
+                const uint32_t next_bar = full0 + 8 * next, next_phase = phase ^ (wrap ? 1u : 0u);
                 bool ready = false;
 #pragma unroll
                 for (int b = 0; b < BATCHES; ++b) {
@@ -308,6 +348,8 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
                 }
                 __syncwarp();
                 mbar_arrive_if(empty0 + 8 * slot, lane == 0);
+                slot = next;
+                phase = next_phase;
             } else {
                 // the last stage (batches loaded past its last row are in bounds and never multiplied)
 #pragma unroll
@@ -322,7 +364,7 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
         const int col = col0 + colw;
 #pragma unroll
         for (int e = 0; e < RT; ++e) {
-            const int r = row0 + e;
+            const int r = rb * SK_ROWS + row0 + e;
             float v[CT];
 #pragma unroll
             for (int j = 0; j < CT; ++j) v[j] = (e & 1) ? c[e >> 1][j].y : c[e >> 1][j].x;
@@ -336,11 +378,25 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
     if (!ok && lane == 0) atomicExch(p.status, (int)ESMM_ERR_TIMEOUT);
 }
 
-// Whether the few-rows kernel takes a problem (otherwise the packed kernel does).
+// Whether this kernel takes a problem (otherwise the tiled kernel does).  Of M <= 32 all; of fewer than two whole panels of 128 rows
+// those for which it takes less time whatever the operands: a strip and row block of 32 rows is counted as 1 per SM, a 64-row tile of
+// eight of them as 5 (a strip takes 13.7 cycles a k with several on an SM, a tile 87, and the tiled kernel is as fast as 1.2 times
+// that on blocks that differ), a 128-row tile as 9.1.  Tiled / strips, us, K = 4096: 64 x 1024 dense 184 / 42, 64 x 4096 185 / 64, 64
+// x 4096 a quarter live 51.8 / 19.8, 96 x 4096 pruned MLP 44.8 / 27.2, 64 x 11008 x 2048 pruned MLP (4.7 per SM) 33.9 / 24.1, 100 x
+// 6000 x 3000 0.5 / 0.5 (5.1) 53.9 / 36.2; on the other side 256 x 4096 dense (6.9) 188 / 205 and pruned MLP 60.4 / 51.7, 1000 x 1508
+// x 2012 0.5 / 0.5 (10.4) 48.5 / 51.2.  Taller problems stay with the tiled kernel and its launch shapes, which callers can ask for
+// (esmm_last_tiled_kernel_warps).
 bool gemm_ab_skinny_applies(int M, int N, int K)
 {
     const int kp = ceil_div(K, BK) * BK;
-    return M <= SK_ROWS && kp <= SK_MAX_KP && N >= 4 * SK_COLS && tuning_get("NO_SKINNY", 0) == 0;
+    if (kp > SK_MAX_KP || M >= 2 * TILE_M || tuning_get("NO_SKINNY", 0)) return false;
+    if (M <= SK_ROWS) return N >= 4 * SK_COLS;
+    if (tiled_kernel_tuned()) return false;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return false;
+    const long units = (long)ceil_div(M, SK_ROWS) * ceil_div(N, SK_COLS), across = ceil_div(N, TILE_N);
+    const long rounds64 = (ceil_div(M, 64) * across + sms - 1) / sms, rounds128 = (ceil_div(M, TILE_M) * across + sms - 1) / sms;
+    return (double)units <= sms * std::min(5.0 * rounds64, 9.1 * rounds128);
 }
 
 int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const float *d_B, float *d_C,
@@ -354,6 +410,7 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
     p.nKB = ceil_div(K, BK);
     p.kp = p.nKB * BK;
     p.cap = p.kp + SK_STAGE_ROWS;
+    p.row_blocks = ceil_div(M, SK_ROWS);
     p.a_pat = d_a_pat;
     p.b_pat = d_b_pat;
     p.a_packed = d_a_packed;
@@ -366,17 +423,22 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
     ESMM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int strips = ceil_div(N, SK_COLS), forced = tuning_get("SKINNY_ROWS", 0);
     const int rows = M > 16 || forced == 32 ? 32 : M > 8 || forced == 16 ? 16 : 8;
+    const long units = (long)strips * p.row_blocks;
     auto launch = [&](auto kernel, int r, int warps) -> int {
-        const size_t smem = sk_smem(r, p.cap);
+        // the ring as deep as it can be with as many CTAs on an SM as there are for it, up to four
+        const size_t room = (size_t)(SMEM_LIMIT + 1024) / std::min(4l, (units + sms - 1) / sms) - 1024;
+        p.stages = SK_MAX_STAGES;
+        while (p.stages > 2 && sk_smem(r, p.stages, p.cap) > room) --p.stages;
+        const size_t smem = sk_smem(r, p.stages, p.cap);
         ESMM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        ESMM_CUDA_TRY(launch_dependent(kernel, dim3(strips), dim3(warps * 32), smem, stream, p));
+        ESMM_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)units), dim3(warps * 32), smem, stream, p));
         ESMM_CUDA_TRY(cudaGetLastError());
         return ESMM_OK;
     };
     // Four multiplying warps where an SM has one or two strips; with three, shared memory bounds the kernel and two warps, which
     // load less of A, are faster.  The multiplying part alone, us, two / four warps, K = 4096: M = 16 dense, one strip per SM 31.1 / 28.6;
     // M = 16 pruned MLP, SMs with two strips 9.2 / 8.6, with three 9.9 / 11.6; M = 32 one strip 10.3 / 7.6, two 14.2 / 11.7, three 14.9 / 16.2.
-    const bool spread = strips <= 2 * sms;
+    const bool spread = units <= 2 * sms;
     if (rows == 8) return launch(esmm_joint_sgemm_skinny_kernel<8, 2, 2, 2>, 8, 4);
     if (rows == 16)
         return spread ? launch(esmm_joint_sgemm_skinny_kernel<16, 4, 2, 2>, 16, 6) : launch(esmm_joint_sgemm_skinny_kernel<16, 2, 2, 4>, 16, 4);

@@ -25,7 +25,8 @@ namespace esmm {
 int gemm_ab_packed_launch_form(int M, int N, int K, const float *d_a_packed, const float *d_B, float *d_C,
                                const uint8_t *d_a_pat, const uint8_t *d_b_pat, cudaStream_t stream, bool follow_hint);
 int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, float *d_packed,
-                             cudaStream_t stream);
+                             cudaStream_t stream, bool beside);
+bool gemm_ab_skinny_applies(int M, int N, int K);
 
 constexpr size_t STATIC_PATTERN_BYTES = ESMM_STATIC_MAX_PATTERN_BYTES;                      // 64 KiB
 constexpr size_t STATIC_PACKED_BYTES = (size_t)ESMM_STATIC_MAX_PACKED_FLOATS * sizeof(float);  // 32 MiB
@@ -81,7 +82,7 @@ extern "C" int esmm_sgemm_joint_static(int M, int N, int K, const float *d_A, co
     if (!scratch) return st;
     uint8_t *a_pat = scratch;
     float *a_packed = reinterpret_cast<float *>(scratch + esmm::STATIC_PATTERN_BYTES);
-    st = esmm::preprocess_a_pack_launch(d_A, M, K, a_pat, a_packed, (cudaStream_t)stream);
+    st = esmm::preprocess_a_pack_launch(d_A, M, K, a_pat, a_packed, (cudaStream_t)stream, esmm::gemm_ab_skinny_applies(M, N, K));
     if (st != ESMM_OK) return st;
     return esmm::gemm_ab_packed_launch_form(M, N, K, a_packed, d_B, d_C, a_pat, d_b_pat, (cudaStream_t)stream, false);
 }

@@ -104,11 +104,11 @@ constexpr int PACK_COLS = 32;
 
 __global__ void __launch_bounds__(PACK_WARPS * 32)
 esmm_preprocess_a_pack32_kernel(const float *A, int M, int K, int nMB, int nKB, int k_chunks,
-                                uint8_t *__restrict__ out, float *__restrict__ packed, int *status)
+                                uint8_t *__restrict__ out, float *__restrict__ packed, int *status, int early)
 {
     // The product kernel, launched as a dependent of this one, may be placed where SMs become free once every CTA of this
     // grid has got here; it waits for this grid's end itself.
-    grid_launch_dependents();
+    if (early) grid_launch_dependents();
     // This kernel is a dependent launch too, of whatever was before it: it is launched as that ends rather than after, which takes 2 us off
     // every call of a train of them (1000 x 1508 x 2012 57.4 -> 55.2 us, 1024^3 at half density 32.9 -> 30.9).  The product kernels don't
     // call it early: strips placed beside those of the call before are 15-100 % slower.  Nothing of A is read before the wait, and what is
@@ -300,8 +300,9 @@ int preprocess_a_launch(const float *d_A, int M, int K, int tile_m, uint8_t *d_o
     return ESMM_OK;
 }
 
+// beside: the kernel after this one has several CTAs per SM.
 int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, float *d_packed,
-                             cudaStream_t stream)
+                             cudaStream_t stream, bool beside)
 {
     if (!d_A || !d_out || !d_packed) return ESMM_ERR_NULL;
     if (M <= 0 || K <= 0 || (K & 3)) return ESMM_ERR_SHAPE;
@@ -327,13 +328,14 @@ int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, flo
         attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (nMB == 1) {
+    if (beside) {
         attr[attrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
         attr[attrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
     }
     cfg.attrs = attr;
     cfg.numAttrs = attrs;
-    ESMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, esmm_preprocess_a_pack32_kernel, d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status));
+    const int early = !beside || blocks <= sms;
+    ESMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, esmm_preprocess_a_pack32_kernel, d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status, early));
     ESMM_CUDA_TRY(cudaGetLastError());
     return ESMM_OK;
 }
@@ -394,7 +396,7 @@ size_t esmm_a_packed_bytes(int M, int K)
 
 int esmm_preprocess_a_packed(const float *d_A, int M, int K, uint8_t *d_out, float *d_packed, void *stream)
 {
-    return esmm::preprocess_a_pack_launch(d_A, M, K, d_out, d_packed, (cudaStream_t)stream);
+    return esmm::preprocess_a_pack_launch(d_A, M, K, d_out, d_packed, (cudaStream_t)stream, M <= 32);
 }
 
 int esmm_preprocess_b(const float *d_B, int K, int N, uint8_t *d_out, void *stream)

@@ -1161,3 +1161,36 @@ def test_packing_kernel_edges(cuda, pkg, oracle_mod, M, K, shift):
         rows = slice((mb % 4) * 32, (mb % 4) * 32 + 32)
         expect[mb // 4, live[mb], rows] = full[mb * 32:mb * 32 + 32, live[mb]].T
     assert np.array_equal(packed.cpu().numpy().view(np.uint32), expect.view(np.uint32))
+
+
+@pytest.mark.parametrize("M", [33, 64, 100, 255])
+@pytest.mark.parametrize("N", [36, 1000, 4740])
+def test_gemm_strips_of_several_row_blocks(cuda, pkg, oracle_mod, M, N):
+    """Problems of two to eight row blocks with too few tiles for the GPU take the strip kernel: ragged rows and columns, one to five
+    strips per SM (two and four multiplying warps), row blocks with lists of their own, empty ones among them, K of one K block, of a ragged
+    one and long enough for a shallower ring; the oracle's bits."""
+    for K, pa, pb in [(8, 1.0, 1.0), (76, 0.8, 0.8), (1028, 0.5, 0.6), (4096, 0.1, 0.4)] + ([(16384, 0.1, 0.2)] if N == 1000 else []):
+        A, B = workloads.tile_random(M, N, K, pa, pb, seed=M + N + K, gran_a=32, gran_b=32)
+        if K == 1028:
+            A[32:64] = 0.0
+        check_all_paths(cuda, pkg, oracle_mod, A, B)
+
+
+def test_gemm_strips_pattern_bits_past_k(cuda, pkg, oracle_mod):
+    """K % 8 == 4 and patterns of the caller that mark k past K live: the strip kernel multiplies none of them."""
+    for M, N, K in [(20, 256, 76), (70, 164, 1020)]:
+        rng = np.random.default_rng(K)
+        A = rng.standard_normal((M, K), dtype=np.float32)
+        B = rng.standard_normal((K, N), dtype=np.float32)
+        nkb = -(-K // 8)
+        dA, dB = cuda.from_numpy(A).cuda(), cuda.from_numpy(B).cuda()
+        ap = cuda.empty((-(-M // 32), nkb), dtype=cuda.uint8, device="cuda")
+        packed = cuda.full((-(-M // 128) * nkb * 8 * 128,), float("nan"), device="cuda")
+        pkg.preprocess_a_packed(dA.data_ptr(), M, K, ap.data_ptr(), packed.data_ptr())
+        ap.fill_(0xFF)
+        bp = cuda.full((-(-N // 32), nkb), 0xFF, dtype=cuda.uint8, device="cuda")
+        c = cuda.full((M, N), float("nan"), device="cuda")
+        pkg.gemm_ab_packed(M, N, K, packed.data_ptr(), dB.data_ptr(), c.data_ptr(), ap.data_ptr(), bp.data_ptr())
+        pkg.device_status()
+        want = oracle_mod.gemm_joint(A, B, np.full((-(-M // 32), nkb), 0xFF, np.uint8), np.full((-(-N // 32), nkb), 0xFF, np.uint8))
+        assert np.array_equal(c.cpu().numpy().view(np.uint32), want.view(np.uint32)), (M, N, K)
