@@ -196,14 +196,12 @@ struct LiveList {
     __device__ __forceinline__ int pending() const { return made - taken; }
 };
 
-// BM_STEP steps of a stage: 8 x 8 outputs per thread, each half-warp on its own rows of X and Y.  SWAP: odd rows hold the upper half
-// of their 128 bytes first (see the copies).
-template <bool SWAP>
+// BM_STEP steps of a stage: 8 x 8 outputs per thread, each half-warp on its own rows of X and Y.
 __device__ __forceinline__ void pair_steps(Acc &acc, const char *sx, const char *sy)
 {
 #pragma unroll
     for (int r = 0; r < BM_STEP; ++r) {
-        const int lo = r * 128 + (SWAP ? (r & 1) * 64 : 0), hi = r * 128 + 64 - (SWAP ? (r & 1) * 64 : 0);
+        const int lo = r * 128, hi = r * 128 + 64;
         KFrag f;
         f.at = *reinterpret_cast<const float4 *>(sx + lo);
         f.ab = *reinterpret_cast<const float4 *>(sx + hi);
@@ -223,6 +221,42 @@ __device__ __forceinline__ void single_steps(Acc &acc, const char *sx, const cha
         f.at = *reinterpret_cast<const float4 *>(((r & 1) ? sx_odd : sx) + r * 128);
         f.b0 = *reinterpret_cast<const float4 *>(sy + r * 128 + (r & 1) * 64);
         f.b1 = *reinterpret_cast<const float4 *>(sy + r * 128 + 64 - (r & 1) * 64);
+        fma_top(acc, f);
+    }
+}
+
+// Row-major A: the eight 16-byte chunks of row r of a stage lie at their number XOR rm_swizzle(r), so that 4-byte copies of eight k of
+// four rows of A fall on all 32 banks; 16-byte copies and the loads below meet as few bank conflicts as without.  (Odd rows' halves
+// swapped and nothing more, block mode of 2048^3 alone: 64-granular 0.5 / 0.5 175 us, 143 so; 32-granular 0.5 / 0.5 207 and 171.)
+__host__ __device__ constexpr int rm_swizzle(int r) { return ((r >> 1) & 3) | ((r & 1) << 2); }
+
+// pair_steps and single_steps on such rows.  The lane's chunks: xg and xg + 4, yg and yg + 4; of a single block lm, ln and ln + 4.
+__device__ __forceinline__ void rm_pair_steps(Acc &acc, const char *sx, const char *sy, int xg, int yg)
+{
+#pragma unroll
+    for (int r = 0; r < BM_STEP; ++r) {
+        const int sw = rm_swizzle(r), lo = r * 128 + (sw & 4) * 16, hi = r * 128 + 64 - (sw & 4) * 16;
+        const char *x = sx + ((xg ^ (sw & 3)) << 4), *y = sy + ((yg ^ (sw & 3)) << 4);
+        KFrag f;
+        f.at = *reinterpret_cast<const float4 *>(x + lo);
+        f.ab = *reinterpret_cast<const float4 *>(x + hi);
+        f.b0 = *reinterpret_cast<const float4 *>(y + lo);
+        f.b1 = *reinterpret_cast<const float4 *>(y + hi);
+        fma_top(acc, f);
+        fma_bottom(acc, f);
+    }
+}
+
+__device__ __forceinline__ void rm_single_steps(Acc &acc, const char *sx, const char *sy, int lm, int ln)
+{
+#pragma unroll
+    for (int r = 0; r < BM_STEP; ++r) {
+        const int sw = rm_swizzle(r);
+        const char *y = sy + ((ln ^ (sw & 3)) << 4);
+        KFrag f;
+        f.at = *reinterpret_cast<const float4 *>(sx + ((lm ^ sw) << 4) + r * 128);
+        f.b0 = *reinterpret_cast<const float4 *>(y + r * 128 + (sw & 4) * 16);
+        f.b1 = *reinterpret_cast<const float4 *>(y + r * 128 + 64 - (sw & 4) * 16);
         fma_top(acc, f);
     }
 }
@@ -260,7 +294,7 @@ __device__ __forceinline__ void fill_16(uint32_t dst, float v)
 
 // One item: blocks x0 and x0 + 1 of X (TWO) or x0 alone, times block y of Y.
 // ROW_MAJOR: A is the caller's matrix instead of the k-major packed copy; 4-byte copies transpose it on the way.
-// EDGE: blocks of B may be cut off by its last column.  AGREE: X's blocks had the same patterns in pairs wherever samples were taken.
+// EDGE: blocks of B may be cut off by its last column, blocks of row-major A by its last row.  AGREE: X's blocks had the same patterns in pairs wherever samples were taken.
 template <bool TWO, bool ROW_MAJOR, bool EDGE, bool AGREE, typename Params>
 __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane, bool wide_b, int x0, int y)
 {
@@ -273,8 +307,8 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     // Copies of a pair from packed A: eight lanes per row, a lane's rows are 4 r4 .. 4 r4 + 3, so that its list entries are one load and the
     // rows of one copy instruction are whole (80 bytes a clock and SM arrive so at most, 64 in the other order).
     const int r4 = lane >> 3, c8 = lane & 7;
-    const uint32_t dst = smem_u32(ring) + (uint32_t)(r4 * 512 + c8 * 16);
-    // Single blocks, and all with row-major A: four lanes per row of the stage, eight rows at a time; a lane moves the 16-byte chunks c4
+    const uint32_t dst = smem_u32(ring) + (uint32_t)(r4 * 512 + ((ROW_MAJOR ? c8 ^ rm_swizzle(r4 * 4) : c8) << 4));
+    // Single blocks: four lanes per row of the stage, eight rows at a time; a lane moves the 16-byte chunks c4
     // and c4 + 4 of its row.  Rows are 128 bytes apart; odd rows have their two halves swapped, so that the eight rows of one copy
     // instruction fall on all banks.  (Fewer addresses: 100 x 6000 x 3000, single blocks only, 54.7 us so, 56.6 in the order above.)
     const int r8 = lane >> 2, c4 = lane & 3;
@@ -295,6 +329,16 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     const int b_chunks = (p.N - b_blk * 32) >> 2;
     const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);
     const int x_chunks = wide_b ? b_chunks : 16, y_chunks = wide_b ? 8 : b_chunks;
+    // Row-major A: the lane's k of a copy, its row within a chunk of four and where it lands.  Rows of A past its last one: one of the rows
+    // before them; columns of B past its last one: others of the same row (what is multiplied there ends in rows and columns of C that do
+    // not exist).
+    const int a_kk = lane & (RM_KL - 1), a_rr = lane / RM_KL;
+    const char *a_rows = reinterpret_cast<const char *>(p.A) + ((size_t)a_blk * 32 + a_rr) * p.K * 4;
+    const char *b_rows = b_src + (!EDGE || c8 < b_chunks ? c8 * 16 : 0);
+    const int b_next = c8 + 8 < b_chunks ? 128 : 0;               // from the lane's chunk of one block of B to the next block's
+    const uint32_t dst_a = smem_u32(ring) + (uint32_t)(a_kk * 128 + (rm_swizzle(a_kk) << 4) + a_rr * 4);
+    const unsigned k16 = (unsigned)p.K * 16u;                     // four rows
+    const bool plain = p.K <= 65536 && (!EDGE || p.M >= 4);       // list entries are whole k; (EDGE) no chunk of four rows is before A
     const bool x_ok0 = c8 < x_chunks, x_ok1 = c8 + 8 < x_chunks, y_ok = c8 < y_chunks;
 
     Acc acc;
@@ -377,59 +421,93 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
         const uint32_t to = BM_SLOT_BYTES - slot;
         bool same_next = false;
         if constexpr (ROW_MAJOR) {
-            const int r16 = lane & 15;
-            auto entry = [&](const LiveList &l, int wrap, int row, int d) {
-                const int pos = l.taken + row;
-                return row < d ? (unsigned)l.list[pos & (BM_LIST - 1)] + (pos >= wrap ? 65536u : 0u) : 0u;
+            auto entry = [&](int blk, int row) {
+                const int pos = (blk ? l1.taken : l0.taken) + row;
+                const uint16_t *list = blk && !one_list ? l1.list : l0.list;
+                return (unsigned)list[pos & (BM_LIST - 1)] + (pos >= (blk && !one_list ? wrap1 : wrap0) ? 65536u : 0u);
             };
             same_next = TWO && d0 == BM_ROWS && d1 == BM_ROWS &&
-                        __all_sync(0xFFFFFFFFu, entry(l0, wrap0, r16, d0) == entry(l1, wrap1, r16, d1));
-            // B: Y of either block, or X
+                        (one_list || __all_sync(0xFFFFFFFFu, entry(0, lane & 15) == entry(1, lane & 15)));
+            // A: X of either block, or Y.  RM_KL lanes on the k, four on the rows of a 16-byte chunk.
+            const bool a_twice = TWO && !(wide_b && same_next), b_twice = TWO && !(!wide_b && same_next);
+            const uint32_t to_a = dst_a + to + (wide_b ? 2 * BM_PART : 0), to_b = dst + to + (wide_b ? 0 : 2 * BM_PART);
+            if (plain && d0 == BM_ROWS && (!TWO || d1 == BM_ROWS)) {
+                auto copy_a = [&](int blk, const uint16_t *list) {
+                    const int down = blk && !wide_b ? 32 : 0;
+                    const char *base = a_rows + (size_t)down * p.K * 4;
+                    const unsigned k0 = list[0], k1 = list[RM_KL];
+                    const char *g0 = base + k0 * 4u, *g1 = base + k1 * 4u;
+                    if (!k_ok(p, k0) || !k_ok(p, k1)) return;
+                    const int last_q = (p.M - 1 - a_blk * 32 - down - a_rr) >> 2;   // (EDGE)
 #pragma unroll
-            for (int h = 0; h < BM_ROWS / 8; ++h) {
-                const int row = h * 8 + r8;
+                    for (int q = 0; q < 8; ++q) {
+                        const uint32_t e = (to_a ^ (q << 4)) + blk * BM_PART;
+                        if (EDGE) {
+                            const long rows = (long)min(q, last_q) * (int)k16;
+                            cp_async_4(e, g0 + rows);
+                            cp_async_4(e + RM_KL * 128, g1 + rows);
+                        } else {
+                            cp_async_4(e, row_of(g0, q, k16));
+                            cp_async_4(e + RM_KL * 128, row_of(g1, q, k16));
+                        }
+                    }
+                };
+                auto copy_b = [&](int blk, const uint16_t *list, bool both) {
+                    const uint2 v = *reinterpret_cast<const uint2 *>(list);
+                    const char *base = b_rows + (wide_b && blk ? (EDGE ? b_next : 128) : 0);
 #pragma unroll
-                for (int blk = 0; blk < (TWO ? 2 : 1); ++blk) {
-                    const int d = blk ? d1 : d0;
-                    if (max(d0, d1) == 0 || (blk && !wide_b && same_next)) continue;
-                    const char *g = b_src + c4 * 16 + (size_t)entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d) * n4 + (wide_b ? blk * 128 : 0);
-                    const uint32_t part = (uint32_t)((wide_b ? 0 : 2) + blk) * BM_PART;
-                    const uint32_t e0 = dst0 + to + h * 1024 + part, e1 = dst1 + to + h * 1024 + part;
-                    if (row < d && k_ok(p, entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d))) {
-                        const int lim = b_chunks - (wide_b ? blk * 8 : 0);
-                        if (!edge || c4 < lim) cp_async_16(e0, g, 16);
-                        if (!edge || c4 + 4 < lim) cp_async_16(e1, g + 64, 16);
-                    } else {
-                        fill_16(e0, wide_b ? -0.0f : 0.0f);
-                        fill_16(e1, wide_b ? -0.0f : 0.0f);
+                    for (int j = 0; j < 4; ++j) {
+                        const unsigned w = j & 2 ? v.y : v.x, k = j & 1 ? w >> 16 : w & 0xFFFFu;
+                        if (!k_ok(p, k)) continue;
+                        const char *g = row_of(base, k, n4);
+                        const uint32_t e = (to_b ^ (rm_swizzle(j) << 4)) + j * 128 + blk * BM_PART;
+                        copy_16<0>(e, g);
+                        if (both) {
+                            if (EDGE) copy_16<0>(e + BM_PART, g + b_next);
+                            else copy_16<128>(e + BM_PART, g);
+                        }
+                    }
+                };
+                // (One body for both lists: its instructions, not their number, are what the loop has too many of.  Unrolled, 32-granular
+                // 0.5 / 0.5, 2048^3: 171 us instead of 154.  Edges in this code for every launch: 4096^3 64-granular 850 instead of 811.)
+                const uint16_t *list0 = l0.list + (l0.taken & (BM_LIST - 1)), *list1 = one_list ? list0 : l1.list + (l1.taken & (BM_LIST - 1));
+
+                if (TWO && wide_b && same_next) {
+                    copy_a(0, list0 + a_kk);
+                    copy_b(0, list0 + r4 * 4, true);
+                } else {
+#pragma unroll 1
+                    for (int blk = 0; blk < (TWO ? 2 : 1); ++blk) {
+                        const uint16_t *list = blk ? list1 : list0;
+                        copy_a(blk, list + a_kk);
+                        if (!blk || b_twice) copy_b(blk, list + r4 * 4, false);
                     }
                 }
-            }
-            // A: X of either block, or Y.  RM_KL lanes on the k, 32 / RM_KL on the rows.
-            constexpr int RL = 32 / RM_KL, STEPS = 32 / RL;
-            const int kk = lane & (RM_KL - 1), rr = lane / RM_KL;
+            } else if (max(d0, d1) > 0) {
+                // Past the end of a list X = -0 and Y = +0 (below).  Rows past the end of A: any row, what is multiplied there ends in
+                // rows of C that do not exist.
+#pragma unroll 1
+                for (int i = 0; i < (a_twice ? 4 : 2); ++i) {
+                    const int blk = i >> 1, row = (i & 1) * RM_KL + a_kk, row0 = (a_blk + (wide_b ? 0 : blk)) * 32 + a_rr;
+                    const bool listed = row < (blk ? d1 : d0);
+                    const unsigned k = listed ? entry(blk, row) : 0u;
+                    if (listed && !k_ok(p, k)) continue;
 #pragma unroll
-            for (int blk = 0; blk < (TWO ? 2 : 1); ++blk) {
-                const int d = blk ? d1 : d0;
-                if (max(d0, d1) == 0 || (blk && wide_b && same_next)) continue;
-                const int row0 = (a_blk + (wide_b ? 0 : blk)) * 32 + rr;
-                const uint32_t part = smem_u32(ring) + to + (uint32_t)((wide_b ? 2 : 0) + blk) * BM_PART + kk * 128 + rr * 4;
-                const uint32_t e0 = part + (kk & 1) * 64, e1 = part + 64 - (kk & 1) * 64;
-#pragma unroll
-                for (int g = 0; g < BM_ROWS / RM_KL; ++g) {
-                    const int row = g * RM_KL + kk;
-                    const float *src = p.A + (size_t)row0 * p.K + entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d);
-                    if (row < d && k_ok(p, entry(blk ? l1 : l0, blk ? wrap1 : wrap0, row, d))) {
-#pragma unroll
-                        for (int q = 0; q < STEPS; ++q) {
-                            // (rows past the end of A: any row, what is multiplied there ends in rows of C that do not exist)
-                            const float *sq = row0 + q * RL < p.M ? src + (size_t)(q * RL) * p.K : p.A;
-                            cp_async_4((q < STEPS / 2 ? e0 : e1) + g * (RM_KL * 128) + (q & (STEPS / 2 - 1)) * (RL * 4), sq);
-                        }
+                    for (int q = 0; q < 8; ++q) {
+                        const uint32_t e = (to_a ^ (q << 4)) + (i & 1) * (RM_KL * 128) + blk * BM_PART;
+                        if (listed) cp_async_4(e, p.A + (size_t)min(row0 + 4 * q, p.M - 1) * p.K + k);
+                        else fill_4(e, wide_b ? 0.0f : -0.0f);
+                    }
+                }
+#pragma unroll 1
+                for (int i = 0; i < (b_twice ? 8 : 4); ++i) {
+                    const int blk = i >> 2, j = i & 3, row = r4 * 4 + j;
+                    const uint32_t e = (to_b ^ (rm_swizzle(j) << 4)) + j * 128 + blk * BM_PART;
+                    if (row < (blk ? d1 : d0)) {
+                        const size_t k = entry(blk, row);
+                        if (k_ok(p, k) && c8 + (wide_b ? blk * 8 : 0) < b_chunks) copy_16<0>(e, b_rows + (wide_b ? blk * 128 : 0) + k * n4);
                     } else {
-#pragma unroll
-                        for (int q = 0; q < STEPS; ++q)
-                            fill_4((q < STEPS / 2 ? e0 : e1) + g * (RM_KL * 128) + (q & (STEPS / 2 - 1)) * (RL * 4), wide_b ? 0.0f : -0.0f);
+                        fill_16(e, wide_b ? -0.0f : 0.0f);
                     }
                 }
             }
@@ -503,10 +581,17 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
         cp_async_commit();
         // ---- the stage itself ----
         const char *st = ring + slot;
-        if (TWO) {
+        if (ROW_MAJOR) {
+            const char *sx = st + (TWO ? half * BM_PART : 0), *sy = st + (TWO && !same ? 2 + half : 2) * BM_PART;
+#pragma unroll 1
+            for (int r = 0; r < count; r += BM_STEP) {
+                if (TWO) rm_pair_steps(acc, sx + r * 128, sy + r * 128, xg, yg);
+                else rm_single_steps(acc, sx + r * 128, sy + r * 128, lm, ln);
+            }
+        } else if (TWO) {
             const char *sx = st + half * BM_PART + xg * 16, *sy = st + (same ? 2 : 2 + half) * BM_PART + yg * 16;
 #pragma unroll 1
-            for (int r = 0; r < count; r += BM_STEP) pair_steps<ROW_MAJOR>(acc, sx + r * 128, sy + r * 128);
+            for (int r = 0; r < count; r += BM_STEP) pair_steps(acc, sx + r * 128, sy + r * 128);
         } else {
             const char *sx = st + lm * 16, *sx_odd = st + (lm ^ 4) * 16, *sy = st + 2 * BM_PART + ln * 16;
 #pragma unroll 1

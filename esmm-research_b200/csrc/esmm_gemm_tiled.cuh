@@ -74,9 +74,10 @@ constexpr int P_TMA_WARP = P_CONSUMER_WARPS;                   // first producer
 // 0.9 / 0.9) 2050 / 2087, 1 (dense) 2130 / 2549.
 constexpr int BM_SIXTEENTHS = 11;
 // The same for row-major A, where block mode has to transpose A for every pair of blocks: kernel alone, pipeline / block mode, share 0.11
-// (32-granular, 0.2 / 0.2) 2048^3 83 / 71 us, 4096^3 455 / 437; share 0.16 (0.3 / 0.3) 123 / 113, 724 / 686; share 0.33 (0.5 / 0.5) 4096^3
-// 1194 / 1402; share 0.44 (64-granular, 0.5 / 0.5) 2048^3 147 / 178.
-constexpr int RM_SIXTEENTHS = 4;
+// (32-granular, 0.2 / 0.2) 2048^3 79 / 64 us; pruned MLP (0.31) 2048 x 11008 x 4096 1267 / 827, 64 x 4096 x 4096 77 / 54; share 0.33
+// (0.5 / 0.5) 2048^3 186 / 151, 1000 x 1508 x 2012 98 / 67; share 0.44 (64-granular, 0.5 / 0.5) 2048^3 142 / 140, 4096^3 882 / 811; share 0.50
+// (32-granular, 0.7 / 0.7) 2048^3 281 / 252, 4096^3 1828 / 1833; share 0.53 (1 / 0.5) 257 / 265, 1683 / 1772.
+constexpr int RM_SIXTEENTHS = 8;
 
 // Optional timeline for tuning (build with -DESMM_TRACE): CTA 0 stamps %globaltimer at a few points
 // into a device array that esmm_trace_read copies out.  Not part of the product build or of the ABI.
@@ -667,9 +668,18 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
                 // 2048 x 11008 x 4096 744 -> 724, 4096^3 64-granular 0.5 / 0.5 692 -> 674 us, 32-granular 0.2 / 0.2 164 either way (165 with one
                 // list until they differ, which is at once).
                 const bool wide_b = (mode & MODE_BLOCKS_WIDE_B) != 0;
-                if (RM || (p.N & 63)) block_mode<RM, true, false>(p, smem, warp, lane, wide_b, next_item);
-                else if (mode & MODE_BLOCKS_AGREE) block_mode<RM, RM, !RM>(p, smem, warp, lane, wide_b, next_item);
-                else block_mode<RM, RM, false>(p, smem, warp, lane, wide_b, next_item);
+                if (RM) {
+                    // (which operand's blocks come in pairs is a constant of the code: 2048 x 11008 x 4096 856 -> 827, ragged 3562 x 724 x 1336
+                    // 85 -> 81)
+                    if ((p.N & 63) || (p.M & 63)) {
+                        if (wide_b) block_mode<RM, true, false>(p, smem, warp, lane, true, next_item);
+                        else block_mode<RM, true, false>(p, smem, warp, lane, false, next_item);
+                    } else if (!wide_b) block_mode<RM, false, false>(p, smem, warp, lane, false, next_item);
+                    else if (mode & MODE_BLOCKS_AGREE) block_mode<RM, false, true>(p, smem, warp, lane, true, next_item);
+                    else block_mode<RM, false, false>(p, smem, warp, lane, true, next_item);
+                } else if (p.N & 63) block_mode<RM, true, false>(p, smem, warp, lane, wide_b, next_item);
+                else if (mode & MODE_BLOCKS_AGREE) block_mode<RM, false, true>(p, smem, warp, lane, wide_b, next_item);
+                else block_mode<RM, false, false>(p, smem, warp, lane, wide_b, next_item);
             }
             return;
         }

@@ -1194,3 +1194,15 @@ def test_gemm_strips_pattern_bits_past_k(cuda, pkg, oracle_mod):
         pkg.device_status()
         want = oracle_mod.gemm_joint(A, B, np.full((-(-M // 32), nkb), 0xFF, np.uint8), np.full((-(-N // 32), nkb), 0xFF, np.uint8))
         assert np.array_equal(c.cpu().numpy().view(np.uint32), want.view(np.uint32)), (M, N, K)
+
+
+@pytest.mark.parametrize("M", [1, 3, 33, 64, 100, 158, 192])
+@pytest.mark.parametrize("N", [4, 36, 64, 100, 192, 228])
+def test_rowmajor_block_mode_edges(cuda, pkg, oracle_mod, tuning, M, N):
+    """Row-major A in block mode: its last rows and B's last columns inside a block or at a block's or a pair's end, fewer rows than a
+    chunk of four; live k that agree in pairs on A's side, on B's, or nowhere; stages that lists fill, and ends of lists; the oracle's bits."""
+    tuning("BLOCK_MODE", 1)
+    tuning("GRID", 2)
+    for K, ga, gb in [(76, 32, 32), (1020, 64, 32), (1020, 32, 64), (2052, 32, 32)]:
+        A, B = workloads.tile_random(M, N, K, 0.6, 0.6, seed=M + N + K, gran_a=ga, gran_b=gb)
+        check_all_paths(cuda, pkg, oracle_mod, A, B)
