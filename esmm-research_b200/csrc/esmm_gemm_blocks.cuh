@@ -294,7 +294,8 @@ __device__ __forceinline__ void fill_16(uint32_t dst, float v)
 
 // One item: blocks x0 and x0 + 1 of X (TWO) or x0 alone, times block y of Y.
 // ROW_MAJOR: A is the caller's matrix instead of the k-major packed copy; 4-byte copies transpose it on the way.
-// EDGE: blocks of B may be cut off by its last column, blocks of row-major A by its last row.  AGREE: X's blocks had the same patterns in pairs wherever samples were taken.
+// EDGE: blocks of B may be cut off by its last column, blocks of row-major A by its last row.  AGREE: X's blocks had the same patterns in
+// pairs wherever samples were taken.
 template <bool TWO, bool ROW_MAJOR, bool EDGE, bool AGREE, typename Params>
 __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane, bool wide_b, int x0, int y)
 {

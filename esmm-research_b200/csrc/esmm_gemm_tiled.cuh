@@ -525,6 +525,7 @@ __device__ __noinline__ int listed_warp_rows(const uint8_t *rmask, int n, int la
 // samples, free again on return.  (A call rather than inline code: it runs once per CTA, and what follows gets better registers: pruned
 // MLP 2048 x 11008 x 4096 765 -> 748 us, 1000 x 1508 x 2012 at 0.5 / 0.5 59.4 -> 57.4, 4096^3 dense 2165 -> 2148.  Block mode as a call
 // spills: 866, 67.6, 2170.)
+// MODE_BLOCKS_WIDE_B: pairs of column blocks; MODE_BLOCKS_AGREE: which had the same patterns wherever samples were taken.
 enum { MODE_PIPELINE = 0, MODE_BLOCKS = 1, MODE_BLOCKS_WIDE_B = 2, MODE_BLOCKS_AGREE = 4 };
 
 template <bool RM>
@@ -583,8 +584,11 @@ __device__ __noinline__ int choose_mode(const PackedParams &p, char *scratch, in
     }
     __syncthreads();   // the samples have been read by all
     if (!blocks) return MODE_PIPELINE;
-    const bool wide_b = RM ? b_differ <= a_differ : b_differ < a_differ;
-    return MODE_BLOCKS | (wide_b ? MODE_BLOCKS_WIDE_B : 0) | ((wide_b ? b_differ : a_differ) == 0 ? MODE_BLOCKS_AGREE : 0);
+    // Pairs on the side whose blocks differ less.  Where neither does more, on B's: an item then has one block of A, which row-major A is
+    // transposed for (16 and not 32 copies a stage), and with packed A the faster code; not at N's edge (1500^3, 64-granular 0.5 / 0.5
+    // 49.3 us, 48.5 with A's).
+    const bool wide_b = RM || !(p.N & 63) ? b_differ <= a_differ : b_differ < a_differ;
+    return MODE_BLOCKS | (wide_b ? MODE_BLOCKS_WIDE_B : 0) | (wide_b && b_differ == 0 ? MODE_BLOCKS_AGREE : 0);
 }
 
 // The CTA's next row list: the tile's next one, or the first of its next tile.
@@ -663,23 +667,20 @@ __device__ __forceinline__ void tiled_sgemm(const PackedMaps &maps, const Packed
         if (mode != MODE_PIPELINE) {
             if (warp < BM_WARPS) {
                 // The code of a whole launch, so that no two kinds of it compete for the instruction cache (items at N's edge alone
-                // with predicates of their own: 2330 x 932 x 5020 128 -> 136 us).  Column blocks all whole: copies without predicates;
-                // blocks that agree in pairs, where samples were taken: one list for both until they differ.  Without / with: pruned MLP
-                // 2048 x 11008 x 4096 744 -> 724, 4096^3 64-granular 0.5 / 0.5 692 -> 674 us, 32-granular 0.2 / 0.2 164 either way (165 with one
-                // list until they differ, which is at once).
+                // with predicates of their own: 2330 x 932 x 5020 128 -> 136 us).  Blocks all whole: copies without predicates; column
+                // blocks that agree in pairs, where samples were taken: one list for both until they differ; and which operand's blocks come in
+                // pairs is a constant.  Without / with the first two: pruned MLP 2048 x 11008 x 4096 744 -> 724, 4096^3 64-granular 0.5 / 0.5
+                // 692 -> 674 us, 32-granular 0.2 / 0.2 164 either way (165 with one list until they differ, which is at once).  The constant:
+                // 720 -> 701, 672 -> 651 (with column blocks in pairs, too: 680 with A's), 162 -> 160, 2330 x 932 x 5020 125 -> 123;
+                // row-major 2048 x 11008 x 4096 856 -> 827.  Row blocks that agree have no code for it: A 64-granular, B 32-granular 677 us
+                // with it, 655 without.
                 const bool wide_b = (mode & MODE_BLOCKS_WIDE_B) != 0;
-                if (RM) {
-                    // (which operand's blocks come in pairs is a constant of the code: 2048 x 11008 x 4096 856 -> 827, ragged 3562 x 724 x 1336
-                    // 85 -> 81)
-                    if ((p.N & 63) || (p.M & 63)) {
-                        if (wide_b) block_mode<RM, true, false>(p, smem, warp, lane, true, next_item);
-                        else block_mode<RM, true, false>(p, smem, warp, lane, false, next_item);
-                    } else if (!wide_b) block_mode<RM, false, false>(p, smem, warp, lane, false, next_item);
-                    else if (mode & MODE_BLOCKS_AGREE) block_mode<RM, false, true>(p, smem, warp, lane, true, next_item);
-                    else block_mode<RM, false, false>(p, smem, warp, lane, true, next_item);
-                } else if (p.N & 63) block_mode<RM, true, false>(p, smem, warp, lane, wide_b, next_item);
-                else if (mode & MODE_BLOCKS_AGREE) block_mode<RM, false, true>(p, smem, warp, lane, wide_b, next_item);
-                else block_mode<RM, false, false>(p, smem, warp, lane, wide_b, next_item);
+                if ((p.N & 63) || (RM && (p.M & 63))) {
+                    if (wide_b) block_mode<RM, true, false>(p, smem, warp, lane, true, next_item);
+                    else block_mode<RM, true, false>(p, smem, warp, lane, false, next_item);
+                } else if (!wide_b) block_mode<RM, false, false>(p, smem, warp, lane, false, next_item);
+                else if (mode & MODE_BLOCKS_AGREE) block_mode<RM, false, true>(p, smem, warp, lane, true, next_item);
+                else block_mode<RM, false, false>(p, smem, warp, lane, true, next_item);
             }
             return;
         }
