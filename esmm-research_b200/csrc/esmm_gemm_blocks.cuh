@@ -5,8 +5,8 @@
 // of 32 such rows, eight warps together.  On operands whose 32-row and 32-column blocks are zero in different places most of
 // a fetched row is of no use to most of the warps, and a step lasts as long as its busiest warp.  Here nothing is shared:
 //
-//   * an item is a pair of adjacent 32 x 32 blocks of C: 64 rows x 32 columns, or 32 rows x 64 columns where B's patterns agree in
-//     pairs of column blocks more often than A's in pairs of row blocks.  The operand that spans 64 is called X, the one that
+//   * an item is a pair of adjacent 32 x 32 blocks of C: 32 rows x 64 columns where B's patterns agree in pairs of column blocks as
+//     often as A's in pairs of row blocks, or more often (and N is a multiple of 64), else 64 rows x 32 columns.  The operand that spans 64 is called X, the one that
 //     spans 32 Y;
 //   * a warp joins the pattern bytes of each block to a list of its live k (ascending, 16 bits each, a ring of 512
 //     that is refilled as it is used up).  Lanes
@@ -24,8 +24,8 @@
 // what the FMAs need: every one of the others costs about 0.7 cycles of it, wherever it stands.  So they are kept few: one load per list
 // for a lane's entries, one instruction per address, no predicates where all of B's blocks are whole, one list for blocks that agree.
 // The rest is lost to the end of a launch (3-4 % between SMs, whose items differ, 2 % inside them).  Measured, whole calls, the tiled pipeline before ->
-// block mode: 2048 x 11008 x 4096 pruned MLP 1016 -> 724 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 164 and at
-// 0.5 / 0.5 921 -> 718, 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 50.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 /
+// block mode: 2048 x 11008 x 4096 pruned MLP 1016 -> 699 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 160 and at
+// 0.5 / 0.5 921 -> 718 (before the pairs' side was a constant), 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 50.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 /
 // 0.5 824), 8 k per stage (971), lists made for all of K before the first copy (762), rows past a list's end skipped in a second code
 // path instead of multiplied by zeros (752: the accumulators are then moved between registers at every stage); eight warps that multiply
 // and four that list and copy for them (pruned MLP 1129: a warp alone on its scheduler's spare slots takes 2000 cycles for a stage's 250

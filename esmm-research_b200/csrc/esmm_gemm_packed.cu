@@ -22,7 +22,7 @@ extern "C" int esmm_trace_read(unsigned long long *host, int n)
 }
 #endif
 
-// esmm_gemm_skinny.cu: the kernel for M <= 32
+// esmm_gemm_skinny.cu: the kernel for few rows
 bool gemm_ab_skinny_applies(int M, int N, int K);
 int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const float *d_B, float *d_C,
                           const uint8_t *d_a_pat, const uint8_t *d_b_pat, cudaStream_t stream);
