@@ -54,7 +54,9 @@ static const char *const kTuningNames[] = {"TILE_M", "STAGES", "BROW_BITS", "ROW
 constexpr int kTuningCount = (int)(sizeof kTuningNames / sizeof kTuningNames[0]);
 static std::atomic<int> g_tuning_value[kTuningCount];
 static std::atomic<bool> g_tuning_set[kTuningCount];
-static std::atomic<bool> g_tuning_any;   // one is set: without, no name is looked up
+// One is set: without, no name is looked up.  Written after a hook that is set and before those that are reset (all of it in one order for
+// every thread), so that a hook set beside a reset is either cleared by it or seen.
+static std::atomic<bool> g_tuning_any;
 
 static int tuning_index(const char *name)
 {
@@ -313,15 +315,15 @@ int esmm_tuning_set(const char *name, int value)
     const int i = esmm::tuning_index(name);
     if (i < 0) return ESMM_ERR_UNSUPPORTED;
     esmm::g_tuning_value[i].store(value);
-    esmm::g_tuning_set[i].store(true, std::memory_order_release);
-    esmm::g_tuning_any.store(true, std::memory_order_release);
+    esmm::g_tuning_set[i].store(true);
+    esmm::g_tuning_any.store(true);
     return ESMM_OK;
 }
 
 void esmm_tuning_reset(void)
 {
-    for (int i = 0; i < esmm::kTuningCount; ++i) esmm::g_tuning_set[i].store(false, std::memory_order_release);
-    esmm::g_tuning_any.store(false, std::memory_order_release);
+    esmm::g_tuning_any.store(false);
+    for (int i = 0; i < esmm::kTuningCount; ++i) esmm::g_tuning_set[i].store(false);
 }
 
 int esmm_pattern_from_string(const char *s)

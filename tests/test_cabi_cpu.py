@@ -185,3 +185,50 @@ def test_multi_gpu_host_side_validation(pkg):
     assert L.esmm_multi_run(None, 1, None, None) == pkg.ERR_NULL and L.esmm_multi_gather(None, None, None) == pkg.ERR_NULL
     assert L.esmm_multi_download(None, None) == pkg.ERR_NULL and L.esmm_multi_destroy(None) == 0
     assert L.esmm_multi_num_gpus(None) == 0 and not L.esmm_multi_gathered_c(None)
+
+
+def test_tuning_set_beside_a_reset_is_not_lost(pkg, tmp_path):
+    """A hook set while another thread resets all of them is either set afterwards or not; it is never set and ignored until some
+    other hook is set."""
+    import subprocess
+    src, exe = tmp_path / "hooks.cc", tmp_path / "hooks"
+    src.write_text(r"""
+#include <atomic>
+#include <cstdio>
+#include <thread>
+extern "C" int esmm_tuning_set(const char *, int);
+extern "C" void esmm_tuning_reset(void);
+namespace esmm { int tuning_get(const char *, int); }
+int main()
+{
+    constexpr int rounds = 200000;
+    std::atomic<int> go{0}, done{0};
+    std::thread other([&] {
+        for (int i = 1; i <= rounds; ++i) {
+            while (go.load() < i) {}
+            esmm_tuning_reset();
+            done.store(i);
+        }
+    });
+    int lost = 0, kept = 0;
+    for (int i = 1; i <= rounds; ++i) {
+        go.store(i);
+        for (volatile int wait = i % 64; wait > 0; wait = wait - 1) {}
+        esmm_tuning_set("TILE_M", 64);
+        while (done.load() < i) {}
+        const bool seen = esmm::tuning_get("TILE_M", 0) == 64;
+        esmm_tuning_set("SWIZZLE", 1);                      // now every hook that is set is looked up
+        lost += seen != (esmm::tuning_get("TILE_M", 0) == 64);
+        kept += seen;
+        esmm_tuning_reset();
+    }
+    other.join();
+    std::printf("%d %d\n", lost, kept);
+    return 0;
+}
+""")
+    libdir, lib = os.path.split(pkg.LIB_PATH)
+    subprocess.check_call(["g++", "-std=c++17", "-O2", "-pthread", "-o", str(exe), str(src), os.path.join(libdir, lib), "-Wl,-rpath," + libdir])
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120, check=True).stdout.split()
+    lost, kept = int(out[0]), int(out[1])
+    assert kept > 0 and lost == 0, (lost, kept)
