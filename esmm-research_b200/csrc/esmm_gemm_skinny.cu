@@ -35,6 +35,7 @@
 // wait is bounded: a wait that runs out raises the abort flag, nothing is stored and the status word tells.
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 
 #include "esmm_gemm_shared.cuh"
 
@@ -378,6 +379,31 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
     if (!ok && lane == 0) atomicExch(p.status, (int)ESMM_ERR_TIMEOUT);
 }
 
+// Once per device: the SM count, and the shared-memory allowance of every variant raised to the device's maximum.  The allowance belongs
+// to the kernel in its context and not to a launch: set to each launch's own size, a call of another thread with a shorter list lowered
+// it between this call's setting and its launch, which was then refused.
+static int skinny_prepare(int dev, int *sms)
+{
+    static std::mutex mu;
+    static int sm_count[64];
+    if (dev < 0 || dev >= 64) return ESMM_ERR_CUDA;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!sm_count[dev]) {
+        int n = 0, smem = 0;
+        auto allow = [&](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); };
+        ESMM_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+        ESMM_CUDA_TRY(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<8, 2, 2, 2>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<16, 4, 2, 2>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<16, 2, 2, 4>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<32, 4, 2, 4>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<32, 2, 2, 4>));
+        sm_count[dev] = n;
+    }
+    *sms = sm_count[dev];
+    return ESMM_OK;
+}
+
 // Whether this kernel takes a problem (otherwise the tiled kernel does).  Of M <= 32 all; of fewer than two whole panels of 128 rows
 // those for which it takes less time whatever the operands: a strip and row block of 32 rows is counted as 1 per SM, a 64-row tile of
 // eight of them as 5 (a strip takes 13.7 cycles a k with several on an SM, a tile 87, and the tiled kernel is as fast as 1.2 times
@@ -420,7 +446,8 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
     if (!p.status) return ESMM_ERR_CUDA;
     int dev = 0, sms = 0;
     ESMM_CUDA_TRY(cudaGetDevice(&dev));
-    ESMM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int pst = skinny_prepare(dev, &sms);
+    if (pst != ESMM_OK) return pst;
     const int strips = ceil_div(N, SK_COLS), forced = tuning_get("SKINNY_ROWS", 0);
     const int rows = M > 16 || forced == 32 ? 32 : M > 8 || forced == 16 ? 16 : 8;
     const long units = (long)strips * p.row_blocks;
@@ -430,7 +457,6 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
         p.stages = SK_MAX_STAGES;
         while (p.stages > 2 && sk_smem(r, p.stages, p.cap) > room) --p.stages;
         const size_t smem = sk_smem(r, p.stages, p.cap);
-        ESMM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         ESMM_CUDA_TRY(launch_dependent(kernel, dim3((unsigned)units), dim3(warps * 32), smem, stream, p));
         ESMM_CUDA_TRY(cudaGetLastError());
         return ESMM_OK;

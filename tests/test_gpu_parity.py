@@ -1206,3 +1206,39 @@ def test_rowmajor_block_mode_edges(cuda, pkg, oracle_mod, tuning, M, N):
     for K, ga, gb in [(76, 32, 32), (1020, 64, 32), (1020, 32, 64), (2052, 32, 32)]:
         A, B = workloads.tile_random(M, N, K, 0.6, 0.6, seed=M + N + K, gran_a=ga, gran_b=gb)
         check_all_paths(cuda, pkg, oracle_mod, A, B)
+
+
+def test_gemm_strips_from_two_threads(cuda, pkg, oracle_mod):
+    """Two host threads, each with a stream and buffers of its own, one with the longest list a strip can have (the most shared memory) and
+    one with a short one: no call is refused and every thread's last C has the oracle's bits.  (With the kernel's shared-memory
+    allowance set by each call to its own size, 33 and 75 of 4000 such calls were refused.)"""
+    import threading
+    jobs = []
+    for seed, (K, pa, pb) in enumerate([(16384, 0.1, 0.2), (64, 1.0, 1.0)]):
+        A, B = workloads.tile_random(16, 256, K, pa, pb, seed=seed, gran_a=32, gran_b=32)
+        dA, dB = cuda.from_numpy(A).cuda(), cuda.from_numpy(B).cuda()
+        bp = cuda.empty((8, K // 8), dtype=cuda.uint8, device="cuda")
+        pkg.preprocess_b(dB.data_ptr(), K, 256, bp.data_ptr())
+        ws = cuda.empty(pkg.sgemm_joint_workspace_bytes(16, K), dtype=cuda.uint8, device="cuda")
+        jobs.append({"K": K, "in": (dA, dB, bp, ws), "c": cuda.empty((16, 256), device="cuda"), "want": oracle_mod.gemm_joint(A, B), "bad": []})
+    cuda.cuda.synchronize()
+    L = pkg.lib()
+
+    def work(job):
+        cuda.cuda.set_device(0)
+        stream = cuda.cuda.Stream()
+        dA, dB, bp, ws = (x.data_ptr() for x in job["in"])
+        for _ in range(4000):
+            st = L.esmm_sgemm_joint(16, 256, job["K"], dA, dB, job["c"].data_ptr(), bp, ws, stream.cuda_stream)
+            if st:
+                job["bad"].append(st)
+        stream.synchronize()
+    threads = [threading.Thread(target=work, args=(job,)) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    pkg.device_status()
+    for job in jobs:
+        assert not job["bad"], (job["K"], len(job["bad"]), job["bad"][0])
+        assert np.array_equal(job["c"].cpu().numpy().view(np.uint32), job["want"].view(np.uint32)), job["K"]
