@@ -196,9 +196,6 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
             }
             q = qn;
         }
-        // (the rest of the last stage: copied like the others, never multiplied)
-        for (int pad = n + (int)threadIdx.x; pad < ((n + SK_STAGE_ROWS - 1) & ~(SK_STAGE_ROWS - 1)); pad += SK_THREADS)
-            if (bounds_ok(pad < p.cap, p.status, 30)) krow[pad] = 0;
         __syncthreads();
     }
     const int num_stages = (n + SK_STAGE_ROWS - 1) / SK_STAGE_ROWS;
@@ -216,14 +213,16 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
         const int a_row = lane / A_LANES * A_N, a_chunk = lane % A_LANES;
         // (columns past B's last one: another chunk of the same row; what is multiplied there is not stored)
         const char *b_src = reinterpret_cast<const char *>(p.B + col0 + (col0 + b_chunk * 4 < p.N ? b_chunk * 4 : 0));
-        const char *a_src = reinterpret_cast<const char *>(p.a_packed + (size_t)(rb >> 2) * p.kp * TILE_M + (rb & 3) * 32 + a_chunk * 4);
+        const char *a_block = reinterpret_cast<const char *>(p.a_packed + (size_t)(rb >> 2) * p.kp * TILE_M + (rb & 3) * 32);
+        const char *a_src = a_block + a_chunk * 16;
         const unsigned n4 = (unsigned)p.N * 4u;
         const uint32_t dst_a = smem_u32(smem) + (uint32_t)(a_row * A_ROW_BYTES + a_chunk * 16);
         const uint32_t dst_b = smem_u32(smem) + (uint32_t)(A_HALF + b_row * SK_ROW_BYTES + b_chunk * 16);
         int slot = role - CW;
         uint32_t phase = 1u;                                        // of the slot's empty barrier that the warp waits for
         static_assert(PW <= 2, "a warp's first slot and its steps along the ring");
-        for (int s = role - CW; s < num_stages; s += PW, slot += PW) {
+        int s = role - CW;
+        for (; s < n / SK_STAGE_ROWS; s += PW, slot += PW) {
             if (slot >= p.stages) {
                 slot -= p.stages;
                 phase ^= 1u;
@@ -260,6 +259,27 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
                 }
             }
             sk_copies_arrive(full0 + 8 * slot);
+        }
+        // The list's end: its rows and no others.  Rows to fill the stage, which nothing multiplies, were the same one of A for all strips
+        // of a row block, which queued for it in L2 (whole stages / the listed rows only, us, product alone: 16 x 11008 x 128 with a quarter
+        // of A's and of B's k live 7.1 / 3.5, 1 x 16000 x 256 likewise 8.1 / 3.5, 33 x 11008 x 8 dense 10.6 / 5.8).
+        const int left = n - s * SK_STAGE_ROWS;
+        if (ok && left > 0) {
+            if (slot >= p.stages) {
+                slot -= p.stages;
+                phase ^= 1u;
+            }
+            ok = mbar_wait(empty0 + 8 * slot, phase, abort_flag);
+            const uint32_t to = smem_u32(smem) + (uint32_t)slot * STAGE_BYTES + b_chunk * 16;
+#pragma unroll 1
+            for (int r = lane >> 3; ok && r < left; r += 4) {
+                if (!bounds_ok(s * SK_STAGE_ROWS + r < p.cap, p.status, 31)) break;
+                const unsigned k = krow[s * SK_STAGE_ROWS + r];
+                if (!bounds_ok(k < (unsigned)p.K, p.status, 32)) continue;
+                sk_copy_16(to + A_HALF + r * SK_ROW_BYTES, b_src + (size_t)k * n4);
+                if (b_chunk < A_LANES) sk_copy_16(to + r * A_ROW_BYTES, a_block + (size_t)k * (TILE_M * 4) + b_chunk * 16);
+            }
+            if (ok) sk_copies_arrive(full0 + 8 * slot);
         }
         cp_async_wait_all();      // nothing of this thread is in flight when it leaves
     } else {

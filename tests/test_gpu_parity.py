@@ -1242,3 +1242,40 @@ def test_gemm_strips_from_two_threads(cuda, pkg, oracle_mod):
     for job in jobs:
         assert not job["bad"], (job["K"], len(job["bad"]), job["bad"][0])
         assert np.array_equal(job["c"].cpu().numpy().view(np.uint32), job["want"].view(np.uint32)), job["K"]
+
+
+@pytest.mark.parametrize("M,K", [(1, 256), (16, 64), (32, 64)])
+def test_strips_of_short_lists_do_not_queue(cuda, pkg, M, K):
+    """Strips with a few live k each (a sixteenth of K), 16 of them and 500: a stage is filled with the list's rows only, so that the 500, all of which
+    fit on the GPU at once, take about as long as the 16 (2.6 to 3.6 times as long when each of them filled its stage with copies of the
+    same row).  The product alone, 20 calls in a graph."""
+    times = []
+    for N in (512, 16000):
+        A, B = workloads.tile_random(M, N, K, 0.25, 0.25, seed=K + M, gran_a=32, gran_b=32)
+        dA, dB = cuda.from_numpy(A).cuda(), cuda.from_numpy(B).cuda()
+        ap = cuda.empty((1, K // 8), dtype=cuda.uint8, device="cuda")
+        bp = cuda.empty((-(-N // 32), K // 8), dtype=cuda.uint8, device="cuda")
+        packed = cuda.empty((K * 128,), device="cuda")
+        pkg.preprocess_b(dB.data_ptr(), K, N, bp.data_ptr())
+        pkg.preprocess_a_packed(dA.data_ptr(), M, K, ap.data_ptr(), packed.data_ptr())
+        c = cuda.empty((M, N), device="cuda")
+
+        def call():
+            pkg.gemm_ab_packed(M, N, K, packed.data_ptr(), dB.data_ptr(), c.data_ptr(), ap.data_ptr(), bp.data_ptr(), cuda.cuda.current_stream().cuda_stream)
+        call()
+        pkg.device_status()
+        graph = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(graph):
+            for _ in range(20):
+                call()
+        best = float("inf")
+        for _ in range(10):
+            t0, t1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+            t0.record()
+            graph.replay()
+            t1.record()
+            cuda.cuda.synchronize()
+            best = min(best, t0.elapsed_time(t1))
+        times.append(best)
+        del graph
+    assert times[1] < 1.8 * times[0], times
