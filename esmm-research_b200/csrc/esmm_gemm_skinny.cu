@@ -430,8 +430,11 @@ static int skinny_prepare(int dev, int *sms)
 // that on blocks that differ), a 128-row tile as 9.1.  Tiled / strips, us, K = 4096: 64 x 1024 dense 184 / 42, 64 x 4096 185 / 64, 64
 // x 4096 a quarter live 51.8 / 19.8, 96 x 4096 pruned MLP 44.8 / 27.2, 64 x 11008 x 2048 pruned MLP (4.7 per SM) 33.9 / 24.1, 100 x
 // 6000 x 3000 0.5 / 0.5 (5.1) 53.9 / 36.2; on the other side 256 x 4096 dense (6.9) 188 / 205 and pruned MLP 60.4 / 51.7, 1000 x 1508
-// x 2012 0.5 / 0.5 (10.4) 48.5 / 51.2.  Taller problems stay with the tiled kernel and its launch shapes, which callers can ask for
-// (esmm_last_tiled_kernel_warps).
+// x 2012 0.5 / 0.5 (10.4) 48.5 / 51.2.  At K up to 256 what a strip costs beside its k counts for more, and the lines are 4 and 8: dense,
+// 64 x 11008 x 128 (4.65 per SM) 12.2 / 15.8, 160 x 4096 x 128 (4.3) 12.1 / 15.4, 160 x 8192 x 64 (8.6) 12.3 / 18.6, 224 x 6000 x 256 (8.9)
+// 26.6 / 29.7; on the other side 64 x 8192 x 128 (3.5) 12.1 / 10.7, 96 x 11008 x 256 (7.0) 25.6 / 24.8.  (Half-density operands of the
+// first group are up to 1.5 us faster in strips.)  Taller problems stay with the tiled kernel and its launch shapes, which callers can ask
+// for (esmm_last_tiled_kernel_warps).
 bool gemm_ab_skinny_applies(int M, int N, int K)
 {
     const int kp = ceil_div(K, BK) * BK;
@@ -442,7 +445,7 @@ bool gemm_ab_skinny_applies(int M, int N, int K)
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return false;
     const long units = (long)ceil_div(M, SK_ROWS) * ceil_div(N, SK_COLS), across = ceil_div(N, TILE_N);
     const long rounds64 = (ceil_div(M, 64) * across + sms - 1) / sms, rounds128 = (ceil_div(M, TILE_M) * across + sms - 1) / sms;
-    return (double)units <= sms * std::min(5.0 * rounds64, 9.1 * rounds128);
+    return K <= 256 ? units <= sms * std::min(4 * rounds64, 8 * rounds128) : (double)units <= sms * std::min(5.0 * rounds64, 9.1 * rounds128);
 }
 
 int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const float *d_B, float *d_C,

@@ -1279,3 +1279,27 @@ def test_strips_of_short_lists_do_not_queue(cuda, pkg, M, K):
         times.append(best)
         del graph
     assert times[1] < 1.8 * times[0], times
+
+
+@pytest.mark.parametrize("M,N,K,strips", [(64, 9472, 256, True), (64, 9476, 256, False), (64, 9476, 260, True), (64, 11840, 260, True), (64, 11844, 260, False),
+                                          (160, 7552, 128, True), (160, 7616, 128, False), (160, 8608, 260, True), (160, 8640, 260, False),
+                                          (255, 128, 8, True), (256, 128, 8, False), (32, 16000, 8, True), (33, 16000, 8, False)])
+def test_gemm_strips_or_tiles(cuda, pkg, oracle_mod, tuning, M, N, K, strips):
+    """Which kernel takes a problem of few rows, on either side of the lines (148 SMs): the tiled kernel's launch shape, 12 warps through the
+    entry point that follows no earlier call, is left at a pinned launch's 16 by the strip kernel.  The oracle's bits from both."""
+    if cuda.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines are those of 148 SMs")
+    mark = Dev(cuda, pkg, *workloads.tile_random(256, 128, 64, 1.0, 1.0, seed=1))
+    mark.patterns()
+    tuning("PRODUCER_WARPS", 7)
+    mark.sgemm_joint()
+    tuning.reset()
+    assert pkg.lib().esmm_last_tiled_kernel_warps() == 16
+    A, B = workloads.tile_random(M, N, K, 0.8, 0.8, seed=M + N + K, gran_a=32, gran_b=32)
+    d = Dev(cuda, pkg, A, B)
+    d.patterns()
+    c = cuda.full((M, N), float("nan"), device="cuda")
+    pkg.check(pkg.lib().esmm_sgemm_joint_static(M, N, K, d.A.data_ptr(), d.B.data_ptr(), c.data_ptr(), d.bp.data_ptr(), None), "esmm_sgemm_joint_static")
+    pkg.device_status()
+    assert pkg.lib().esmm_last_tiled_kernel_warps() == (16 if strips else 12)
+    assert np.array_equal(c.cpu().numpy().view(np.uint32), oracle_mod.gemm_joint(A, B).view(np.uint32))
