@@ -204,85 +204,7 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
     const int role = CW == 2 ? (warp + wsum[SK_WARPS]) & 3 : warp;
     bool ok = true;
 
-    if (role >= CW) {
-        // ---------------- copies: a warp takes every PW-th stage ----------------
-        // 32 rows at a time.  B: 8 lanes per row, 4 rows an instruction, rows 8 apart, so that a lane's 8 list entries are one load;
-        // A likewise.  (Rows of 128 bytes are too short for the tensor copy engine: about 57 cycles of issue per copy and warp.)
-        constexpr int A_LANES = ROWS / 4, A_N = A_LANES;            // lanes per row of A; instructions per 32 rows
-        const int b_row = (lane >> 3) * 8, b_chunk = lane & 7;
-        const int a_row = lane / A_LANES * A_N, a_chunk = lane % A_LANES;
-        // (columns past B's last one: another chunk of the same row; what is multiplied there is not stored)
-        const char *b_src = reinterpret_cast<const char *>(p.B + col0 + (col0 + b_chunk * 4 < p.N ? b_chunk * 4 : 0));
-        const char *a_block = reinterpret_cast<const char *>(p.a_packed + (size_t)(rb >> 2) * p.kp * TILE_M + (rb & 3) * 32);
-        const char *a_src = a_block + a_chunk * 16;
-        const unsigned n4 = (unsigned)p.N * 4u;
-        const uint32_t dst_a = smem_u32(smem) + (uint32_t)(a_row * A_ROW_BYTES + a_chunk * 16);
-        const uint32_t dst_b = smem_u32(smem) + (uint32_t)(A_HALF + b_row * SK_ROW_BYTES + b_chunk * 16);
-        int slot = role - CW;
-        uint32_t phase = 1u;                                        // of the slot's empty barrier that the warp waits for
-        static_assert(PW <= 2, "a warp's first slot and its steps along the ring");
-        int s = role - CW;
-        for (; s < n / SK_STAGE_ROWS; s += PW, slot += PW) {
-            if (slot >= p.stages) {
-                slot -= p.stages;
-                phase ^= 1u;
-            }
-            if (!bounds_ok((s + 1) * SK_STAGE_ROWS <= p.cap, p.status, 31)) break;
-            ok = mbar_wait(empty0 + 8 * slot, phase, abort_flag);
-            if (!ok) break;
-#pragma unroll
-            for (int h = 0; h < SK_STAGE_ROWS / 32; ++h) {
-                const uint32_t s_off = (uint32_t)slot * STAGE_BYTES;
-                const uint16_t *list = krow + s * SK_STAGE_ROWS + h * 32;
-                const uint4 bk = *reinterpret_cast<const uint4 *>(list + b_row);
-                unsigned ka[8];
-                const unsigned kb[8] = {bk.x & 0xFFFFu, bk.x >> 16, bk.y & 0xFFFFu, bk.y >> 16, bk.z & 0xFFFFu, bk.z >> 16, bk.w & 0xFFFFu, bk.w >> 16};
-                if (A_N == 8) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) ka[j] = kb[j];
-                } else if (A_N == 4) {
-                    const uint2 v = *reinterpret_cast<const uint2 *>(list + a_row);
-                    ka[0] = v.x & 0xFFFFu, ka[1] = v.x >> 16, ka[2] = v.y & 0xFFFFu, ka[3] = v.y >> 16;
-                } else {
-                    const unsigned v = *reinterpret_cast<const unsigned *>(list + a_row);
-                    ka[0] = v & 0xFFFFu, ka[1] = v >> 16;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (!bounds_ok(kb[j] < (unsigned)p.K, p.status, 32)) continue;   // site 32: a k outside B / the packed panel
-                    sk_copy_16(dst_b + s_off + (h * 32 + j) * SK_ROW_BYTES, b_src + (size_t)kb[j] * n4);
-                }
-#pragma unroll
-                for (int j = 0; j < A_N; ++j) {
-                    if (!bounds_ok(ka[j] < (unsigned)p.kp, p.status, 32)) continue;
-                    sk_copy_16(dst_a + s_off + (h * 32 + j) * A_ROW_BYTES, a_src + (size_t)ka[j] * (TILE_M * 4));
-                }
-            }
-            sk_copies_arrive(full0 + 8 * slot);
-        }
-        // The list's end: its rows and no others.  Rows to fill the stage, which nothing multiplies, were the same one of A for all strips
-        // of a row block, which queued for it in L2 (whole stages / the listed rows only, us, product alone: 16 x 11008 x 128 with a quarter
-        // of A's and of B's k live 7.1 / 3.5, 1 x 16000 x 256 likewise 8.1 / 3.5, 33 x 11008 x 8 dense 10.6 / 5.8).
-        const int left = n - s * SK_STAGE_ROWS;
-        if (ok && left > 0) {
-            if (slot >= p.stages) {
-                slot -= p.stages;
-                phase ^= 1u;
-            }
-            ok = mbar_wait(empty0 + 8 * slot, phase, abort_flag);
-            const uint32_t to = smem_u32(smem) + (uint32_t)slot * STAGE_BYTES + b_chunk * 16;
-#pragma unroll 1
-            for (int r = lane >> 3; ok && r < left; r += 4) {
-                if (!bounds_ok(s * SK_STAGE_ROWS + r < p.cap, p.status, 31)) break;
-                const unsigned k = krow[s * SK_STAGE_ROWS + r];
-                if (!bounds_ok(k < (unsigned)p.K, p.status, 32)) continue;
-                sk_copy_16(to + A_HALF + r * SK_ROW_BYTES, b_src + (size_t)k * n4);
-                if (b_chunk < A_LANES) sk_copy_16(to + r * A_ROW_BYTES, a_block + (size_t)k * (TILE_M * 4) + b_chunk * 16);
-            }
-            if (ok) sk_copies_arrive(full0 + 8 * slot);
-        }
-        cp_async_wait_all();      // nothing of this thread is in flight when it leaves
-    } else {
+    if (role < CW) {
         // ---------------- multiplying warps: WROWS rows x WCOLS columns each, 4 rows x CT columns per thread ----------------
         constexpr int WROWS = ROWS < 16 ? ROWS : 16, ROW_SPLIT = ROWS / WROWS, WCOLS = SK_COLS * ROW_SPLIT / CW;
         constexpr int RG = WROWS / RT, CG = 32 / RG, CT = WCOLS / CG;     // groups of lanes on the rows, on the columns
@@ -395,6 +317,113 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
                 else *reinterpret_cast<float2 *>(dst) = make_float2(v[0], v[1]);
             }
         }
+    } else {
+        // ---------------- copies: a warp takes every PW-th stage ----------------
+        // 32 rows at a time.  B: 8 lanes per row, 4 rows an instruction, rows 8 apart, so that a lane's 8 list entries are one load;
+        // A likewise.  (Rows of 128 bytes are too short for the tensor copy engine: about 57 cycles of issue per copy and warp.)
+        constexpr int A_LANES = ROWS / 4, A_N = A_LANES;            // lanes per row of A; instructions per 32 rows
+        const int b_row = (lane >> 3) * 8, b_chunk = lane & 7;
+        const int a_row = lane / A_LANES * A_N, a_chunk = lane % A_LANES;
+        // (columns past B's last one: another chunk of the same row; what is multiplied there is not stored)
+        const char *b_src = reinterpret_cast<const char *>(p.B + col0 + (col0 + b_chunk * 4 < p.N ? b_chunk * 4 : 0));
+        const char *a_src = reinterpret_cast<const char *>(p.a_packed + (size_t)(rb >> 2) * p.kp * TILE_M + (rb & 3) * 32 + a_chunk * 4);
+        const unsigned n4 = (unsigned)p.N * 4u;
+        const uint32_t dst_a = smem_u32(smem) + (uint32_t)(a_row * A_ROW_BYTES + a_chunk * 16);
+        const uint32_t dst_b = smem_u32(smem) + (uint32_t)(A_HALF + b_row * SK_ROW_BYTES + b_chunk * 16);
+        int slot = role - CW;
+        uint32_t phase = 1u;                                        // of the slot's empty barrier that the warp waits for
+        static_assert(PW <= 2, "a warp's first slot and its steps along the ring");
+        int s = role - CW;
+        for (; (s + 1) * SK_STAGE_ROWS <= n; s += PW, slot += PW) {
+            if (slot >= p.stages) {
+                slot -= p.stages;
+                phase ^= 1u;
+            }
+            if (!bounds_ok((s + 1) * SK_STAGE_ROWS <= p.cap, p.status, 31)) break;
+            ok = mbar_wait(empty0 + 8 * slot, phase, abort_flag);
+            if (!ok) break;
+#pragma unroll
+            for (int h = 0; h < SK_STAGE_ROWS / 32; ++h) {
+                const uint32_t s_off = (uint32_t)slot * STAGE_BYTES;
+                const uint16_t *list = krow + s * SK_STAGE_ROWS + h * 32;
+                const uint4 bk = *reinterpret_cast<const uint4 *>(list + b_row);
+                unsigned ka[8];
+                const unsigned kb[8] = {bk.x & 0xFFFFu, bk.x >> 16, bk.y & 0xFFFFu, bk.y >> 16, bk.z & 0xFFFFu, bk.z >> 16, bk.w & 0xFFFFu, bk.w >> 16};
+                if (A_N == 8) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) ka[j] = kb[j];
+                } else if (A_N == 4) {
+                    const uint2 v = *reinterpret_cast<const uint2 *>(list + a_row);
+                    ka[0] = v.x & 0xFFFFu, ka[1] = v.x >> 16, ka[2] = v.y & 0xFFFFu, ka[3] = v.y >> 16;
+                } else {
+                    const unsigned v = *reinterpret_cast<const unsigned *>(list + a_row);
+                    ka[0] = v & 0xFFFFu, ka[1] = v >> 16;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (!bounds_ok(kb[j] < (unsigned)p.K, p.status, 32)) continue;   // site 32: a k outside B / the packed panel
+                    sk_copy_16(dst_b + s_off + (h * 32 + j) * SK_ROW_BYTES, b_src + (size_t)kb[j] * n4);
+                }
+#pragma unroll
+                for (int j = 0; j < A_N; ++j) {
+                    if (!bounds_ok(ka[j] < (unsigned)p.kp, p.status, 32)) continue;
+                    sk_copy_16(dst_a + s_off + (h * 32 + j) * A_ROW_BYTES, a_src + (size_t)ka[j] * (TILE_M * 4));
+                }
+            }
+            sk_copies_arrive(full0 + 8 * slot);
+        }
+        // The list's end: its rows and no others.  Rows to fill the stage, which nothing multiplies, were the same one of A for all strips
+        // of a row block, which queued for it in L2 (whole stages / the listed rows only, us, product alone: 16 x 11008 x 128 with a quarter
+        // of A's and of B's k live 6.6 / 2.9, 1 x 16000 x 256 likewise 7.6 / 2.9, 33 x 8192 x 8 dense 8.4 / 3.2).
+        // For 8 and 16 rows as a whole stage is copied (in the other form, a loop, lists of one stage take 0.7 us longer), for 32 a loop.  What
+        // the compiler makes of the loops over whole stages, here and above, depends on this part and on its place: so, and after the
+        // multiplying warps' code, nothing is slower than without it (128 x 4096 x 4096 dense 101.3 us, 102.7 without it, 101 to 121 in nine
+        // other forms and places; one strip of 48 k 3.1 and 3.1).
+        const int left = n - s * SK_STAGE_ROWS;
+        if (ok && left > 0) {
+            if (slot >= p.stages) {
+                slot -= p.stages;
+                phase ^= 1u;
+            }
+            ok = mbar_wait(empty0 + 8 * slot, phase, abort_flag);
+            const uint32_t s_off = (uint32_t)slot * STAGE_BYTES;
+            if constexpr (ROWS < 32) {
+#pragma unroll 2
+                for (int h = 0; h < SK_STAGE_ROWS / 32; ++h) {
+                    if (!ok || h * 32 >= left) break;
+                    const uint16_t *list = krow + s * SK_STAGE_ROWS + h * 32;
+                    const uint4 bk = *reinterpret_cast<const uint4 *>(list + b_row);
+                    const unsigned kb[8] = {bk.x & 0xFFFFu, bk.x >> 16, bk.y & 0xFFFFu, bk.y >> 16, bk.z & 0xFFFFu, bk.z >> 16, bk.w & 0xFFFFu, bk.w >> 16};
+                    const int b_left = left - h * 32 - b_row, a_left = left - h * 32 - a_row;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (j >= b_left || !bounds_ok(kb[j] < (unsigned)p.K, p.status, 32)) continue;
+                        sk_copy_16(dst_b + s_off + (h * 32 + j) * SK_ROW_BYTES, b_src + (size_t)kb[j] * n4);
+                    }
+#pragma unroll
+                    for (int j = 0; j < A_N; ++j) {
+                        const unsigned k = list[a_row + j];
+                        if (j >= a_left || !bounds_ok(k < (unsigned)p.kp, p.status, 32)) continue;
+                        sk_copy_16(dst_a + s_off + (h * 32 + j) * A_ROW_BYTES, a_src + (size_t)k * (TILE_M * 4));
+                    }
+                }
+            } else {
+                const uint32_t to = smem_u32(smem) + s_off + b_chunk * 16;   // (a row of A is as long as one of B)
+#pragma unroll (CW == 4 ? 1 : 2)
+                for (int r = (lane >> 3) * 4; ok && r < left; r += 16) {
+                    const uint2 v = *reinterpret_cast<const uint2 *>(krow + s * SK_STAGE_ROWS + r);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const unsigned w = j & 2 ? v.y : v.x, k = j & 1 ? w >> 16 : w & 0xFFFFu;
+                        if (r + j >= left || !bounds_ok(k < (unsigned)p.K, p.status, 32)) continue;
+                        sk_copy_16(to + A_HALF + (r + j) * SK_ROW_BYTES, b_src + (size_t)k * n4);
+                        sk_copy_16(to + (r + j) * A_ROW_BYTES, a_src + (size_t)k * (TILE_M * 4));
+                    }
+                }
+            }
+            if (ok) sk_copies_arrive(full0 + 8 * slot);
+        }
+        cp_async_wait_all();      // nothing of this thread is in flight when it leaves
     }
     if (!ok && lane == 0) atomicExch(p.status, (int)ESMM_ERR_TIMEOUT);
 }
