@@ -909,7 +909,7 @@ int esmm_run_kernel_pattern(int kernel_id, int rows, int cols, int inners, float
                         st = esmm_preprocess_b(d_B, inners, cols, d_bp, 0);
                     }
                 }
-                if (st == ESMM_OK) st = esmm::preprocess_a_pack_launch(d_A, rows, inners, d_ap, d_packed, 0, rows <= 32);
+                if (st == ESMM_OK) st = esmm::preprocess_a_pack_launch(d_A, rows, inners, d_ap, d_packed, 0, esmm::gemm_ab_skinny_applies(rows, cols, inners));
                 if (st == ESMM_OK)
                     st = esmm::gemm_ab_packed_launch(rows, cols, inners, d_packed, d_B, d_C, d_ap, d_bp, 0);
                 cudaDeviceSynchronize();
@@ -921,7 +921,7 @@ int esmm_run_kernel_pattern(int kernel_id, int rows, int cols, int inners, float
             st = esmm_preprocess_ab(d_A, d_B, rows, cols, inners, a_tile, d_b_pat_cached, &meta);
             if (st != ESMM_OK) break;
             if (d_packed) {
-                st = esmm::preprocess_a_pack_launch(d_A, rows, inners, meta.d_a_patterns, d_packed, 0, rows <= 32);
+                st = esmm::preprocess_a_pack_launch(d_A, rows, inners, meta.d_a_patterns, d_packed, 0, esmm::gemm_ab_skinny_applies(rows, cols, inners));
                 if (st == ESMM_OK)
                     st = esmm::gemm_ab_packed_launch(rows, cols, inners, d_packed, d_B, d_C, meta.d_a_patterns,
                                                      meta.d_b_patterns, 0);

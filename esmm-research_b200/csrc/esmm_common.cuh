@@ -11,6 +11,7 @@ namespace esmm {
 
 constexpr int BK = 8;    // K offsets per pattern byte (the reference's BK)
 constexpr int PAT_N = 32;  // columns of B per pattern byte (the reference's WN)
+constexpr int STRIP_ROW_LIMIT = 256;   // problems of fewer rows may go to the strip kernel (gemm_ab_skinny_applies)
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 

@@ -467,7 +467,7 @@ static int skinny_prepare(int dev, int *sms)
 bool gemm_ab_skinny_applies(int M, int N, int K)
 {
     const int kp = ceil_div(K, BK) * BK;
-    if (kp > SK_MAX_KP || M >= 2 * TILE_M || tuning_get("NO_SKINNY", 0)) return false;
+    if (kp > SK_MAX_KP || M >= STRIP_ROW_LIMIT || tuning_get("NO_SKINNY", 0)) return false;
     if (M <= SK_ROWS) return N >= 4 * SK_COLS;
     if (tiled_kernel_tuned()) return false;
     int dev = 0, sms = 0;

@@ -300,9 +300,9 @@ int preprocess_a_launch(const float *d_A, int M, int K, int tile_m, uint8_t *d_o
     return ESMM_OK;
 }
 
-// beside: the kernel after this one has several CTAs per SM.
+// strips: the strip kernel comes next, or may.
 int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, float *d_packed,
-                             cudaStream_t stream, bool beside)
+                             cudaStream_t stream, bool strips)
 {
     if (!d_A || !d_out || !d_packed) return ESMM_ERR_NULL;
     if (M <= 0 || K <= 0 || (K & 3)) return ESMM_ERR_SHAPE;
@@ -320,21 +320,24 @@ int preprocess_a_pack_launch(const float *d_A, int M, int K, uint8_t *d_out, flo
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(PACK_WARPS * 32);
     cfg.stream = stream;
-    // Few rows: the strip kernel's CTAs are placed while this kernel ends, and an SM whose shared memory is carved out for less
-    // than they need takes none of them until it has (M = 16, K = 4096: 344 strips on 132 of 148 SMs).
+    // The strip kernel's CTAs are placed while this kernel ends, and an SM whose shared memory is carved out for less than they need takes
+    // none of them until it has (M = 16, K = 4096: 344 strips on 132 of 148 SMs; packing and product by calls of their own, dense, 100 x 1000
+    // x 4096 95.5 us without the carve-out, 42.6 with it, 33 x 4096 x 2048 50.1 and 35.0; before tiles it makes no difference).
     cudaLaunchAttribute attr[2];
     int attrs = 0;
     if (!tuning_get("NO_DEPENDENT_LAUNCH", 0)) {
         attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (beside) {
+    if (strips) {
         attr[attrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
         attr[attrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
     }
     cfg.attrs = attr;
     cfg.numAttrs = attrs;
-    const int early = !beside || blocks <= sms;
+    // Strips of one row block are placed late where this grid fills the GPU.  Of several row blocks they take the same either way (33 x 4096 x
+    // 2048 dense 35.0 and 35.1 us), and tiles, which may come instead, lose by it (255 x 11008 x 8192 dense 1082 us early, 1090 late).
+    const int early = !strips || M > 32 || blocks <= sms;
     ESMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, esmm_preprocess_a_pack32_kernel, d_A, M, K, nMB, nKB, k_chunks, d_out, d_packed, status, early));
     ESMM_CUDA_TRY(cudaGetLastError());
     return ESMM_OK;
@@ -396,7 +399,7 @@ size_t esmm_a_packed_bytes(int M, int K)
 
 int esmm_preprocess_a_packed(const float *d_A, int M, int K, uint8_t *d_out, float *d_packed, void *stream)
 {
-    return esmm::preprocess_a_pack_launch(d_A, M, K, d_out, d_packed, (cudaStream_t)stream, M <= 32);
+    return esmm::preprocess_a_pack_launch(d_A, M, K, d_out, d_packed, (cudaStream_t)stream, M < esmm::STRIP_ROW_LIMIT);
 }
 
 int esmm_preprocess_b(const float *d_B, int K, int N, uint8_t *d_out, void *stream)

@@ -1303,3 +1303,46 @@ def test_gemm_strips_or_tiles(cuda, pkg, oracle_mod, tuning, M, N, K, strips):
     pkg.device_status()
     assert pkg.lib().esmm_last_tiled_kernel_warps() == (16 if strips else 12)
     assert np.array_equal(c.cpu().numpy().view(np.uint32), oracle_mod.gemm_joint(A, B).view(np.uint32))
+
+
+@pytest.mark.parametrize("M,N", [(16, 1024), (100, 1024), (255, 1000), (256, 1024), (512, 1024)])
+def test_packing_before_strips_is_launched_alike(cuda, pkg, M, N):
+    """The packing kernel asks for the same division of an SM's shared memory whether its product comes in the same call or in one of its
+    own, and before strips that is the largest one (100 x 1000 x 4096 as two calls took 2.2 times as long where it was asked for up to 32
+    rows only).  Read from the launches as a graph holds them."""
+    cudart = pytest.importorskip("cuda.bindings.runtime")
+    K = 512
+    A, B = workloads.tile_random(M, N, K, 0.5, 0.5, seed=M, gran_a=32, gran_b=32)
+    d = Dev(cuda, pkg, A, B)
+    d.patterns()
+    packed = cuda.empty((-(-M // 128) * 128 * K,), device="cuda")
+    ws = cuda.empty(pkg.sgemm_joint_workspace_bytes(M, K), dtype=cuda.uint8, device="cuda")
+    c = d.C()
+
+    def joint(stream):
+        pkg.sgemm_joint(M, N, K, d.A.data_ptr(), d.B.data_ptr(), c.data_ptr(), d.bp.data_ptr(), ws.data_ptr(), stream)
+
+    def two(stream):
+        pkg.preprocess_a_packed(d.A.data_ptr(), M, K, d.ap.data_ptr(), packed.data_ptr(), stream)
+        pkg.gemm_ab_packed(M, N, K, packed.data_ptr(), d.B.data_ptr(), c.data_ptr(), d.ap.data_ptr(), d.bp.data_ptr(), stream)
+
+    def carveouts(call):
+        call(cuda.cuda.current_stream().cuda_stream)                  # (set-up of a first call)
+        pkg.device_status()
+        graph = cuda.cuda.CUDAGraph(keep_graph=True)
+        with cuda.cuda.graph(graph):
+            call(cuda.cuda.current_stream().cuda_stream)
+        raw = cudart.cudaGraph_t(graph.raw_cuda_graph())
+        err, _, count = cudart.cudaGraphGetNodes(raw)
+        assert int(err) == 0 and count == 2
+        err, nodes, count = cudart.cudaGraphGetNodes(raw, count)
+        assert int(err) == 0
+        got = []
+        for node in nodes:
+            err, value = cudart.cudaGraphKernelNodeGetAttribute(node, cudart.cudaLaunchAttributeID.cudaLaunchAttributePreferredSharedMemoryCarveout)
+            assert int(err) == 0
+            got.append(int(value.sharedMemCarveout))
+        return sorted(got)
+    one_call, two_calls = carveouts(joint), carveouts(two)
+    assert one_call == two_calls
+    assert (100 in one_call) == (M < 256), one_call                   # cudaSharedmemCarveoutMaxShared
