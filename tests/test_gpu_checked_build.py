@@ -82,23 +82,28 @@ def test_guarded_buffers_and_bounds_checks(cuda, pkg, libs, oracle_mod, which, M
     ap = Guarded(t, -(-M // 32) * nkb)
     bp = Guarded(t, -(-N // 32) * nkb)
     c1 = Guarded(t, M * N * 4, fill=0xFF)
-    c2 = Guarded(t, M * N * 4, fill=0xFF)
+    c2, c3 = Guarded(t, M * N * 4, fill=0xFF), Guarded(t, M * N * 4, fill=0xFF)
     ws = Guarded(t, int(L.esmm_sgemm_joint_workspace_bytes(M, K)), fill=0xFF)
-    # pattern preprocessors, the row-major kernel, then the per-call path (packing preprocess + packed / strip kernel)
+    # pattern preprocessors, the row-major kernel, then the per-call path (packing preprocess + strip or tiled kernel, then the tiled one)
     assert L.esmm_preprocess_a(dA.data_ptr(), M, K, 32, ap.ptr, None) == 0
     assert L.esmm_preprocess_b(dB.data_ptr(), K, N, bp.ptr, None) == 0
     assert L.esmm_gemm_ab(M, N, K, dA.data_ptr(), dB.data_ptr(), c1.ptr, ap.ptr, bp.ptr, 32, None) == 0
     assert L.esmm_sgemm_joint(M, N, K, dA.data_ptr(), dB.data_ptr(), c2.ptr, bp.ptr, ws.ptr, None) == 0
+    assert L.esmm_tuning_set(b"NO_SKINNY", 1) == 0
+    try:
+        assert L.esmm_sgemm_joint(M, N, K, dA.data_ptr(), dB.data_ptr(), c3.ptr, bp.ptr, ws.ptr, None) == 0
+    finally:
+        L.esmm_tuning_reset()
     st = L.esmm_device_status(None)
     assert st == 0, (st, L.esmm_last_cuda_error())
     for name, g in (("A patterns", ap), ("B patterns", bp), ("C (row-major kernel)", c1), ("C (per-call path)", c2),
-                    ("workspace", ws)):
+                    ("C (tiled kernel)", c3), ("workspace", ws)):
         assert g.intact(), f"{which} build wrote outside {name}"
     oap, obp = oracle_mod.preprocess_a(A), oracle_mod.preprocess_b(B)
     assert np.array_equal(ap.view(t.uint8, oap.shape).cpu().numpy(), oap)
     assert np.array_equal(bp.view(t.uint8, obp.shape).cpu().numpy(), obp)
     want = oracle_mod.gemm_joint(A, B, oap, obp)
-    for g in (c1, c2):
+    for g in (c1, c2, c3):
         got = g.view(t.float32, (M, N)).cpu().numpy()
         assert not np.isnan(got).any() and np.array_equal(got, want)
 

@@ -65,6 +65,8 @@ def pin_mode(tuning, mode):
 
 
 def check_all_paths(cuda, pkg, oracle_mod, A, B, expect_bits=True):
+    """Row-major and packed kernel against the oracle.  Problems of 33 to 255 rows, most of which the strip kernel takes, go through the
+    tiled kernel as well."""
     d = Dev(cuda, pkg, A, B)
     ap, bp = d.patterns()
     oap, obp = oracle_mod.preprocess_a(A), oracle_mod.preprocess_b(B)
@@ -74,7 +76,14 @@ def check_all_paths(cuda, pkg, oracle_mod, A, B, expect_bits=True):
     C1 = d.gemm_rowmajor()
     C2, ap2 = d.sgemm_joint()
     assert np.array_equal(ap2, oap), "packing preprocessor: A pattern bytes differ from the oracle"
-    for name, Cg in (("row-major kernel", C1), ("packed kernel", C2)):
+    results = [("row-major kernel", C1), ("packed kernel", C2)]
+    if 32 < A.shape[0] < 256:
+        assert pkg.lib().esmm_tuning_set(b"NO_SKINNY", 1) == 0
+        try:
+            results.append(("tiled kernel", d.sgemm_joint()[0]))
+        finally:
+            pkg.lib().esmm_tuning_set(b"NO_SKINNY", 0)                # what it is where it is not set
+    for name, Cg in results:
         assert not np.isnan(Cg).any(), name
         assert oracle_mod.rel_inf_err(Cg, Cref) <= TOL, name
         if expect_bits:
@@ -377,23 +386,20 @@ def test_gemm_block_structured(cuda, pkg, oracle_mod, tuning, rows):
     check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
-def test_packing_kernel_variants(cuda, pkg, oracle_mod, tuning):
-    """The packing preprocessor has a 32 x 64 task per warp (default) and a 32 x 128 one; both must give the
-    oracle's pattern bytes and a packed copy the GEMM turns into the oracle's C (workspace poisoned with NaN
-    bit patterns: a dead entry that were read would show)."""
-    for variant in ("128", "64"):
-        tuning("PACK", int(variant))
-        for M, N, K, pa, pb in [(256, 256, 512, 0.5, 0.5), (100, 132, 8 * 37, 0.3, 0.7), (384, 128, 4 * 75, 0.8, 0.4),
-                                (16, 256, 256, 0.5, 0.5), (200, 64, 64, 1.0, 1.0)]:
-            A, B = workloads.tile_random(M, N, K, pa, pb, seed=M + K, gran_a=32, gran_b=32)
-            check_all_paths(cuda, pkg, oracle_mod, A, B)
-        A, B = workloads.all_byte_values(seed=31)
+def test_packing_kernel_variants(cuda, pkg, oracle_mod):
+    """The packing preprocessor gives the oracle's pattern bytes and a packed copy that the strip and the tiled kernel turn into the oracle's C
+    (workspace poisoned with NaN bit patterns: a dead entry that were read would show)."""
+    for M, N, K, pa, pb in [(256, 256, 512, 0.5, 0.5), (100, 132, 8 * 37, 0.3, 0.7), (384, 128, 4 * 75, 0.8, 0.4),
+                            (16, 256, 256, 0.5, 0.5), (200, 64, 64, 1.0, 1.0)]:
+        A, B = workloads.tile_random(M, N, K, pa, pb, seed=M + K, gran_a=32, gran_b=32)
         check_all_paths(cuda, pkg, oracle_mod, A, B)
+    A, B = workloads.all_byte_values(seed=31)
+    check_all_paths(cuda, pkg, oracle_mod, A, B)
 
 
 def test_gemm_random_shapes(cuda, pkg, oracle_mod):
-    """Seeded random shapes and densities (ragged M, N % 4 == 0, K % 4 == 0, all three kernels and both tilings get
-    their share through the launch heuristics): same bits as the oracle everywhere."""
+    """Seeded random shapes and densities (ragged M, N % 4 == 0, K % 4 == 0; up to 255 rows the strip kernel and the tiled kernel,
+    above the tiled one, row-major A besides): same bits as the oracle everywhere."""
     rng = np.random.default_rng(2024)
     for case in range(40):
         M = int(rng.integers(1, 320))
@@ -1087,6 +1093,73 @@ def test_calls_wait_for_what_is_before_them(cuda, pkg, M, captured):
         run()
         cuda.cuda.synchronize()
         assert all(cuda.equal(x, w) for row, wrow in zip(out, want) for x, w in zip(row, wrow))
+    pkg.device_status()
+    if captured:
+        del graph
+
+
+@pytest.mark.parametrize("M", [16, 512])
+@pytest.mark.parametrize("captured", [False, True])
+def test_calls_wait_for_a_kernel_that_triggers_early(cuda, pkg, M, captured):
+    """The same kernels after one that lets its dependents be placed at its start, long before it has written what they read: the packing of
+    8192 x 4096 elements, in more than one wave of CTAs.  A is the end of the packed copy, which the last CTAs write.  (A kernel that lets nothing be
+    placed early, as a copy or one of torch's, has ended when a dependent starts, whether the dependent waits or not.)"""
+    N, K, rounds, XM, XK = 768, 2048, 4, 8192, 4096
+    gen = cuda.Generator(device="cuda")
+    gen.manual_seed(17)
+    B = cuda.randn((K, N), generator=gen, device="cuda")
+    B.view(K, N // 32, 32).mul_((cuda.rand((K, N // 32, 1), generator=gen, device="cuda") < 0.5).float())
+    xs = [cuda.randn((XM, XK), generator=gen, device="cuda") for _ in range(2)]
+    nkb = K // 8
+    bp = cuda.empty((N // 32, nkb), dtype=cuda.uint8, device="cuda")
+    pkg.preprocess_b(B.data_ptr(), K, N, bp.data_ptr())
+    cuda.cuda.synchronize()
+    handle = pkg.Tf32x3B(B.data_ptr(), K, N)
+    xp = cuda.empty((XM // 32, XK // 8), dtype=cuda.uint8, device="cuda")
+    packed = cuda.empty((XM * XK,), device="cuda")
+    A = packed[-M * K:]
+    ap = cuda.empty((-(-M // 32), nkb), dtype=cuda.uint8, device="cuda")
+    ws = cuda.empty(pkg.sgemm_joint_workspace_bytes(M, K), dtype=cuda.uint8, device="cuda")
+    ws2 = cuda.empty(pkg.tf32x3_workspace_bytes(M, K), dtype=cuda.uint8, device="cuda")
+    out = [[cuda.empty((M, N), device="cuda") for _ in range(3)] for _ in range(rounds)]
+    pats = [cuda.empty_like(ap) for _ in range(rounds)]
+
+    def train(wait):
+        st = cuda.cuda.current_stream().cuda_stream
+        for i in range(rounds):
+            for which in range(3):
+                packed.zero_()                                        # (read too early: zeros, whose patterns are empty)
+                pkg.preprocess_a_packed(xs[i % 2].data_ptr(), XM, XK, xp.data_ptr(), packed.data_ptr(), st)
+                if wait:
+                    cuda.cuda.synchronize()
+                c = out[i][which].data_ptr()
+                if which == 0:
+                    pkg.sgemm_joint(M, N, K, A.data_ptr(), B.data_ptr(), c, bp.data_ptr(), ws.data_ptr(), st)
+                elif which == 1:
+                    pkg.preprocess_a(A.data_ptr(), M, K, ap.data_ptr(), 32, st)
+                    pkg.gemm_ab(M, N, K, A.data_ptr(), B.data_ptr(), c, ap.data_ptr(), bp.data_ptr(), 32, st)
+                    pats[i].copy_(ap)
+                else:
+                    pkg.sgemm_joint_tf32x3(M, A.data_ptr(), handle, c, ws2.data_ptr(), st)
+                if wait:
+                    cuda.cuda.synchronize()
+
+    train(True)
+    flat = [x for row in out for x in row] + pats
+    want = [x.clone() for x in flat]
+    assert not cuda.equal(want[0], want[3]) and bool((want[-1] == 0xFF).all())
+    run = lambda: train(False)
+    if captured:
+        graph = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(graph):
+            train(False)
+        run = graph.replay
+    for _ in range(5):
+        for x in flat:
+            x.zero_()
+        run()
+        cuda.cuda.synchronize()
+        assert all(cuda.equal(x, w) for x, w in zip(flat, want))
     pkg.device_status()
     if captured:
         del graph
