@@ -328,7 +328,6 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     const char *b_src = reinterpret_cast<const char *>(p.B + b_blk * 32);
     const char *xs = (wide_b ? b_src : a_src) + c8 * 16, *ys = (wide_b ? a_src : b_src) + c8 * 16;
     const int b_chunks = (p.N - b_blk * 32) >> 2;
-    const bool edge = b_chunks < (wide_b && TWO ? 16 : 8);
     const int x_chunks = wide_b ? b_chunks : 16, y_chunks = wide_b ? 8 : b_chunks;
     // Row-major A: the lane's k of a copy, its row within a chunk of four and where it lands.  Rows of A past its last one: one of the rows
     // before them; columns of B past its last one: others of the same row (what is multiplied there ends in rows and columns of C that do

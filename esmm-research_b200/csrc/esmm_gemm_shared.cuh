@@ -87,12 +87,6 @@ __device__ __forceinline__ void fma_bottom(Acc &c, const KFrag &f)
     fma_pair_row(c, 3, make_float2(f.ab.z, f.ab.w), f);
 }
 
-// 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros instead
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, int src_bytes)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-
 __device__ __forceinline__ void cp_async_commit()
 {
     asm volatile("cp.async.commit_group;" ::: "memory");

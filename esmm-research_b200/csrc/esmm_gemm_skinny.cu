@@ -47,6 +47,7 @@ constexpr int SK_STAGE_ROWS = 64;               // k per stage
 constexpr int SK_ROW_BYTES = 128;               // one k of B in shared memory
 constexpr int SK_MAX_STAGES = 4;                // of the ring; two at least
 constexpr int SK_MAX_KP = 16384;                // longest K the row list is sized for
+constexpr int SK_COPY_WARPS = 2;                // warps that copy
 constexpr int SK_BATCH = 4;                     // k per register set of operands
 constexpr int SK_SETS = 2;                      // register sets
 
@@ -110,15 +111,15 @@ __host__ __device__ constexpr size_t sk_smem(int rows, int stages, int cap)
     return sk_sum_off(rows, stages, cap) + 32 + 2 * SK_MAX_STAGES * 8 + 16;
 }
 
-// ROWS: rows of C that are fetched and multiplied, 8, 16 or 32.  CW: warps that multiply, PW: warps that copy.  RT: rows per thread.
-template <int ROWS, int CW, int PW, int RT>
-__global__ void __launch_bounds__((CW + PW) * 32)
+// ROWS: rows of C that are fetched and multiplied, 8, 16 or 32.  CW: warps that multiply.  RT: rows per thread.
+template <int ROWS, int CW, int RT>
+__global__ void __launch_bounds__((CW + SK_COPY_WARPS) * 32)
 esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
 {
     constexpr int A_ROW_BYTES = ROWS * 4;                           // one k of A in shared memory
     constexpr int A_HALF = SK_STAGE_ROWS * A_ROW_BYTES;             // A rows, then B rows
     constexpr int STAGE_BYTES = sk_stage_bytes(ROWS);
-    constexpr int SK_WARPS = CW + PW, SK_THREADS = SK_WARPS * 32;
+    constexpr int SK_WARPS = CW + SK_COPY_WARPS, SK_THREADS = SK_WARPS * 32;
     static_assert(SK_WARPS < 8 && (CW == 2 ? SK_WARPS == 4 : CW == 4), "warp sums; roles");
     extern __shared__ __align__(1024) char smem[];
     uint16_t *krow = reinterpret_cast<uint16_t *>(smem + (size_t)p.stages * STAGE_BYTES);
@@ -318,7 +319,7 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
             }
         }
     } else {
-        // ---------------- copies: a warp takes every PW-th stage ----------------
+        // ---------------- copies: a warp takes every other stage ----------------
         // 32 rows at a time.  B: 8 lanes per row, 4 rows an instruction, rows 8 apart, so that a lane's 8 list entries are one load;
         // A likewise.  (Rows of 128 bytes are too short for the tensor copy engine: about 57 cycles of issue per copy and warp.)
         constexpr int A_LANES = ROWS / 4, A_N = A_LANES;            // lanes per row of A; instructions per 32 rows
@@ -332,9 +333,9 @@ esmm_joint_sgemm_skinny_kernel(const SkinnyParams p)
         const uint32_t dst_b = smem_u32(smem) + (uint32_t)(A_HALF + b_row * SK_ROW_BYTES + b_chunk * 16);
         int slot = role - CW;
         uint32_t phase = 1u;                                        // of the slot's empty barrier that the warp waits for
-        static_assert(PW <= 2, "a warp's first slot and its steps along the ring");
+        static_assert(SK_COPY_WARPS <= 2, "a warp's first slot and its steps along the ring");
         int s = role - CW;
-        for (; (s + 1) * SK_STAGE_ROWS <= n; s += PW, slot += PW) {
+        for (; (s + 1) * SK_STAGE_ROWS <= n; s += SK_COPY_WARPS, slot += SK_COPY_WARPS) {
             if (slot >= p.stages) {
                 slot -= p.stages;
                 phase ^= 1u;
@@ -442,11 +443,11 @@ static int skinny_prepare(int dev, int *sms)
         auto allow = [&](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); };
         ESMM_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
         ESMM_CUDA_TRY(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<8, 2, 2, 2>));
-        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<16, 4, 2, 2>));
-        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<16, 2, 2, 4>));
-        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<32, 4, 2, 4>));
-        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<32, 2, 2, 4>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<8, 2, 2>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<16, 4, 2>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<16, 2, 4>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<32, 4, 4>));
+        ESMM_CUDA_TRY(allow(esmm_joint_sgemm_skinny_kernel<32, 2, 4>));
         sm_count[dev] = n;
     }
     *sms = sm_count[dev];
@@ -517,10 +518,10 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
     // load less of A, are faster.  The multiplying part alone, us, two / four warps, K = 4096: M = 16 dense, one strip per SM 31.1 / 28.6;
     // M = 16 pruned MLP, SMs with two strips 9.2 / 8.6, with three 9.9 / 11.6; M = 32 one strip 10.3 / 7.6, two 14.2 / 11.7, three 14.9 / 16.2.
     const bool spread = units <= 2 * sms;
-    if (rows == 8) return launch(esmm_joint_sgemm_skinny_kernel<8, 2, 2, 2>, 8, 4);
+    if (rows == 8) return launch(esmm_joint_sgemm_skinny_kernel<8, 2, 2>, 8, 4);
     if (rows == 16)
-        return spread ? launch(esmm_joint_sgemm_skinny_kernel<16, 4, 2, 2>, 16, 6) : launch(esmm_joint_sgemm_skinny_kernel<16, 2, 2, 4>, 16, 4);
-    return spread ? launch(esmm_joint_sgemm_skinny_kernel<32, 4, 2, 4>, 32, 6) : launch(esmm_joint_sgemm_skinny_kernel<32, 2, 2, 4>, 32, 4);
+        return spread ? launch(esmm_joint_sgemm_skinny_kernel<16, 4, 2>, 16, 6) : launch(esmm_joint_sgemm_skinny_kernel<16, 2, 4>, 16, 4);
+    return spread ? launch(esmm_joint_sgemm_skinny_kernel<32, 4, 4>, 32, 6) : launch(esmm_joint_sgemm_skinny_kernel<32, 2, 4>, 32, 4);
 }
 
 }  // namespace esmm
