@@ -19,13 +19,13 @@
 //   * the warps of a CTA draw items from a counter in shared memory; the last ones come as single blocks spread over the whole
 //     warp, so that the warps finish together (a problem with few blocks consists of nothing else).
 //
-// What bounds it: the FMA pipe together with everything else that is issued.  A stage (16 steps) is 512 two-wide FMAs and 64 loads; where it
-// took 210 instructions more for copies, addresses and lists, a scheduler's three warps got through one in 1310 cycles each, 1113 being
-// what the FMAs need: every one of the others costs about 0.7 cycles of it, wherever it stands.  So they are kept few: one load per list
+// What bounds it: the FMA pipe together with everything else that is issued.  A stage (16 steps) is 512 two-wide FMAs and 64 loads; with
+// everything, items' starts and ends included, it is 739 instructions at 4096^3 64-granular 0.5 / 0.5, where it was 785 (ncu), and the
+// kernel takes 670 us instead of 716, the FMA pipe active 75 % of the time instead of 71.  So the others are kept few: one load per list
 // for a lane's entries, one instruction per address, no predicates where all of B's blocks are whole, one list for blocks that agree.
 // The rest is lost to the end of a launch (3-4 % between SMs, whose items differ, 2 % inside them).  Measured, whole calls, the tiled pipeline before ->
-// block mode: 2048 x 11008 x 4096 pruned MLP 1016 -> 699 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 160 and at
-// 0.5 / 0.5 921 -> 718 (before the pairs' side was a constant), 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 50.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 /
+// block mode: 2048 x 11008 x 4096 pruned MLP 1016 -> 701 us, 4096^3 with independent 32-granular patterns at 0.2 / 0.2 308 -> 163 and at
+// 0.5 / 0.5 921 -> 710, 1000 x 1508 x 2012 at 0.5 / 0.5 80.7 -> 49.  Also measured: one block after the other on the whole warp (4096^3 at 0.5 /
 // 0.5 824), 8 k per stage (971), lists made for all of K before the first copy (762), rows past a list's end skipped in a second code
 // path instead of multiplied by zeros (752: the accumulators are then moved between registers at every stage); eight warps that multiply
 // and four that list and copy for them (pruned MLP 1129: a warp alone on its scheduler's spare slots takes 2000 cycles for a stage's 250
@@ -306,7 +306,7 @@ __device__ __forceinline__ void block_item(const Params &p, char *ring, int lane
     const int half = lane >> 4, xg = (lane >> 1) & 3, yg = (lane & 1) | ((lane >> 2) & 2);   // pair: 4 x 4 lanes per block
     const int lm = (lane >> 1) & 7, ln = (lane & 1) | ((lane >> 4) << 1);                    // single block: 8 x 4 lanes
     // Copies of a pair from packed A: eight lanes per row, a lane's rows are 4 r4 .. 4 r4 + 3, so that its list entries are one load and the
-    // rows of one copy instruction are whole (80 bytes a clock and SM arrive so at most, 64 in the other order).
+    // rows of one copy instruction are whole.
     const int r4 = lane >> 3, c8 = lane & 7;
     const uint32_t dst = smem_u32(ring) + (uint32_t)(r4 * 512 + ((ROW_MAJOR ? c8 ^ rm_swizzle(r4 * 4) : c8) << 4));
     // Single blocks: four lanes per row of the stage, eight rows at a time; a lane moves the 16-byte chunks c4
@@ -652,7 +652,8 @@ __device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp
     // pairs and the rest single 55.2 us, all single 49.9).  Up to 12 what is over when every scheduler (SM sub-partition) has as many pairs as
     // every other (7 and 8 items as 2 and 4 pairs and 10 and 8 single blocks: 1500^3 at 0.5 / 0.5 50.1 -> 53.2, 512 x 4096 x 4096 pruned MLP
     // 107.4 -> 108.6).  Then the end of a row of rounds: 4 of 56 items 692 us (4096^3, 64-granular 0.5 / 0.5), 6 700, 2 701; but
-    // 1024 x 11008 x 4096 pruned MLP, 14 items, 6 181, 4 185.
+    // 1024 x 11008 x 4096 pruned MLP, 14 items, 6 181, 4 185.  (All measured with packed A, between 15 and 55 items at no other number;
+    // row-major A, whose single blocks are dearer, goes by the same rule.)
     const int tail = mine <= 6 ? mine : mine <= BM_WARPS ? (mine & 3) % 3 : mine <= 24 ? 6 : 4, whole = mine - tail;
 
     for (int v = warp; v < whole + 2 * tail;) {

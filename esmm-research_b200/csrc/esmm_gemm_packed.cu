@@ -33,12 +33,13 @@ int gemm_ab_skinny_launch(int M, int N, int K, const float *d_a_packed, const fl
 // the first launch) where the word said otherwise when the host launched it (a launch's end waits for the store across
 // PCIe: 512 x 1024 x 704, 32-granular 0.2 / 0.2, 16.4 us with a note every time, 14.4 now), and the next launch on that
 // device reads the word, without waiting for anything: repeated products of like operands - what a benchmark loop or a
-// layer with fixed weights issues - get the right shape from the second call on, and a stale or missing note only costs
-// that difference.  The results are bit-identical in both shapes.  esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins the
+// layer with fixed weights issues - get the right shape from the second call on, and a stale or missing note costs one
+// launch in the other.  The results are bit-identical in both shapes.  esmm_tuning_set("PRODUCER_WARPS", 3 | 7 | 0) pins the
 // shape instead.  (Scattered rows reach the pipeline in launches too short to look at the samples.  Larger operands of that
-// kind go to block mode, where twelve warps work in either shape and the 12-warp form is the faster one or as fast; there
-// the note is set only with no more pairs of blocks than CTAs, where both take the same time: 512 x 1024 x 2048 at 0.3 / 0.3
-// 25.3 and 24.9 us.)
+// kind go to block mode, where twelve warps work in either shape and the 16-warp form, whose registers do not hold block mode's
+// accumulators without spilling, is as a rule the slower one: whole calls, 12 / 16 warps, 4096^3 32-granular 0.2 / 0.2 158 / 182 us,
+// 64-granular 0.5 / 0.5 652 / 731, 1000 x 1508 x 2012 at 0.5 / 0.5 47.9 / 50.7; 2048^3 32-granular 0.5 / 0.5 118 / 115.  There the note
+// is set only with no more pairs of blocks than CTAs: 512 x 512 x 4096 at 0.3 / 0.3 24.1 / 24.7.)
 static std::atomic<int> g_last_tiled_warps[64];   // per device: warps per CTA of the last launch of the tiled kernel
 
 struct FormHint {

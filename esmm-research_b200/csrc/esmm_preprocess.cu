@@ -98,7 +98,7 @@ esmm_preprocess_a_patterns_kernel(const float *A, int M, int K, int tile_m, int 
 // of 128 bytes per chunk follow, of live columns only.
 // What bounds it: HBM.  In a train of calls 4096^2 takes 11.4 us with a fifth of the columns live, 16.2 with half and 21.8 with all (12.3, 15.4
 // and 20.5 us of bytes at the measured copy bandwidth); 32 x 64 columns per warp with every element's own test, store and load through shared
-// memory, 1280 instructions per task where these two have 320, took 15.2, 18.5 and 22.3 and had 16 warps per SM for these 32.
+// memory, 1277 instructions for 64 live columns where these tasks have 796 (ncu), took 15.2, 18.5 and 22.3 and had 16 warps per SM for these 32.
 constexpr int PACK_WARPS = 4;
 constexpr int PACK_COLS = 32;
 
