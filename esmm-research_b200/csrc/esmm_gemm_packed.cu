@@ -247,6 +247,7 @@ static int tiled_launch(int M, int N, int K, const float *d_a_packed, const floa
     int grid = tuning_get("GRID", sms);
     const long pairs = std::max((long)ceil_div(p.a_rows, 2) * p.b_rows, (long)p.a_rows * ceil_div(p.b_rows, 2));
     p.few_blocks = pairs <= grid;
+    p.rm_shape = row_major_shape(M, N, p.num_tiles, pairs, sms);
     // Where blocks differ the samples cost a launch a microsecond or two, which short ones do not win back: the pipeline, without looking, where an SM
     // has fewer than 768 k of tiles to go through (58 x 7368 x 648: 15.2 us, 17.4 with the look; 2502 x 1112 x 456, 912 k of tiles
     // per SM: 37.1 in the pipeline, 31.5 in block mode).

@@ -76,7 +76,8 @@ constexpr int BM_SIXTEENTHS = 11;
 // The same for row-major A, where block mode has to transpose A for every pair of blocks: kernel alone, pipeline / block mode, share 0.11
 // (32-granular, 0.2 / 0.2) 2048^3 79 / 64 us; pruned MLP (0.31) 2048 x 11008 x 4096 1267 / 827, 64 x 4096 x 4096 77 / 54; share 0.33
 // (0.5 / 0.5) 2048^3 186 / 151, 1000 x 1508 x 2012 98 / 67; share 0.44 (64-granular, 0.5 / 0.5) 2048^3 142 / 140, 4096^3 882 / 811; share 0.50
-// (32-granular, 0.7 / 0.7) 2048^3 281 / 252, 4096^3 1828 / 1833; share 0.53 (1 / 0.5) 257 / 265, 1683 / 1772.
+// (32-granular, 0.7 / 0.7) 2048^3 281 / 252, 4096^3 1828 / 1833; share 0.53 (1 / 0.5) 257 / 265, 1683 / 1772.  Some problems above a
+// quarter stay with the pipeline all the same: row_major_pipeline_pays.
 constexpr int RM_SIXTEENTHS = 8;
 
 // Optional timeline for tuning (build with -DESMM_TRACE): CTA 0 stamps %globaltimer at a few points
@@ -117,6 +118,7 @@ struct PackedParams {
     int pat_words;     // pattern rows may be read as 32-bit words
     unsigned last_bits;  // of the last K block's byte: the bits whose k is < K, in all four bytes of the word
     int few_blocks;    // no more pairs of blocks than CTAs
+    int rm_shape;      // row-major A: RmShape
     // row-major A: 32-row block mb uses A pattern rows (mb / a_div) * a_mul + [0, a_mul) of a_pat_rows
     int a_div, a_mul, a_pat_rows;
     int list_kb, lists;  // row-major A: K blocks per row list, row lists per tile
@@ -569,7 +571,16 @@ __device__ __noinline__ int choose_mode(const PackedParams &p, char *scratch, in
         a_differ += x.z;
         b_differ += x.w;
     }
-    const bool blocks = p.block_mode > 0 || block_mode_pays(work, slots, RM ? RM_SIXTEENTHS : BM_SIXTEENTHS);
+    bool blocks = p.block_mode > 0 || block_mode_pays(work, slots, RM ? RM_SIXTEENTHS : BM_SIXTEENTHS);
+    if (RM && blocks && p.block_mode <= 0 && (p.rm_shape & RM_FILLS)) {
+        int listed = 0, rows64 = 0;
+        for (int i = 0; i < BM_SAMPLES; ++i) {
+            const int4 y = stats[BM_SAMPLES + i];
+            listed += y.x;
+            rows64 += y.y;
+        }
+        blocks = !row_major_pipeline_pays(work, slots, rows64, listed, BM_SAMPLES * min(32 * 4 * BK, p.K), p.rm_shape);
+    }
     if (blocks && blockIdx.x == 0 && threadIdx.x == 0 && p.form_hint != nullptr) {
         // the note for the next launch (see gemm_ab_packed_launch_form)
         int listed = 0, rows64 = 0, single = 0;

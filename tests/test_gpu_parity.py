@@ -1419,3 +1419,46 @@ def test_packing_before_strips_is_launched_alike(cuda, pkg, M, N):
     one_call, two_calls = carveouts(joint), carveouts(two)
     assert one_call == two_calls
     assert (100 in one_call) == (M < 256), one_call                   # cudaSharedmemCarveoutMaxShared
+
+
+@pytest.mark.parametrize("M,N,K,gran,pa,pb", [(1024, 1024, 1024, 64, 0.2, 0.2), (1024, 1024, 1024, 64, 0.1, 0.1), (1024, 1024, 1028, 64, 0.3, 0.3), (1500, 1500, 800, 32, 0.7, 0.7),
+                                              (1024, 1024, 1024, 32, 0.5, 0.5)])
+def test_rowmajor_mode_rule_bits(cuda, pkg, oracle_mod, M, N, K, gran, pa, pb):
+    """Row-major A on operands that the rule sends to either way of working, by its own choice: the oracle's bits."""
+    A, B = workloads.tile_random(M, N, K, pa, pb, seed=M + K, gran_a=gran, gran_b=gran)
+    d = Dev(cuda, pkg, A, B)
+    d.patterns()
+    assert np.array_equal(d.gemm_rowmajor().view(np.uint32), oracle_mod.gemm_joint(A, B).view(np.uint32))
+
+
+def test_rowmajor_mode_rule_time(cuda, pkg, tuning):
+    """Row-major A with a fifth of A's and of B's 64-granular k live, 1024 x 1024 x 4096: left to the rule the product takes no longer than the
+    pipeline does, but for the look at the samples (1.1 times; 1.35 in block mode, where it went for a time).  20 calls in a graph."""
+    M, N, K = 1024, 1024, 4096
+    A, B = workloads.tile_random(M, N, K, 0.2, 0.2, seed=3, gran_a=64, gran_b=64)
+    d = Dev(cuda, pkg, A, B)
+    d.patterns()
+    c = d.C()
+
+    def graph_ms():
+        call = lambda: pkg.gemm_ab(M, N, K, d.A.data_ptr(), d.B.data_ptr(), c.data_ptr(), d.ap.data_ptr(), d.bp.data_ptr(), stream=cuda.cuda.current_stream().cuda_stream)
+        call()
+        pkg.device_status()
+        graph = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(graph):
+            for _ in range(20):
+                call()
+        best = float("inf")
+        for _ in range(10):
+            t0, t1 = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+            t0.record()
+            graph.replay()
+            t1.record()
+            cuda.cuda.synchronize()
+            best = min(best, t0.elapsed_time(t1))
+        del graph
+        return best
+    own = graph_ms()
+    tuning("BLOCK_MODE", 0)
+    pipeline = graph_ms()
+    assert own < 1.2 * pipeline, (own, pipeline)

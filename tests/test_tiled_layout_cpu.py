@@ -20,6 +20,11 @@ extern "C" void layout(int stages, int stage_bytes, int cap, int blocks, unsigne
     for (int i = 0; i < 9; ++i) out[i] = v[i];
 }
 extern "C" int pays(int work, int slots, int sixteenths) { return block_mode_pays(work, slots, sixteenths); }
+extern "C" int pipeline_pays(int work, int slots, int rows64, int listed, int span, int shape)
+{
+    return row_major_pipeline_pays(work, slots, rows64, listed, span, shape);
+}
+extern "C" int shape(int M, int N, long tiles, long pairs, int sms) { return row_major_shape(M, N, tiles, pairs, sms); }
 extern "C" int constant(int i)
 {
     const int v[] = {SMEM_LIMIT, BM_SMEM, PSTAGE_BYTES, P_MAX_STAGES, P_CONSUMER_WARPS, RM_STAGE_A_BYTES + STAGE_HALF_BYTES};
@@ -72,6 +77,34 @@ def test_block_mode_rule(shim):
             assert shim.pays(slots * sixteenths // 16, slots, sixteenths)
             assert not shim.pays(slots * sixteenths // 16 + 1, slots, sixteenths)
             assert not shim.pays(slots, slots, sixteenths)
+
+
+def test_row_major_rule(shim):
+    """Row-major A: which problems stay with the pipeline although their share of live slots is one for block mode.  Samples as the kinds of operands
+    give them (per k looked at: listed, work and rows64 of a tile of 4 x 4 blocks), shapes on 148 SMs, and the side each was measured on."""
+    shim.shape.argtypes = [C.c_int, C.c_int, C.c_long, C.c_long, C.c_int]
+    span = 8 * 1024
+
+    def pipeline(M, N, rows, gran, pa, pb):
+        across = -(-N // 128)
+        tiles = -(-M // rows) * across
+        ra, rb = -(-M // 32), -(-N // 32)
+        pairs = max(-(-ra // 2) * rb, ra * -(-rb // 2))
+        na, nb = (2, 2) if gran == 64 else (4, 4)                       # patterns of their own per tile
+        listed = span * (1 - (1 - pa) ** na) * (1 - (1 - pb) ** nb)
+        work = span * 16 * pa * pb
+        rows64 = span * 8 * pb * (pa if gran == 64 else 1 - (1 - pa) ** 2)
+        return bool(shim.pipeline_pays(int(work), int(16 * listed), int(rows64), int(listed), span, shim.shape(M, N, tiles, pairs, 148)))
+
+    for shape in [(4096, 4096, 128), (2048, 2048, 128), (1024, 1024, 64), (512, 4096, 128), (2048, 11008, 128)]:
+        assert pipeline(*shape, 64, 0.2, 0.2) and not pipeline(*shape, 64, 0.1, 0.1) and not pipeline(*shape, 64, 0.5, 0.5)
+        assert not pipeline(*shape, 32, 0.5, 0.5) and not pipeline(*shape, 32, 0.2, 0.2)
+        assert pipeline(*shape, 64, 0.3, 0.3) == (shape[0] == 1024)
+    for shape, even in [((4096, 4096, 128), True), ((3000, 3000, 128), True), ((512, 4096, 128), True), ((2048, 2048, 128), False), ((2048, 11008, 128), False)]:
+        assert pipeline(*shape, 32, 0.7, 0.7) == even and pipeline(*shape, 32, 1.0, 0.4) == even
+    assert not pipeline(3000, 3000, 128, 64, 0.2, 0.2)                  # ragged
+    assert not any(pipeline(64, 4096, 64, 32, pa, pb) for pa, pb in [(0.7, 0.7), (1.0, 0.4)])   # 32 tiles
+    assert not pipeline(128, 2048, 128, 64, 0.2, 0.2)
 
 
 def test_copies_that_signal_a_barrier_are_waited_for():
