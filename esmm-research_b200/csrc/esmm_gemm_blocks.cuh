@@ -647,14 +647,7 @@ __device__ __forceinline__ void block_mode(const Params &p, char *smem, int warp
     const int tiles_m = wide_b ? y_blocks : pairs_x, tiles_n = wide_b ? pairs_x : y_blocks;
     const long items = (long)tiles_m * tiles_n;
     const int mine = blockIdx.x < items ? (int)((items - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
-    // The last `tail` items go as two single blocks each.  Up to 6 items all of them: twelve warps then have a block or none, and a warp
-    // alone takes longer for a pair than three do for their blocks beside each other (1000 x 1508 x 2012 at 0.5 / 0.5, 5 or 6 items, four
-    // pairs and the rest single 55.2 us, all single 49.9).  Up to 12 what is over when every scheduler (SM sub-partition) has as many pairs as
-    // every other (7 and 8 items as 2 and 4 pairs and 10 and 8 single blocks: 1500^3 at 0.5 / 0.5 50.1 -> 53.2, 512 x 4096 x 4096 pruned MLP
-    // 107.4 -> 108.6).  Then the end of a row of rounds: 4 of 56 items 692 us (4096^3, 64-granular 0.5 / 0.5), 6 700, 2 701; but
-    // 1024 x 11008 x 4096 pruned MLP, 14 items, 6 181, 4 185.  (All measured with packed A, between 15 and 55 items at no other number;
-    // row-major A, whose single blocks are dearer, goes by the same rule.)
-    const int tail = mine <= 6 ? mine : mine <= BM_WARPS ? (mine & 3) % 3 : mine <= 24 ? 6 : 4, whole = mine - tail;
+    const int tail = block_tail(mine), whole = mine - tail;   // the last `tail` items go as two single blocks each
 
     for (int v = warp; v < whole + 2 * tail;) {
         const int item = blockIdx.x + (v < whole ? v : whole + ((v - whole) >> 1)) * gridDim.x;

@@ -51,6 +51,22 @@ ESMM_HOST_DEVICE inline bool block_mode_pays(int work, int slots, int sixteenths
     return slots > 0 && 16 * work <= sixteenths * slots;
 }
 
+// How many of a CTA's items (pairs of blocks) go as two single blocks each, at the end.  Up to 6 all of them: twelve warps then have a
+// block or none, and a warp alone takes longer for a pair than three do for their blocks beside each other (1000 x 1508 x 2012 at 0.5 / 0.5, 5 or 6
+// items, four pairs and the rest single 55.2 us, all single 49.9).  Up to 12 what is over when every scheduler (SM sub-partition) has as many
+// pairs as every other (7 and 8 items as 2 and 4 pairs and 10 and 8 single blocks: 1500^3 at 0.5 / 0.5 50.1 -> 53.2, 512 x 4096 x 4096 pruned
+// MLP 107.4 -> 108.6).  Then the end of a row of rounds: six, which are a round of single blocks, up to 24 items and where 5 or 6 are over
+// after whole rounds; four elsewhere.  Whole calls, 4 / 6, 32-granular 0.5 / 0.5, 2048 x N x 1024, by items per CTA: 17.7 78.0 / 69.6 us, 29.8
+// 113.9 / 106.6 (row-major A 173.8 / 163.6), 42 154.5 / 149.6, 53.6 191.4 / 187.1; 32 119.0 / 120.6, 45 158.9 / 160.7; 3000 x 3000 x 1000 at
+// 0.7 / 0.7 (29.9) 207 / 190; 4096^3 64-granular (55.4) 652 / 662.  (Two are as good or better with 8 to 12 over, eight nowhere.)
+ESMM_HOST_DEVICE inline int block_tail(int mine)
+{
+    if (mine <= 6) return mine;
+    if (mine <= BM_WARPS) return (mine & 3) % 3;
+    const int over = mine % BM_WARPS;
+    return mine <= 2 * BM_WARPS || over == 5 || over == 6 ? 6 : 4;
+}
+
 // Row-major A: problems for which block_mode_pays has the pipeline as the faster one all the same, at shares above a quarter.  listed: k that
 // are live for a sample's tile; span: k looked at; rows64: live (64-row half of a tile, column block, k); shape: RmShape of the problem.
 //   * Row blocks that agree in pairs (work is twice rows64), so that the pipeline's warps, 64 rows each, waste nothing, and few k listed: an

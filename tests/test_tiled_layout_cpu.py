@@ -25,6 +25,7 @@ extern "C" int pipeline_pays(int work, int slots, int rows64, int listed, int sp
     return row_major_pipeline_pays(work, slots, rows64, listed, span, shape);
 }
 extern "C" int shape(int M, int N, long tiles, long pairs, int sms) { return row_major_shape(M, N, tiles, pairs, sms); }
+extern "C" int tail(int mine) { return block_tail(mine); }
 extern "C" int constant(int i)
 {
     const int v[] = {SMEM_LIMIT, BM_SMEM, PSTAGE_BYTES, P_MAX_STAGES, P_CONSUMER_WARPS, RM_STAGE_A_BYTES + STAGE_HALF_BYTES};
@@ -77,6 +78,23 @@ def test_block_mode_rule(shim):
             assert shim.pays(slots * sixteenths // 16, slots, sixteenths)
             assert not shim.pays(slots * sixteenths // 16 + 1, slots, sixteenths)
             assert not shim.pays(slots, slots, sixteenths)
+
+
+def test_items_cut_in_halves(shim):
+    """Block mode's end: twelve warps that draw a CTA's items, pairs first, then single blocks at 0.55 of a pair, finish no later (0.15 of a pair)
+    than with four or six of the last items cut in halves, whichever is better."""
+    def finish(mine, tail):
+        warps = [0.0] * 12
+        for cost in [1.0] * (mine - tail) + [0.55] * (2 * tail):
+            i = warps.index(min(warps))
+            warps[i] += cost
+        return max(warps)
+
+    for mine in range(1, 300):
+        tail = shim.tail(mine)
+        assert 0 <= tail <= mine
+        if mine > 12:
+            assert finish(mine, tail) <= min(finish(mine, 4), finish(mine, 6)) + 0.15, mine
 
 
 def test_row_major_rule(shim):
