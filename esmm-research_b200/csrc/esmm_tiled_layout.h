@@ -72,18 +72,18 @@ ESMM_HOST_DEVICE inline int block_tail(int mine)
 //   * Row blocks that agree in pairs (work is twice rows64), so that the pipeline's warps, 64 rows each, waste nothing, and few k listed: an
 //     item's start and end then outweigh its stages in block mode.  Whole call, pipeline / block mode, 64-granular 0.2 / 0.2 (0.13 listed)
 //     4096^3 270 / 300 us, 2048^3 55 / 57, 1024^2 x 4096 32 / 39; but 0.1 / 0.1 (0.04) 2048^3 42 / 34, and 0.3 / 0.3 (0.26) 2048 x 11008 x 4096
-//     589 / 537, while with at most six pairs of blocks per SM, single blocks all, 1024^2 x 4096 47 / 54.  Not at ragged edges, which cost the
-//     pipeline more: 3000 x 3000 x 1000 at 0.2 / 0.2 98 / 66.
+//     589 / 537, while with at most six pairs of blocks per SM, single blocks all, 1024^2 x 4096 47 / 54 and 1100 x 700 x 12000 at 0.2 / 0.2
+//     88 / 98.  Of more pairs not at ragged edges, which cost the pipeline more: 3000 x 3000 x 1000 at 0.2 / 0.2 98 / 66.
 //   * Most k listed and more than 7/16 of them used, where the tiles come out even (a last round nearly full) or the blocks do not (seven
 //     or eight pairs for twelve warps): 32-granular 0.7 / 0.7 4096^3 1798 / 1830, 3000 x 3000 x 1000 279 / 289, 512 x 4096 x 4096 285 / 314;
 //     not so 2048^3 (0.86 of two rounds) 279 / 253.
-// Neither where the tiles do not fill the GPU (64 x 4096 x 4096 at 1 / 0.4 149 / 85).
+// Neither where fewer than seven SMs of ten have a tile (64 x 4096 x 4096 at 1 / 0.4 149 / 85; 1000 x 1508 x 2012, 96 tiles, at 0.3 / 0.3 49 / 45).
 enum RmShape { RM_FILLS = 1, RM_WHOLE = 2, RM_FEW = 4, RM_EVEN = 8 };
 
 ESMM_HOST_DEVICE inline bool row_major_pipeline_pays(int work, int slots, int rows64, int listed, int span, int shape)
 {
     if (!(shape & RM_FILLS) || 4 * work <= slots) return false;
-    const bool short_lists = (shape & RM_WHOLE) && 10 * work >= 19 * rows64 && 12 * listed >= span && ((shape & RM_FEW) ? 3 : 6) * listed <= span;
+    const bool short_lists = (shape & (RM_WHOLE | RM_FEW)) && 10 * work >= 19 * rows64 && 12 * listed >= span && ((shape & RM_FEW) ? 3 : 6) * listed <= span;
     return short_lists || (16 * work > 7 * slots && 4 * listed >= 3 * span && (shape & RM_EVEN));
 }
 
@@ -91,7 +91,7 @@ inline int row_major_shape(int M, int N, long tiles, long pairs, int sms)
 {
     const long rounds = (tiles + sms - 1) / sms;
     const bool even = 20 * tiles >= 19 * rounds * sms || (pairs > 6l * sms && pairs <= 8l * sms);
-    return (5 * tiles >= 4l * sms ? RM_FILLS : 0) | (M % 64 == 0 && N % 64 == 0 ? RM_WHOLE : 0) | (pairs <= 6l * sms ? RM_FEW : 0) | (even ? RM_EVEN : 0);
+    return (10 * tiles >= 7l * sms ? RM_FILLS : 0) | (M % 64 == 0 && N % 64 == 0 ? RM_WHOLE : 0) | (pairs <= 6l * sms ? RM_FEW : 0) | (even ? RM_EVEN : 0);
 }
 
 struct PackedSmem {

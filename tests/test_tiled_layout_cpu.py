@@ -120,7 +120,9 @@ def test_row_major_rule(shim):
         assert pipeline(*shape, 64, 0.3, 0.3) == (shape[0] == 1024)
     for shape, even in [((4096, 4096, 128), True), ((3000, 3000, 128), True), ((512, 4096, 128), True), ((2048, 2048, 128), False), ((2048, 11008, 128), False)]:
         assert pipeline(*shape, 32, 0.7, 0.7) == even and pipeline(*shape, 32, 1.0, 0.4) == even
-    assert not pipeline(3000, 3000, 128, 64, 0.2, 0.2)                  # ragged
+    assert not pipeline(3000, 3000, 128, 64, 0.2, 0.2)                  # ragged, many pairs
+    assert pipeline(1100, 700, 64, 64, 0.2, 0.2) and pipeline(1100, 700, 64, 64, 0.2, 0.6)      # ragged, single blocks all
+    assert not pipeline(1000, 1508, 128, 64, 0.3, 0.3)                  # 96 tiles
     assert not any(pipeline(64, 4096, 64, 32, pa, pb) for pa, pb in [(0.7, 0.7), (1.0, 0.4)])   # 32 tiles
     assert not pipeline(128, 2048, 128, 64, 0.2, 0.2)
 
