@@ -27,8 +27,8 @@
 // What bounds it: a multiplying warp is alone or nearly so on its SM sub-partition, so its loads' issue and its multiply-adds add up:
 // 13 cycles a k for 4 x 2 outputs (8 of multiply-adds) with no copies and no barriers at all, 15 with them; on SMs with three or more
 // strips shared memory (10 of its wavefronts per strip of 32 rows and k, 7.5 of 16).  Measured, whole calls, the kernel before -> this
-// one: M = 16, N = 11008, K = 4096 pruned MLP (819 live k per strip, 344 strips) 28.5 -> 19.3 us; M = 8 28.4 -> 14.1; M = 1 19.4 ->
-// 10.6; M = 32 34.1 -> 27.3; dense, N = 4096, K = 4096, M = 16 61.5 -> 33.5; dense, N = 11008, M = 1 100.5 -> 47.4; N = 512, K =
+// one: M = 16, N = 11008, K = 4096 pruned MLP (819 live k per strip, 344 strips) 28.5 -> 19.0 us; M = 8 28.4 -> 14.5; M = 1 19.4 ->
+// 9.7; M = 32 34.1 -> 27.3; dense, N = 4096, K = 4096, M = 16 61.5 -> 33.5; dense, N = 11008, M = 1 100.5 -> 47.4; N = 512, K =
 // 16384, M = 6 148 -> 70.  Also measured: stages of 32 k 10-20 % slower, of 128 in a ring of two as fast, k of a batch 2 or 8 and
 // three batches ahead as fast, counters in shared memory with release / acquire instead of barriers 3-5 % slower; lanes past B's last
 // column that all copy the matrix's first bytes instead of others of their row: N = 300, 32 row blocks 118 us instead of 61. Every
