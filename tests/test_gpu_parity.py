@@ -1320,7 +1320,7 @@ def test_gemm_strips_from_two_threads(cuda, pkg, oracle_mod):
 @pytest.mark.parametrize("M,K", [(1, 256), (16, 64), (32, 64)])
 def test_strips_of_short_lists_do_not_queue(cuda, pkg, M, K):
     """Strips with a few live k each (a sixteenth of K), 16 of them and 500: a stage is filled with the list's rows only, so that the 500, all of which
-    fit on the GPU at once, take about as long as the 16 (2.6 to 3.6 times as long when each of them filled its stage with copies of the
+    fit on the GPU at once, take about as long as the 16 (1.1 to 1.4 times; 2.6 to 3.6 when each of them filled its stage with copies of the
     same row).  The product alone, 20 calls in a graph."""
     times = []
     for N in (512, 16000):
@@ -1433,7 +1433,8 @@ def test_rowmajor_mode_rule_bits(cuda, pkg, oracle_mod, M, N, K, gran, pa, pb):
 
 def test_rowmajor_mode_rule_time(cuda, pkg, tuning):
     """Row-major A with a fifth of A's and of B's 64-granular k live, 1024 x 1024 x 4096: left to the rule the product takes no longer than the
-    pipeline does, but for the look at the samples (1.1 times; 1.35 in block mode, where it went for a time).  20 calls in a graph."""
+    pipeline does, but for the look at the samples (measured 1.14 times; 1.43 in block mode, where it went for a time: the line is halfway).
+    20 calls in a graph."""
     M, N, K = 1024, 1024, 4096
     A, B = workloads.tile_random(M, N, K, 0.2, 0.2, seed=3, gran_a=64, gran_b=64)
     d = Dev(cuda, pkg, A, B)
@@ -1461,4 +1462,4 @@ def test_rowmajor_mode_rule_time(cuda, pkg, tuning):
     own = graph_ms()
     tuning("BLOCK_MODE", 0)
     pipeline = graph_ms()
-    assert own < 1.2 * pipeline, (own, pipeline)
+    assert own < 1.28 * pipeline, (own, pipeline)
